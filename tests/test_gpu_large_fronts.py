@@ -1,0 +1,90 @@
+"""Schur complements and solutions of blocked fronts (too large for one CTA's
+shared memory) against 64-bit numpy, at sizes around the kernels' edges:
+64-column steps, 256-column outer panels, 128 x 128 update tiles, 16-column
+row blocks.
+
+Two leaf fronts (fs own rows, ss shared rows) below a root of the ss shared
+rows.  The element matrices are random symmetric positive definite (LU:
+plus a random skew part) with eigenvalues in [1, 4], so the Schur complement
+is well conditioned.  Tolerance, elementwise: the factorisation's backward
+error is at most (fs + 8) u sqrt(a_ii a_jj) for the front's unit roundoff u, and it
+reaches ABR multiplied by at most (1 + ||A21 A11^-1||)^2 <= 25 for this
+spectrum."""
+import numpy as np
+import pytest
+
+from oracle import uhm_oracle as uo
+from uhm_gb300 import api
+
+pytestmark = pytest.mark.gpu
+
+U = {"fp64": 2.0 ** -53, "fp32": 2.0 ** -24}
+
+
+def _matrix(n, symmetric, rng):
+    q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    a = (q * rng.uniform(1.0, 4.0, n)) @ q.T
+    a = 0.5 * (a + a.T)
+    if not symmetric:
+        s = rng.standard_normal((n, n)) / np.sqrt(n)
+        a = a + 0.5 * (s - s.T)
+    return a
+
+
+def _mesh(fs, ss, symmetric, seed):
+    rng = np.random.default_rng(seed)
+    m = api.Mesh()
+    nodes = [m.add_node(0, fs), m.add_node(1, fs), m.add_node(2, ss)]
+    leaves = [m.add_element(0), m.add_element(0)]
+    root = m.add_element(-1)
+    for k, e in enumerate(leaves):
+        m.element_add_node(e, nodes[k])
+        m.element_add_node(e, nodes[2])
+        m.set_parent(e, root)
+        m.add_child(root, e)
+    m.lock()
+    m.create_matrix_without_buffer(api.UHM_REAL, 1)
+    mats = [_matrix(fs + ss, symmetric, rng) for _ in leaves]
+    rhs = [rng.standard_normal((fs + ss, 1)) for _ in leaves]
+    for k, e in enumerate(leaves):
+        m.copy_in(e, [k, 2], api.UHM_LHS, mats[k])
+        m.copy_in(e, [k, 2], api.UHM_RHS, rhs[k])
+    return m, leaves, mats, rhs
+
+
+def _check(method, prec, fs, ss, seed):
+    m, leaves, mats, rhs = _mesh(fs, ss, method == uo.CHOL, seed)
+    if prec == "fp32":
+        m.set_mode(1, api.PREC_FP32, 1e-12, 10)
+    m.factor(method)
+    eid = m.fronts()[0]
+    tol = 25 * (fs + 8) * U[prec]
+    for k in range(2):
+        a = mats[k]
+        exact = a[fs:, fs:] - a[fs:, :fs] @ np.linalg.solve(a[:fs, :fs], a[:fs, fs:])
+        got = m.front_block(int(eid[k]), "ABR")
+        if method == uo.CHOL:
+            exact = np.tril(exact)
+        d = np.abs(np.diag(a)[fs:])
+        assert (np.abs(got - exact) <= tol * np.sqrt(np.outer(d, d))).all(), (k, np.abs(got - exact).max())
+    m.solve(method)
+    n = 2 * fs + ss
+    full, b = np.zeros((n, n)), np.zeros(n)
+    for k in range(2):
+        i = np.concatenate([np.arange(fs) + k * fs, np.arange(2 * fs, n)])
+        full[np.ix_(i, i)] += mats[k]
+        b[i] += rhs[k][:, 0]
+    x = m.node_solution(np.arange(3, dtype=np.int32), np.array([fs, fs, ss]))[:, 0]
+    ref = np.linalg.solve(full, b)
+    assert np.abs(x - ref).max() <= 1e-11 * np.abs(ref).max()
+
+
+# (fs, ss): one step; a step and one column; the outer panel's edge; one column past
+# it; two panels with a remainder; one column
+SIZES = [(64, 165), (65, 200), (256, 1), (257, 128), (300, 129), (449, 255), (1, 240)]
+
+
+@pytest.mark.parametrize("fs,ss", SIZES)
+@pytest.mark.parametrize("method,prec", [(uo.LU_PIV, "fp64"), (uo.LU_NOPIV, "fp32")])
+def test_lu_front(native_lib, method, prec, fs, ss):
+    _check(method, prec, fs, ss, 100 + fs)

@@ -24,7 +24,7 @@ static constexpr int ASM_SCATTER_MAX = 26624; // the FP64 column fits 208 KB of 
 static constexpr int TRSM_RB = 64;
 static constexpr int FWD_RB = 256;            // k_solve.cu
 static constexpr int BWD_RB = 512;
-static constexpr int LUROW_CB = 64;
+static constexpr int LUROW_CB = 16;         // k_lu_row_update (k_factor.cu)
 static constexpr int TILE = 64;             // trailing-update tile (k_tile_update)
 
 #define CK(x)                                                                          \

@@ -1146,59 +1146,67 @@ void launch_laswp(const DevCtx& c, const Item* items, int n_items, int dtype, in
   else k_laswp<float><<<n_items, 256, 0, s>>>(c, items, nb);
 }
 
-constexpr int LUROW_CB = 64;   // columns per row-panel block
+constexpr int LUROW_CB = 16;   // columns per row-panel block
+constexpr int LUROW_LQ = 18;   // row of a lane's 16 L entries in shared memory (16-byte rows, no bank conflicts)
 
 // A[k0:k0+kb, cols] <- L11^{-1} A[k0:k0+kb, cols]  (unit lower), cols >= k0+kb;
 // item: front, a = k0, b = first column of the chunk, c = column limit (0: n)
-template <typename T, int NT>
-__global__ void __launch_bounds__(NT) k_lu_row_update(DevCtx c, const Item* __restrict__ items,
-                                                      int nb) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+//
+// Substitution in registers: four lanes hold one column (lane q rows q, q+4,
+// ..), a step's solved entry goes to the other three by one shuffle, L comes
+// from shared memory in the lanes' order, and nothing waits at a block
+// barrier after L is staged.  Two warps take 16 columns; bound by the
+// multiply-adds (2016 per column; FP64 at about 2 per clock and SM, which
+// is why the chunk is narrow: 16 columns spread a panel over every SM) and,
+// FP32, by latency.  Measured on GB300 against the form it replaces (64
+// columns per CTA, a block barrier per row): 24^3 p = 3 BF16-split LU, 534
+// launches, 38.7 -> 7.9 ms; 12^3 p = 3 FP64, 115 launches, 8.6 ->
+// 4.0 ms.
+template <typename T>
+__global__ void __launch_bounds__(4 * LUROW_CB) k_lu_row_update(DevCtx c, const Item* __restrict__ items, int nb) {
+  __shared__ __align__(16) T L[64 * 4 * LUROW_LQ];   // L[(4 k + q) LUROW_LQ + u] = L11[q + 4 u][k]
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
-  const int n = f.n, k0 = it.a, c0 = it.b;
+  const int n = f.n, k0 = it.a;
   const int kb = min(nb, f.fs - k0);
   const int cend = it.c > 0 ? min(it.c, n) : n;    // columns < cend (item c; 0: all)
-  const int cb = min(LUROW_CB, cend - c0);
-  T* L = reinterpret_cast<T*>(smem_raw);      // kb x kb
-  T* X = L + nb * nb;                         // kb x LUROW_CB, ld nb
   T* __restrict__ G = arena<T>(c) + f.off;
-  for (int idx = threadIdx.x; idx < kb * kb; idx += NT) {
-    const int i = idx % kb, j = idx / kb;
-    L[idx] = i > j ? G[(k0 + i) + (int64_t)(k0 + j) * n] : (T)0;
-  }
-  for (int idx = threadIdx.x; idx < nb * LUROW_CB; idx += NT) {
-    const int i = idx % nb, j = idx / nb;
-    X[idx] = (i < kb && j < cb) ? G[(k0 + i) + (int64_t)(c0 + j) * n] : (T)0;
+  const int q = threadIdx.x & 3, col = it.b + (threadIdx.x >> 2);
+  const bool in = col < cend;
+  T* __restrict__ X = G + k0 + q + (int64_t)col * n;
+  T x[16];
+#pragma unroll
+  for (int u = 0; u < 16; ++u) x[u] = in && q + 4 * u < kb ? X[4 * u] : T(0);
+  {
+    const int i = threadIdx.x;                     // row of L11 (64 threads)
+#pragma unroll 16
+    for (int k = 0; k < 64; ++k)
+      L[(4 * k + (i & 3)) * LUROW_LQ + (i >> 2)] = i > k && i < kb ? G[(k0 + i) + (int64_t)(k0 + k) * n] : T(0);
   }
   __syncthreads();
-  for (int k = 0; k < kb; ++k) {
-    const int h = kb - k - 1;
-    for (int idx = threadIdx.x; idx < h * LUROW_CB; idx += NT) {
-      const int i = k + 1 + idx % h, j = idx / h;
-      X[i + j * nb] -= L[i + k * kb] * X[k + j * nb];
+#pragma unroll
+  for (int b = 0; b < 16; ++b) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const T xk = __shfl_sync(0xffffffffu, x[b], r, 4);
+      const T* __restrict__ l = L + (4 * (4 * b + r) + q) * LUROW_LQ;
+      if (q > r) x[b] -= l[b] * xk;
+#pragma unroll
+      for (int u = b + 1; u < 16; ++u) x[u] -= l[u] * xk;
     }
-    __syncthreads();
   }
-  for (int idx = threadIdx.x; idx < nb * LUROW_CB; idx += NT) {
-    const int i = idx % nb, j = idx / nb;
-    if (i < kb && j < cb) G[(k0 + i) + (int64_t)(c0 + j) * n] = X[idx];
-  }
+#pragma unroll
+  for (int u = 0; u < 16; ++u)
+    if (in && q + 4 * u < kb) X[4 * u] = x[u];
 }
 
 void launch_lu_row_update(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
                           int pivot, cudaStream_t s) {
   (void)pivot;
   if (!n_items) return;
-  if (dtype == F64) {
-    size_t sm = (size_t)(nb * nb + nb * LUROW_CB) * sizeof(double);
-    cudaFuncSetAttribute(k_lu_row_update<double, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_lu_row_update<double, 256><<<n_items, 256, sm, s>>>(c, items, nb);
-  } else {
-    size_t sm = (size_t)(nb * nb + nb * LUROW_CB) * sizeof(float);
-    cudaFuncSetAttribute(k_lu_row_update<float, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_lu_row_update<float, 256><<<n_items, 256, sm, s>>>(c, items, nb);
-  }
+  if (nb != 64) throw std::invalid_argument("lu_row_update: panels are 64 columns wide");
+  if (dtype == F64) k_lu_row_update<double><<<n_items, 4 * LUROW_CB, 0, s>>>(c, items, nb);
+  else k_lu_row_update<float><<<n_items, 4 * LUROW_CB, 0, s>>>(c, items, nb);
 }
 
 // ---------------------------------------------------------------------------
