@@ -26,6 +26,7 @@ int set_wait_limit_solve(long long v);
 int set_wait_limit_tc(long long v);
 int set_wait_limit_noalloc(long long v);
 int set_wait_limit_chol_tc(long long v);
+int set_wait_limit_xs(long long v);
 }  // namespace uhm_gpu
 
 namespace {
@@ -513,6 +514,7 @@ int uhm_gpu_set_wait_limit(long long iters) {
   rc |= uhm_gpu::set_wait_limit_tc(iters);
   rc |= uhm_gpu::set_wait_limit_noalloc(iters);
   rc |= uhm_gpu::set_wait_limit_chol_tc(iters);
+  rc |= uhm_gpu::set_wait_limit_xs(iters);
   return rc ? 7 : 0;
 }
 

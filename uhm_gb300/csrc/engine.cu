@@ -90,6 +90,8 @@ void Engine::free_device() {
   d_ws2 = nullptr;
   d_ws2_row0 = nullptr;
   d_ws2b_row0 = d_linv_row0 = nullptr;
+  d_xs = nullptr;
+  xs_ctx = XsCtx{};
   d_pflags = nullptr;
   d_hand = nullptr;
   d_err = nullptr;
@@ -679,6 +681,7 @@ void Engine::build_plan(int method) {
     for (auto& f : fronts) {
       const int dt = f.prec == PREC_FP64 ? F64 : F32;
       f.blocked = f.tc || f.n > small_max_f[dt];
+      f.xs = f.blocked && !f.tc;
       f.flag_off = (int)flags_n;
       f.dinv_off = 0;
       if (!f.blocked || method != UHM_CHOL) continue;
@@ -689,6 +692,27 @@ void Engine::build_plan(int method) {
       flags_n += nfb;
     }
   }
+  // operand slices of the current panel of every front with sliced updates;
+  // the levels run one after the other and share the workspace
+  xs_rows = xs_exps = 0;
+  for (auto& lv : levels) {
+    int64_t rows = 0, exps = 0;
+    for (int s : lv) {
+      HostFront& f = fronts[s];
+      if (!f.xs) continue;
+      const int64_t r = (int64_t)(f.prec == PREC_FP64 ? XS_S64 : XS_S32) *
+                        ((std::min(f.fs, XS_NBO) + 63) / 64) * f.n;
+      f.xs_row0 = rows;
+      rows += r;
+      f.xs_row0b = method == UHM_CHOL ? f.xs_row0 : rows;
+      if (method != UHM_CHOL) rows += r;
+      f.xs_exp0 = exps;
+      exps += (method == UHM_CHOL ? 1 : 2) * (int64_t)f.n;
+    }
+    xs_rows = std::max(xs_rows, rows);
+    xs_exps = std::max(xs_exps, exps);
+  }
+  if (xs_rows + XS_SPARE_ROWS > ((int64_t)1 << 31) - 1) fail("operand workspace beyond the tensor map's row range", 4);
   // assembly sources in summation order: the element matrix (copy_in), then
   // the children in child order (op_merge, UHM/src/operation/element.cxx:150-162)
   for (auto& f : fronts) {
@@ -969,6 +993,32 @@ void Engine::build_programs(int method) {
       i0 = i1;
     }
   };
+  // sliced updates: pack items of rows [r0, r1), update tiles of rows
+  // [r0, r1) x columns [c0, c1) (Cholesky: those reaching the lower
+  // triangle; returns the update's flops and adds its bytes to by), and the
+  // launches of one update
+  auto xs_pack_rows = [](std::vector<Item>& it, int s, int k0, int r0, int r1, int cols) {
+    for (int r = r0; r < r1; r += XS_PACK_ROWS) it.push_back(Item{s, k0, r, cols});
+  };
+  auto xs_tiles = [](std::vector<Item>& it, const HostFront& f, int k0, int kb, int r0, int r1, int c0, int c1,
+                     bool lower, double& by) {
+    for (int r = r0; r < r1; r += XS_TILE)
+      for (int c = c0; c < c1 && (!lower || c < r + XS_TILE); c += XS_TILE) it.push_back(Item{f.slot, r, c, k0});
+    const double m = r1 - r0, w = c1 - c0;
+    const double area = lower ? m * w - 0.5 * w * (w - 1) : m * w, esz = f.prec == PREC_FP64 ? 8.0 : 4.0;
+    by += 2.0 * esz * area + 2.0 * (f.prec == PREC_FP64 ? XS_S64 : XS_S32) * kb * (lower ? m : m + w);
+    return 2.0 * kb * area;
+  };
+  auto push_xs = [&](int dt, int nb, int region, const std::vector<Item>& pk, const std::vector<Item>& tiles,
+                     double fl, double by) {
+    if (tiles.empty()) return;
+    push(fac_ops, OP_XS_PACK, dt, nb, 0, pk);
+    Op op{OP_XS_UPDATE, dt, nb, chol ? 1 : 0, add_items(tiles), (int)tiles.size()};
+    op.q0 = region;
+    op.flops = fl;
+    op.bytes = by;
+    fac_ops.push_back(op);
+  };
   const int small_max[2] = {tune.small_max_f64, tune.small_max_f32};
   for (auto& lv : levels) {
     for (int dt = 0; dt < 2; ++dt) {
@@ -1027,47 +1077,87 @@ void Engine::build_programs(int method) {
       push(fac_ops, OP_ASSEMBLE, dt, 0, chol ? 1 : 0, asm_items, 0, asm_items.empty() ? 0.0 : asm_bytes);
       push(fac_ops, OP_ASSEMBLE_SCATTER, dt, n_big, chol ? 1 : 0, asm_big, 0, asm_items.empty() ? asm_bytes : 0.0);
       push(fac_ops, OP_SMALL_FACTOR, dt, 0, max_small, small_items, small_flops);
+      // large FP64 / FP32 fronts: outer panels of XS_NBO columns factored 64
+      // columns at a time, every update by sliced tensor-core products
+      // (k_xs.cu): the panel's own columns after each step (K = 64), the
+      // trailing block once per outer panel (K = XS_NBO)
       int maxfs = 0;
       for (int s : large) maxfs = std::max(maxfs, fronts[s].fs);
-      for (int k0 = 0; k0 < maxfs; k0 += NB) {
-        std::vector<Item> p_items, t_items, u_items;
-        double fp = 0, ft = 0, fu = 0;
+      for (int K0 = 0; K0 < maxfs; K0 += XS_NBO) {
+        const int k_end = std::min(K0 + XS_NBO, maxfs);
+        for (int k0 = K0; k0 < k_end; k0 += NB) {
+          std::vector<Item> p_items, t_items, pk, ut;
+          double fp = 0, ft = 0, fu = 0, bu = 0;
+          for (int s : large) {
+            const HostFront& f = fronts[s];
+            if (f.fs <= k0) continue;
+            const int kb = std::min(NB, f.fs - k0), base = k0 + kb;
+            const int B = std::min(K0 + XS_NBO, f.fs);       // end of the front's outer panel
+            p_items.push_back(Item{s, k0, 0, 0});
+            if (chol) {
+              fp += get_flop_chol(0, kb);
+              ft += get_flop_trsm_lower(0, kb, f.n - base);
+              for (int r0 = base; r0 < f.n; r0 += TRSM_RB) t_items.push_back(Item{s, k0, r0, 0});
+            } else {
+              fp += get_flop_lu(0, f.n - k0, kb);
+              ft += get_flop_trsm_lower(0, kb, B - base);
+              for (int c0 = base; c0 < B; c0 += LUROW_CB) t_items.push_back(Item{s, k0, c0, B});
+            }
+            if (base >= B) continue;
+            xs_pack_rows(pk, s, k0, base, f.n, 0);
+            if (!chol) xs_pack_rows(pk, s, k0, base, B, 1);
+            fu += xs_tiles(ut, f, k0, kb, base, f.n, base, B, chol, bu);
+          }
+          if (chol) {
+            push_potrf_trsm(dt, p_items, t_items, fp, ft);
+          } else {
+            push_lu_panel(dt, p_items, fp, XS_NBO);
+            push(fac_ops, OP_LUROW, dt, NB, 0, t_items, ft);
+          }
+          push_xs(dt, NB, 1, pk, ut, fu, bu);
+        }
+        if (method == UHM_LU_PIV) {
+          // the outer panel's row swaps on the columns right of it
+          std::vector<Item> sw;
+          for (int s : large) {
+            const HostFront& f = fronts[s];
+            if (f.fs <= K0) continue;
+            for (int c0 = std::min(K0 + XS_NBO, f.fs); c0 < f.n; c0 += 256) sw.push_back(Item{s, K0, c0, 0});
+          }
+          push(fac_ops, OP_LASWP, dt, XS_NBO, 0, sw);
+        }
+        // LU: the outer panel's rows of U right of it, 64-row block by block
+        for (int k0 = K0; !chol && k0 < k_end; k0 += NB) {
+          std::vector<Item> t_items, pk, ut;
+          double ft = 0, fu = 0, bu = 0;
+          for (int s : large) {
+            const HostFront& f = fronts[s];
+            if (f.fs <= k0) continue;
+            const int kb = std::min(NB, f.fs - k0), base = k0 + kb;
+            const int B = std::min(K0 + XS_NBO, f.fs);
+            for (int c0 = B; c0 < f.n; c0 += LUROW_CB) t_items.push_back(Item{s, k0, c0, 0});
+            ft += get_flop_trsm_lower(0, kb, f.n - B);
+            if (base >= B || B >= f.n) continue;
+            xs_pack_rows(pk, s, k0, base, B, 0);
+            xs_pack_rows(pk, s, k0, B, f.n, 1);
+            fu += xs_tiles(ut, f, k0, kb, base, B, B, f.n, false, bu);
+          }
+          push(fac_ops, OP_LUROW, dt, NB, 0, t_items, ft);
+          push_xs(dt, NB, 2, pk, ut, fu, bu);
+        }
+        // the trailing block
+        std::vector<Item> pk, ut;
+        double fu = 0, bu = 0;
         for (int s : large) {
           const HostFront& f = fronts[s];
-          if (f.fs <= k0) continue;
-          const int kb = std::min(NB, f.fs - k0);
-          const int base = k0 + kb;
-          const int mrest = f.n - base;
-          if (chol) {
-            fp += get_flop_chol(0, kb);
-            ft += get_flop_trsm_lower(0, kb, mrest);
-            fu += get_flop_syrk(0, kb, mrest);
-          } else {
-            fp += get_flop_lu(0, f.n - k0, kb);
-            ft += get_flop_trsm_lower(0, kb, mrest);
-            fu += get_flop_gemm(0, mrest, mrest, kb);
-          }
-          p_items.push_back(Item{s, k0, 0, 0});
-          if (chol) {
-            for (int r0 = base; r0 < f.n; r0 += TRSM_RB) t_items.push_back(Item{s, k0, r0, 0});
-            const int T = (f.n - base + TILE - 1) / TILE;
-            for (int ti = 0; ti < T; ++ti)
-              for (int tj = 0; tj <= ti; ++tj) u_items.push_back(Item{s, k0, ti, tj});
-          } else {
-            for (int c0 = base; c0 < f.n; c0 += LUROW_CB) t_items.push_back(Item{s, k0, c0, 0});
-            const int T = (f.n - base + TILE - 1) / TILE;
-            for (int ti = 0; ti < T; ++ti)
-              for (int tj = 0; tj < T; ++tj) u_items.push_back(Item{s, k0, ti, tj});
-          }
+          if (f.fs <= K0) continue;
+          const int KB = std::min(XS_NBO, f.fs - K0), base = K0 + KB;
+          if (base >= f.n) continue;
+          xs_pack_rows(pk, s, K0, base, f.n, 0);
+          if (!chol) xs_pack_rows(pk, s, K0, base, f.n, 1);
+          fu += xs_tiles(ut, f, K0, KB, base, f.n, base, f.n, chol, bu);
         }
-        if (chol) {
-          push_potrf_trsm(dt, p_items, t_items, fp, ft);
-          push(fac_ops, OP_SYRK, dt, NB, 0, u_items, fu);
-        } else {
-          push_lu_panel(dt, p_items, fp, 0);
-          push(fac_ops, OP_LUROW, dt, NB, 0, t_items, ft);
-          push(fac_ops, OP_GEMM, dt, NB, 0, u_items, fu);
-        }
+        push_xs(dt, XS_NBO, 0, pk, ut, fu, bu);
       }
       // tensor-core fronts: outer panels of tc_nbo columns; inside a panel the
       // SIMT kernels factor 64 columns at a time and update only the panel's
@@ -1675,6 +1765,27 @@ void Engine::alloc_device(int method) {
     up64(d_linv_row0, rl);
     CK(cudaStreamSynchronize(stream));
   }
+  if (xs_rows > 0) {
+    const size_t bytes = 128 * (size_t)(xs_rows + XS_SPARE_ROWS);
+    d_xs = dmalloc(bytes);
+    CK(cudaMemsetAsync(d_xs, 0, bytes, stream));     // rows never packed are read by tiles that run over
+    if (!tcc_encode(&xs_map, d_xs, xs_rows + XS_SPARE_ROWS)) fail("tensor map encoding failed", 4);
+    std::vector<int64_t> v(3 * fronts.size(), 0);
+    for (auto& f : fronts)
+      if (f.xs) {
+        v[f.slot] = f.xs_row0;
+        v[fronts.size() + f.slot] = f.xs_row0b;
+        v[2 * fronts.size() + f.slot] = f.xs_exp0;
+      }
+    int64_t* d = (int64_t*)dmalloc(sizeof(int64_t) * v.size());
+    CK(cudaMemcpyAsync(d, v.data(), sizeof(int64_t) * v.size(), cudaMemcpyHostToDevice, stream));
+    CK(cudaStreamSynchronize(stream));
+    xs_ctx.ws = d_xs;
+    xs_ctx.row0 = d;
+    xs_ctx.row0b = d + fronts.size();
+    xs_ctx.exp0 = d + 2 * fronts.size();
+    xs_ctx.exps = (int*)dmalloc(sizeof(int) * (size_t)xs_exps);
+  }
   if (pflags_n > 0) d_pflags = (int*)dmalloc(sizeof(int) * (size_t)pflags_n);
   if (hand_n > 0) {
     // zero: no word carries a tag (every tag has its top bit set)
@@ -1922,6 +2033,10 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
       case OP_TC_SYRK:
         launch_tc_syrk(ctx, ws_map, d_ws_off, d_ws_stride, it, op.n_items, op.nb, op.param == 3 ? 6 : 3,
                        op.param == 3 ? TC_TERMS_BF16X6 : TC_TERMS_BF16X3, 1, d_err, st);
+        break;
+      case OP_XS_PACK: launch_xs_pack(ctx, xs_ctx, it, op.n_items, op.dtype, op.nb, st); break;
+      case OP_XS_UPDATE:
+        launch_xs_update(ctx, xs_ctx, xs_map, it, op.n_items, op.dtype, op.nb, op.q0, op.param, d_err, st);
         break;
       case OP_GETRF: launch_getrf_panel(ctx, it, op.n_items, op.dtype, op.nb, op.param, st); break;
       case OP_GETRF_COOP:

@@ -15,6 +15,7 @@
 #include "kernels.cuh"
 #include "k_tc.cuh"
 #include "k_chol_tc.cuh"
+#include "k_xs.cuh"
 #include "mesh.hpp"
 
 namespace uhm {
@@ -32,6 +33,8 @@ struct HostFront {
   int prec = PREC_FP64;
   bool tc = false;                 // trailing updates on tensor cores (BF16-split)
   bool tcc = false;                // ... through the cooperative panel kernel (BF16X3 Cholesky, k_chol_tc.cu)
+  bool xs = false;                 // large FP64 / FP32 front: sliced tensor-core updates (k_xs.cu)
+  int64_t xs_row0 = 0, xs_row0b = 0, xs_exp0 = 0;   // its slices and row exponents in the level's workspace
   int64_t ws_off = 0, ws_stride = 0;
   int64_t ws2_row0 = 0;            // first 128-byte row of its parts in the chunk-major workspace
   int64_t ws2b_row0 = 0;           // ... of the panel rows before their TRSM (tc_panel 256)
@@ -65,7 +68,8 @@ struct Op {
   double flops = 0;   // algorithmic flops of this launch (LAWN-41 terms)
   double bytes = 0;   // algorithmic HBM bytes of this launch
   int q0 = 0;         // first right-hand side (flag-driven solves) / CTAs (cooperative LU panel) /
-                      // SMs left free for a concurrent launch (tensor-core Cholesky update)
+                      // SMs left free for a concurrent launch (tensor-core Cholesky update) /
+                      // region of the front (sliced update)
   int aux = 0;        // rows per CTA (cooperative LU panel, flag-driven solves)
   int strm = 0;       // 0: the engine's stream, 1: its side stream (panel lookahead)
 };
@@ -82,7 +86,7 @@ enum OpKind : int {
   OP_TRSV_B, OP_BWD_STORE, OP_TC_PACK, OP_TC_SYRK, OP_FWD_FLAGS, OP_BWD_FLAGS, OP_GETRF_COOP,
   OP_LASWP, OP_POTRF_TRSM, OP_ASSEMBLE_SCATTER, OP_TC_GEMM, OP_CHOL_PANEL, OP_TC_CHOL_TRAIL,
   OP_TC_CHOL_SCHUR, OP_CLEAR_FLAGS, OP_CHOL_DIAG, OP_CHOL_PACK, OP_TC_CHOL_TRSM, OP_EV_RECORD, OP_EV_WAIT,
-  OP_FWD_CHAIN, OP_BWD_CHAIN, OP_KIND_END
+  OP_FWD_CHAIN, OP_BWD_CHAIN, OP_XS_PACK, OP_XS_UPDATE, OP_KIND_END
 };
 static_assert(OP_KIND_END <= N_OP_KINDS, "profile arrays hold N_OP_KINDS op kinds");
 
@@ -295,6 +299,10 @@ class Engine {
   int64_t ws2_rows = 0;              // its size in rows of 64 BF16
   int64_t* d_ws2_row0 = nullptr;     // per front: first row of its parts
   CUtensorMap ws2_map;
+  void* d_xs = nullptr;              // operand slices of the current level's sliced updates
+  int64_t xs_rows = 0, xs_exps = 0;  // its rows of 64 BF16 and row exponents (the largest level)
+  uhm_gpu::XsCtx xs_ctx{};
+  CUtensorMap xs_map;
   int* d_pflags = nullptr;           // tickets and flags of the panel launches (cleared per factorisation)
   int64_t* d_ws2b_row0 = nullptr;
   int64_t* d_linv_row0 = nullptr;

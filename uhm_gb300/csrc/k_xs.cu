@@ -1,0 +1,502 @@
+// Trailing updates C -= A B^T of FP64 and FP32 fronts on the tensor cores,
+// without loss of precision: the operands are cut into 8-bit slices whose
+// BF16 products add up exactly.
+//
+// Restates the trailing SYRK / GEMM of the front's blocked factorisation
+// (LINAL/src/dense/chol.cxx:78-82, lu_piv.cxx:95-105 and the front-level
+// updates of UHM/src/matrix/uhm/fla/chol/decompose.cxx:94-95,
+// fla/lu_piv/decompose.cxx:148-149).
+//
+// Slices (the error-free splitting of Ozaki, Ogita, Oishi and Rump, "Error-
+// free transformations of matrix multiplication by using fast routines of
+// matrix multiplication", 2012, with digits in place of floating parts): every
+// row of a panel of W <= 256 columns gets one exponent e, |a| < 2^e, and each
+// entry becomes the integer X = round(a 2^(62-e)) (FP64; 2^(30-e) for FP32),
+// written in balanced base 256, X = sum_p d_p 256^(S-1-p), -128 <= d_p <=
+// 127, |d_0| <= 64, S = 8 (4).  Digits are exact in BF16.  A product a b is
+// 2^(ea+eb-124) sum_d 256^(14-d) sum_{p+q=d} d_p d'_q; the sums over k of
+// one diagonal d are integers below 2^24 for d <= 4 (W <= 256), so FP32
+// accumulation in tensor memory is exact; d = 5..7 stay below 1.75 2^24, where
+// a rounding is worth 2^-60 of the row maxima's product.  Diagonals d > 7
+// (> 3 for FP32) are left out: about 2^-66 (2^-32) of W times the product of
+// the row maxima.  36 (10) of the 64 (16) slice products remain.  The
+// diagonals are added up in 64-bit integers, whose last place is 2^-54 (2^-36)
+// of the product of the row bounds, and applied to C with one rounding per panel
+// instead of one per column.  Measured against 64 bits the solutions are as
+// close as the SIMT update's (seven slices without diagonal 7 were 3 to 10
+// times further off).
+//
+// Why: GB300 does about 2 FP64 multiply-adds per clock per SM (1.17 TFLOP/s
+// measured for the SIMT update), against 1,906 TFLOP/s of BF16 products:
+// 36 products per FP64 one still leave 53.  FP32 fronts: 10 products leave
+// 190 TFLOP/s against 15 measured for the SIMT update.  Measured on GB300, the
+// updates of one factorisation: 16^3 p = 4 FP64 906 -> 46 ms (and 6 for the
+// slices), 13^3 p = 4 FP32 23.0 -> 7.9 (2.9), 12^3 p = 3 FP64 LU 196 -> 14.5 (3.3).
+#include <cuda.h>
+
+#include <stdexcept>
+
+#include "k_common.cuh"
+#include "k_tc_ptx.cuh"
+#include "k_xs.cuh"
+
+namespace uhm_gpu {
+
+UHM_DEFINE_WAIT_LIMIT(set_wait_limit_xs, 1u << 22)
+
+// exponent of a row holding a NaN or an infinity: the update is NaN in that
+// whole row and column (an infinity becomes one in the panel's TRSM already:
+// the product with the zeros of the diagonal block's inverse)
+constexpr int XS_BAD = 1 << 28;
+constexpr int XS_ERR = 7;
+
+// 64-column chunks per slice of a front's layout in a launch of panel width nb
+__device__ __forceinline__ int xs_chunks(int nb, int fs) { return (min(nb, fs) + 63) / 64; }
+
+// ---------------------------------------------------------------------------
+// slices
+// ---------------------------------------------------------------------------
+template <typename T> struct XsType;
+template <> struct XsType<double> {
+  static constexpr int S = XS_S64;
+  static __device__ __forceinline__ int field(double v) { return (__double2hiint(v) >> 20) & 0x7FF; }
+  static constexpr int FMAX = 0x7FF, EBIAS = 1022;
+  // round(v 2^(62 - e)), e = fmax - EBIAS, fmax the largest exponent field of the row (at least 1)
+  static __device__ __forceinline__ long long fixed(double v, int fmax) {
+    const long long b = __double_as_longlong(v);
+    int f = (int)((b >> 52) & 0x7FF);
+    long long m = b & 0xFFFFFFFFFFFFFll;
+    if (f) m |= 1ll << 52;
+    else f = 1;
+    const int sh = fmax - f;
+    m <<= 9;
+    if (sh > 0) m = sh > 62 ? 0 : (m + (1ll << (sh - 1))) >> sh;
+    return b < 0 ? -m : m;
+  }
+};
+template <> struct XsType<float> {
+  static constexpr int S = XS_S32;
+  static __device__ __forceinline__ int field(float v) { return (__float_as_int(v) >> 23) & 0xFF; }
+  static constexpr int FMAX = 0xFF, EBIAS = 126;
+  // round(v 2^(30 - e))
+  static __device__ __forceinline__ long long fixed(float v, int fmax) {
+    const int b = __float_as_int(v);
+    int f = (b >> 23) & 0xFF;
+    int m = b & 0x7FFFFF;
+    if (f) m |= 1 << 23;
+    else f = 1;
+    const int sh = fmax - f;
+    m <<= 6;
+    if (sh > 0) m = sh > 31 ? 0 : (m + (1 << (sh - 1))) >> sh;
+    return b < 0 ? -m : m;
+  }
+};
+
+// A CTA cuts 64 rows: thread r + 64 g holds 16 columns 16 g .. of row r per
+// 64-column chunk (a warp's loads of one column are 32 consecutive rows) and
+// writes each slice's 16 digits as one whole 32-byte sector.  Memory bound:
+// 8 (4) bytes read twice (the second time from L2) and 16 (8) written per
+// entry; the digits come from integer shifts and byte extraction, no FP64.
+template <typename T>
+__global__ void __launch_bounds__(256) k_xs_pack(DevCtx c, XsCtx x, const Item* __restrict__ items, int nb) {
+  constexpr int S = XsType<T>::S;
+  __shared__ int s_f[4][64];
+  const Item it = items[blockIdx.x];
+  const FrontDev f = c.fronts[it.front];
+  const int n = f.n, K0 = it.a, trans = it.c;
+  const int W = min(nb, f.fs - K0), nch = xs_chunks(nb, f.fs);
+  const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
+  const int row = it.b + r;
+  const T* __restrict__ G = arena<T>(c) + f.off;
+  const int64_t base = trans ? (int64_t)row * n + K0 : row + (int64_t)K0 * n;
+  const int64_t step = trans ? 1 : n;
+  const bool in = row < n;
+  int fm = 0;
+  for (int k0 = 0; k0 < W; k0 += 64) {
+    T v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int k = k0 + 16 * g + u;
+      v[u] = in && k < W ? G[base + k * step] : T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) fm = max(fm, XsType<T>::field(v[u]));
+  }
+  s_f[g][r] = fm;
+  __syncthreads();
+  fm = max(max(s_f[0][r], s_f[1][r]), max(max(s_f[2][r], s_f[3][r]), 1));
+  if (!in) return;
+  const bool bad = fm == XsType<T>::FMAX;
+  if (g == 0) x.exps[x.exp0[it.front] + (trans ? n : 0) + row] = bad ? XS_BAD : fm - XsType<T>::EBIAS;
+  uint8_t* const w0 = reinterpret_cast<uint8_t*>(x.ws) + 128 * ((trans ? x.row0b : x.row0)[it.front] + row) + 32 * g;
+  for (int k0 = 0; k0 < W; k0 += 64) {
+    uint32_t d[S][8];
+#pragma unroll
+    for (int u = 0; u < 16; u += 2) {
+      uint32_t lo[S];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int k = k0 + 16 * g + u + e;
+        const long long X = (k < W && !bad) ? XsType<T>::fixed(G[base + k * step], fm) : 0;
+        // balanced digits: adding 128 to every place but the top turns each
+        // into its byte; float(2^23 + byte) - (2^23 + 128) is the digit
+        constexpr long long BIAS = S == 8 ? 0x0080808080808080ll : 0x0000000000808080ll;
+        const long long Y = X + BIAS;
+#pragma unroll
+        for (int p = 0; p < S; ++p) {
+          float dg;
+          if (p == 0) {
+            const int t = (int)(Y >> (8 * (S - 1)));
+            dg = __int_as_float(0x4B400000 + t) - 12582912.0f;
+          } else {
+            const uint32_t b = (uint32_t)(Y >> (8 * (S - 1 - p))) & 0xFFu;
+            dg = __int_as_float((int)(0x4B000000u | b)) - 8388736.0f;
+          }
+          const uint32_t h = __float_as_uint(dg);
+          if (e == 0) lo[p] = h;
+          else d[p][u / 2] = __byte_perm(lo[p], h, 0x7632);
+        }
+      }
+    }
+    const int kc = k0 >> 6;
+#pragma unroll
+    for (int p = 0; p < S; ++p) {
+      uint4* w = reinterpret_cast<uint4*>(w0 + 128 * (int64_t)(p * nch + kc) * n);
+      w[0] = make_uint4(d[p][0], d[p][1], d[p][2], d[p][3]);
+      w[1] = make_uint4(d[p][4], d[p][5], d[p][6], d[p][7]);
+    }
+  }
+}
+
+void launch_xs_pack(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, int dtype, int nb,
+                    cudaStream_t s) {
+  if (!n_items) return;
+  if (dtype == F64) k_xs_pack<double><<<n_items, 256, 0, s>>>(c, x, items, nb);
+  else k_xs_pack<float><<<n_items, 256, 0, s>>>(c, x, items, nb);
+}
+
+// ---------------------------------------------------------------------------
+// update
+// ---------------------------------------------------------------------------
+constexpr int XS_EPI_WARPS = 16;
+constexpr int XS_THREADS = 32 * (XS_EPI_WARPS + 2);     // epilogue warps, TMA producer, MMA issuer
+constexpr uint32_t XS_BOX = 128 * 64;                   // 128 rows of 32 BF16 = 8 KB
+constexpr uint32_t XS_SLOT = 2 * XS_BOX;                // one slice of A and of B, 32 columns
+constexpr int XS_SLOTS = 14;
+constexpr uint32_t XS_SMEM = 1024 + XS_SLOTS * XS_SLOT + 512;
+
+#define XS_LD16(taddr, v)                                                                        \
+  asm volatile(                                                                                  \
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14," \
+      "%15}, [%16];"                                                                              \
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),      \
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),   \
+        "=r"(v[14]), "=r"(v[15])                                                                  \
+      : "r"(taddr))
+
+// One tile takes S = 8 (FP64) in two passes over its columns: diagonals 4 ..
+// 7 (26 products of all slices), then diagonals 0 .. 3 (10 products of slices
+// 0 .. 3); S = 4 (FP32) only the second pass.  Diagonal d goes to accumulator
+// d mod 4, 128 x 128 FP32; the four fill tensor memory.
+
+// a += v 2^SH, v a diagonal's integer sum
+template <int SH>
+__device__ __forceinline__ void xs_add(long long& a, uint32_t v) {
+  a += (long long)__float2int_rn(__uint_as_float(v)) << SH;
+}
+
+// value 2^E of the integer a (E may leave the exponent range)
+__device__ __forceinline__ double xs_scaled(long long a, int E, double) {
+  const double x = __ll2double_rn(a);
+  const int hi = __double2hiint(x), f = (hi >> 20) & 0x7FF;
+  if (a == 0) return 0.0;
+  if ((unsigned)(f + E - 1) < 2045u) return __hiloint2double(hi + (E << 20), __double2loint(x));
+  const int e1 = max(-2000, min(2000, E)) / 2, e2 = max(-2000, min(2000, E)) - e1;
+  return x * __hiloint2double((1023 + e1) << 20, 0) * __hiloint2double((1023 + e2) << 20, 0);
+}
+__device__ __forceinline__ float xs_scaled(long long a, int E, float) {
+  const float x = __ll2float_rn(a);
+  const int b = __float_as_int(x), f = (b >> 23) & 0xFF;
+  if (a == 0) return 0.f;
+  if ((unsigned)(f + E - 1) < 253u) return __int_as_float(b + (E << 23));
+  const int e1 = max(-240, min(240, E)) / 2, e2 = max(-240, min(240, E)) - e1;
+  return x * __int_as_float((127 + e1) << 23) * __int_as_float((127 + e2) << 23);
+}
+
+// Persistent: one CTA per SM walks the 128 x 128 tiles.  Warp 16 loads one
+// slice of A and B (32 columns, 64-byte swizzle) per ring slot, one thread of
+// warp 17 issues the products of a chunk as soon as its slices are there,
+// warps 0..15 (a lane quarter and 32 columns each) take the accumulators to
+// 64-bit integers in registers while the next pass runs, then update C
+// (column by column: a warp's loads and stores are 32 consecutive rows).
+// 14 slots of 16 KB.  Bound: tensor pipe /
+// shared-memory reads of the 128 x 128 products.
+template <typename T>
+__global__ void __launch_bounds__(XS_THREADS, 1)
+k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const Item* __restrict__ items, int n_items,
+            int nb, int region, int lower, int* err) {
+  constexpr int S = XsType<T>::S;
+  extern __shared__ __align__(1024) uint8_t xs_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(xs_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + XS_SLOTS * XS_SLOT);
+  uint64_t* empty = bars + XS_SLOTS;
+  uint64_t* acc_full = empty + XS_SLOTS;
+  uint64_t* acc_empty = acc_full + 4;
+  uint64_t* drain_bar = acc_empty + 4;
+  volatile int* s_abort = reinterpret_cast<volatile int*>(drain_bar + 1);
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(drain_bar + 2);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < XS_SLOTS; ++s) {
+      mbar_init(smem_u32(&bars[s]), 1);
+      mbar_init(smem_u32(&empty[s]), 1);
+    }
+    for (int b = 0; b < 4; ++b) {
+      mbar_init(smem_u32(&acc_full[b]), 1);
+      mbar_init(smem_u32(&acc_empty[b]), XS_EPI_WARPS);
+    }
+    mbar_init(smem_u32(drain_bar), 1);
+    *s_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)),
+                 "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *s_tmem;
+  const uint32_t lim = g_wait_limit;
+
+  if (warp == XS_EPI_WARPS) {
+    if (lane == 0) {
+      // TMA producer
+      int s = 0;
+      uint32_t ph = 1;               // parity of the empty wait (the first round passes)
+      uint32_t issued = 0;
+      bool live = true;
+      for (int t = blockIdx.x; t < n_items && live; t += gridDim.x) {
+        const Item it = items[t];
+        const FrontDev f = c.fronts[it.front];
+        const int n = f.n, nch = xs_chunks(nb, f.fs);
+        const int nk = (min(nb, f.fs - it.c) + 31) / 32;
+        const int64_t ya = x.row0[it.front] + it.a;
+        const int64_t yb = (lower ? x.row0[it.front] : x.row0b[it.front]) + it.b;
+        for (int pass = S == 8 ? 0 : 1; pass < 2 && live; ++pass) {
+          const int np = pass == 0 ? S : 4;
+          for (int k = 0; k < nk && live; ++k)
+            for (int p = 0; p < np; ++p) {
+              if (issued >= XS_SLOTS &&
+                  !mbar_wait_lim(smem_u32(&empty[s]), ph, s_abort, err, XS_ERR, lim)) {
+                live = false;
+                break;
+              }
+              const uint32_t fb = smem_u32(&bars[s]), st = smem_u32(smem + s * XS_SLOT);
+              mbar_expect_tx(fb, XS_SLOT);
+              const int64_t dr = (int64_t)(p * nch + (k >> 1)) * n;
+              tma_load_2d(st, &wsmap, 32 * (k & 1), (int)(ya + dr), fb);
+              tma_load_2d(st + XS_BOX, &wsmap, 32 * (k & 1), (int)(yb + dr), fb);
+              ++issued;
+              if (++s == XS_SLOTS) { s = 0; ph ^= 1; }
+            }
+        }
+      }
+      // the last loads issued (one per slot at most) land before the CTA exits
+      const uint32_t cnt = issued < XS_SLOTS ? issued : XS_SLOTS;
+      for (uint32_t q = issued - cnt; q < issued; ++q)
+        mbar_drain(smem_u32(&bars[q % XS_SLOTS]), (q / XS_SLOTS) & 1);
+    }
+  } else if (warp == XS_EPI_WARPS + 1) {
+    if (lane == 0) {
+      // MMA issuer
+      const uint32_t idesc = idesc_bf16_f32(XS_TILE, XS_TILE);
+      const uint32_t ring = smem_u32(smem);
+      int s = 0;
+      uint32_t ph = 0;               // parity of the full wait at slot s
+      uint32_t use[4] = {0, 0, 0, 0};
+      bool live = true;
+      // the products of diagonals D0..D1 of one chunk: NP slices from slot s
+      auto wait_slot = [&](int p) {
+        int q = s + p;
+        uint32_t qp = ph;
+        if (q >= XS_SLOTS) { q -= XS_SLOTS; qp ^= 1; }
+        return mbar_wait_lim(smem_u32(&bars[q]), qp, s_abort, err, XS_ERR, lim);
+      };
+      auto slot_addr = [&](int p) {
+        int q = s + p;
+        if (q >= XS_SLOTS) q -= XS_SLOTS;
+        return ring + (uint32_t)q * XS_SLOT;
+      };
+      auto diag = [&](auto dd, bool first) {
+        constexpr int d = decltype(dd)::value, a = d & 3, np = d >= 4 ? S : 4;
+        if (first) {
+          if (use[a] >= 1 &&
+              !mbar_wait_lim(smem_u32(&acc_empty[a]), (use[a] - 1) & 1, s_abort, err, XS_ERR, lim))
+            return false;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        }
+        const uint32_t acc = tmem + a * XS_TILE;
+        uint32_t on = first ? 0u : 1u;
+#pragma unroll
+        for (int p = 0; p <= d; ++p) {
+          const int q = d - p;
+          if (p >= np || q >= np) continue;
+          const uint32_t A = slot_addr(p), B = slot_addr(q) + XS_BOX;
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            umma_bf16(acc, sdesc_sw64(A + k * 32), sdesc_sw64(B + k * 32), idesc, on);
+            on = 1u;
+          }
+        }
+        return true;
+      };
+      auto release = [&](int np) {
+        for (int p = 0; p < np; ++p) {
+          int q = s + p;
+          if (q >= XS_SLOTS) q -= XS_SLOTS;
+          umma_commit(smem_u32(&empty[q]));
+        }
+        s += np;
+        if (s >= XS_SLOTS) { s -= XS_SLOTS; ph ^= 1; }
+      };
+      auto finish = [&](int a) {
+        umma_commit(smem_u32(&acc_full[a]));
+        ++use[a];
+      };
+      for (int t = blockIdx.x; t < n_items && live; t += gridDim.x) {
+        const Item it = items[t];
+        const int nk = (min(nb, c.fronts[it.front].fs - it.c) + 31) / 32;
+        // a chunk's products, each diagonal once its last slice has arrived
+        auto step = [&](auto dd, bool first) {
+          if (!wait_slot(decltype(dd)::value)) return false;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          return diag(dd, first);
+        };
+        if constexpr (S == 8) {
+          for (int k = 0; k < nk && live; ++k) {
+            for (int p = 0; p < 4 && live; ++p) live = wait_slot(p);
+            live = live && step(std::integral_constant<int, 4>{}, k == 0) &&
+                   step(std::integral_constant<int, 5>{}, k == 0) && step(std::integral_constant<int, 6>{}, k == 0) &&
+                   step(std::integral_constant<int, 7>{}, k == 0);
+            if (live) release(8);
+          }
+          if (live)
+            for (int a = 0; a < 4; ++a) finish(a);
+        }
+        for (int k = 0; k < nk && live; ++k) {
+          live = step(std::integral_constant<int, 0>{}, k == 0) && step(std::integral_constant<int, 1>{}, k == 0) &&
+                 step(std::integral_constant<int, 2>{}, k == 0) && step(std::integral_constant<int, 3>{}, k == 0);
+          if (live) release(4);
+        }
+        if (live)
+          for (int a = 0; a < 4; ++a) finish(a);
+      }
+      // every MMA issued has completed before tensor memory is freed
+      umma_commit(smem_u32(drain_bar));
+      mbar_drain(smem_u32(drain_bar), 0);
+    }
+  } else {
+    // epilogue
+    const int quarter = warp & 3, cg = warp >> 2;
+    const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + cg * 32;
+    uint32_t par = 0;              // bit a: parity of the next use of accumulator a
+    bool live = true;
+    for (int t = blockIdx.x; t < n_items && live; t += gridDim.x) {
+      long long acc[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) acc[j] = 0;
+      auto take = [&](auto dd) {
+        constexpr int d = decltype(dd)::value, a = d & 3;
+        constexpr int SH = d >= 4 ? 8 * (7 - d) : 8 * (3 - d) + (S == 8 ? 18 : 0);
+        if (!mbar_wait_lim(smem_u32(&acc_full[a]), (par >> a) & 1, s_abort, err, XS_ERR, lim)) return false;
+        par ^= 1u << a;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t v[16];
+          XS_LD16(tbase + a * XS_TILE + 16 * h, v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (h == 1) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&acc_empty[a]));
+          }
+#pragma unroll
+          for (int j = 0; j < 16; ++j) xs_add<SH>(acc[16 * h + j], v[j]);
+        }
+        return true;
+      };
+      if constexpr (S == 8) {
+        // the low diagonals, then rounded to the last place kept
+        live = take(std::integral_constant<int, 4>{}) && take(std::integral_constant<int, 5>{}) &&
+               take(std::integral_constant<int, 6>{}) && take(std::integral_constant<int, 7>{});
+#pragma unroll
+        for (int j = 0; j < 32; ++j) acc[j] = (acc[j] + (1 << 13)) >> 14;
+      }
+      live = live && take(std::integral_constant<int, 0>{}) && take(std::integral_constant<int, 1>{}) &&
+             take(std::integral_constant<int, 2>{}) && take(std::integral_constant<int, 3>{});
+      if (!live || *s_abort) break;
+      // C -= acc 2^(ea + eb - 54) (FP32: - 36); |acc| < 2^62 (2^44)
+      const Item it = items[t];
+      const FrontDev& f = c.fronts[it.front];
+      const int n = f.n, K0 = it.c;
+      const int Bnd = region ? min((K0 / XS_NBO) * XS_NBO + XS_NBO, f.fs) : n;
+      const int rmax = region == 2 ? Bnd : n, cmax = region == 1 ? Bnd : n;
+      const int row = it.a + quarter * 32 + lane, c0 = it.b + cg * 32;
+      if (row < rmax) {
+        const int* __restrict__ ex = x.exps + x.exp0[it.front];
+        const int* __restrict__ ebp = ex + (lower ? 0 : n);
+        const int ea = ex[row] - (S == 8 ? 54 : 36);
+        const int cend = min(cmax, lower ? row + 1 : cmax) - c0;      // columns j < cend are updated
+        T* __restrict__ G = arena<T>(c) + f.off + row + (int64_t)c0 * n;
+#pragma unroll
+        for (int j0 = 0; j0 < 32; j0 += 4) {
+          T cv[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) cv[j] = j0 + j < cend ? __ldcg(G + (int64_t)j * n) : T(0);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (j0 + j < cend) {
+              const int E = ea + __ldg(ebp + c0 + j0 + j);
+              T d = xs_scaled(acc[j0 + j], E, T(0));
+              if (E > XS_BAD / 2) d = T(NAN);
+              G[(int64_t)j * n] = cv[j] - d;
+            }
+          G += 4 * (int64_t)n;
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+  }
+}
+
+template <typename T>
+static void xs_update_t(const DevCtx& c, const XsCtx& x, const CUtensorMap& map, const Item* items, int n_items,
+                        int nb, int region, int lower, int* err, cudaStream_t s) {
+  static int n_sm = 0;
+  if (!n_sm) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    if (n_sm <= 0) n_sm = 1;
+  }
+  cudaFuncSetAttribute(k_xs_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XS_SMEM);
+  const int grid = n_items < n_sm ? n_items : n_sm;
+  k_xs_update<T><<<grid, XS_THREADS, XS_SMEM, s>>>(c, x, map, items, n_items, nb, region, lower, err);
+}
+
+void launch_xs_update(const DevCtx& c, const XsCtx& x, const CUtensorMap& map, const Item* items, int n_items,
+                      int dtype, int nb, int region, int lower, int* err, cudaStream_t s) {
+  if (!n_items) return;
+  if (nb > XS_NBO) throw std::invalid_argument("sliced update: panel wider than 256");
+  if (dtype == F64) xs_update_t<double>(c, x, map, items, n_items, nb, region, lower, err, s);
+  else xs_update_t<float>(c, x, map, items, n_items, nb, region, lower, err, s);
+}
+
+}  // namespace uhm_gpu

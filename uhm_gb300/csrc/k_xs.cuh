@@ -1,0 +1,38 @@
+// Launchers of the sliced tensor-core updates of FP64 and FP32 fronts (k_xs.cu).
+#pragma once
+#include <cuda.h>
+#include <cstdint>
+#include "kernels.cuh"
+
+namespace uhm_gpu {
+
+constexpr int XS_NBO = 256;       // outer panel width: columns whose slices share a row exponent at most
+constexpr int XS_TILE = 128;      // update tiles are XS_TILE x XS_TILE
+constexpr int XS_PACK_ROWS = 64;  // rows per pack item
+constexpr int XS_S64 = 8, XS_S32 = 4;   // slices of an FP64 / FP32 front's operands
+constexpr int XS_SPARE_ROWS = 256;      // workspace rows past the last front's (tiles run over)
+
+// Where the operand slices live: 128-byte rows of 64 BF16, per front first
+// row row0[front] (A and, Cholesky, B) and row0b[front] (LU: B = U12^T), one
+// exponent per front row at exp0[front] / exp0 + nb_off.
+struct XsCtx {
+  void* ws;
+  const int64_t* row0;
+  const int64_t* row0b;
+  const int64_t* exp0;     // first exponent of the front's A rows; its B rows follow at + n
+  int* exps;
+};
+
+// slices of 64 panel rows, columns K0 .. K0 + W, W = min(nb, fs - K0) (item:
+// front, a = K0, b = first row, c = 0; c = 1: the rows are the front's
+// columns (U12^T: entries (K0 + k, row)), written to the B region)
+void launch_xs_pack(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, int dtype, int nb,
+                    cudaStream_t s);
+// C -= A B^T over 128 x 128 tiles (item: front, a = first row, b = first
+// column, c = K0 of the packed columns, W = min(nb, fs - K0)); lower: B is A
+// and only entries col <= row are updated.  region as for k_tile_update: 0
+// every entry, 1 columns below the outer panel's end, 2 rows below it
+void launch_xs_update(const DevCtx& c, const XsCtx& x, const CUtensorMap& map, const Item* items, int n_items,
+                      int dtype, int nb, int region, int lower, int* err, cudaStream_t s);
+
+}  // namespace uhm_gpu
