@@ -909,9 +909,10 @@ void Engine::build_programs(int method) {
   auto push_potrf_trsm = [&](int dt, const std::vector<Item>& p_items, const std::vector<Item>& t_items,
                              double fp, double ft) {
     // every fused CTA repeats the latency-bound diagonal factorisation: fuse
-    // only while the launch fits fuse_potrf_trsm waves of one CTA per SM
+    // only while the launch fits fuse_potrf_trsm waves of one CTA per SM.
+    // Not for FP64, whose diagonal kernel (k_potrf_inv64) takes a wider block.
     const size_t n_fused = t_items.size() + p_items.size();
-    if (!tune.fuse_potrf_trsm || n_fused > (size_t)tune.fuse_potrf_trsm * n_sm) {
+    if (dt == F64 || !tune.fuse_potrf_trsm || n_fused > (size_t)tune.fuse_potrf_trsm * n_sm) {
       push(fac_ops, OP_POTRF, dt, NB, 0, p_items, fp);
       push(fac_ops, OP_TRSM, dt, NB, 0, t_items, ft);
       return;

@@ -480,12 +480,120 @@ __global__ void __launch_bounds__(256) k_potrf_diag(DevCtx c, const Item* __rest
   if (nb == 64 && Dinv) potrf_store_inverse<T>(kb, x, Dinv + f.dinv_off + (int64_t)(k0 / 64) * 4096);
 }
 
+// The same for FP64 fronts: only the inverse is formed (the solves and the
+// TRSM use nothing else), and no multiply-add is spent on zeros.  GB300 does
+// about 2 FP64 multiply-adds per clock per SM, so a warp instruction costs its
+// scheduler ~64 clocks whatever its lanes do: the block is bound by their
+// count.  Tile (i, j), i >= j, of the 16 x 16 lower tiles (4 x 4 entries)
+// holds A until step j and X = L^{-1} after it; either way step q < i takes
+// the one rank-4 update  t -= L[tile i, q] B[:, tile j],  B[m][c] = L(c, P+m)
+// right of the pivot columns P .. P+3 (j > q) and X(P+m, c) left of them (j
+// <= q): 2 x 136 half tiles on 9 warps, in order of i, so that finished rows
+// leave whole warps idle.  The step's 64 vectors (rows of A below the pivot,
+// columns of X) take the same 4-step substitution, one thread each: warps 9
+// and 10 factor the pivot block (every thread) and solve them.  Measured on
+// GB300: 294 -> 67 us per block against the tile-per-thread form (k_potrf_diag),
+// which updates the full squares.
+constexpr int PD_BULK = 288, PD_THREADS = PD_BULK + 64;
+
+__global__ void __launch_bounds__(PD_THREADS) k_potrf_inv64(DevCtx c, const Item* __restrict__ items) {
+  __shared__ __align__(16) double V[4][64], B[4][64];
+  const Item it = items[blockIdx.x];
+  const FrontDev f = c.fronts[it.front];
+  const int n = f.n, k0 = it.a;
+  const int kb = min(64, f.fs - k0);
+  const double* __restrict__ G = c.a64 + f.off + k0 + (int64_t)k0 * n;
+  double* __restrict__ D = c.dinv64 + f.dinv_off + (int64_t)(k0 / 64) * 4096;
+  const int tid = threadIdx.x;
+  int i = -1, j = -1;                       // this thread's tile (none: i = -1)
+  if (tid < 2 * 136) {
+    const int t = tid >> 1;
+    i = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
+    while (i * (i + 1) / 2 > t) --i;
+    while ((i + 1) * (i + 2) / 2 <= t) ++i;
+    j = t - i * (i + 1) / 2;
+  }
+  const int r0 = 4 * i, c0 = 4 * j + 2 * (tid & 1);   // rows r0 .. r0+3, columns c0, c0+1
+  double a[4][2];
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const int r = r0 + u, cc = c0 + v;
+      a[u][v] = i < 0 || r < cc ? 0.0 : (r < kb && cc < kb) ? G[r + (int64_t)cc * n] : (r == cc ? 1.0 : 0.0);
+    }
+  bool bad = false;
+#pragma unroll 1
+  for (int q = 0; q < 16; ++q) {
+    const int P = 4 * q;
+    if (i >= q && j == q) {                 // A below (and on) the pivot columns
+#pragma unroll
+      for (int v = 0; v < 2; ++v) Vec4<double>::st(&V[c0 + v - P][r0], {a[0][v], a[1][v], a[2][v], a[3][v]});
+    } else if (i == q) {                    // X in the pivot rows
+#pragma unroll
+      for (int u = 0; u < 4; ++u) *reinterpret_cast<double2*>(&V[u][c0]) = make_double2(a[u][0], a[u][1]);
+    }
+    __syncthreads();
+    if (tid >= PD_BULK) {
+      const int cc = tid - PD_BULK;
+      double lb[4][4], rd[4], t[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        double s = V[m][P + m];
+#pragma unroll
+        for (int l = 0; l < m; ++l) s -= lb[m][l] * lb[m][l];
+        if (!(s > 0.0)) { bad = true; s = 1.0; }
+        rd[m] = rsqrt(s);
+#pragma unroll
+        for (int r = m + 1; r < 4; ++r) {
+          double w = V[m][P + r];
+#pragma unroll
+          for (int l = 0; l < m; ++l) w -= lb[r][l] * lb[m][l];
+          lb[r][m] = w * rd[m];
+        }
+      }
+      const bool piv = cc >= P && cc < P + 4;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        double w = piv ? (cc == P + m ? 1.0 : 0.0) : V[m][cc];
+#pragma unroll
+        for (int l = 0; l < m; ++l) w -= lb[m][l] * t[l];
+        t[m] = w * rd[m];
+        B[m][cc] = t[m];
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+        if (cc >= P + 4 || P + m >= kb || cc >= kb) t[m] = 0.0;
+      Vec4<double>::st(D + (int64_t)cc * 64 + P, t);
+    }
+    __syncthreads();
+    if (i > q) {
+      if (j == q) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) a[u][0] = a[u][1] = 0.0;
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        double l[4];
+        Vec4<double>::ld(&B[m][r0], l);
+        const double2 b = *reinterpret_cast<const double2*>(&B[m][c0]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          a[u][0] -= l[u] * b.x;
+          a[u][1] -= l[u] * b.y;
+        }
+      }
+    }
+  }
+  if (tid == PD_BULK && bad) set_status(c, it.front, ST_NOT_SPD);
+}
+
 void launch_potrf_diag(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
                        cudaStream_t s) {
   if (!n_items) return;
   if (nb > 64) throw std::invalid_argument("potrf_diag: block wider than 64");
   if (dtype == F64)
-    k_potrf_diag<double><<<n_items, 256, 0, s>>>(c, items, nb);
+    k_potrf_inv64<<<n_items, PD_THREADS, 0, s>>>(c, items);
   else
     k_potrf_diag<float><<<n_items, 256, 0, s>>>(c, items, nb);
 }
@@ -533,7 +641,9 @@ __global__ void __launch_bounds__(NT) k_trsm_panel(DevCtx c, const Item* __restr
     T acc[16];
 #pragma unroll
     for (int u = 0; u < 16; ++u) acc[u] = T(0);
-    for (int t = 0; t < kb; ++t) {
+    // Linv is lower triangular: columns jg * 16 .. need t <= jg * 16 + 15
+    const int te = min(kb, 16 * jg + 16);
+    for (int t = 0; t < te; ++t) {
       const T x = X[i + t * TRSM_RB];
 #pragma unroll
       for (int u4 = 0; u4 < 16; u4 += 4) {
@@ -679,15 +789,10 @@ __global__ void __launch_bounds__(256) k_potrf_trsm(DevCtx c, const Item* __rest
 
 void launch_potrf_trsm(const DevCtx& c, const Item* items, int n_items, int dtype, cudaStream_t s) {
   if (!n_items) return;
-  if (dtype == F64) {
-    const size_t sm = ((sizeof(PotrfShared<double>) + 15) / 16) * 16 + sizeof(double) * 64 * PT_LD;
-    cudaFuncSetAttribute(k_potrf_trsm<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_potrf_trsm<double><<<n_items, 256, sm, s>>>(c, items);
-  } else {
-    const size_t sm = ((sizeof(PotrfShared<float>) + 15) / 16) * 16 + sizeof(float) * 64 * PT_LD;
-    cudaFuncSetAttribute(k_potrf_trsm<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_potrf_trsm<float><<<n_items, 256, sm, s>>>(c, items);
-  }
+  if (dtype == F64) throw std::invalid_argument("potrf_trsm: FP64 fronts take potrf_diag and trsm_panel");
+  const size_t sm = ((sizeof(PotrfShared<float>) + 15) / 16) * 16 + sizeof(float) * 64 * PT_LD;
+  cudaFuncSetAttribute(k_potrf_trsm<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_potrf_trsm<float><<<n_items, 256, sm, s>>>(c, items);
 }
 
 // Trailing update of one BM x BN tile of the front:
@@ -820,16 +925,16 @@ void launch_syrk_update(const DevCtx& c, const Item* items, int n_items, int dty
   if (!n_items) return;
   if (nb > 64) throw std::invalid_argument("trailing update: panel width above 64");
   const int region = nbo > 0 ? 1 : 0;
-  if (dtype == F64) k_tile_update<double, 64, 64, 16, 4, 4, false><<<n_items, 256, 0, s>>>(c, items, nb, nbo, region);
-  else k_tile_update<float, 64, 64, 16, 4, 4, false><<<n_items, 256, 0, s>>>(c, items, nb, nbo, region);
+  if (dtype == F64) throw std::invalid_argument("trailing update: FP64 fronts take the sliced update");
+  k_tile_update<float, 64, 64, 16, 4, 4, false><<<n_items, 256, 0, s>>>(c, items, nb, nbo, region);
 }
 
 void launch_gemm_update(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, int nbo,
                         int region, cudaStream_t s) {
   if (nb > 64) throw std::invalid_argument("trailing update: panel width above 64");
   if (!n_items) return;
-  if (dtype == F64) k_tile_update<double, 64, 64, 16, 4, 4, true><<<n_items, 256, 0, s>>>(c, items, nb, nbo, region);
-  else k_tile_update<float, 64, 64, 16, 4, 4, true><<<n_items, 256, 0, s>>>(c, items, nb, nbo, region);
+  if (dtype == F64) throw std::invalid_argument("trailing update: FP64 fronts take the sliced update");
+  k_tile_update<float, 64, 64, 16, 4, 4, true><<<n_items, 256, 0, s>>>(c, items, nb, nbo, region);
 }
 
 // ---------------------------------------------------------------------------
