@@ -25,6 +25,13 @@ static constexpr int TRSM_RB = 64;
 static constexpr int FWD_RB = 256;            // k_solve.cu
 static constexpr int BWD_RB = 512;
 static constexpr int LUROW_CB = 16;         // k_lu_row_update (k_factor.cu)
+// LU panels (k_getrf_smem): clusters grow until a CTA holds at most this many rows
+static constexpr int LU_GOAL_F64 = 64, LU_GOAL_F32 = 192;
+// more rows than this per CTA of the largest cluster go to the whole GPU.
+// Measured on GB300 (us per 64-column panel): FP32, 16 CTAs, 130 at 100 rows each,
+// 205 at 400, 290 at 750, against 195 for the whole GPU on 14,911 rows; FP64, 16
+// CTAs, 185 at 96 rows each, against 240 for the whole GPU on 6,938 rows
+static constexpr int LU_CLUSTER_ROWS_F64 = 128, LU_CLUSTER_ROWS_F32 = 384;
 static constexpr int TILE = 64;             // trailing-update tile (k_tile_update)
 
 #define CK(x)                                                                          \
@@ -98,7 +105,6 @@ void Engine::free_device() {
   d_dof_tree = nullptr;
   d_tree_red = nullptr;
   d_gc_xbuf = nullptr;
-  d_gc_ctr = nullptr;
   d_gen = nullptr;
   d_gen_bytes = 0;
   d_items_part = nullptr;
@@ -942,17 +948,53 @@ void Engine::build_programs(int method) {
   // trailing block, whose swaps come after the outer panel
   auto push_lu_panel = [&](int dt, const std::vector<Item>& p_items, double fp, int nbo) {
     const int piv = method == UHM_LU_PIV ? 1 : 0;
-    const int rcap = dt == F64 ? GC_RMAX_F64 : GC_RMAX_F32;
+    const int rcap = dt == F64 ? GC_RMAX_F64 : GC_RMAX_F32, rgoal = dt == F64 ? LU_GOAL_F64 : LU_GOAL_F32;
     auto col_end = [&](const Item& it) {
       if (nbo <= 0) return 0;
       return std::min((it.a / nbo) * nbo + nbo, fronts[it.front].fs);
     };
-    std::vector<Item> one, tall;
+    // a cluster per front up to the rows that fit its shared memory, the whole
+    // GPU for the rest; in global memory where gc_min_rows was raised to ask for
+    // one CTA on more rows than its shared memory holds
+    const int n_cta = std::min(n_sm, GC_MAX_CTAS);
+    std::vector<Item> glob, tall, sw, cl[5];
+    int rmax_cl[5] = {1, 1, 1, 1, 1};
+    // clusters that keep the launch within one wave
+    const int per_item = std::max(1, n_cta / std::max(1, (int)p_items.size()));
     for (const Item& it : p_items) {
-      if (fronts[it.front].n - it.a >= tune.gc_min_rows) tall.push_back(it);
-      else one.push_back(Item{it.front, it.a, col_end(it), 0});
+      const int rows = fronts[it.front].n - it.a;
+      bool own_swaps = false;
+      if (rows > rcap && rows < tune.gc_min_rows && tune.gc_min_rows > 512) {
+        glob.push_back(Item{it.front, it.a, col_end(it), 0});
+        own_swaps = true;
+      } else {
+        int lc = 0;
+        while (lc < 4 && ((rows + (1 << lc) - 1) >> lc) > rcap) ++lc;                      // must
+        while (lc < 4 && (2 << lc) <= per_item && (rows >> lc) > rgoal) ++lc;              // worth it
+        const int per = (rows + (1 << lc) - 1) >> lc, most = dt == F64 ? LU_CLUSTER_ROWS_F64 : LU_CLUSTER_ROWS_F32;
+        if (per > rcap || (lc == 4 && per > most && rows >= tune.gc_min_rows)) {
+          tall.push_back(it);
+        } else {
+          cl[lc].push_back(it);
+          rmax_cl[lc] = std::max(rmax_cl[lc], per);
+        }
+      }
+      if (!piv) continue;
+      const int ce = col_end(it), lim = ce > 0 ? ce : fronts[it.front].n;
+      for (int c0 = 0; !own_swaps && c0 < lim; c0 += 256) sw.push_back(Item{it.front, it.a, c0, ce});
     }
-    push(fac_ops, OP_GETRF, dt, NB, piv, one, tall.empty() ? fp : 0.0);
+    double fl = fp;                  // the panel's operations, on its first launch
+    push(fac_ops, OP_GETRF, dt, NB, piv, glob, glob.empty() ? 0.0 : fl);
+    if (!glob.empty()) fl = 0;
+    for (int lc = 0; lc < 5; ++lc) {
+      if (cl[lc].empty()) continue;
+      Op op{OP_GETRF_COOP, dt, NB, piv, add_items(cl[lc]), (int)cl[lc].size()};
+      op.q0 = -(1 << lc);            // CTAs per item (a cluster)
+      op.aux = rmax_cl[lc];
+      op.flops = fl;
+      fl = 0;
+      fac_ops.push_back(op);
+    }
     size_t i0 = 0;
     while (i0 < tall.size()) {
       // a group whose minimum CTA counts fit one cooperative launch
@@ -962,14 +1004,14 @@ void Engine::build_programs(int method) {
       while (i1 < tall.size()) {
         const int rows = fronts[tall[i1].front].n - tall[i1].a;
         const int mn = (rows + rcap - 1) / rcap;
-        if (i1 > i0 && need + mn > n_sm) break;
+        if (i1 > i0 && need + mn > n_cta) break;
         need += mn;
         rows_sum += rows;
         ++i1;
       }
       std::vector<Item> g;
       int b = 0, rmax = 1;
-      const int spare = std::max(0, n_sm - need);
+      const int spare = std::max(0, n_cta - need);
       for (size_t i = i0; i < i1; ++i) {
         const int rows = fronts[tall[i].front].n - tall[i].a;
         int P = (rows + rcap - 1) / rcap + (int)(spare * (rows / rows_sum));
@@ -981,18 +1023,12 @@ void Engine::build_programs(int method) {
       Op op{OP_GETRF_COOP, dt, NB, piv, add_items(g), (int)g.size()};
       op.q0 = b;
       op.aux = rmax;
-      if (i0 == 0) op.flops = fp;
+      op.flops = fl;
+      fl = 0;
       fac_ops.push_back(op);
-      if (piv) {
-        std::vector<Item> sw;
-        for (const Item& it : g) {
-          const int ce = col_end(it), lim = ce > 0 ? ce : fronts[it.front].n;
-          for (int c0 = 0; c0 < lim; c0 += 256) sw.push_back(Item{it.front, it.a, c0, ce});
-        }
-        push(fac_ops, OP_LASWP, dt, NB, 0, sw);
-      }
       i0 = i1;
     }
+    push(fac_ops, OP_LASWP, dt, NB, 0, sw);
   };
   // sliced updates: pack items of rows [r0, r1), update tiles of rows
   // [r0, r1) x columns [c0, c1) (Cholesky: those reaching the lower
@@ -1741,8 +1777,7 @@ void Engine::alloc_device(int method) {
   d_err = (int*)dmalloc(sizeof(int));
   CK(cudaMemsetAsync(d_err, 0, sizeof(int), stream));
   if (method != UHM_CHOL) {
-    d_gc_xbuf = (double*)dmalloc(sizeof(double) * (size_t)std::max(1, n_sm) * (2 * 66 + 2 * 64));
-    d_gc_ctr = (unsigned int*)dmalloc(2 * sizeof(unsigned int));
+    d_gc_xbuf = (uint64_t*)dmalloc(sizeof(uint64_t) * (size_t)gc_words(GC_MAX_CTAS, GC_MAX_CTAS));
   }
   if (ws2_rows > 0) {
     // 512 spare rows: tiles that run past the last front's rows stay inside the tensor
@@ -2041,8 +2076,8 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
         break;
       case OP_GETRF: launch_getrf_panel(ctx, it, op.n_items, op.dtype, op.nb, op.param, st); break;
       case OP_GETRF_COOP:
-        launch_getrf_coop(ctx, it, op.n_items, op.q0, op.dtype, op.nb, op.param, op.aux, d_gc_xbuf, d_gc_ctr, d_err,
-                          st);
+        launch_getrf_smem(ctx, it, op.n_items, std::max(op.q0, 0), std::max(-op.q0, 0), op.dtype, op.nb, op.param,
+                          op.aux, d_gc_xbuf, d_err, st);
         break;
       case OP_LASWP: launch_laswp(ctx, it, op.n_items, op.dtype, op.nb, st); break;
       case OP_LUROW: launch_lu_row_update(ctx, it, op.n_items, op.dtype, op.nb, 0, st); break;

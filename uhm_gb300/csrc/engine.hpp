@@ -67,7 +67,7 @@ struct Op {
   int n_items;
   double flops = 0;   // algorithmic flops of this launch (LAWN-41 terms)
   double bytes = 0;   // algorithmic HBM bytes of this launch
-  int q0 = 0;         // first right-hand side (flag-driven solves) / CTAs (cooperative LU panel) /
+  int q0 = 0;         // first right-hand side (flag-driven solves) / CTAs (LU panel; -CTAs per item of clusters) /
                       // SMs left free for a concurrent launch (tensor-core Cholesky update) /
                       // region of the front (sliced update)
   int aux = 0;        // rows per CTA (cooperative LU panel, flag-driven solves)
@@ -318,8 +318,7 @@ class Engine {
   int* d_err = nullptr;              // bounded-wait error flag of device kernels
   unsigned char* d_gen = nullptr;    // recipe of the element generator (one block)
   size_t d_gen_bytes = 0;
-  double* d_gc_xbuf = nullptr;       // exchange buffer of the cooperative LU panel
-  unsigned int* d_gc_ctr = nullptr;  // its grid-barrier counter and abort word
+  uint64_t* d_gc_xbuf = nullptr;     // exchange words of the cooperative LU panel
   int n_sm = 0;
   int64_t ws_total = 0;
   int64_t* d_emat_off = nullptr;

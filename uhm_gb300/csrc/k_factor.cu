@@ -996,228 +996,425 @@ void launch_getrf_panel(const DevCtx& c, const Item* items, int n_items, int dty
 }
 
 // ---------------------------------------------------------------------------
-// LU panel of a tall front on many CTAs (cooperative launch)
+// LU panel in shared memory: one CTA, a cluster, or a whole grid per front
 // ---------------------------------------------------------------------------
 // The panel (rows k0..n-1, columns k0..k0+kb-1) of each item is split into
-// row chunks of R rows, one per CTA, held in shared memory (column-major,
-// leading dimension R).  For each column k of the panel, every CTA
-//   1. finds its candidate pivot: the largest |a| in column k among its rows
+// chunks of R rows, one per CTA, held in shared memory (column-major, leading
+// dimension rmax).  For each column k of the panel, every CTA
+//   1. offers its candidate pivot: the largest |a| in column k among its rows
 //      in [k0+k, fs) (the reference searches the eliminated rows only), ties
-//      to the lowest row, and publishes value, row and the row's kb values
-//      in the exchange buffer; the CTA holding row k0+k also publishes that
-//      row;
-//   2. passes one grid barrier (the exchange buffers alternate by column
-//      parity, so a barrier per column is enough);
-//   3. picks the item's pivot from all its CTAs' candidates (same rule: the
-//      largest value, the lowest row on ties; this is the first maximum of a
-//      sequential search), swaps the two rows in its chunk when it holds
-//      them, and applies l_r = a_rk / a_kk, a_rj -= l_r u_j to its rows below
-//      the pivot row.
+//      to the lowest row, with the row's kb values; the CTA holding row k0+k
+//      also hands out that row;
+//   2. picks the pivot from all its item's candidates (same rule: the largest
+//      value, the lowest row on ties; this is the first maximum of a sequential
+//      search; compared as integers, the bits of |a|);
+//   3. swaps the two rows in its chunk when it holds them, and applies l_r =
+//      a_rk / a_kk, a_rj -= l_r u_j to its rows below the pivot row, column
+//      k + 1 first, whose candidates are found on the way.
 // The result is the reference's partial pivoting (FLA_LU_piv inside the
 // eliminated block) exactly; only the panel's own columns are swapped here,
-// the other columns of the front by k_laswp afterwards.  Item: front,
-// a = k0, b = first CTA, c = number of CTAs.  The grid barrier is an arrival
-// counter with a bounded spin; a CTA that gives up raises the abort word and
-// the error flag, and every CTA then skips the remaining barriers.
-constexpr int GC_THREADS = 256;
+// the other columns of the front by k_laswp afterwards.
+//
+// Two ways to hand candidates and rows over:
+// CL: the item's CTAs are a cluster (1 .. 16 of them) and write into each
+// other's shared memory; one cluster barrier per column orders it (buffers
+// alternate by column: nobody writes column k + 2 before everybody has
+// passed the barrier of k + 1, that is, has used column k).  Item: front, a = k0.
+// !CL (rows beyond a cluster's shared memory, or FP64 fronts whose update
+// wants more SMs): 8-byte words in global memory whose upper bits hold the
+// column (k + 1) beside the data, polled until they carry it; no counter, flag
+// or fence.  The same argument holds for their reuse, since a CTA publishes its
+// candidate of k + 1 only when it has read all of column k (also without
+// pivoting, where no candidate wins).  The words are cleared before the
+// launch; the launch is cooperative, every wait is bounded, and a CTA that
+// gives up raises the error word, which ends the others' waits.  Item: front, a
+// = k0, b = first CTA, c = number of CTAs.
+//
+// Bound by the latency of a column: about 3 us in either form (two or three
+// block barriers, one exchange, the reductions), then by the update's shared-
+// memory traffic (FP32) or multiply-adds (FP64).  Measured on GB300, the panels
+// of one factorisation, against a grid barrier on a counter per column: 24^3 p =
+// 3 FP32 141 + 2.5 (one-CTA panels in global memory) -> 69.0 ms, 12^3 p = 3
+// FP64 55.9 + 4.8 -> 25.7, 6^3 p = 3 4.9 + 2.0 -> 4.4.
+constexpr int GC_ERR = 3;
+constexpr int GC_BATCH = 4;                     // columns a thread updates at a time
+constexpr int GC_POLL = (GC_MAX_CTAS + 31) / 32;
+constexpr int64_t GC_REC = 2 + 2 * 64;          // words of one record: candidate, then a row (two per FP64 value)
+static_assert(gc_words(1, 1) == 4 * GC_REC, "record size of the launcher's callers");
 
 UHM_DEFINE_WAIT_LIMIT(set_wait_limit_factor, 1u << 22)
 
-__device__ __forceinline__ unsigned int gc_ld_acquire(const unsigned int* p) {
-  unsigned int v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+template <typename T> struct LuBits;
+template <> struct LuBits<double> {
+  static constexpr int WORDS = 2;               // exchange words per value
+  static __device__ __forceinline__ uint64_t key(double v) {
+    return v == v ? (uint64_t)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull : 0ull;
+  }
+  static __device__ __forceinline__ uint32_t half(double v, int h) {
+    return h ? (uint32_t)__double2loint(v) : (uint32_t)__double2hiint(v);
+  }
+  static __device__ __forceinline__ double make(uint32_t hi, uint32_t lo) { return __hiloint2double((int)hi, (int)lo); }
+};
+template <> struct LuBits<float> {
+  static constexpr int WORDS = 1;
+  static __device__ __forceinline__ uint64_t key(float v) {
+    return v == v ? (uint64_t)(__float_as_uint(v) & 0x7FFFFFFFu) : 0ull;
+  }
+  static __device__ __forceinline__ uint32_t half(float v, int) { return __float_as_uint(v); }
+  static __device__ __forceinline__ float make(uint32_t hi, uint32_t) { return __uint_as_float(hi); }
+};
+constexpr int LU_NONE = 0x7fffffff;             // no candidate row
+
+// the warp's best candidate: the largest key, the lowest row on ties (LU_NONE
+// where no lane has one)
+template <typename T>
+__device__ __forceinline__ void lu_best(uint64_t& key, int& r) {
+  const uint32_t all = 0xffffffffu;
+  if constexpr (sizeof(T) == 4) {
+    const uint32_t k = r == LU_NONE ? 0u : (uint32_t)key + 1, mx = __reduce_max_sync(all, k);
+    r = (int)__reduce_min_sync(all, k == mx ? (uint32_t)r : (uint32_t)LU_NONE);
+    key = mx ? mx - 1 : 0;
+  } else {
+    const uint32_t h = r == LU_NONE ? 0u : (uint32_t)(key >> 32) + 1, mh = __reduce_max_sync(all, h);
+    const uint32_t l = h == mh && mh ? (uint32_t)key : 0u, ml = __reduce_max_sync(all, l);
+    r = (int)__reduce_min_sync(all, h == mh && l == ml ? (uint32_t)r : (uint32_t)LU_NONE);
+    key = mh ? (uint64_t)(mh - 1) << 32 | ml : 0;
+  }
+}
+
+__device__ __forceinline__ void gc_put(uint64_t* p, uint64_t v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ uint64_t gc_get(const uint64_t* p) {
+  uint64_t v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-
-// barrier number `round` (1, 2, ...) of a launch of `total` CTAs; false once
-// any CTA gave up
-__device__ __forceinline__ bool gc_grid_barrier(unsigned int* ctr, unsigned int round, unsigned int total,
-                                                int* err, int* s_ok) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    bool ok = *s_ok != 0;
-    if (ok) {
-      __threadfence();
-      atomicAdd(ctr, 1u);
-      const unsigned int target = round * total;
-      ok = false;
-      const uint32_t lim = g_wait_limit;
-      for (uint32_t i = 0; i < lim; ++i) {
-        if (gc_ld_acquire(ctr) >= target) { ok = true; break; }
-        if (gc_ld_acquire(ctr + 1)) break;          // another CTA gave up
-        __nanosleep(20);
-      }
-      if (!ok) {
-        atomicExch(ctr + 1, 1u);
-        atomicExch(err, 3);
-      }
-      __threadfence();
-    }
-    *s_ok = ok ? 1 : 0;
+// words p[32 e + lane] (e < N, while < cnt), all loads in flight, until every
+// one carries the tag; false (and the error word set) when the wait gives up
+template <int N>
+__device__ __forceinline__ bool gc_poll(const uint64_t* p, int stride, int cnt, uint32_t tag, uint64_t (&x)[N], int* err) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t lim = g_wait_limit;
+  uint32_t open = 0;
+#pragma unroll
+  for (int e = 0; e < N; ++e) open |= (lane + 32 * e < cnt ? 1u : 0u) << e;
+  for (uint32_t i = 0; open; ++i) {
+    uint64_t y[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+      if ((open >> e) & 1) y[e] = gc_get(p + (int64_t)(lane + 32 * e) * stride);
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+      if (((open >> e) & 1) && (uint32_t)(y[e] >> 56) == tag) { x[e] = y[e]; open &= ~(1u << e); }
+    if (!open) break;
+    if (i >= lim) { atomicExch(err, GC_ERR); return false; }
+    if ((i & 255) == 255 && *(volatile int*)err) return false;
+    if (i > 64) __nanosleep(20);
   }
-  __syncthreads();
-  return *s_ok != 0;
+  return true;
 }
+__device__ __forceinline__ uint32_t lu_smem(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ uint32_t lu_mapa(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void lu_put(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void lu_put(uint32_t a, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void lu_put(uint32_t a, uint64_t v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+__device__ __forceinline__ void lu_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float lu_rcp(float v) { return 1.0f / v; }
+__device__ __forceinline__ double lu_rcp(double v) { return __drcp_rn(v); }
 
-template <typename T>
-__global__ void __launch_bounds__(GC_THREADS) k_getrf_coop(DevCtx c, const Item* __restrict__ items, int n_items,
-                                                           int nb, int pivot, int rmax, double* __restrict__ xbuf,
-                                                           unsigned int* ctr, int* err) {
+// rows received in one column: of every candidate (CL) or of the pivot, then row k0 + k
+template <typename T, bool CL>
+struct LuRecv {
+  T row[CL ? GC_CLUSTER : 1][64];
+  T diag[64];
+  uint64_t key[CL ? GC_CLUSTER : 1];
+  uint64_t at[CL ? GC_CLUSTER : 1];
+};
+
+template <typename T, bool CL, int NT>
+__global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restrict__ items, int n_items, int nb,
+                                                   int pivot, int rmax, int csize, uint64_t* __restrict__ xbuf,
+                                                   int* err) {
   extern __shared__ __align__(16) unsigned char gc_smem[];
-  T* S = reinterpret_cast<T*>(gc_smem);        // chunk, column-major, leading dimension R
-  __shared__ T s_u[64], s_old[64];
-  __shared__ double s_cv[GC_THREADS / 32];
-  __shared__ int s_ci[GC_THREADS / 32];
-  __shared__ int s_ok, s_item, s_p, s_w;
-  const unsigned int total = gridDim.x;
-  if (threadIdx.x == 0) {
-    s_ok = 1;
+  constexpr int NW = NT / 32, WORDS = LuBits<T>::WORDS;
+  __shared__ __align__(16) LuRecv<T, CL> recv[2];
+  __shared__ uint64_t s_key[NW];
+  __shared__ int s_row[NW];
+  __shared__ int s_item, s_p;
+  __shared__ T s_rinv;
+  T* S = reinterpret_cast<T*>(gc_smem);        // chunk, column-major, leading dimension rmax
+  const int total = gridDim.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
     int k = 0;
-    while (k + 1 < n_items && (int)blockIdx.x >= items[k + 1].b) ++k;
-    s_item = k;
+    if (!CL) while (k + 1 < n_items && (int)blockIdx.x >= items[k + 1].b) ++k;
+    s_item = CL ? blockIdx.x / csize : k;
   }
   __syncthreads();
   const Item it = items[s_item];
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, fs = f.fs, k0 = it.a;
   const int kb = min(nb, fs - k0);
-  const int P = it.c, q = blockIdx.x - it.b;
+  const int P = CL ? csize : it.c, q = CL ? (int)blockIdx.x % csize : (int)blockIdx.x - it.b;
   const int rows = n - k0;
   const int R = (rows + P - 1) / P;
   const int rbeg = k0 + q * R, rend = min(rbeg + R, n);   // my rows [rbeg, rend)
   const int nr_my = max(0, rend - rbeg);
   T* __restrict__ G = arena<T>(c) + f.off;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // exchange buffer: per parity, per CTA {value, row, kb values}, then per item the row k0+k
-  constexpr int XS = 66;
-  auto cand = [&](int par, int b) { return xbuf + ((size_t)par * total + b) * XS; };
-  auto diag_row = [&](int par, int itx) { return xbuf + (size_t)2 * total * XS + ((size_t)par * n_items + itx) * 64; };
-  for (int idx = threadIdx.x; idx < nr_my * kb; idx += GC_THREADS) {
-    const int r = idx % nr_my, j = idx / nr_my;
-    S[j * rmax + r] = G[(rbeg + r) + (int64_t)(k0 + j) * n];
-  }
+  // !CL: exchange records: per parity, one per CTA, then one per item (the row k0 + k)
+  auto rec = [&](int par, int b) { return xbuf + ((int64_t)par * (total + n_items) + b) * GC_REC; };
+  // thread layout of the chunk: rows along lanes, ng column groups
+  const int rw = min(NT, (max(nr_my, 1) + 31) / 32 * 32), ng = NT / rw;
+  const int tr = tid % rw, tg = tid / rw;
+  uint64_t mk = 0;                             // this thread's best candidate of the next column
+  int mr = LU_NONE;
+  auto offer = [&](T v, int r) {
+    const uint64_t key = LuBits<T>::key(v);
+    if (v == v && (mr == LU_NONE || key > mk || (key == mk && r < mr))) { mk = key; mr = r; }
+  };
+  if (tg < ng)
+    for (int j = tg; j < kb; j += ng)
+      for (int r = tr; r < nr_my; r += rw) {
+        const T v = G[(rbeg + r) + (int64_t)(k0 + j) * n];
+        S[j * rmax + r] = v;
+        if (pivot && j == 0 && rbeg + r < fs) offer(v, rbeg + r);
+      }
+  lu_best<T>(mk, mr);
+  if (lane == 0) { s_key[warp] = mk; s_row[warp] = mr; }
+  if (CL && csize > 1) lu_cluster_sync();      // every CTA of the cluster runs before anyone writes to it
   __syncthreads();
   for (int k = 0; k < kb; ++k) {
     const int gk = k0 + k, par = k & 1;
-    // 1. candidate of this chunk
-    double bv = -1.0;
-    int bi = 0x7fffffff;
-    if (pivot) {
-      const int lo = max(rbeg, gk), hi = min(rend, fs);
-      for (int r = lo + threadIdx.x; r < hi; r += GC_THREADS) {
-        const double v = (double)my_abs<T>(S[k * rmax + (r - rbeg)]);
-        if (v > bv) { bv = v; bi = r; }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_down_sync(0xffffffffu, bv, o);
-        const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-      }
-      if (lane == 0) { s_cv[warp] = bv; s_ci[warp] = bi; }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        for (int w = 1; w < GC_THREADS / 32; ++w)
-          if (s_cv[w] > bv || (s_cv[w] == bv && s_ci[w] < bi)) { bv = s_cv[w]; bi = s_ci[w]; }
-        s_ci[0] = bi;
-        double* cb = cand(par, blockIdx.x);
-        cb[0] = bv;
-        cb[1] = (double)bi;
-      }
-      __syncthreads();
-      bi = s_ci[0];
-      if (bi != 0x7fffffff && threadIdx.x < kb) cand(par, blockIdx.x)[2 + threadIdx.x] = (double)S[threadIdx.x * rmax + (bi - rbeg)];
-    }
-    if (gk >= rbeg && gk < rend && threadIdx.x < kb)
-      diag_row(par, s_item)[threadIdx.x] = (double)S[threadIdx.x * rmax + (gk - rbeg)];
-    // 2. one grid barrier per column
-    if (!gc_grid_barrier(ctr, (unsigned int)(k + 1), total, err, &s_ok)) return;
-    // 3. the item's pivot
-    if (warp == 0) {
-      double v = -1.0;
-      int r = 0x7fffffff, w = -1;
-      if (pivot) {
-        for (int b = lane; b < P; b += 32) {
-          const double* cb = cand(par, it.b + b);
-          const double cv = __ldcg(cb);
-          const int ci = (int)__ldcg(cb + 1);
-          if (cv > v || (cv == v && ci < r)) { v = cv; r = ci; w = it.b + b; }
+    const bool diag_mine = gk >= rbeg && gk < rend;
+    LuRecv<T, CL>& rc = recv[par];
+    // 1. this chunk's candidate, known to every warp
+    uint64_t bk = lane < NW ? s_key[lane] : 0;
+    int bi = lane < NW ? s_row[lane] : LU_NONE;
+    lu_best<T>(bk, bi);
+    const T* u;                                // the pivot's row and the old row k0 + k
+    const T* old = rc.diag;
+    int p = gk;
+    if constexpr (CL) {
+      // warp w serves CTAs w, w + NW, ..
+      for (int d = warp; d < csize; d += NW) {
+        if (lane == 0) {
+          lu_put(lu_mapa(lu_smem(&rc.key[q]), d), bk);
+          lu_put(lu_mapa(lu_smem(&rc.at[q]), d), (uint64_t)bi);
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const double ov = __shfl_down_sync(0xffffffffu, v, o);
-          const int oi = __shfl_down_sync(0xffffffffu, r, o);
-          const int ow = __shfl_down_sync(0xffffffffu, w, o);
-          if (ov > v || (ov == v && oi < r)) { v = ov; r = oi; w = ow; }
+        if (bi != LU_NONE) {
+          const uint32_t a = lu_mapa(lu_smem(&rc.row[q][0]), d);
+          for (int j = lane; j < kb; j += 32) lu_put(a + j * (uint32_t)sizeof(T), S[j * rmax + (bi - rbeg)]);
+        }
+        if (diag_mine) {
+          const uint32_t a = lu_mapa(lu_smem(&rc.diag[0]), d);
+          for (int j = lane; j < kb; j += 32) lu_put(a + j * (uint32_t)sizeof(T), S[j * rmax + (gk - rbeg)]);
         }
       }
-      if (lane == 0) {
-        if (!pivot || r == 0x7fffffff) { r = gk; w = -1; }
-        s_p = r;
-        s_w = w;
+      if (csize > 1) lu_cluster_sync();
+      else __syncthreads();
+      // 2. the item's pivot
+      uint64_t key = lane < csize ? rc.key[lane] : 0;
+      int r = lane < csize ? (int)rc.at[lane] : LU_NONE;
+      lu_best<T>(key, r);
+      if (r != LU_NONE) p = r;
+      u = p == gk ? rc.diag : rc.row[(p - k0) / R];
+    } else {
+      const uint64_t tag56 = (uint64_t)(k + 1) << 56;
+      bool ok = true;
+      if (warp == 0) {
+        uint64_t* cb = rec(par, blockIdx.x);
+        if (lane < 2)
+          // key bits 63..32 and the row (24 bits) in the first word, key bits 31..0 in the second
+          gc_put(cb + lane, tag56 | (lane == 0 ? (uint64_t)(bi == LU_NONE ? 0xFFFFFFu : (uint32_t)(bi - k0)) << 32 | (bk >> 32)
+                                               : (bk & 0xFFFFFFFFull)));
+        if (bi != LU_NONE)
+          for (int w = lane; w < kb * WORDS; w += 32)
+            gc_put(cb + 2 + w, tag56 | LuBits<T>::half(S[(w / WORDS) * rmax + (bi - rbeg)], w % WORDS));
+        // 2. the item's pivot
+        uint64_t x0[GC_POLL], x1[GC_POLL], key = 0;
+        int r = LU_NONE, w = -1;
+        ok = gc_poll<GC_POLL>(rec(par, it.b), (int)GC_REC, P, k + 1, x0, err) &&
+             gc_poll<GC_POLL>(rec(par, it.b) + 1, (int)GC_REC, P, k + 1, x1, err);
+        if (ok) {
+#pragma unroll
+          for (int e = 0; e < GC_POLL; ++e) {
+            if (lane + 32 * e >= P) continue;
+            const uint64_t ck = x0[e] << 32 | (x1[e] & 0xFFFFFFFFull);
+            const uint32_t row = (uint32_t)(x0[e] >> 32) & 0xFFFFFFu;
+            const int cr = k0 + (int)row;
+            if (row != 0xFFFFFFu && (r == LU_NONE || ck > key || (ck == key && cr < r))) { key = ck; r = cr; }
+          }
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        lu_best<T>(key, r);
+        if (r != LU_NONE) p = r;
+        if (lane == 0) s_p = p;
+        w = it.b + (p - k0) / R;
+        if (ok && p != gk) {
+          if (p >= rbeg && p < rend) {
+            for (int j = lane; j < kb; j += 32) rc.row[0][j] = S[j * rmax + (p - rbeg)];
+          } else {
+            uint64_t x[2 * WORDS];
+            ok = gc_poll<2 * WORDS>(rec(par, w) + 2, 1, kb * WORDS, k + 1, x, err);
+#pragma unroll
+            for (int e = 0; e < 2 * WORDS; ++e) {
+              const uint32_t v = (uint32_t)x[e], lo = __shfl_down_sync(0xffffffffu, v, 1);
+              const int t = lane + 32 * e;
+              if (ok && t < kb * WORDS && t % WORDS == 0) rc.row[0][t / WORDS] = LuBits<T>::make(v, lo);
+            }
+          }
+        }
+      } else if (warp == 1) {
+        // the old row k0 + k
+        uint64_t* dr = rec(par, total + s_item);
+        if (diag_mine) {
+          for (int w = lane; w < kb * WORDS; w += 32)
+            gc_put(dr + w, tag56 | LuBits<T>::half(S[(w / WORDS) * rmax + (gk - rbeg)], w % WORDS));
+          for (int j = lane; j < kb; j += 32) rc.diag[j] = S[j * rmax + (gk - rbeg)];
+        } else {
+          uint64_t x[2 * WORDS];
+          ok = gc_poll<2 * WORDS>(dr, 1, kb * WORDS, k + 1, x, err);
+#pragma unroll
+          for (int e = 0; e < 2 * WORDS; ++e) {
+            const uint32_t v = (uint32_t)x[e], lo = __shfl_down_sync(0xffffffffu, v, 1);
+            const int t = lane + 32 * e;
+            if (ok && t < kb * WORDS && t % WORDS == 0) rc.diag[t / WORDS] = LuBits<T>::make(v, lo);
+          }
+        }
       }
+      if (__syncthreads_or(!ok)) return;
+      p = s_p;
+      u = p == gk ? rc.diag : rc.row[0];
     }
-    __syncthreads();
-    const int p = s_p;
-    if (threadIdx.x < kb) {
-      const double* dr = diag_row(par, s_item);
-      s_old[threadIdx.x] = (T)__ldcg(dr + threadIdx.x);                        // old row gk
-      s_u[threadIdx.x] = p == gk ? s_old[threadIdx.x] : (T)__ldcg(cand(par, s_w) + 2 + threadIdx.x);
-    }
-    __syncthreads();
-    if (threadIdx.x < kb) {
-      if (gk >= rbeg && gk < rend) S[threadIdx.x * rmax + (gk - rbeg)] = s_u[threadIdx.x];
-      if (p != gk && p >= rbeg && p < rend) S[threadIdx.x * rmax + (p - rbeg)] = s_old[threadIdx.x];
-    }
-    if (q == 0 && threadIdx.x == 0) c.piv[f.piv_off + gk] = p;
-    __syncthreads();
-    T akk = s_u[k];
+    if (q == 0 && tid == 0) c.piv[f.piv_off + gk] = p;
+    T akk = u[k];
     if (akk == (T)0 || akk != akk) {
-      if (q == 0 && threadIdx.x == 0) set_status(c, it.front, akk != akk ? ST_NAN : ST_ZERO_PIVOT);
+      if (q == 0 && tid == 0) set_status(c, it.front, akk != akk ? ST_NAN : ST_ZERO_PIVOT);
       akk = (T)1;
     }
-    const T rinv = (T)1 / akk;
-    // rows below the pivot row: multiplier and rank-1 update of the panel's later columns
-    for (int r = max(rbeg, gk + 1) + threadIdx.x; r < rend; r += GC_THREADS) {
-      const int rl = r - rbeg;
-      const T l = S[k * rmax + rl] * rinv;
-      S[k * rmax + rl] = l;
-      for (int j = k + 1; j < kb; ++j) S[j * rmax + rl] -= l * s_u[j];
+    T rinv;
+    if constexpr (sizeof(T) == 8) {            // a reciprocal costs every FP64 warp that takes it
+      if (warp == 0) {
+        rinv = lu_rcp(akk);
+        if (lane == 0) s_rinv = rinv;
+      }
+      __syncthreads();
+      rinv = s_rinv;
+    } else {
+      rinv = lu_rcp(akk);
     }
+    // 3. rows from the pivot row on: the two rows swapped, multiplier and
+    // rank-1 update of the panel's later columns below it
+    mk = 0;
+    mr = LU_NONE;
+    if (tg < ng)
+      for (int rl = max(rbeg, gk) - rbeg + tr; rl < nr_my; rl += rw) {
+        const int r = rbeg + rl;
+        if (r == gk) {
+          if (p != gk)
+            for (int j = tg; j < kb; j += ng) S[j * rmax + rl] = u[j];
+          continue;
+        }
+        const bool sw = r == p;
+        const T l = (sw ? old[k] : S[k * rmax + rl]) * rinv;
+        if (sw)
+          for (int j = tg; j < k; j += ng) S[j * rmax + rl] = old[j];
+        int j = k + 1 + tg;
+        if (tg == 0 && j < kb) {
+          const T v = (sw ? old[j] : S[j * rmax + rl]) - l * u[j];
+          S[j * rmax + rl] = v;
+          if (pivot && r < fs) offer(v, r);
+          j += ng;
+        }
+        for (; j + (GC_BATCH - 1) * ng < kb; j += GC_BATCH * ng) {
+          T a[GC_BATCH], b[GC_BATCH];
+#pragma unroll
+          for (int e = 0; e < GC_BATCH; ++e) {
+            a[e] = sw ? old[j + e * ng] : S[(j + e * ng) * rmax + rl];
+            b[e] = u[j + e * ng];
+          }
+#pragma unroll
+          for (int e = 0; e < GC_BATCH; ++e) S[(j + e * ng) * rmax + rl] = a[e] - l * b[e];
+        }
+        for (; j < kb; j += ng) S[j * rmax + rl] = (sw ? old[j] : S[j * rmax + rl]) - l * u[j];
+      }
+    lu_best<T>(mk, mr);
+    if (lane == 0) { s_key[warp] = mk; s_row[warp] = mr; }
+    __syncthreads();
+    // the multipliers, once every group has read column k
+    if (tg == 0)
+      for (int rl = max(rbeg, gk + 1) - rbeg + tr; rl < nr_my; rl += rw) {
+        T* e = &S[k * rmax + rl];
+        *e = (rbeg + rl == p ? old[k] : *e) * rinv;
+      }
     __syncthreads();
   }
-  for (int idx = threadIdx.x; idx < nr_my * kb; idx += GC_THREADS) {
-    const int r = idx % nr_my, j = idx / nr_my;
-    G[(rbeg + r) + (int64_t)(k0 + j) * n] = S[j * rmax + r];
-  }
+  if (tg < ng)
+    for (int j = tg; j < kb; j += ng)
+      for (int r = tr; r < nr_my; r += rw) G[(rbeg + r) + (int64_t)(k0 + j) * n] = S[j * rmax + r];
 }
 
-void launch_getrf_coop(const DevCtx& c, const Item* items, int n_items, int n_ctas, int dtype, int nb, int pivot,
-                       int rmax, double* xbuf, unsigned int* ctr, int* err, cudaStream_t s) {
-  if (!n_items) return;
-  if (nb > 64) throw std::invalid_argument("getrf_coop: panel wider than 64");
-  cudaMemsetAsync(ctr, 0, 2 * sizeof(unsigned int), s);
-  const size_t smem = (size_t)rmax * nb * (dtype == F64 ? sizeof(double) : sizeof(float));
+constexpr int GC_NT_CLUSTER = 512, GC_NT_GRID = 256;
+
+template <typename T, bool CL>
+static cudaError_t getrf_smem_t(const DevCtx& c, const Item* items, int n_items, int n_ctas, int csize, int nb,
+                                int pivot, int rmax, uint64_t* xbuf, int* err, cudaStream_t s) {
+  constexpr int NT = CL ? GC_NT_CLUSTER : GC_NT_GRID;
+  const size_t smem = (size_t)rmax * nb * sizeof(T);
+  cudaFuncSetAttribute(k_getrf_smem<T, CL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(n_ctas);
-  cfg.blockDim = dim3(GC_THREADS);
+  cfg.blockDim = dim3(NT);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e;
-  if (dtype == F64) {
-    cudaFuncSetAttribute(k_getrf_coop<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    e = cudaLaunchKernelEx(&cfg, k_getrf_coop<double>, c, items, n_items, nb, pivot, rmax, xbuf, ctr, err);
+  if (CL) {
+    if (csize > 8) cudaFuncSetAttribute(k_getrf_smem<T, CL, NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = csize;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
   } else {
-    cudaFuncSetAttribute(k_getrf_coop<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    e = cudaLaunchKernelEx(&cfg, k_getrf_coop<float>, c, items, n_items, nb, pivot, rmax, xbuf, ctr, err);
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = CL && csize == 1 ? 0 : 1;
+  return cudaLaunchKernelEx(&cfg, k_getrf_smem<T, CL, NT>, c, items, n_items, nb, pivot, rmax, csize, xbuf, err);
+}
+
+void launch_getrf_smem(const DevCtx& c, const Item* items, int n_items, int n_ctas, int csize, int dtype, int nb,
+                       int pivot, int rmax, uint64_t* xbuf, int* err, cudaStream_t s) {
+  if (!n_items) return;
+  if (nb > 64) throw std::invalid_argument("getrf_smem: panel wider than 64");
+  if (csize > GC_CLUSTER) throw std::invalid_argument("getrf_smem: cluster too large");
+  cudaError_t e;
+  if (csize > 0) {
+    e = dtype == F64 ? getrf_smem_t<double, true>(c, items, n_items, n_items * csize, csize, nb, pivot, rmax, nullptr, err, s)
+                     : getrf_smem_t<float, true>(c, items, n_items, n_items * csize, csize, nb, pivot, rmax, nullptr, err, s);
+  } else {
+    if (n_ctas > GC_MAX_CTAS) throw std::invalid_argument("getrf_smem: too many CTAs");
+    cudaMemsetAsync(xbuf, 0, sizeof(uint64_t) * (size_t)gc_words(n_ctas, n_items), s);
+    e = dtype == F64 ? getrf_smem_t<double, false>(c, items, n_items, n_ctas, 0, nb, pivot, rmax, xbuf, err, s)
+                     : getrf_smem_t<float, false>(c, items, n_items, n_ctas, 0, nb, pivot, rmax, xbuf, err, s);
   }
   if (e != cudaSuccess)
-    throw std::runtime_error(std::string("cooperative LU panel launch failed: ") + cudaGetErrorString(e));
+    throw std::runtime_error(std::string("LU panel launch failed: ") + cudaGetErrorString(e));
 }
 
 // Row interchanges of a panel (pivots of rows k0..k0+kb-1, kb = min(nb,
