@@ -31,7 +31,7 @@ def _matrix(n, symmetric, rng):
     return a
 
 
-def _mesh(fs, ss, symmetric, seed):
+def _mesh(fs, ss, symmetric, seed, n_rhs=1):
     rng = np.random.default_rng(seed)
     m = api.Mesh()
     nodes = [m.add_node(0, fs), m.add_node(1, fs), m.add_node(2, ss)]
@@ -43,9 +43,9 @@ def _mesh(fs, ss, symmetric, seed):
         m.set_parent(e, root)
         m.add_child(root, e)
     m.lock()
-    m.create_matrix_without_buffer(api.UHM_REAL, 1)
+    m.create_matrix_without_buffer(api.UHM_REAL, n_rhs)
     mats = [_matrix(fs + ss, symmetric, rng) for _ in leaves]
-    rhs = [rng.standard_normal((fs + ss, 1)) for _ in leaves]
+    rhs = [rng.standard_normal((fs + ss, n_rhs)) for _ in leaves]
     for k, e in enumerate(leaves):
         m.copy_in(e, [k, 2], api.UHM_LHS, mats[k])
         m.copy_in(e, [k, 2], api.UHM_RHS, rhs[k])
@@ -68,15 +68,18 @@ def _check(method, prec, fs, ss, seed):
         d = np.abs(np.diag(a)[fs:])
         assert (np.abs(got - exact) <= tol * np.sqrt(np.outer(d, d))).all(), (k, np.abs(got - exact).max())
     m.solve(method)
-    n = 2 * fs + ss
-    full, b = np.zeros((n, n)), np.zeros(n)
+    x, ref = _solutions(m, fs, ss, mats, rhs)
+    assert np.abs(x - ref).max() <= 3e-10 * np.abs(ref).max()   # 1e-12 times the condition number
+
+
+def _solutions(m, fs, ss, mats, rhs):
+    n, nr = 2 * fs + ss, rhs[0].shape[1]
+    full, b = np.zeros((n, n)), np.zeros((n, nr))
     for k in range(2):
         i = np.concatenate([np.arange(fs) + k * fs, np.arange(2 * fs, n)])
         full[np.ix_(i, i)] += mats[k]
-        b[i] += rhs[k][:, 0]
-    x = m.node_solution(np.arange(3, dtype=np.int32), np.array([fs, fs, ss]))[:, 0]
-    ref = np.linalg.solve(full, b)
-    assert np.abs(x - ref).max() <= 3e-10 * np.abs(ref).max()   # 1e-12 times the condition number
+        b[i] += rhs[k]
+    return m.node_solution(np.arange(3, dtype=np.int32), np.array([fs, fs, ss]), nr), np.linalg.solve(full, b)
 
 
 # (fs, ss): one step; a step and one column; the outer panel's edge; one column past
@@ -88,6 +91,19 @@ SIZES = [(64, 165), (65, 200), (256, 1), (257, 128), (300, 129), (449, 255), (1,
 @pytest.mark.parametrize("method,prec", [(uo.LU_PIV, "fp64"), (uo.LU_NOPIV, "fp32")])
 def test_lu_front(native_lib, method, prec, fs, ss):
     _check(method, prec, fs, ss, 100 + fs)
+
+
+@pytest.mark.parametrize("n_rhs", [2, 3, 5, 16])
+@pytest.mark.parametrize("method", [uo.LU_PIV, uo.LU_NOPIV])
+def test_lu_right_hand_sides(native_lib, method, n_rhs):
+    """Groups of four, two and one right-hand sides through the flag-driven LU
+    solves of blocked fronts (a ragged last block); tolerance 3 n u times a
+    condition number of 40."""
+    m, leaves, mats, rhs = _mesh(300, 129, False, 31, n_rhs)
+    m.factor(method)
+    m.solve(method)
+    x, ref = _solutions(m, 300, 129, mats, rhs)
+    assert np.abs(x - ref).max() <= 3 * 729 * U["fp64"] * 40 * np.abs(ref).max()
 
 
 @pytest.mark.parametrize("fs,ss", SIZES)

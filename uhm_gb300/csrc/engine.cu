@@ -22,8 +22,6 @@ static constexpr int ASM_TJ = 16;           // assembly column tile (k_factor.cu
 static constexpr int ASM_SCATTER_MIN = 2048;  // fronts this large: one column per CTA, shared-memory scatter
 static constexpr int ASM_SCATTER_MAX = 26624; // the FP64 column fits 208 KB of shared memory
 static constexpr int TRSM_RB = 64;
-static constexpr int FWD_RB = 256;            // k_solve.cu
-static constexpr int BWD_RB = 512;
 static constexpr int LUROW_CB = 16;         // k_lu_row_update (k_factor.cu)
 // LU panels (k_getrf_smem): clusters grow until a CTA holds at most this many rows
 static constexpr int LU_GOAL_F64 = 64, LU_GOAL_F32 = 192;
@@ -90,7 +88,7 @@ void Engine::free_device() {
   dev_ok = false;
   ctx = DevCtx{};
   d_items = nullptr;
-  d_b = d_x = d_r = d_d = d_erhs = d_y = d_red = d_scratch = nullptr;
+  d_b = d_x = d_r = d_d = d_erhs = d_y = d_red = nullptr;
   d_sel = nullptr;
   d_ws = nullptr;
   d_ws_off = d_ws_stride = nullptr;
@@ -679,7 +677,7 @@ void Engine::build_plan(int method) {
     f.piv_off = piv_n;
     piv_n += f.fs;
   }
-  // large Cholesky fronts: inverses of their 64 x 64 diagonal blocks and one
+  // large fronts: inverses of their 64 x 64 diagonal blocks and one
   // completion flag per block for the flag-driven solves
   dinv64_n = dinv32_n = flags_n = 0;
   {
@@ -690,11 +688,11 @@ void Engine::build_plan(int method) {
       f.xs = f.blocked && !f.tc;
       f.flag_off = (int)flags_n;
       f.dinv_off = 0;
-      if (!f.blocked || method != UHM_CHOL) continue;
+      if (!f.blocked) continue;
       const int nfb = (f.fs + NB - 1) / NB;
       int64_t& dn = dt == F64 ? dinv64_n : dinv32_n;
       f.dinv_off = dn;
-      dn += (int64_t)nfb * NB * NB;
+      dn += (method == UHM_CHOL ? 1 : 2) * (int64_t)nfb * NB * NB;   // LU: of L's blocks, then of U's
       flags_n += nfb;
     }
   }
@@ -981,7 +979,8 @@ void Engine::build_programs(int method) {
       }
       if (!piv) continue;
       const int ce = col_end(it), lim = ce > 0 ? ce : fronts[it.front].n;
-      for (int c0 = 0; !own_swaps && c0 < lim; c0 += 256) sw.push_back(Item{it.front, it.a, c0, ce});
+      if (own_swaps) sw.push_back(Item{it.front, it.a, -1, 0});      // the permutation only
+      else for (int c0 = 0; c0 < lim; c0 += 256) sw.push_back(Item{it.front, it.a, c0, ce});
     }
     double fl = fp;                  // the panel's operations, on its first launch
     push(fac_ops, OP_GETRF, dt, NB, piv, glob, glob.empty() ? 0.0 : fl);
@@ -1350,6 +1349,13 @@ void Engine::build_programs(int method) {
         push(fac_ops, OP_TC_PACK, dt, NBO, parts, pk);
         push(fac_ops, OP_TC_SYRK, dt, NBO, parts, tt, ftc, btc);
       }
+      if (!chol) {
+        std::vector<Item> di;
+        for (int s : fl)
+          if (fronts[s].blocked)
+            for (int b = 0; b * NB < fronts[s].fs; ++b) di.push_back(Item{s, b, 0, 0});
+        push(fac_ops, OP_LU_DINV, dt, NB, 0, di);
+      }
       // BF16X3 Cholesky fronts (k_chol_tc.cu): per outer panel of W1 columns
       // one cooperative panel launch (factor, TRSM, in-panel updates, BF16
       // parts) and one tensor-core launch over the factor block's trailing
@@ -1556,12 +1562,12 @@ void Engine::build_programs(int method) {
   for (auto& lv : levels) {
     std::vector<Item> g_items;
     for (int s : lv) {
-      if (gm == M_LU_PIV) {
-        g_items.push_back(Item{s, 0, 0, 0});
+      // c = 1: the front takes the flag-driven (or chain) solves, whose
+      // forward hand-off words the gather empties
+      const int hand = nr <= NR_FLAGS_MAX && !solve_small(fronts[s], h_fronts[s].dtype);
+      if (gm == M_LU_PIV && !hand) {
+        g_items.push_back(Item{s, 0, 0, 0});        // applies the pivots: the whole front
       } else {
-        // c = 1: the front takes the flag-driven (or chain) solves, whose
-        // forward hand-off words the gather empties
-        const int hand = chol && nr <= NR_FLAGS_MAX && !solve_small(fronts[s], h_fronts[s].dtype);
         for (int r0 = 0; r0 < fronts[s].n; r0 += GATHER_ROWS) g_items.push_back(Item{s, r0, GATHER_ROWS, hand});
       }
     }
@@ -1602,11 +1608,11 @@ void Engine::build_programs(int method) {
         }
         large.clear();
       }
-      if (chol && nr <= NR_FLAGS_MAX && !large.empty()) {
+      if (nr <= NR_FLAGS_MAX && !large.empty()) {
         // one flag-driven launch for every large front of this level (per
         // group of FLAG_NR right-hand sides)
         std::vector<Item> fi, ai;
-        const int RB = tune.solve_rows;     // rows per CTA: 64 (k_fwd_flags) or 256 (k_fwd_flags4)
+        const int RB = chol ? tune.solve_rows : 64;     // rows per CTA: 64 (k_fwd_flags) or 256 (k_fwd_flags4)
         const int per = RB / NB;
         int maxb = 0;
         for (int s : large) maxb = std::max(maxb, ((fronts[s].fs + NB - 1) / NB + per - 1) / per);
@@ -1631,20 +1637,6 @@ void Engine::build_programs(int method) {
           op.aux = RB;
           fwd_ops.push_back(op);
         }
-        large.clear();
-      }
-      int maxfs = 0;
-      for (int s : large) maxfs = std::max(maxfs, fronts[s].fs);
-      for (int k0 = 0; k0 < maxfs; k0 += NB) {
-        std::vector<Item> fv;
-        for (int s : large) {
-          const HostFront& f = fronts[s];
-          if (f.fs <= k0) continue;
-          const int kb = std::min(NB, f.fs - k0);
-          const int nch = std::max(1, (f.n - k0 - kb + FWD_RB - 1) / FWD_RB);
-          for (int ch = 0; ch < nch; ++ch) fv.push_back(Item{s, k0, ch, 0});
-        }
-        push(fwd_ops, OP_TRSV_F, dt, NB, gm, fv);
       }
     }
   }
@@ -1687,7 +1679,7 @@ void Engine::build_programs(int method) {
         }
         large.clear();
       }
-      if (chol && nr <= NR_FLAGS_MAX && !large.empty()) {
+      if (nr <= NR_FLAGS_MAX && !large.empty()) {
         std::vector<Item> bi;
         const int per = 1;                       // 64-column blocks per CTA
         int maxb = 0;
@@ -1701,28 +1693,13 @@ void Engine::build_programs(int method) {
           f1 = std::max(f1, fronts[s].flag_off + (fronts[s].fs + NB - 1) / NB);
         }
         const int64_t io = add_items(bi);
-        const int qstep = per > 1 ? FLAG_NR : (dt == F64 ? FLAG_NR_BWD_F64 : FLAG_NR);
+        const int qstep = chol && dt == F64 ? FLAG_NR_BWD_F64 : FLAG_NR;
         for (int q0 = 0; q0 < nr; q0 += qstep) {
           Op op{OP_BWD_FLAGS, dt, f1 - f0, f0, io, (int)bi.size()};
           op.q0 = q0;
           op.aux = NB;
           bwd_ops.push_back(op);
         }
-        large.clear();
-      }
-      int maxfs = 0;
-      for (int s : large) maxfs = std::max(maxfs, fronts[s].fs);
-      int last = maxfs == 0 ? -1 : ((maxfs - 1) / NB) * NB;
-      for (int k0 = last; k0 >= 0; k0 -= NB) {
-        std::vector<Item> bv;
-        for (int s : large) {
-          const HostFront& f = fronts[s];
-          if (f.fs <= k0) continue;
-          const int kb = std::min(NB, f.fs - k0);
-          const int nch = (f.n - k0 - kb + BWD_RB - 1) / BWD_RB;
-          for (int ch = 0; ch < std::max(1, nch); ++ch) bv.push_back(Item{s, k0, ch, nch});
-        }
-        push(bwd_ops, OP_TRSV_B, dt, NB, gm, bv);
       }
       push(bwd_ops, OP_BWD_STORE, dt, 0, gm, st);
     }
@@ -1762,6 +1739,7 @@ void Engine::alloc_device(int method) {
   ctx.colsrc = (int2*)dmalloc(sizeof(int2) * std::max<size_t>(1, h_colsrc.size()));
   ctx.sgi = (int32_t*)dmalloc(sizeof(int32_t) * std::max<size_t>(1, h_sgi.size()));
   ctx.piv = (int32_t*)dmalloc(sizeof(int32_t) * std::max<int64_t>(1, piv_n));
+  ctx.perm = (int32_t*)dmalloc(sizeof(int32_t) * std::max<int64_t>(1, method == UHM_LU_PIV ? piv_n : 0));
   ctx.a64 = (double*)dmalloc(sizeof(double) * std::max<int64_t>(1, arena64_n));
   ctx.a32 = (float*)dmalloc(sizeof(float) * std::max<int64_t>(1, arena32_n));
   ctx.emat = (double*)dmalloc(sizeof(double) * std::max<int64_t>(1, emat_total));
@@ -1846,19 +1824,6 @@ void Engine::alloc_device(int method) {
     CK(cudaMemcpyAsync(d_ws_off, wo.data(), sizeof(int64_t) * wo.size(), cudaMemcpyHostToDevice, stream));
     CK(cudaMemcpyAsync(d_ws_stride, wst.data(), sizeof(int64_t) * wst.size(), cudaMemcpyHostToDevice, stream));
     CK(cudaStreamSynchronize(stream));
-  }
-  {
-    std::vector<int64_t> so(fronts.size());
-    int64_t tot = 0;
-    for (auto& f : fronts) {
-      so[f.slot] = tot;
-      tot += (int64_t)((f.n + BWD_RB - 1) / BWD_RB + 1) * nr * NB;
-    }
-    d_scratch = (double*)dmalloc(sizeof(double) * std::max<int64_t>(1, tot));
-    d_scr_off = (int64_t*)dmalloc(sizeof(int64_t) * so.size());
-    d_counters = (int*)dmalloc(sizeof(int) * fronts.size());
-    CK(cudaMemcpyAsync(d_scr_off, so.data(), sizeof(int64_t) * so.size(), cudaMemcpyHostToDevice, stream));
-    CK(cudaMemsetAsync(d_counters, 0, sizeof(int) * fronts.size(), stream));
   }
   const size_t gv = sizeof(double) * (size_t)std::max<int64_t>(1, n_global) * nr;
   d_b = (double*)dmalloc(gv);
@@ -2059,7 +2024,12 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
         break;
       case OP_FWD_CHAIN: launch_fwd_chain(ctx, it, op.n_items, d_ticket, d_err, op.q0, st); break;
       case OP_BWD_CHAIN: launch_bwd_chain(ctx, it, op.n_items, d_ticket, d_err, op.q0, st); break;
+      case OP_LU_DINV: launch_lu_dinv(ctx, it, op.n_items, op.dtype, st); break;
       case OP_BWD_FLAGS:
+        if (!ctx.symmetric) {
+          launch_lu_bwd_flags(ctx, it, op.n_items, op.dtype, d_ticket, d_err, op.q0, st);
+          break;
+        }
         launch_bwd_flags(ctx, it, op.n_items, op.dtype, d_ticket, ctx.flags + op.param, op.nb, d_err, op.q0,
                            st);
         break;
@@ -2109,13 +2079,9 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
         break;
       case OP_FWD_GATHER: launch_fwd_gather(ctx, it, op.n_items, g_in, n_global, op.param, st); break;
       case OP_FWD_SMALL: launch_fwd_small(ctx, it, op.n_items, op.dtype, op.param, op.nb, st); break;
-      case OP_TRSV_F: launch_fwd_step(ctx, it, op.n_items, op.dtype, op.param, st); break;
       case OP_BWD_PREP: launch_bwd_prepare(ctx, it, op.n_items, 0, op.param, g_out, n_global, st); break;
       case OP_BWD_SMALL:
         launch_bwd_small(ctx, it, op.n_items, op.dtype, op.param, g_out, n_global, op.nb, st);
-        break;
-      case OP_TRSV_B:
-        launch_bwd_step(ctx, it, op.n_items, op.dtype, op.param, d_scratch, d_scr_off, d_counters, st);
         break;
       case OP_BWD_STORE: launch_bwd_store(ctx, it, op.n_items, g_out, n_global, st); break;
     }

@@ -86,7 +86,7 @@ enum OpKind : int {
   OP_TRSV_B, OP_BWD_STORE, OP_TC_PACK, OP_TC_SYRK, OP_FWD_FLAGS, OP_BWD_FLAGS, OP_GETRF_COOP,
   OP_LASWP, OP_POTRF_TRSM, OP_ASSEMBLE_SCATTER, OP_TC_GEMM, OP_CHOL_PANEL, OP_TC_CHOL_TRAIL,
   OP_TC_CHOL_SCHUR, OP_CLEAR_FLAGS, OP_CHOL_DIAG, OP_CHOL_PACK, OP_TC_CHOL_TRSM, OP_EV_RECORD, OP_EV_WAIT,
-  OP_FWD_CHAIN, OP_BWD_CHAIN, OP_XS_PACK, OP_XS_UPDATE, OP_KIND_END
+  OP_FWD_CHAIN, OP_BWD_CHAIN, OP_XS_PACK, OP_XS_UPDATE, OP_LU_DINV, OP_KIND_END
 };
 static_assert(OP_KIND_END <= N_OP_KINDS, "profile arrays hold N_OP_KINDS op kinds");
 
@@ -291,10 +291,7 @@ class Engine {
   double* d_erhs = nullptr;     // element rhs (FP64)
   double* d_y = nullptr;        // per-element A_e x_e
   double* d_red = nullptr;      // reduction scratch
-  double* d_scratch = nullptr;  // backward-solve partial sums
   float* d_sel = nullptr;       // selector scratch: element statistics, features, parameters, probabilities
-  int64_t* d_scr_off = nullptr;
-  int* d_counters = nullptr;
   void* d_ws2 = nullptr;             // chunk-major BF16 parts of the cooperative-panel fronts
   int64_t ws2_rows = 0;              // its size in rows of 64 BF16
   int64_t* d_ws2_row0 = nullptr;     // per front: first row of its parts

@@ -1420,18 +1420,39 @@ void launch_getrf_smem(const DevCtx& c, const Item* items, int n_items, int n_ct
 // Row interchanges of a panel (pivots of rows k0..k0+kb-1, kb = min(nb,
 // fs - k0), applied in order) on the front's columns outside the panel and
 // below a column limit.  Item: front, a = k0, b = first column of a
-// 256-column chunk, c = column limit (0: n); one thread per column.
+// 256-column chunk, c = column limit (0: n); one thread per column.  The
+// last warp of chunk 0 (of b = -1: no columns) applies them to the front's
+// row permutation, which the solves gather by.
+constexpr int LASWP_THREADS = 256 + 32;
+
 template <typename T>
-__global__ void __launch_bounds__(256) k_laswp(DevCtx c, const Item* __restrict__ items, int nb) {
+__global__ void __launch_bounds__(LASWP_THREADS) k_laswp(DevCtx c, const Item* __restrict__ items, int nb) {
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, k0 = it.a;
   const int kb = min(nb, f.fs - k0);
+  const int32_t* __restrict__ pv = c.piv + f.piv_off;
+  if (threadIdx.x >= 256) {
+    if (it.b > 0) return;
+    int32_t* __restrict__ perm = c.perm + f.piv_off;
+    if (k0 == 0)
+      for (int i = threadIdx.x - 256; i < f.fs; i += 32) perm[i] = i;
+    __syncwarp();
+    if (threadIdx.x == 256)
+      for (int k = k0; k < k0 + kb; ++k) {
+        const int p = pv[k];
+        if (p != k) {
+          const int32_t t = perm[k];
+          perm[k] = perm[p];
+          perm[p] = t;
+        }
+      }
+    return;
+  }
   const int j = it.b + threadIdx.x;
   const int jend = it.c > 0 ? min(it.c, n) : n;
-  if (j >= jend || (j >= k0 && j < k0 + kb)) return;
+  if (it.b < 0 || j >= jend || (j >= k0 && j < k0 + kb)) return;
   T* __restrict__ col = arena<T>(c) + f.off + (int64_t)j * n;
-  const int32_t* __restrict__ pv = c.piv + f.piv_off;
   for (int k = k0; k < k0 + kb; ++k) {
     const int p = pv[k];
     if (p != k) {
@@ -1444,8 +1465,8 @@ __global__ void __launch_bounds__(256) k_laswp(DevCtx c, const Item* __restrict_
 
 void launch_laswp(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, cudaStream_t s) {
   if (!n_items) return;
-  if (dtype == F64) k_laswp<double><<<n_items, 256, 0, s>>>(c, items, nb);
-  else k_laswp<float><<<n_items, 256, 0, s>>>(c, items, nb);
+  if (dtype == F64) k_laswp<double><<<n_items, LASWP_THREADS, 0, s>>>(c, items, nb);
+  else k_laswp<float><<<n_items, LASWP_THREADS, 0, s>>>(c, items, nb);
 }
 
 constexpr int LUROW_CB = 16;   // columns per row-panel block
@@ -1509,6 +1530,65 @@ void launch_lu_row_update(const DevCtx& c, const Item* items, int n_items, int d
   if (nb != 64) throw std::invalid_argument("lu_row_update: panels are 64 columns wide");
   if (dtype == F64) k_lu_row_update<double><<<n_items, 4 * LUROW_CB, 0, s>>>(c, items, nb);
   else k_lu_row_update<float><<<n_items, 4 * LUROW_CB, 0, s>>>(c, items, nb);
+}
+
+// Inverses of a large LU front's diagonal blocks, for the flag-driven solves:
+// L_bb (unit lower) and U_bb, 64 x 64, zero outside their triangles and past
+// the block's kb rows.  Item: front, a = b.  Substitution in registers as in
+// k_lu_row_update, four lanes per column of the identity; U through its
+// transpose, (U^T)^{-1} by rows being U^{-1} by columns.  One launch per level
+// after its fronts are factored: every block of every front at once.
+template <typename T>
+__global__ void __launch_bounds__(256) k_lu_dinv(DevCtx c, const Item* __restrict__ items) {
+  __shared__ __align__(16) T L[64 * 4 * LUROW_LQ];   // L[(4 k + q) LUROW_LQ + u] = M[q + 4 u][k]
+  __shared__ T rd[64];
+  const Item it = items[blockIdx.x];
+  const FrontDev f = c.fronts[it.front];
+  const int n = f.n, fs = f.fs, k0 = 64 * it.a;
+  const int kb = min(64, fs - k0), nfb = (fs + 63) / 64;
+  const T* __restrict__ G = arena<T>(c) + f.off + k0 + (int64_t)k0 * n;
+  T* __restrict__ D = (sizeof(T) == 8 ? (T*)c.dinv64 : (T*)c.dinv32) + f.dinv_off + (int64_t)it.a * 4096;
+  const int q = threadIdx.x & 3, col = threadIdx.x >> 2;
+#pragma unroll 1
+  for (int upper = 0; upper < 2; ++upper) {
+    for (int e = threadIdx.x; e < 4096; e += 256) {
+      const int i = e & 63, k = e >> 6;              // entry (i, k) of the block, column k
+      const T v = i < kb && k < kb ? G[i + (int64_t)k * n] : (i == k ? T(1) : T(0));
+      if (!upper) L[(4 * k + (i & 3)) * LUROW_LQ + (i >> 2)] = i > k ? v : T(0);
+      else L[(4 * i + (k & 3)) * LUROW_LQ + (k >> 2)] = k > i ? v : T(0);   // U^T: entry (k, i)
+      if (i == k) rd[i] = upper ? v : T(1);
+    }
+    __syncthreads();
+    T x[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) x[u] = q + 4 * u == col ? T(1) : T(0);
+#pragma unroll
+    for (int b = 0; b < 16; ++b) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        if (upper && q == r) x[b] /= rd[4 * b + r];
+        const T xk = __shfl_sync(0xffffffffu, x[b], r, 4);
+        const T* __restrict__ l = L + (4 * (4 * b + r) + q) * LUROW_LQ;
+        if (q > r) x[b] -= l[b] * xk;
+#pragma unroll
+        for (int u = b + 1; u < 16; ++u) x[u] -= l[u] * xk;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int i = q + 4 * u;                       // entry (i, col) of M^{-1}
+      const T v = i < kb && col < kb && i >= col ? x[u] : T(0);
+      if (!upper) D[col * 64 + i] = v;
+      else D[(int64_t)nfb * 4096 + i * 64 + col] = v;
+    }
+    __syncthreads();
+  }
+}
+
+void launch_lu_dinv(const DevCtx& c, const Item* items, int n_items, int dtype, cudaStream_t s) {
+  if (!n_items) return;
+  if (dtype == F64) k_lu_dinv<double><<<n_items, 256, 0, s>>>(c, items);
+  else k_lu_dinv<float><<<n_items, 256, 0, s>>>(c, items);
 }
 
 // ---------------------------------------------------------------------------

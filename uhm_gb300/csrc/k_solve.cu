@@ -24,7 +24,8 @@ constexpr unsigned long long HAND_EMPTY = 0x7FF4DEAD7FF4DEADull;
 
 // z = [g[g0 .. g0+fs); 0] + sum over children of their xb (extend-add);
 // item: front, a = first row, b = rows (0: all), c = 1 for a front of the
-// 64-row flag-driven solves
+// 64-row flag-driven solves (LU with pivoting: its factor rows are gathered in
+// the order of the front's row permutation)
 __global__ void __launch_bounds__(256) k_fwd_gather(DevCtx c, const Item* __restrict__ items,
                                                     const double* __restrict__ g, int64_t ldg,
                                                     int method) {
@@ -38,6 +39,7 @@ __global__ void __launch_bounds__(256) k_fwd_gather(DevCtx c, const Item* __rest
   // rows [it.a, it.a + it.b) of the front (it.b == 0: all rows; only then
   // are pivots applied, which needs the whole gathered vector)
   const int I0 = it.a, I1 = it.b > 0 ? min(n, it.a + it.b) : n;
+  const int32_t* __restrict__ perm = method == M_LU_PIV && it.c ? c.perm + f.piv_off : nullptr;
   // the sources decoded once per CTA (in source order): a child's updated
   // bottom block and its leading dimension, null for an element source
   constexpr int GMAXSRC = 64;
@@ -57,7 +59,8 @@ __global__ void __launch_bounds__(256) k_fwd_gather(DevCtx c, const Item* __rest
   }
   __syncthreads();
   for (int q = 0; q < c.n_rhs; ++q) {
-    for (int I = I0 + threadIdx.x; I < I1; I += blockDim.x) {
+    for (int R = I0 + threadIdx.x; R < I1; R += blockDim.x) {
+      const int I = perm && R < f.fs ? perm[R] : R;
       double acc = I < f.fs ? g[(f.g0 + I) + q * ldg] : 0.0;
       for (int s = 0; s < ns; ++s) {
         const double* xb = s_xb[s];
@@ -74,13 +77,13 @@ __global__ void __launch_bounds__(256) k_fwd_gather(DevCtx c, const Item* __rest
           acc += c.vec[ch.voff + ch.fs + is + (int64_t)q * ch.n];
         }
       }
-      z[I + (int64_t)q * n] = acc;
+      z[R + (int64_t)q * n] = acc;
       // fronts of the 64-row flag-driven and chain solves: their y factor
       // rows (solutions) and w factor rows (partial sums) are forward
       // hand-offs, emptied here (the forward launch comes after)
-      if (it.c && I < f.fs) {
-        y[I + (int64_t)q * n] = __longlong_as_double((long long)HAND_EMPTY);
-        w[I + (int64_t)q * n] = __longlong_as_double((long long)HAND_EMPTY);
+      if (it.c && R < f.fs) {
+        y[R + (int64_t)q * n] = __longlong_as_double((long long)HAND_EMPTY);
+        w[R + (int64_t)q * n] = __longlong_as_double((long long)HAND_EMPTY);
       }
     }
   }
@@ -356,197 +359,6 @@ void launch_bwd_small(const DevCtx& c, const Item* items, int n_items, int dtype
     cudaFuncSetAttribute(k_bwd_small<float, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     k_bwd_small<float, 256><<<n_items, 256, sm, s>>>(c, items, method, g, ldg);
   }
-}
-
-// ---------------------------------------------------------------------------
-// Large fronts, blocked by SB = 64 columns.
-// Forward step k (item: front, a = k0, b = row chunk): every CTA solves the
-// diagonal block x_k = L_kk^{-1} z_k (warp-synchronous substitution, unit
-// diagonal for LU), chunk 0 stores x_k in the y slab, and each CTA updates
-// its chunk of rows below:  z[r] -= L[r, k-block] x_k.  Step k reads only
-// z_k and writes only rows >= k0+kb and y_k, so CTAs never race.
-// Backward step k (item: front, a = k0, b = chunk, c = number of chunks):
-// each CTA forms partial dot products of its tail chunk (Chol: L^T, LU: U)
-// with y; the last CTA to arrive (threadfence reduction) sums the partials in
-// chunk order -- deterministic -- and solves the diagonal block into y_k.
-// ---------------------------------------------------------------------------
-constexpr int SB = 64;          // diagonal block of the blocked solves
-constexpr int FWD_RB = 256;     // rows per forward-update CTA
-constexpr int BWD_RB = 512;     // tail rows per backward partial CTA
-constexpr int NR_MAX = 16;      // right-hand sides of large fronts
-
-// lower-triangular substitution of one diagonal block by one warp;
-// x (shared, length kb) in, solution out
-template <typename T, typename CT>
-__device__ __forceinline__ void warp_lower_solve(const T* D, int kb, CT* x, bool unit) {
-  const int lane = threadIdx.x & 31;
-  CT v0 = lane < kb ? x[lane] : CT(0), v1 = lane + 32 < kb ? x[lane + 32] : CT(0);
-  for (int j = 0; j < kb; ++j) {
-    CT xj = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, j & 31);
-    if (!unit) xj /= (CT)D[j + j * SB];
-    if (lane == (j & 31)) { if (j < 32) v0 = xj; else v1 = xj; }
-    if (lane > j && lane < kb) v0 -= (CT)D[lane + j * SB] * xj;
-    if (lane + 32 > j && lane + 32 < kb) v1 -= (CT)D[lane + 32 + j * SB] * xj;
-  }
-  if (lane < kb) x[lane] = v0;
-  if (lane + 32 < kb) x[lane + 32] = v1;
-}
-
-// upper substitution: Chol uses L_kk^T (A(i,j) = D[j,i]), LU uses U_kk
-template <typename T, typename CT>
-__device__ __forceinline__ void warp_upper_solve(const T* D, int kb, CT* x, bool chol) {
-  const int lane = threadIdx.x & 31;
-  CT v0 = lane < kb ? x[lane] : CT(0), v1 = lane + 32 < kb ? x[lane + 32] : CT(0);
-  for (int j = kb - 1; j >= 0; --j) {
-    CT xj = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, j & 31);
-    xj /= (CT)D[j + j * SB];
-    if (lane == (j & 31)) { if (j < 32) v0 = xj; else v1 = xj; }
-    if (lane < j) v0 -= (CT)(chol ? D[j + lane * SB] : D[lane + j * SB]) * xj;
-    if (lane + 32 < j) v1 -= (CT)(chol ? D[j + (lane + 32) * SB] : D[lane + 32 + j * SB]) * xj;
-  }
-  if (lane < kb) x[lane] = v0;
-  if (lane + 32 < kb) x[lane + 32] = v1;
-}
-
-template <typename T, int NT>
-__global__ void __launch_bounds__(NT) k_fwd_step(DevCtx c, const Item* __restrict__ items, int method) {
-  using CT = T;   // compute in the storage precision of the factor
-  __shared__ T D[SB * SB];
-  __shared__ CT xk[SB * NR_MAX];
-  const Item it = items[blockIdx.x];
-  const FrontDev f = c.fronts[it.front];
-  const int n = f.n, k0 = it.a, nr = c.n_rhs;
-  const int kb = min(SB, f.fs - k0);
-  const T* __restrict__ G = arena<T>(c) + f.off;
-  double* __restrict__ z = c.vec + f.voff;
-  double* __restrict__ y = z + (int64_t)n * nr;
-  for (int idx = threadIdx.x; idx < SB * kb; idx += NT) {
-    const int i = idx % SB, j = idx / SB;
-    D[idx] = i < kb ? G[(k0 + i) + (int64_t)(k0 + j) * n] : T(0);
-  }
-  for (int idx = threadIdx.x; idx < kb * nr; idx += NT) {
-    const int i = idx % kb, q = idx / kb;
-    xk[i + q * SB] = (CT)z[(k0 + i) + (int64_t)q * n];
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5;
-  for (int q = warp; q < nr; q += NT / 32) warp_lower_solve<T, CT>(D, kb, xk + q * SB, method != M_CHOL);
-  __syncthreads();
-  if (it.b == 0)
-    for (int idx = threadIdx.x; idx < kb * nr; idx += NT) {
-      const int i = idx % kb, q = idx / kb;
-      y[(k0 + i) + (int64_t)q * n] = (double)xk[i + q * SB];
-    }
-  const int r0 = k0 + kb + it.b * FWD_RB;
-  const int r1 = min(r0 + FWD_RB, n);
-  for (int r = r0 + threadIdx.x; r < r1; r += NT) {
-    for (int q = 0; q < nr; ++q) {
-      CT acc = CT(0);
-      for (int t = 0; t < kb; ++t) acc += (CT)G[r + (int64_t)(k0 + t) * n] * xk[t + q * SB];
-      z[r + (int64_t)q * n] -= (double)acc;
-    }
-  }
-}
-
-template <typename T, int NT>
-__global__ void __launch_bounds__(NT) k_bwd_step(DevCtx c, const Item* __restrict__ items, int method,
-                                                 double* __restrict__ scratch,
-                                                 const int64_t* __restrict__ scr_off,
-                                                 int* __restrict__ counters) {
-  using CT = T;
-  // the diagonal block (last CTA) and the partial-sum tile (all CTAs) share storage
-  __shared__ __align__(16) unsigned char s_raw[sizeof(CT) * SB * (SB + 1)];
-  T* D = reinterpret_cast<T*>(s_raw);
-  CT (*tileT)[SB + 1] = reinterpret_cast<CT (*)[SB + 1]>(s_raw);
-  __shared__ CT part[4][SB];
-  __shared__ CT xk[SB * NR_MAX];
-  __shared__ CT ys[SB];
-  __shared__ int s_last;
-  const Item it = items[blockIdx.x];
-  const FrontDev f = c.fronts[it.front];
-  const int n = f.n, k0 = it.a, nr = c.n_rhs;
-  const int kb = min(SB, f.fs - k0);
-  const T* __restrict__ G = arena<T>(c) + f.off;
-  double* __restrict__ y = c.vec + f.voff + (int64_t)n * nr;
-  const int t0 = k0 + kb;
-  const int nch = it.c;
-  const bool chol = method == M_CHOL;
-  double* __restrict__ sc = scratch + scr_off[it.front];
-  if (nch > 0) {
-    const int c0 = t0 + it.b * BWD_RB, c1 = min(c0 + BWD_RB, n);
-    const int i = threadIdx.x % SB, g = threadIdx.x / SB;   // NT = 256: 4 groups
-    for (int q = 0; q < nr; ++q) {
-      CT acc = CT(0);
-      if (chol) {
-        // rows of the chunk in tiles of 64: load L[rows, k-block] coalesced
-        // along rows, then thread (i, g) sums 16 rows of column i
-        for (int t0r = c0; t0r < c1; t0r += SB) {
-          __syncthreads();
-          for (int idx = threadIdx.x; idx < SB * SB; idx += NT) {
-            const int rr = idx % SB, cc = idx / SB;
-            tileT[rr][cc] = (t0r + rr < c1 && cc < kb) ? (CT)G[(t0r + rr) + (int64_t)(k0 + cc) * n] : CT(0);
-          }
-          for (int rr = threadIdx.x; rr < SB; rr += NT)
-            ys[rr] = t0r + rr < c1 ? (CT)y[t0r + rr + (int64_t)q * n] : CT(0);
-          __syncthreads();
-#pragma unroll 4
-          for (int rr = g * 16; rr < g * 16 + 16; ++rr) acc += tileT[rr][i] * ys[rr];
-        }
-      } else if (i < kb) {
-        {
-          for (int cc = c0 + g; cc < c1; cc += 4)
-            acc += (CT)G[(k0 + i) + (int64_t)cc * n] * (CT)y[cc + (int64_t)q * n];
-        }
-      }
-      part[g][i] = acc;
-      __syncthreads();
-      if (threadIdx.x < SB)
-        sc[((int64_t)it.b * nr + q) * SB + threadIdx.x] =
-            (double)(part[0][threadIdx.x] + part[1][threadIdx.x] + part[2][threadIdx.x] + part[3][threadIdx.x]);
-      __syncthreads();
-    }
-    __threadfence();
-    if (threadIdx.x == 0) s_last = (atomicAdd(&counters[it.front], 1) == nch - 1);
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    if (threadIdx.x == 0) counters[it.front] = 0;
-  }
-  // last CTA (or the only one): sum partials in chunk order, solve the block
-  for (int idx = threadIdx.x; idx < SB * kb; idx += NT) {
-    const int ii = idx % SB, j = idx / SB;
-    D[idx] = ii < kb ? G[(k0 + ii) + (int64_t)(k0 + j) * n] : T(0);
-  }
-  for (int idx = threadIdx.x; idx < kb * nr; idx += NT) {
-    const int ii = idx % kb, q = idx / kb;
-    double s = 0.0;
-    for (int ch = 0; ch < nch; ++ch) s += sc[((int64_t)ch * nr + q) * SB + ii];
-    xk[ii + q * SB] = (CT)(y[(k0 + ii) + (int64_t)q * n] - s);
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5;
-  for (int q = warp; q < nr; q += NT / 32) warp_upper_solve<T, CT>(D, kb, xk + q * SB, chol);
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < kb * nr; idx += NT) {
-    const int ii = idx % kb, q = idx / kb;
-    y[(k0 + ii) + (int64_t)q * n] = (double)xk[ii + q * SB];
-  }
-}
-
-void launch_fwd_step(const DevCtx& c, const Item* items, int n_items, int dtype, int method,
-                     cudaStream_t s) {
-  if (!n_items) return;
-  if (dtype == F64) k_fwd_step<double, 256><<<n_items, 256, 0, s>>>(c, items, method);
-  else k_fwd_step<float, 256><<<n_items, 256, 0, s>>>(c, items, method);
-}
-
-void launch_bwd_step(const DevCtx& c, const Item* items, int n_items, int dtype, int method,
-                     double* scratch, const int64_t* scr_off, int* counters, cudaStream_t s) {
-  if (!n_items) return;
-  if (dtype == F64)
-    k_bwd_step<double, 256><<<n_items, 256, 0, s>>>(c, items, method, scratch, scr_off, counters);
-  else
-    k_bwd_step<float, 256><<<n_items, 256, 0, s>>>(c, items, method, scratch, scr_off, counters);
 }
 
 __global__ void __launch_bounds__(256) k_bwd_store(DevCtx c, const Item* __restrict__ items,
@@ -1474,6 +1286,156 @@ void launch_bwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype
   const int nq = c.n_rhs - q0 < grp ? c.n_rhs - q0 : grp;
   if (dtype == F64) bwd_flags_t<double>(c, items, n_items, ticket, err, q0, nq, s);
   else bwd_flags_t<float>(c, items, n_items, ticket, err, q0, nq, s);
+}
+
+// ===========================================================================
+// Backward flag-driven solve of large LU fronts: x_b = U_bb^{-1} (y_b - sum_{c
+// right of block b} U_bc x_c), the forward kernel's row blocks from the last
+// one up.  Item: front, a = factor block, tickets in descending block order.
+// The columns right of the factor block (x known from the parent) come
+// first, then the factor blocks as their hand-off words arrive.  U_bb^{-1}
+// is formed at factorisation (k_lu_dinv).  Bound by the chain of hand-offs
+// as the Cholesky solves are; measured on GB300 (24^3 p = 3, root 14,911
+// rows, FP32): 1.9 ms for the two backward solves of a step against 44
+// for a launch per 64 columns with the block substituted by one warp.
+// ===========================================================================
+template <typename T, int NQ>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_lu_bwd_flags(DevCtx c, const Item* __restrict__ items,
+                                                                              int* ticket, int* err, int q0) {
+  __shared__ int s_t;
+  __shared__ T red[4][FB][NQ];
+  __shared__ T v[FB][NQ];
+  __shared__ T dsh[FB * (FB + 1)];
+  __shared__ T xsh[2][NQ][FB];
+  if (threadIdx.x == 0) s_t = atomicAdd(ticket, 1);
+  __syncthreads();
+  const Item it = items[s_t];
+  const FrontDev f = c.fronts[it.front];
+  const int n = f.n, fs = f.fs, nr = c.n_rhs, b = it.a;
+  const int nq = min(NQ, nr - q0), nfb = (fs + FB - 1) / FB;
+  const T* __restrict__ G = arena<T>(c) + f.off;
+  {
+    const T* __restrict__ Dg = dinv_arena<T>(c) + f.dinv_off + (int64_t)(nfb + b) * FB * FB;
+    for (int idx = threadIdx.x; idx < FB * FB; idx += 256) dsh[(idx / FB) * (FB + 1) + idx % FB] = Dg[idx];
+  }
+  double* __restrict__ hx = c.vec + f.voff;                  // hand-off: the z slab's factor rows
+  double* __restrict__ y = hx + (int64_t)n * nr;
+  const int i = threadIdx.x % FB, g = threadIdx.x / FB;
+  const int row = b * FB + i;
+  const bool rv = row < fs;
+  T acc[NQ], yb[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    acc[q] = T(0);
+    yb[q] = (rv && q < nq && g == 0) ? (T)y[row + (int64_t)(q0 + q) * n] : T(0);   // before any wait
+  }
+  // columns fs .. n-1: group g takes 16 of every 64, all loads of a round in flight
+  for (int cs = fs; cs < n; cs += FB) {
+    T gv[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int cc = cs + g * 16 + u;
+      gv[u] = rv && cc < n ? G[row + (int64_t)cc * n] : T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int cc = min(cs + g * 16 + u, n - 1);
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        if (q < nq) acc[q] += gv[u] * (T)y[cc + (int64_t)(q0 + q) * n];
+    }
+  }
+  T tile[16];
+  auto load_tile = [&](int j) {
+    const int kbj = min(FB, fs - j * FB);
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int cc = g * 16 + u;
+      tile[u] = (rv && cc < kbj) ? G[row + (int64_t)(j * FB + cc) * n] : T(0);
+    }
+  };
+  const bool w0 = threadIdx.x < 32;
+  HandWords hw;
+  bool live = true;      // warp 0: false once a wait has run out (no more waiting)
+  if (nfb - 1 > b) {
+    load_tile(nfb - 1);
+    if (w0) hw.load(hx + (nfb - 1) * FB + (int64_t)q0 * n, min(FB, fs - (nfb - 1) * FB));
+  }
+  for (int j = nfb - 1; j > b; --j) {
+    const int buf = j & 1;
+    if (w0) {
+      const int kbj = min(FB, fs - j * FB);
+      const double* xj = hx + j * FB;
+      if (live) live = hw.wait(xj + (int64_t)q0 * n, kbj, err, wait_code(2, j, b));
+      hw.stage(xsh[buf][0]);
+      for (int q = 1; q < nq; ++q) {
+        HandWords hq;
+        hq.load(xj + (int64_t)(q0 + q) * n, kbj);
+        if (live) live = hq.wait(xj + (int64_t)(q0 + q) * n, kbj, err, wait_code(2, j, b));
+        hq.stage(xsh[buf][q]);
+      }
+      if (j - 1 > b) hw.load(hx + (j - 1) * FB + (int64_t)q0 * n, min(FB, fs - (j - 1) * FB));
+    }
+    T cur[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) cur[u] = tile[u];
+    if (j - 1 > b) load_tile(j - 1);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        if (q < nq) acc[q] += cur[u] * xsh[buf][q][g * 16 + u];
+  }
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) red[g][i][q] = acc[q];
+  __syncthreads();
+  if (threadIdx.x < FB) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+      v[i][q] = (rv && q < nq) ? yb[q] - (red[0][i][q] + red[1][i][q] + red[2][i][q] + red[3][i][q]) : T(0);
+  }
+  __syncthreads();
+  // x = Uinv v by four column groups (zero below its diagonal and past the block)
+  T xp[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) xp[q] = T(0);
+#pragma unroll
+  for (int u = 0; u < 16; ++u) {
+    const int t = g * 16 + u;
+    const T d = dsh[t * (FB + 1) + i];     // Uinv[i][t], column t staged as row t
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) xp[q] += d * v[t][q];
+  }
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) red[g][i][q] = xp[q];
+  __syncthreads();
+  if (threadIdx.x < FB && rv) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+      if (q < nq) {
+        const double x = (double)(red[0][i][q] + red[1][i][q] + red[2][i][q] + red[3][i][q]);
+        y[row + (int64_t)(q0 + q) * n] = x;
+        st_hand(hx + row + (int64_t)(q0 + q) * n, x);
+      }
+  }
+}
+
+template <typename T>
+static void lu_bwd_flags_t(const DevCtx& c, const Item* items, int n_items, int* ticket, int* err, int q0, int nq,
+                           cudaStream_t s) {
+  if (nq >= 3) k_lu_bwd_flags<T, 4><<<n_items, 256, 0, s>>>(c, items, ticket, err, q0);
+  else if (nq == 2) k_lu_bwd_flags<T, 2><<<n_items, 256, 0, s>>>(c, items, ticket, err, q0);
+  else k_lu_bwd_flags<T, 1><<<n_items, 256, 0, s>>>(c, items, ticket, err, q0);
+}
+
+void launch_lu_bwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket, int* err, int q0,
+                         cudaStream_t s) {
+  if (!n_items) return;
+  cudaMemsetAsync(ticket, 0, sizeof(int), s);
+  const int nq = c.n_rhs - q0 < FLAG_NR ? c.n_rhs - q0 : FLAG_NR;
+  if (dtype == F64) lu_bwd_flags_t<double>(c, items, n_items, ticket, err, q0, nq, s);
+  else lu_bwd_flags_t<float>(c, items, n_items, ticket, err, q0, nq, s);
 }
 
 // ===========================================================================

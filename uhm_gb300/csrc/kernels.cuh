@@ -62,6 +62,7 @@ struct DevCtx {
   int2* colsrc;       // (source local index, source column)
   int32_t* sgi;       // schur-row global dofs
   int32_t* piv;       // pivots (LU), relative to the front's first row
+  int32_t* perm;      // large LU fronts with pivoting: row of the gathered vector at each factor row
   double* a64;        // FP64 panel arena
   float* a32;         // FP32 panel arena
   double* emat;       // element matrices (FP64, retained for the residual)
@@ -155,11 +156,12 @@ void launch_bwd_chain(const DevCtx& c, const Item* items, int n_items, int* tick
 // where the first hand-off wait of the solves gave up (0: none; kind * 10^8 +
 // awaited block * 10^4 + waiting block), cleared when read
 int solve_wait_where();
-// blocked solve steps of large fronts (64-column diagonal blocks)
-void launch_fwd_step(const DevCtx& c, const Item* items, int n_items, int dtype, int method,
-                     cudaStream_t s);
-void launch_bwd_step(const DevCtx& c, const Item* items, int n_items, int dtype, int method,
-                     double* scratch, const int64_t* scr_off, int* counters, cudaStream_t s);
+// large LU fronts: inverses of the 64 x 64 diagonal blocks of L (unit lower)
+// and U (item: front, a = block; L's at dinv_off, U's behind them), and the
+// backward flag-driven solve (the forward one is launch_fwd_flags)
+void launch_lu_dinv(const DevCtx& c, const Item* items, int n_items, int dtype, cudaStream_t s);
+void launch_lu_bwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket, int* err, int q0,
+                         cudaStream_t s);
 void launch_bwd_prepare(const DevCtx& c, const Item* items, int n_items, int dtype, int method,
                         const double* g, int64_t ldg, cudaStream_t s);
 void launch_bwd_store(const DevCtx& c, const Item* items, int n_items, double* g, int64_t ldg,
