@@ -913,10 +913,9 @@ void Engine::build_programs(int method) {
   auto push_potrf_trsm = [&](int dt, const std::vector<Item>& p_items, const std::vector<Item>& t_items,
                              double fp, double ft) {
     // every fused CTA repeats the latency-bound diagonal factorisation: fuse
-    // only while the launch fits fuse_potrf_trsm waves of one CTA per SM.
-    // Not for FP64, whose diagonal kernel (k_potrf_inv64) takes a wider block.
+    // only while the launch fits fuse_potrf_trsm waves of one CTA per SM
     const size_t n_fused = t_items.size() + p_items.size();
-    if (dt == F64 || !tune.fuse_potrf_trsm || n_fused > (size_t)tune.fuse_potrf_trsm * n_sm) {
+    if (!tune.fuse_potrf_trsm || n_fused > (size_t)tune.fuse_potrf_trsm * n_sm) {
       push(fac_ops, OP_POTRF, dt, NB, 0, p_items, fp);
       push(fac_ops, OP_TRSM, dt, NB, 0, t_items, ft);
       return;
@@ -1033,8 +1032,8 @@ void Engine::build_programs(int method) {
   // [r0, r1) x columns [c0, c1) (Cholesky: those reaching the lower
   // triangle; returns the update's flops and adds its bytes to by), and the
   // launches of one update
-  auto xs_pack_rows = [](std::vector<Item>& it, int s, int k0, int r0, int r1, int cols) {
-    for (int r = r0; r < r1; r += XS_PACK_ROWS) it.push_back(Item{s, k0, r, cols});
+  auto xs_pack_items = [](std::vector<Item>& it, int nb, int s, int k0, int r0, int r1, int cols) {
+    for (int r = r0; r < r1; r += xs_pack_rows(nb)) it.push_back(Item{s, k0, r, cols});
   };
   auto xs_tiles = [](std::vector<Item>& it, const HostFront& f, int k0, int kb, int r0, int r1, int c0, int c1,
                      bool lower, double& by) {
@@ -1045,12 +1044,27 @@ void Engine::build_programs(int method) {
     by += 2.0 * esz * area + 2.0 * (f.prec == PREC_FP64 ? XS_S64 : XS_S32) * kb * (lower ? m : m + w);
     return 2.0 * kb * area;
   };
-  auto push_xs = [&](int dt, int nb, int region, const std::vector<Item>& pk, const std::vector<Item>& tiles,
+  auto push_xs = [&](int dt, int nb, int region, const std::vector<Item>& pk, std::vector<Item>& tiles,
                      double fl, double by) {
     if (tiles.empty()) return;
     push(fac_ops, OP_XS_PACK, dt, nb, 0, pk);
+    // fewer tiles than SMs: tiles of half the width (a launch is as long as its
+    // slowest CTA; one round of half tiles of K = 64 takes 23 us and two 38,
+    // against 29 and 49 for whole ones)
+    const bool narrow = (int)tiles.size() < n_sm;
+    if (narrow) {
+      std::vector<Item> h;
+      for (const Item& t : tiles)
+        for (int e = 0; e < 2; ++e) {
+          const HostFront& f = fronts[t.front];
+          const int c = t.b + 64 * e, B = std::min(t.c / XS_NBO * XS_NBO + XS_NBO, f.fs);
+          if (c < (region == 1 ? B : f.n) && (!chol || c < t.a + XS_TILE)) h.push_back(Item{t.front, t.a, c, t.c});
+        }
+      tiles.swap(h);
+    }
     Op op{OP_XS_UPDATE, dt, nb, chol ? 1 : 0, add_items(tiles), (int)tiles.size()};
     op.q0 = region;
+    op.aux = narrow ? 64 : XS_TILE;
     op.flops = fl;
     op.bytes = by;
     fac_ops.push_back(op);
@@ -1133,18 +1147,25 @@ void Engine::build_programs(int method) {
             if (chol) {
               fp += get_flop_chol(0, kb);
               ft += get_flop_trsm_lower(0, kb, f.n - base);
-              for (int r0 = base; r0 < f.n; r0 += TRSM_RB) t_items.push_back(Item{s, k0, r0, 0});
+              if (dt == F64)
+                for (int r0 = base; r0 < f.n; r0 += XS_TRSM_ROWS) t_items.push_back(Item{s, k0, r0, base < B});
+              else
+                for (int r0 = base; r0 < f.n; r0 += TRSM_RB) t_items.push_back(Item{s, k0, r0, 0});
             } else {
               fp += get_flop_lu(0, f.n - k0, kb);
               ft += get_flop_trsm_lower(0, kb, B - base);
               for (int c0 = base; c0 < B; c0 += LUROW_CB) t_items.push_back(Item{s, k0, c0, B});
             }
             if (base >= B) continue;
-            xs_pack_rows(pk, s, k0, base, f.n, 0);
-            if (!chol) xs_pack_rows(pk, s, k0, base, B, 1);
+            // (FP64 Cholesky: the TRSM writes the slices)
+            if (!chol || dt == F32) xs_pack_items(pk, NB, s, k0, base, f.n, 0);
+            if (!chol) xs_pack_items(pk, NB, s, k0, base, B, 1);
             fu += xs_tiles(ut, f, k0, kb, base, f.n, base, B, chol, bu);
           }
-          if (chol) {
+          if (chol && dt == F64) {
+            push(fac_ops, OP_POTRF, dt, NB, 0, p_items, fp);
+            push(fac_ops, OP_TRSM, dt, NB, 0, t_items, ft);
+          } else if (chol) {
             push_potrf_trsm(dt, p_items, t_items, fp, ft);
           } else {
             push_lu_panel(dt, p_items, fp, XS_NBO);
@@ -1174,8 +1195,8 @@ void Engine::build_programs(int method) {
             for (int c0 = B; c0 < f.n; c0 += LUROW_CB) t_items.push_back(Item{s, k0, c0, 0});
             ft += get_flop_trsm_lower(0, kb, f.n - B);
             if (base >= B || B >= f.n) continue;
-            xs_pack_rows(pk, s, k0, base, B, 0);
-            xs_pack_rows(pk, s, k0, B, f.n, 1);
+            xs_pack_items(pk, NB, s, k0, base, B, 0);
+            xs_pack_items(pk, NB, s, k0, B, f.n, 1);
             fu += xs_tiles(ut, f, k0, kb, base, B, B, f.n, false, bu);
           }
           push(fac_ops, OP_LUROW, dt, NB, 0, t_items, ft);
@@ -1189,8 +1210,8 @@ void Engine::build_programs(int method) {
           if (f.fs <= K0) continue;
           const int KB = std::min(XS_NBO, f.fs - K0), base = K0 + KB;
           if (base >= f.n) continue;
-          xs_pack_rows(pk, s, K0, base, f.n, 0);
-          if (!chol) xs_pack_rows(pk, s, K0, base, f.n, 1);
+          xs_pack_items(pk, XS_NBO, s, K0, base, f.n, 0);
+          if (!chol) xs_pack_items(pk, XS_NBO, s, K0, base, f.n, 1);
           fu += xs_tiles(ut, f, K0, KB, base, f.n, base, f.n, chol, bu);
         }
         push_xs(dt, XS_NBO, 0, pk, ut, fu, bu);
@@ -2012,7 +2033,10 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
                             op.param, st);
         break;
       case OP_POTRF: launch_potrf_diag(ctx, it, op.n_items, op.dtype, op.nb, st); break;
-      case OP_TRSM: launch_trsm_panel(ctx, it, op.n_items, op.dtype, op.nb, st); break;
+      case OP_TRSM:
+        if (op.dtype == F64) launch_xs_trsm(ctx, xs_ctx, it, op.n_items, st);
+        else launch_trsm_panel(ctx, it, op.n_items, op.dtype, op.nb, st);
+        break;
       case OP_POTRF_TRSM: launch_potrf_trsm(ctx, it, op.n_items, op.dtype, st); break;
       case OP_SYRK: launch_syrk_update(ctx, it, op.n_items, op.dtype, op.nb, op.param, st); break;
       case OP_FWD_FLAGS:
@@ -2042,7 +2066,7 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
         break;
       case OP_XS_PACK: launch_xs_pack(ctx, xs_ctx, it, op.n_items, op.dtype, op.nb, st); break;
       case OP_XS_UPDATE:
-        launch_xs_update(ctx, xs_ctx, xs_map, it, op.n_items, op.dtype, op.nb, op.q0, op.param, d_err, st);
+        launch_xs_update(ctx, xs_ctx, xs_map, it, op.n_items, op.dtype, op.nb, op.q0, op.param, op.aux, d_err, st);
         break;
       case OP_GETRF: launch_getrf_panel(ctx, it, op.n_items, op.dtype, op.nb, op.param, st); break;
       case OP_GETRF_COOP:

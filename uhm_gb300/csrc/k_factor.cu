@@ -689,15 +689,10 @@ __global__ void __launch_bounds__(NT) k_trsm_panel(DevCtx c, const Item* __restr
 void launch_trsm_panel(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
                        cudaStream_t s) {
   if (!n_items) return;
-  if (dtype == F64) {
-    size_t sm = (size_t)(64 * 68 + TRSM_RB * nb) * sizeof(double);
-    cudaFuncSetAttribute(k_trsm_panel<double, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_trsm_panel<double, 256><<<n_items, 256, sm, s>>>(c, items, nb);
-  } else {
-    size_t sm = (size_t)(64 * 68 + TRSM_RB * nb) * sizeof(float);
-    cudaFuncSetAttribute(k_trsm_panel<float, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_trsm_panel<float, 256><<<n_items, 256, sm, s>>>(c, items, nb);
-  }
+  if (dtype == F64) throw std::invalid_argument("trsm_panel: FP64 fronts take xs_trsm");
+  size_t sm = (size_t)(64 * 68 + TRSM_RB * nb) * sizeof(float);
+  cudaFuncSetAttribute(k_trsm_panel<float, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_trsm_panel<float, 256><<<n_items, 256, sm, s>>>(c, items, nb);
 }
 
 // Diagonal block and panel TRSM of one 64-column step in one launch.  Every

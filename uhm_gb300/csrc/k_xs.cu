@@ -92,87 +92,172 @@ template <> struct XsType<float> {
   }
 };
 
-// A CTA cuts 64 rows: thread r + 64 g holds 16 columns 16 g .. of row r per
-// 64-column chunk (a warp's loads of one column are 32 consecutive rows) and
-// writes each slice's 16 digits as one whole 32-byte sector.  Memory bound:
-// 8 (4) bytes read twice (the second time from L2) and 16 (8) written per
-// entry; the digits come from integer shifts and byte extraction, no FP64.
-template <typename T>
+// the digits of one entry, as bits of exact floats (d[p] = slice p)
+template <int S>
+__device__ __forceinline__ void xs_digits(long long X, uint32_t (&d)[S]) {
+  // balanced digits: adding 128 to every place but the top turns each into its
+  // byte; float(2^23 + byte) - (2^23 + 128) is the digit
+  constexpr long long BIAS = S == 8 ? 0x0080808080808080ll : 0x0000000000808080ll;
+  const long long Y = X + BIAS;
+#pragma unroll
+  for (int p = 0; p < S; ++p) {
+    float dg;
+    if (p == 0) {
+      dg = __int_as_float(0x4B400000 + (int)(Y >> (8 * (S - 1)))) - 12582912.0f;
+    } else {
+      const uint32_t b = (uint32_t)(Y >> (8 * (S - 1 - p))) & 0xFFu;
+      dg = __int_as_float((int)(0x4B000000u | b)) - 8388736.0f;
+    }
+    d[p] = __float_as_uint(dg);
+  }
+}
+
+// A CTA cuts 256 / NG rows: thread r + (256 / NG) g holds 16 columns 16 g .. of
+// row r (a warp's loads of one column are consecutive rows), all its loads in
+// flight, and writes each slice's 16 digits as one whole 32-byte sector.  NG =
+// 4 (64 columns) or 16 (256).  Memory bound: 8 (4) bytes read and 16 (8)
+// written per entry; the digits come from integer shifts and byte extraction,
+// no FP64.  Measured on GB300 for 256 columns: 29 us with 64 rows per CTA and
+// its 64-column chunks in turn (whatever their number), 11 with 16 rows.
+template <typename T, int NG>
 __global__ void __launch_bounds__(256) k_xs_pack(DevCtx c, XsCtx x, const Item* __restrict__ items, int nb) {
-  constexpr int S = XsType<T>::S;
-  __shared__ int s_f[4][64];
+  constexpr int S = XsType<T>::S, ROWS = 256 / NG;
+  __shared__ int s_f[NG][ROWS];
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, K0 = it.a, trans = it.c;
   const int W = min(nb, f.fs - K0), nch = xs_chunks(nb, f.fs);
-  const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
+  const int r = threadIdx.x % ROWS, g = threadIdx.x / ROWS;
   const int row = it.b + r;
   const T* __restrict__ G = arena<T>(c) + f.off;
   const int64_t base = trans ? (int64_t)row * n + K0 : row + (int64_t)K0 * n;
   const int64_t step = trans ? 1 : n;
   const bool in = row < n;
-  int fm = 0;
-  for (int k0 = 0; k0 < W; k0 += 64) {
-    T v[16];
+  T v[16];
 #pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int k = k0 + 16 * g + u;
-      v[u] = in && k < W ? G[base + k * step] : T(0);
-    }
+  for (int u = 0; u < 16; ++u) v[u] = in && 16 * g + u < W ? G[base + (16 * g + u) * step] : T(0);
+  int fm = 1;
 #pragma unroll
-    for (int u = 0; u < 16; ++u) fm = max(fm, XsType<T>::field(v[u]));
-  }
+  for (int u = 0; u < 16; ++u) fm = max(fm, XsType<T>::field(v[u]));
   s_f[g][r] = fm;
   __syncthreads();
-  fm = max(max(s_f[0][r], s_f[1][r]), max(max(s_f[2][r], s_f[3][r]), 1));
-  if (!in) return;
+#pragma unroll
+  for (int e = 0; e < NG; ++e) fm = max(fm, s_f[e][r]);
+  if (!in || 16 * g >= 64 * nch) return;
   const bool bad = fm == XsType<T>::FMAX;
   if (g == 0) x.exps[x.exp0[it.front] + (trans ? n : 0) + row] = bad ? XS_BAD : fm - XsType<T>::EBIAS;
-  uint8_t* const w0 = reinterpret_cast<uint8_t*>(x.ws) + 128 * ((trans ? x.row0b : x.row0)[it.front] + row) + 32 * g;
-  for (int k0 = 0; k0 < W; k0 += 64) {
-    uint32_t d[S][8];
+  uint8_t* const w0 = reinterpret_cast<uint8_t*>(x.ws) +
+                      128 * ((trans ? x.row0b : x.row0)[it.front] + (int64_t)(g >> 2) * n + row) + 32 * (g & 3);
+  uint32_t d[S][8];
 #pragma unroll
-    for (int u = 0; u < 16; u += 2) {
-      uint32_t lo[S];
+  for (int u = 0; u < 16; u += 2) {
+    uint32_t d0[S], d1[S];
+    xs_digits<S>(bad ? 0 : XsType<T>::fixed(v[u], fm), d0);
+    xs_digits<S>(bad ? 0 : XsType<T>::fixed(v[u + 1], fm), d1);
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int k = k0 + 16 * g + u + e;
-        const long long X = (k < W && !bad) ? XsType<T>::fixed(G[base + k * step], fm) : 0;
-        // balanced digits: adding 128 to every place but the top turns each
-        // into its byte; float(2^23 + byte) - (2^23 + 128) is the digit
-        constexpr long long BIAS = S == 8 ? 0x0080808080808080ll : 0x0000000000808080ll;
-        const long long Y = X + BIAS;
+    for (int p = 0; p < S; ++p) d[p][u / 2] = __byte_perm(d0[p], d1[p], 0x7632);
+  }
 #pragma unroll
-        for (int p = 0; p < S; ++p) {
-          float dg;
-          if (p == 0) {
-            const int t = (int)(Y >> (8 * (S - 1)));
-            dg = __int_as_float(0x4B400000 + t) - 12582912.0f;
-          } else {
-            const uint32_t b = (uint32_t)(Y >> (8 * (S - 1 - p))) & 0xFFu;
-            dg = __int_as_float((int)(0x4B000000u | b)) - 8388736.0f;
-          }
-          const uint32_t h = __float_as_uint(dg);
-          if (e == 0) lo[p] = h;
-          else d[p][u / 2] = __byte_perm(lo[p], h, 0x7632);
-        }
-      }
-    }
-    const int kc = k0 >> 6;
-#pragma unroll
-    for (int p = 0; p < S; ++p) {
-      uint4* w = reinterpret_cast<uint4*>(w0 + 128 * (int64_t)(p * nch + kc) * n);
-      w[0] = make_uint4(d[p][0], d[p][1], d[p][2], d[p][3]);
-      w[1] = make_uint4(d[p][4], d[p][5], d[p][6], d[p][7]);
-    }
+  for (int p = 0; p < S; ++p) {
+    uint4* w = reinterpret_cast<uint4*>(w0 + 128 * (int64_t)(p * nch) * n);
+    w[0] = make_uint4(d[p][0], d[p][1], d[p][2], d[p][3]);
+    w[1] = make_uint4(d[p][4], d[p][5], d[p][6], d[p][7]);
   }
 }
 
 void launch_xs_pack(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, int dtype, int nb,
                     cudaStream_t s) {
   if (!n_items) return;
-  if (dtype == F64) k_xs_pack<double><<<n_items, 256, 0, s>>>(c, x, items, nb);
-  else k_xs_pack<float><<<n_items, 256, 0, s>>>(c, x, items, nb);
+  if (nb != 64 && nb != XS_NBO) throw std::invalid_argument("slices: panel width must be 64 or 256");
+  if (dtype == F64) {
+    if (nb == 64) k_xs_pack<double, 4><<<n_items, 256, 0, s>>>(c, x, items, nb);
+    else k_xs_pack<double, 16><<<n_items, 256, 0, s>>>(c, x, items, nb);
+  } else {
+    if (nb == 64) k_xs_pack<float, 4><<<n_items, 256, 0, s>>>(c, x, items, nb);
+    else k_xs_pack<float, 16><<<n_items, 256, 0, s>>>(c, x, items, nb);
+  }
+}
+
+// FP64 Cholesky panel TRSM, X = A Linv^T below a 64-column diagonal block (its
+// inverse from k_potrf_inv64), and the slices of X for the panel's own update.
+// 16 rows per CTA: thread (i, j) sums columns j, j + 16, j + 32, j + 48 of row
+// i, each up to its diagonal (Linv is lower triangular), so every warp issues
+// the same 160 of 256 multiply-adds per row.  Bound by those (2 per clock and
+// SM); 16 rows instead of 64 spread a panel over every SM: the smallest launch
+// took 55 us with 64 rows, 17 with 16, slices included (they were a launch of 12 us
+// of their own).  Item: front, a = k0, b = first row, c = 1: slices too.
+constexpr int XT_ROWS = XS_TRSM_ROWS;
+__global__ void __launch_bounds__(256) k_xs_trsm64(DevCtx c, XsCtx x, const Item* __restrict__ items) {
+  constexpr int S = XS_S64;
+  __shared__ double Lt[64 * 64];               // Lt[t][j] = Linv[j][t]
+  __shared__ double Xs[64][XT_ROWS];           // A, then X
+  __shared__ int s_f[XT_ROWS];
+  const Item it = items[blockIdx.x];
+  const FrontDev f = c.fronts[it.front];
+  const int n = f.n, k0 = it.a, r0 = it.b;
+  const int kb = min(64, f.fs - k0);
+  double* __restrict__ G = c.a64 + f.off + r0 + (int64_t)k0 * n;
+  const double* __restrict__ D = c.dinv64 + f.dinv_off + (int64_t)(k0 / 64) * 4096;
+  const int tid = threadIdx.x, i = tid & 15, jg = tid >> 4;
+  const bool rv = r0 + i < n;
+  {
+    double dv[16], xv[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int t = jg + 16 * u;
+      xv[u] = rv && t < kb ? G[i + (int64_t)t * n] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) dv[u] = D[tid + 256 * u];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) Xs[jg + 16 * u][i] = xv[u];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) Lt[tid + 256 * u] = dv[u];
+    if (tid < XT_ROWS) s_f[tid] = 1;
+  }
+  __syncthreads();
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+#pragma unroll 4
+    for (int t = 16 * h; t < 16 * h + 16; ++t) {
+      const double xt = Xs[t][i];
+#pragma unroll
+      for (int u = h; u < 4; ++u) acc[u] += xt * Lt[t * 64 + jg + 16 * u];
+    }
+  }
+  int fm = 1;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int j = jg + 16 * u;
+    if (rv && j < kb) G[i + (int64_t)j * n] = acc[u];
+    fm = max(fm, XsType<double>::field(acc[u]));
+  }
+  if (!it.c) return;
+  atomicMax(&s_f[i], fm);
+  __syncthreads();                             // A has been read
+#pragma unroll
+  for (int u = 0; u < 4; ++u) Xs[jg + 16 * u][i] = acc[u];
+  __syncthreads();
+  // thread (row tid / 16, columns 4 (tid % 16) ..): 8 bytes of every slice
+  const int r = tid >> 4, c4 = 4 * (tid & 15), row = r0 + r;
+  if (row >= n) return;
+  fm = s_f[r];
+  const bool bad = fm == XsType<double>::FMAX;
+  if (c4 == 0) x.exps[x.exp0[it.front] + row] = bad ? XS_BAD : fm - XsType<double>::EBIAS;
+  uint32_t d[4][S];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) xs_digits<S>(bad ? 0 : XsType<double>::fixed(Xs[c4 + e][r], fm), d[e]);
+  uint8_t* const w0 = reinterpret_cast<uint8_t*>(x.ws) + 128 * (x.row0[it.front] + row) + 2 * c4;
+#pragma unroll
+  for (int p = 0; p < S; ++p)
+    *reinterpret_cast<uint2*>(w0 + 128 * (int64_t)p * n) =
+        make_uint2(__byte_perm(d[0][p], d[1][p], 0x7632), __byte_perm(d[2][p], d[3][p], 0x7632));
+}
+
+void launch_xs_trsm(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, cudaStream_t s) {
+  if (!n_items) return;
+  k_xs_trsm64<<<n_items, 256, 0, s>>>(c, x, items);
 }
 
 // ---------------------------------------------------------------------------
@@ -205,14 +290,24 @@ __device__ __forceinline__ void xs_add(long long& a, uint32_t v) {
   a += (long long)__float2int_rn(__uint_as_float(v)) << SH;
 }
 
-// value 2^E of the integer a (E may leave the exponent range)
+// a 2^E, rounded to nearest (E may leave the exponent range).  FP64 without
+// conversions, which run at the FP64 rate: the leading bit by clz, the bits
+// below the 53rd rounded to even in integers.
 __device__ __forceinline__ double xs_scaled(long long a, int E, double) {
-  const double x = __ll2double_rn(a);
-  const int hi = __double2hiint(x), f = (hi >> 20) & 0x7FF;
-  if (a == 0) return 0.0;
-  if ((unsigned)(f + E - 1) < 2045u) return __hiloint2double(hi + (E << 20), __double2loint(x));
-  const int e1 = max(-2000, min(2000, E)) / 2, e2 = max(-2000, min(2000, E)) - e1;
-  return x * __hiloint2double((1023 + e1) << 20, 0) * __hiloint2double((1023 + e2) << 20, 0);
+  unsigned long long m = a < 0 ? 0ull - (unsigned long long)a : (unsigned long long)a;
+  const int lz = __clzll((long long)m);
+  const int e = 1023 + 63 - lz + E;
+  if (m == 0) return 0.0;
+  if ((unsigned)(e - 1) >= 2044u) {
+    const int e1 = max(-2000, min(2000, E)) / 2, e2 = max(-2000, min(2000, E)) - e1;
+    return __ll2double_rn(a) * __hiloint2double((1023 + e1) << 20, 0) * __hiloint2double((1023 + e2) << 20, 0);
+  }
+  m <<= lz;
+  const unsigned rem = (unsigned)m & 0x7FFu;
+  unsigned long long q = (m >> 11) + ((rem + ((unsigned)(m >> 11) & 1u)) > 0x400u ? 1u : 0u);
+  q += (unsigned long long)(e - 1) << 52;      // the leading bit adds the last 1 to the exponent
+  if (a < 0) q |= 1ull << 63;
+  return __longlong_as_double((long long)q);
 }
 __device__ __forceinline__ float xs_scaled(long long a, int E, float) {
   const float x = __ll2float_rn(a);
@@ -229,9 +324,14 @@ __device__ __forceinline__ float xs_scaled(long long a, int E, float) {
 // warps 0..15 (a lane quarter and 32 columns each) take the accumulators to
 // 64-bit integers in registers while the next pass runs, then update C
 // (column by column: a warp's loads and stores are 32 consecutive rows).
-// 14 slots of 16 KB.  Bound: tensor pipe /
-// shared-memory reads of the 128 x 128 products.
-template <typename T>
+// 14 slots of 16 KB.  BN = 64: tiles of half the width
+// for launches with fewer 128 x 128 tiles than SMs, where a tile's own time
+// counts: half the products and half the FP64 additions of the epilogue, whose C
+// entries are loaded while the products run.  Bound: tensor pipe / shared-memory
+// reads of the 128 x 128 products; a tile of a small launch by its epilogue.
+// Measured on GB300 for up to 80 tiles
+// of K = 64 (256): 29 (60) -> 23 (50) us.
+template <typename T, int BN>
 __global__ void __launch_bounds__(XS_THREADS, 1)
 k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const Item* __restrict__ items, int n_items,
             int nb, int region, int lower, int* err) {
@@ -311,7 +411,7 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
   } else if (warp == XS_EPI_WARPS + 1) {
     if (lane == 0) {
       // MMA issuer
-      const uint32_t idesc = idesc_bf16_f32(XS_TILE, XS_TILE);
+      const uint32_t idesc = idesc_bf16_f32(XS_TILE, BN);
       const uint32_t ring = smem_u32(smem);
       int s = 0;
       uint32_t ph = 0;               // parity of the full wait at slot s
@@ -399,14 +499,30 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
     }
   } else {
     // epilogue
+    constexpr int NC = BN / 4;       // columns per thread
     const int quarter = warp & 3, cg = warp >> 2;
-    const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + cg * 32;
+    const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + cg * NC;
     uint32_t par = 0;              // bit a: parity of the next use of accumulator a
     bool live = true;
     for (int t = blockIdx.x; t < n_items && live; t += gridDim.x) {
-      long long acc[32];
+      const Item it = items[t];
+      const FrontDev& f = c.fronts[it.front];
+      const int n = f.n, K0 = it.c;
+      const int Bnd = region ? min((K0 / XS_NBO) * XS_NBO + XS_NBO, f.fs) : n;
+      const int rmax = region == 2 ? Bnd : n, cmax = region == 1 ? Bnd : n;
+      const int row = it.a + quarter * 32 + lane, c0 = it.b + cg * NC;
+      // columns c0 + j, j < cend, of this thread's row are updated
+      const int cend = row < rmax ? min(cmax, lower ? row + 1 : cmax) - c0 : 0;
+      T* __restrict__ G = arena<T>(c) + f.off + row + (int64_t)c0 * n;
+      constexpr bool EARLY = BN == 64;
+      T ce[EARLY ? NC : 1];
+      if constexpr (EARLY) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) acc[j] = 0;
+        for (int j = 0; j < NC; ++j) ce[j] = j < cend ? __ldcg(G + (int64_t)j * n) : T(0);
+      }
+      long long acc[NC];
+#pragma unroll
+      for (int j = 0; j < NC; ++j) acc[j] = 0;
       auto take = [&](auto dd) {
         constexpr int d = decltype(dd)::value, a = d & 3;
         constexpr int SH = d >= 4 ? 8 * (7 - d) : 8 * (3 - d) + (S == 8 ? 18 : 0);
@@ -414,11 +530,11 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
         par ^= 1u << a;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < NC / 16; ++h) {
           uint32_t v[16];
           XS_LD16(tbase + a * XS_TILE + 16 * h, v);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (h == 1) {
+          if (h == NC / 16 - 1) {
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&acc_empty[a]));
@@ -433,33 +549,28 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
         live = take(std::integral_constant<int, 4>{}) && take(std::integral_constant<int, 5>{}) &&
                take(std::integral_constant<int, 6>{}) && take(std::integral_constant<int, 7>{});
 #pragma unroll
-        for (int j = 0; j < 32; ++j) acc[j] = (acc[j] + (1 << 13)) >> 14;
+        for (int j = 0; j < NC; ++j) acc[j] = (acc[j] + (1 << 13)) >> 14;
       }
       live = live && take(std::integral_constant<int, 0>{}) && take(std::integral_constant<int, 1>{}) &&
              take(std::integral_constant<int, 2>{}) && take(std::integral_constant<int, 3>{});
       if (!live || *s_abort) break;
       // C -= acc 2^(ea + eb - 54) (FP32: - 36); |acc| < 2^62 (2^44)
-      const Item it = items[t];
-      const FrontDev& f = c.fronts[it.front];
-      const int n = f.n, K0 = it.c;
-      const int Bnd = region ? min((K0 / XS_NBO) * XS_NBO + XS_NBO, f.fs) : n;
-      const int rmax = region == 2 ? Bnd : n, cmax = region == 1 ? Bnd : n;
-      const int row = it.a + quarter * 32 + lane, c0 = it.b + cg * 32;
-      if (row < rmax) {
+      if (cend > 0) {
         const int* __restrict__ ex = x.exps + x.exp0[it.front];
-        const int* __restrict__ ebp = ex + (lower ? 0 : n);
+        const int* __restrict__ ebp = ex + (lower ? 0 : n) + c0;
         const int ea = ex[row] - (S == 8 ? 54 : 36);
-        const int cend = min(cmax, lower ? row + 1 : cmax) - c0;      // columns j < cend are updated
-        T* __restrict__ G = arena<T>(c) + f.off + row + (int64_t)c0 * n;
 #pragma unroll
-        for (int j0 = 0; j0 < 32; j0 += 4) {
+        for (int j0 = 0; j0 < NC; j0 += 4) {
           T cv[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) cv[j] = j0 + j < cend ? __ldcg(G + (int64_t)j * n) : T(0);
+          for (int j = 0; j < 4; ++j) {
+            if constexpr (EARLY) cv[j] = ce[j0 + j];
+            else cv[j] = j0 + j < cend ? __ldcg(G + (int64_t)j * n) : T(0);
+          }
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             if (j0 + j < cend) {
-              const int E = ea + __ldg(ebp + c0 + j0 + j);
+              const int E = ea + __ldg(ebp + j0 + j);
               T d = xs_scaled(acc[j0 + j], E, T(0));
               if (E > XS_BAD / 2) d = T(NAN);
               G[(int64_t)j * n] = cv[j] - d;
@@ -476,7 +587,7 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
   }
 }
 
-template <typename T>
+template <typename T, int BN>
 static void xs_update_t(const DevCtx& c, const XsCtx& x, const CUtensorMap& map, const Item* items, int n_items,
                         int nb, int region, int lower, int* err, cudaStream_t s) {
   static int n_sm = 0;
@@ -486,17 +597,23 @@ static void xs_update_t(const DevCtx& c, const XsCtx& x, const CUtensorMap& map,
     cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
     if (n_sm <= 0) n_sm = 1;
   }
-  cudaFuncSetAttribute(k_xs_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XS_SMEM);
+  cudaFuncSetAttribute(k_xs_update<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XS_SMEM);
   const int grid = n_items < n_sm ? n_items : n_sm;
-  k_xs_update<T><<<grid, XS_THREADS, XS_SMEM, s>>>(c, x, map, items, n_items, nb, region, lower, err);
+  k_xs_update<T, BN><<<grid, XS_THREADS, XS_SMEM, s>>>(c, x, map, items, n_items, nb, region, lower, err);
 }
 
 void launch_xs_update(const DevCtx& c, const XsCtx& x, const CUtensorMap& map, const Item* items, int n_items,
-                      int dtype, int nb, int region, int lower, int* err, cudaStream_t s) {
+                      int dtype, int nb, int region, int lower, int tile_n, int* err, cudaStream_t s) {
   if (!n_items) return;
   if (nb > XS_NBO) throw std::invalid_argument("sliced update: panel wider than 256");
-  if (dtype == F64) xs_update_t<double>(c, x, map, items, n_items, nb, region, lower, err, s);
-  else xs_update_t<float>(c, x, map, items, n_items, nb, region, lower, err, s);
+  if (tile_n != 64 && tile_n != XS_TILE) throw std::invalid_argument("sliced update: tiles are 64 or 128 columns wide");
+  if (dtype == F64) {
+    if (tile_n == 64) xs_update_t<double, 64>(c, x, map, items, n_items, nb, region, lower, err, s);
+    else xs_update_t<double, 128>(c, x, map, items, n_items, nb, region, lower, err, s);
+  } else {
+    if (tile_n == 64) xs_update_t<float, 64>(c, x, map, items, n_items, nb, region, lower, err, s);
+    else xs_update_t<float, 128>(c, x, map, items, n_items, nb, region, lower, err, s);
+  }
 }
 
 }  // namespace uhm_gpu

@@ -7,8 +7,9 @@
 namespace uhm_gpu {
 
 constexpr int XS_NBO = 256;       // outer panel width: columns whose slices share a row exponent at most
-constexpr int XS_TILE = 128;      // update tiles are XS_TILE x XS_TILE
-constexpr int XS_PACK_ROWS = 64;  // rows per pack item
+constexpr int XS_TILE = 128;      // update tiles: XS_TILE rows, XS_TILE or 64 columns
+constexpr int xs_pack_rows(int nb) { return nb == 64 ? 64 : 16; }   // rows per pack item
+constexpr int XS_TRSM_ROWS = 16;  // rows per item of the FP64 panel TRSM
 constexpr int XS_S64 = 8, XS_S32 = 4;   // slices of an FP64 / FP32 front's operands
 constexpr int XS_SPARE_ROWS = 256;      // workspace rows past the last front's (tiles run over)
 
@@ -23,16 +24,19 @@ struct XsCtx {
   int* exps;
 };
 
-// slices of 64 panel rows, columns K0 .. K0 + W, W = min(nb, fs - K0) (item:
+// slices of xs_pack_rows(nb) panel rows, columns K0 .. K0 + W, W = min(nb, fs - K0), nb 64 or XS_NBO (item:
 // front, a = K0, b = first row, c = 0; c = 1: the rows are the front's
 // columns (U12^T: entries (K0 + k, row)), written to the B region)
 void launch_xs_pack(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, int dtype, int nb,
                     cudaStream_t s);
-// C -= A B^T over 128 x 128 tiles (item: front, a = first row, b = first
+// FP64 Cholesky: panel rows times the inverse of the diagonal block and, c = 1,
+// their slices for an update with nb = 64 (item: front, a = k0, b = first row)
+void launch_xs_trsm(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, cudaStream_t s);
+// C -= A B^T over 128 x tile_n tiles (item: front, a = first row, b = first
 // column, c = K0 of the packed columns, W = min(nb, fs - K0)); lower: B is A
 // and only entries col <= row are updated.  region as for k_tile_update: 0
 // every entry, 1 columns below the outer panel's end, 2 rows below it
 void launch_xs_update(const DevCtx& c, const XsCtx& x, const CUtensorMap& map, const Item* items, int n_items,
-                      int dtype, int nb, int region, int lower, int* err, cudaStream_t s);
+                      int dtype, int nb, int region, int lower, int tile_n, int* err, cudaStream_t s);
 
 }  // namespace uhm_gpu
