@@ -57,13 +57,11 @@ int guard(Mesh m, F&& f) {
 }
 
 void account_flops(Mesh m, int method, bool factor) {
-  double dec = 0, sol = 0, buf = 0;
-  unsigned nnz = 0;
-  m->estimate_cost(method, m->datatype, m->n_rhs, dec, sol, nnz, buf);
-  g_flop += factor ? dec : sol;
+  const uhm::Engine::PlanCost& c = m->eng().plan_cost(method);
+  g_flop += factor ? c.dec : c.sol;
   if (factor) {
-    g_buffer = buf;
-    g_buffer_max = std::max(g_buffer_max, buf);
+    g_buffer = c.buf;
+    g_buffer_max = std::max(g_buffer_max, c.buf);
   }
 }
 }  // namespace

@@ -119,6 +119,7 @@ void Engine::free_device() {
 // ---------------------------------------------------------------------------
 void Engine::ensure_plan() {
   if (plan_ok) return;
+  for (PlanCost& c : plan_costs) c.known = false;
   if (!mesh->is_locked()) fail("mesh is not locked", 5);
   fronts.clear();
   levels.clear();
@@ -195,6 +196,17 @@ void Engine::ensure_plan() {
   dev_ok = false;
   factored = false;
   h_x_valid = false;
+}
+
+const Engine::PlanCost& Engine::plan_cost(int method) {
+  ensure_plan();
+  PlanCost& c = plan_costs[method & 7];
+  if (!c.known) {
+    unsigned nnz = 0;
+    mesh->estimate_cost(method, mesh->datatype, mesh->n_rhs, c.dec, c.sol, nnz, c.buf);
+    c.known = true;
+  }
+  return c;
 }
 
 void Engine::release_staging() {

@@ -218,6 +218,14 @@ class Engine {
   int64_t n_global = 0;
   void ensure_plan();
   int method_built = 0;
+  // the mesh's cost estimate for a method (LAWN-41 operations, buffer), a
+  // function of the plan's structure: walked once per plan, not per call (0.28
+  // us per front and call: 2 x 4 ms of a 24^3 step)
+  struct PlanCost {
+    bool known = false;
+    double dec = 0, sol = 0, buf = 0;
+  };
+  const PlanCost& plan_cost(int method);
 
  private:
   Mesh_* mesh;
@@ -330,6 +338,7 @@ class Engine {
   std::vector<int> h_elem_m;
   std::vector<int32_t> h_emap;
   int64_t y_total = 0;
+  PlanCost plan_costs[8];
   std::vector<void*> allocations;
   double anorm_inf = -1.0;
   std::vector<double> h_x;      // cached solution on host
