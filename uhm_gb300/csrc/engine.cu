@@ -1061,8 +1061,7 @@ void Engine::build_programs(int method) {
     if (tiles.empty()) return;
     push(fac_ops, OP_XS_PACK, dt, nb, 0, pk);
     // fewer tiles than SMs: tiles of half the width (a launch is as long as its
-    // slowest CTA; one round of half tiles of K = 64 takes 23 us and two 38,
-    // against 29 and 49 for whole ones)
+    // slowest CTA; one round of half tiles of K = 64 takes 19 us)
     const bool narrow = (int)tiles.size() < n_sm;
     if (narrow) {
       std::vector<Item> h;
@@ -1816,7 +1815,7 @@ void Engine::alloc_device(int method) {
     const size_t bytes = 128 * (size_t)(xs_rows + XS_SPARE_ROWS);
     d_xs = dmalloc(bytes);
     CK(cudaMemsetAsync(d_xs, 0, bytes, stream));     // rows never packed are read by tiles that run over
-    if (!tcc_encode(&xs_map, d_xs, xs_rows + XS_SPARE_ROWS)) fail("tensor map encoding failed", 4);
+    if (!xs_encode(&xs_map, d_xs, xs_rows + XS_SPARE_ROWS)) fail("tensor map encoding failed", 4);
     std::vector<int64_t> v(3 * fronts.size(), 0);
     for (auto& f : fronts)
       if (f.xs) {

@@ -122,6 +122,40 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
+// one lane of the (converged) warp
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t e;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.b32 %0, 1, 0, p;\n}\n" : "=r"(e));
+  return e;
+}
+
+// the low word of a K-major shared-memory descriptor at saddr (sdesc_sw128's
+// high word is SDESC_SW128_HI); 32 bytes further along a row is + 2
+__device__ __forceinline__ uint32_t sdesc_lo(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | 1u << 16; }
+constexpr uint32_t SDESC_SW128_HI = (1024u >> 4) | 1u << 14 | 2u << 29;
+
+// umma_bf16 by the elected lane of a converged warp, descriptors by their low
+// words: the whole warp runs the issue loop, so that its addresses and barriers
+// stay in uniform registers, which the instruction takes its operands from.
+// From one thread's branch every operand is moved there first: the sliced update
+// took 170 clocks per 128 x 128 x 16 MMA that way, 118 so (a kernel whose MMAs
+// wait for HBM, k_tc_chol or k_tc_syrk, gains nothing).
+__device__ __forceinline__ void umma_bf16_w(uint32_t elected, uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t hi,
+                                            uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p, e;\n .reg .b64 da, db;\n setp.ne.b32 e, %0, 0;\n setp.ne.b32 p, %6, 0;\n"
+      " mov.b64 da, {%2, %4};\n mov.b64 db, {%3, %4};\n"
+      " @e tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %5, p;\n}\n" ::"r"(elected),
+      "r"(tmem_d), "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate));
+}
+__device__ __forceinline__ void umma_commit_w(uint32_t elected, uint32_t bar) {
+  asm volatile(
+      "{\n .reg .pred e;\n setp.ne.b32 e, %0, 0;\n"
+      " @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n}\n" ::"r"(elected),
+      "r"(bar)
+      : "memory");
+}
+
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");

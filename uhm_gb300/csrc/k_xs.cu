@@ -30,9 +30,10 @@
 // measured for the SIMT update), against 1,906 TFLOP/s of BF16 products:
 // 36 products per FP64 one still leave 53.  FP32 fronts: 10 products leave
 // 190 TFLOP/s against 15 measured for the SIMT update.  Measured on GB300, the
-// updates of one factorisation: 16^3 p = 4 FP64 906 -> 46 ms (and 6 for the
-// slices), 13^3 p = 4 FP32 23.0 -> 7.9 (2.9), 12^3 p = 3 FP64 LU 196 -> 14.5 (3.3).
+// updates of one factorisation: 16^3 p = 4 FP64 906 -> 34.5 ms (and 2.3 for the
+// slices), 13^3 p = 4 FP32 23.0 -> 6.5 (2.0), 12^3 p = 3 FP64 LU 196 -> 10.3 (2.7).
 #include <cuda.h>
+#include <cudaTypedefs.h>
 
 #include <stdexcept>
 
@@ -114,7 +115,7 @@ __device__ __forceinline__ void xs_digits(long long X, uint32_t (&d)[S]) {
 
 // A CTA cuts 256 / NG rows: thread r + (256 / NG) g holds 16 columns 16 g .. of
 // row r (a warp's loads of one column are consecutive rows), all its loads in
-// flight, and writes each slice's 16 digits as one whole 32-byte sector.  NG =
+// flight, and writes its digits as one or two whole rows of the workspace.  NG =
 // 4 (64 columns) or 16 (256).  Memory bound: 8 (4) bytes read and 16 (8)
 // written per entry; the digits come from integer shifts and byte extraction,
 // no FP64.  Measured on GB300 for 256 columns: 29 us with 64 rows per CTA and
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(256) k_xs_pack(DevCtx c, XsCtx x, const Item* 
   const bool bad = fm == XsType<T>::FMAX;
   if (g == 0) x.exps[x.exp0[it.front] + (trans ? n : 0) + row] = bad ? XS_BAD : fm - XsType<T>::EBIAS;
   uint8_t* const w0 = reinterpret_cast<uint8_t*>(x.ws) +
-                      128 * ((trans ? x.row0b : x.row0)[it.front] + (int64_t)(g >> 2) * n + row) + 32 * (g & 3);
+                      128 * ((trans ? x.row0b : x.row0)[it.front] + (int64_t)g * n + row);
   uint32_t d[S][8];
 #pragma unroll
   for (int u = 0; u < 16; u += 2) {
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(256) k_xs_pack(DevCtx c, XsCtx x, const Item* 
   }
 #pragma unroll
   for (int p = 0; p < S; ++p) {
-    uint4* w = reinterpret_cast<uint4*>(w0 + 128 * (int64_t)(p * nch) * n);
+    uint4* w = reinterpret_cast<uint4*>(w0 + 128 * (int64_t)((p >> 2) * 4 * nch) * n + 32 * (p & 3));
     w[0] = make_uint4(d[p][0], d[p][1], d[p][2], d[p][3]);
     w[1] = make_uint4(d[p][4], d[p][5], d[p][6], d[p][7]);
   }
@@ -248,10 +249,11 @@ __global__ void __launch_bounds__(256) k_xs_trsm64(DevCtx c, XsCtx x, const Item
   uint32_t d[4][S];
 #pragma unroll
   for (int e = 0; e < 4; ++e) xs_digits<S>(bad ? 0 : XsType<double>::fixed(Xs[c4 + e][r], fm), d[e]);
-  uint8_t* const w0 = reinterpret_cast<uint8_t*>(x.ws) + 128 * (x.row0[it.front] + row) + 2 * c4;
+  uint8_t* const w0 =
+      reinterpret_cast<uint8_t*>(x.ws) + 128 * (x.row0[it.front] + (int64_t)(c4 >> 4) * n + row) + 2 * (c4 & 15);
 #pragma unroll
   for (int p = 0; p < S; ++p)
-    *reinterpret_cast<uint2*>(w0 + 128 * (int64_t)p * n) =
+    *reinterpret_cast<uint2*>(w0 + 128 * (int64_t)((p >> 2) * 4) * n + 32 * (p & 3)) =
         make_uint2(__byte_perm(d[0][p], d[1][p], 0x7632), __byte_perm(d[2][p], d[3][p], 0x7632));
 }
 
@@ -265,9 +267,9 @@ void launch_xs_trsm(const DevCtx& c, const XsCtx& x, const Item* items, int n_it
 // ---------------------------------------------------------------------------
 constexpr int XS_EPI_WARPS = 16;
 constexpr int XS_THREADS = 32 * (XS_EPI_WARPS + 2);     // epilogue warps, TMA producer, MMA issuer
-constexpr uint32_t XS_BOX = 128 * 64;                   // 128 rows of 32 BF16 = 8 KB
-constexpr uint32_t XS_SLOT = 2 * XS_BOX;                // one slice of A and of B, 32 columns
-constexpr int XS_SLOTS = 14;
+constexpr uint32_t XS_BOX = 128 * 128;                  // 128 rows of four slices x 16 columns = 16 KB
+constexpr uint32_t XS_SLOT = 2 * XS_BOX;                // four slices of A and of B, 16 columns
+constexpr int XS_SLOTS = 7;
 constexpr uint32_t XS_SMEM = 1024 + XS_SLOTS * XS_SLOT + 512;
 
 #define XS_LD16(taddr, v)                                                                        \
@@ -318,19 +320,22 @@ __device__ __forceinline__ float xs_scaled(long long a, int E, float) {
   return x * __int_as_float((127 + e1) << 23) * __int_as_float((127 + e2) << 23);
 }
 
-// Persistent: one CTA per SM walks the 128 x 128 tiles.  Warp 16 loads one
-// slice of A and B (32 columns, 64-byte swizzle) per ring slot, one thread of
-// warp 17 issues the products of a chunk as soon as its slices are there,
+// Persistent: one CTA per SM walks the 128 x 128 tiles.  Warp 16 loads four
+// slices of A and B (16 columns, 128-byte swizzle) per ring slot, one thread of
+// warp 17 issues the products of a chunk,
 // warps 0..15 (a lane quarter and 32 columns each) take the accumulators to
 // 64-bit integers in registers while the next pass runs, then update C
 // (column by column: a warp's loads and stores are 32 consecutive rows).
-// 14 slots of 16 KB.  BN = 64: tiles of half the width
+// Seven slots of 32 KB.  The four slices share
+// 128-byte rows because TMA takes a row at a time: with 32-byte rows a tile of K =
+// 256 took 64 us, with 64- and 128-byte ones 42, with the converged issue loop
+// (umma_bf16_w) 30; the tensor pipe alone needs 18.  BN = 64: tiles of half the width
 // for launches with fewer 128 x 128 tiles than SMs, where a tile's own time
 // counts: half the products and half the FP64 additions of the epilogue, whose C
 // entries are loaded while the products run.  Bound: tensor pipe / shared-memory
 // reads of the 128 x 128 products; a tile of a small launch by its epilogue.
 // Measured on GB300 for up to 80 tiles
-// of K = 64 (256): 29 (60) -> 23 (50) us.
+// of K = 64 (256): 29 (60) us with whole tiles, 19 (35) with these.
 template <typename T, int BN>
 __global__ void __launch_bounds__(XS_THREADS, 1)
 k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const Item* __restrict__ items, int n_items,
@@ -381,11 +386,11 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
         const Item it = items[t];
         const FrontDev f = c.fronts[it.front];
         const int n = f.n, nch = xs_chunks(nb, f.fs);
-        const int nk = (min(nb, f.fs - it.c) + 31) / 32;
+        const int nk = (min(nb, f.fs - it.c) + 15) / 16;
         const int64_t ya = x.row0[it.front] + it.a;
         const int64_t yb = (lower ? x.row0[it.front] : x.row0b[it.front]) + it.b;
         for (int pass = S == 8 ? 0 : 1; pass < 2 && live; ++pass) {
-          const int np = pass == 0 ? S : 4;
+          const int np = pass == 0 ? 2 : 1;      // groups of four slices
           for (int k = 0; k < nk && live; ++k)
             for (int p = 0; p < np; ++p) {
               if (issued >= XS_SLOTS &&
@@ -395,9 +400,9 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
               }
               const uint32_t fb = smem_u32(&bars[s]), st = smem_u32(smem + s * XS_SLOT);
               mbar_expect_tx(fb, XS_SLOT);
-              const int64_t dr = (int64_t)(p * nch + (k >> 1)) * n;
-              tma_load_2d(st, &wsmap, 32 * (k & 1), (int)(ya + dr), fb);
-              tma_load_2d(st + XS_BOX, &wsmap, 32 * (k & 1), (int)(yb + dr), fb);
+              const int64_t dr = (int64_t)(p * 4 * nch + k) * n;
+              tma_load_2d(st, &wsmap, 0, (int)(ya + dr), fb);
+              tma_load_2d(st + XS_BOX, &wsmap, 0, (int)(yb + dr), fb);
               ++issued;
               if (++s == XS_SLOTS) { s = 0; ph ^= 1; }
             }
@@ -409,94 +414,81 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
         mbar_drain(smem_u32(&bars[q % XS_SLOTS]), (q / XS_SLOTS) & 1);
     }
   } else if (warp == XS_EPI_WARPS + 1) {
-    if (lane == 0) {
-      // MMA issuer
-      const uint32_t idesc = idesc_bf16_f32(XS_TILE, BN);
-      const uint32_t ring = smem_u32(smem);
-      int s = 0;
-      uint32_t ph = 0;               // parity of the full wait at slot s
-      uint32_t use[4] = {0, 0, 0, 0};
-      bool live = true;
-      // the products of diagonals D0..D1 of one chunk: NP slices from slot s
-      auto wait_slot = [&](int p) {
-        int q = s + p;
-        uint32_t qp = ph;
-        if (q >= XS_SLOTS) { q -= XS_SLOTS; qp ^= 1; }
-        return mbar_wait_lim(smem_u32(&bars[q]), qp, s_abort, err, XS_ERR, lim);
-      };
-      auto slot_addr = [&](int p) {
-        int q = s + p;
-        if (q >= XS_SLOTS) q -= XS_SLOTS;
-        return ring + (uint32_t)q * XS_SLOT;
-      };
-      auto diag = [&](auto dd, bool first) {
-        constexpr int d = decltype(dd)::value, a = d & 3, np = d >= 4 ? S : 4;
-        if (first) {
-          if (use[a] >= 1 &&
-              !mbar_wait_lim(smem_u32(&acc_empty[a]), (use[a] - 1) & 1, s_abort, err, XS_ERR, lim))
-            return false;
+    // MMA issuer: the whole warp, one elected lane issuing
+    const uint32_t elected = elect_one();
+    const uint32_t idesc = idesc_bf16_f32(XS_TILE, BN);
+    const uint32_t ring = smem_u32(smem), bar0 = smem_u32(bars), acc_bar = smem_u32(acc_full);
+    int s = 0;
+    uint32_t ph = 0;               // parity of the full wait at slot s
+    uint32_t used = 0, par = 0;    // bit a: accumulator a has been used / parity of its next reuse
+    bool live = true;
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbar_wait_lim(bar, parity, s_abort, err, XS_ERR, lim)) != 0;
+    };
+    // the products of diagonal d of one chunk, slices 0..3 in slot s0 and 4..7 in s1
+    auto diag = [&](auto dd, uint32_t s0, uint32_t s1, int k, int nk) {
+      constexpr int d = decltype(dd)::value, a = d & 3, np = d >= 4 ? S : 4;
+      if (k == 0) {
+        if ((used >> a) & 1) {
+          if (!wait(acc_bar + 8 * (4 + a), (par >> a) & 1)) return false;
+          par ^= 1u << a;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
-        const uint32_t acc = tmem + a * XS_TILE;
-        uint32_t on = first ? 0u : 1u;
-#pragma unroll
-        for (int p = 0; p <= d; ++p) {
-          const int q = d - p;
-          if (p >= np || q >= np) continue;
-          const uint32_t A = slot_addr(p), B = slot_addr(q) + XS_BOX;
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            umma_bf16(acc, sdesc_sw64(A + k * 32), sdesc_sw64(B + k * 32), idesc, on);
-            on = 1u;
-          }
-        }
-        return true;
-      };
-      auto release = [&](int np) {
-        for (int p = 0; p < np; ++p) {
-          int q = s + p;
-          if (q >= XS_SLOTS) q -= XS_SLOTS;
-          umma_commit(smem_u32(&empty[q]));
-        }
-        s += np;
-        if (s >= XS_SLOTS) { s -= XS_SLOTS; ph ^= 1; }
-      };
-      auto finish = [&](int a) {
-        umma_commit(smem_u32(&acc_full[a]));
-        ++use[a];
-      };
-      for (int t = blockIdx.x; t < n_items && live; t += gridDim.x) {
-        const Item it = items[t];
-        const int nk = (min(nb, c.fronts[it.front].fs - it.c) + 31) / 32;
-        // a chunk's products, each diagonal once its last slice has arrived
-        auto step = [&](auto dd, bool first) {
-          if (!wait_slot(decltype(dd)::value)) return false;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          return diag(dd, first);
-        };
-        if constexpr (S == 8) {
-          for (int k = 0; k < nk && live; ++k) {
-            for (int p = 0; p < 4 && live; ++p) live = wait_slot(p);
-            live = live && step(std::integral_constant<int, 4>{}, k == 0) &&
-                   step(std::integral_constant<int, 5>{}, k == 0) && step(std::integral_constant<int, 6>{}, k == 0) &&
-                   step(std::integral_constant<int, 7>{}, k == 0);
-            if (live) release(8);
-          }
-          if (live)
-            for (int a = 0; a < 4; ++a) finish(a);
-        }
-        for (int k = 0; k < nk && live; ++k) {
-          live = step(std::integral_constant<int, 0>{}, k == 0) && step(std::integral_constant<int, 1>{}, k == 0) &&
-                 step(std::integral_constant<int, 2>{}, k == 0) && step(std::integral_constant<int, 3>{}, k == 0);
-          if (live) release(4);
-        }
-        if (live)
-          for (int a = 0; a < 4; ++a) finish(a);
+        used |= 1u << a;
       }
-      // every MMA issued has completed before tensor memory is freed
-      umma_commit(smem_u32(drain_bar));
-      mbar_drain(smem_u32(drain_bar), 0);
+      const uint32_t acc = tmem + a * XS_TILE;
+      uint32_t on = k == 0 ? 0u : 1u;
+#pragma unroll
+      for (int p = 0; p <= d; ++p) {
+        const int q = d - p;
+        if (p >= np || q >= np) continue;
+        umma_bf16_w(elected, acc, (p < 4 ? s0 : s1) + 2 * (p & 3), (q < 4 ? s0 : s1) + (XS_BOX >> 4) + 2 * (q & 3),
+                    SDESC_SW128_HI, idesc, on);
+        on = 1u;
+      }
+      // the last chunk hands each accumulator over as soon as its diagonal is
+      // issued, so that the epilogue reads one while the others fill
+      if (k == nk - 1) umma_commit_w(elected, acc_bar + 8 * a);
+      return true;
+    };
+    auto lo_of = [&](int q) { return sdesc_lo(ring + (uint32_t)q * XS_SLOT); };
+    for (int t = blockIdx.x; t < n_items && live; t += gridDim.x) {
+      const Item it = items[t];
+      const int nk = __shfl_sync(0xffffffffu, (min(nb, c.fronts[it.front].fs - it.c) + 15) / 16, 0);
+      if constexpr (S == 8) {
+        for (int k = 0; k < nk && live; ++k) {
+          const int q = s + 1 == XS_SLOTS ? 0 : s + 1;
+          const uint32_t qp = q ? ph : ph ^ 1;
+          live = wait(bar0 + 8 * s, ph) && wait(bar0 + 8 * q, qp);
+          if (!live) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t s0 = lo_of(s), s1 = lo_of(q);
+          live = diag(std::integral_constant<int, 4>{}, s0, s1, k, nk) &&
+                 diag(std::integral_constant<int, 5>{}, s0, s1, k, nk) &&
+                 diag(std::integral_constant<int, 6>{}, s0, s1, k, nk) &&
+                 diag(std::integral_constant<int, 7>{}, s0, s1, k, nk);
+          umma_commit_w(elected, bar0 + 8 * (XS_SLOTS + s));
+          umma_commit_w(elected, bar0 + 8 * (XS_SLOTS + q));
+          s = q + 1 == XS_SLOTS ? 0 : q + 1;
+          ph = s ? qp : qp ^ 1;
+        }
+      }
+      for (int k = 0; k < nk && live; ++k) {
+        live = wait(bar0 + 8 * s, ph);
+        if (!live) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t s0 = lo_of(s);
+        live = diag(std::integral_constant<int, 0>{}, s0, s0, k, nk) &&
+               diag(std::integral_constant<int, 1>{}, s0, s0, k, nk) &&
+               diag(std::integral_constant<int, 2>{}, s0, s0, k, nk) &&
+               diag(std::integral_constant<int, 3>{}, s0, s0, k, nk);
+        umma_commit_w(elected, bar0 + 8 * (XS_SLOTS + s));
+        if (++s == XS_SLOTS) { s = 0; ph ^= 1; }
+      }
     }
+    // every MMA issued has completed before tensor memory is freed
+    umma_commit_w(elected, smem_u32(drain_bar));
+    mbar_drain(smem_u32(drain_bar), 0);
   } else {
     // epilogue
     constexpr int NC = BN / 4;       // columns per thread
@@ -585,6 +577,27 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
   if (warp == 0) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
   }
+}
+
+bool xs_encode(CUtensorMap* map, void* base, int64_t rows) {
+  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+  if (!encode) {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess || !fn) {
+      cudaGetLastError();
+      return false;
+    }
+    encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+  }
+  cuuint64_t dims[2] = {64, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {128};
+  cuuint32_t box[2] = {64, 128};
+  cuuint32_t estr[2] = {1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <typename T, int BN>

@@ -13,7 +13,8 @@ constexpr int XS_TRSM_ROWS = 16;  // rows per item of the FP64 panel TRSM
 constexpr int XS_S64 = 8, XS_S32 = 4;   // slices of an FP64 / FP32 front's operands
 constexpr int XS_SPARE_ROWS = 256;      // workspace rows past the last front's (tiles run over)
 
-// Where the operand slices live: 128-byte rows of 64 BF16, per front first
+// Where the operand slices live: 128-byte rows of four slices x 16 columns (BF16),
+// row ((group of slices) (16-column chunks) + chunk) n + r, per front first
 // row row0[front] (A and, Cholesky, B) and row0b[front] (LU: B = U12^T), one
 // exponent per front row at exp0[front] / exp0 + nb_off.
 struct XsCtx {
@@ -24,6 +25,8 @@ struct XsCtx {
   int* exps;
 };
 
+// 2D map over the workspace's 128-byte rows: box 128 rows, 128-byte swizzle
+bool xs_encode(CUtensorMap* map, void* base, int64_t rows);
 // slices of xs_pack_rows(nb) panel rows, columns K0 .. K0 + W, W = min(nb, fs - K0), nb 64 or XS_NBO (item:
 // front, a = K0, b = first row, c = 0; c = 1: the rows are the front's
 // columns (U12^T: entries (K0 + k, row)), written to the B region)
