@@ -1,5 +1,5 @@
 """Schur complements and solutions of blocked fronts (too large for one CTA's
-shared memory) against 64-bit numpy, at sizes around the kernels' edges:
+shared memory), and of small ones, against 64-bit numpy, at sizes around the kernels' edges:
 64-column steps, 256-column outer panels, 128 x 128 update tiles, 16-column
 row blocks.
 
@@ -123,3 +123,25 @@ def test_non_finite_front_reports_status(native_lib, value):
     with pytest.raises(api.UHMError) as ei:
         m.chol_with_free()
     assert ei.value.code == 13
+
+
+@pytest.mark.parametrize("n_rhs", [1, 3, 4, 9])
+@pytest.mark.parametrize("prec,fs,ss", [("fp64", 1, 5), ("fp64", 5, 3), ("fp64", 62, 98), ("fp64", 97, 30),
+                                        ("fp32", 30, 1), ("fp32", 131, 93)])
+def test_small_cholesky_front(native_lib, prec, fs, ss, n_rhs):
+    """Fronts that fit one CTA: four-column steps with remainders, and the solves
+    by whole blocks (up to three right-hand sides) or a warp each."""
+    m, leaves, mats, rhs = _mesh(fs, ss, True, 300 + fs, n_rhs)
+    if prec == "fp32":
+        m.set_mode(1, api.PREC_FP32, 1e-12, 10)
+    m.factor(uo.CHOL)
+    eid = m.fronts()[0]
+    for k in range(2):
+        a = mats[k]
+        exact = np.tril(a[fs:, fs:] - a[fs:, :fs] @ np.linalg.solve(a[:fs, :fs], a[:fs, fs:]))
+        d = np.abs(np.diag(a)[fs:])
+        got = m.front_block(int(eid[k]), "ABR")
+        assert (np.abs(got - exact) <= 25 * (fs + 8) * U[prec] * np.sqrt(np.outer(d, d))).all(), k
+    m.solve(uo.CHOL)
+    x, ref = _solutions(m, fs, ss, mats, rhs)
+    assert np.abs(x - ref).max() <= 3e-10 * np.abs(ref).max()

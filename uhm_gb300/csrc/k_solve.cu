@@ -144,52 +144,86 @@ __global__ void __launch_bounds__(NT) k_fwd_small(DevCtx c, const Item* __restri
 
 // Cholesky small fronts with the factor panel (n x fs) staged in shared
 // memory by one batch of loads: every column step then works on shared data
-// (one barrier per column instead of a global round trip per column).  The
-// right-hand sides are solved in the factor's precision (as in the
-// flag-driven solves of large fronts): FP32 fronts take no FP64 arithmetic,
-// which runs at a small fraction of the FP32 rate on this GPU.
+// (no global round trip per column).  The right-hand sides are solved in the
+// factor's precision (as in the flag-driven solves of large fronts): FP32
+// fronts take no FP64 arithmetic, which runs at a small fraction of the FP32 rate
+// on this GPU.  The pivots' reciprocals are formed once, all at a time (a
+// division per column was most of an FP64 step); the solved entries are scaled by them
+// where they are used.  From WARP_RHS right-hand sides on each warp takes its own
+// ones and no block barrier is left in the sweep; below, the block shares
+// the rows and crosses one per column.  Measured on GB300: 125-row FP64 front,
+// one right-hand side, forward 121 -> 35 us, backward 172 -> 31 (its panel now
+// staged too); 4,096 fronts of 125 (27) 106 -> 77 and 240 -> 68; 12 meshes, 16
+// right-hand sides, FP32 1.08 -> 0.80 ms and 1.95 -> 1.03.
+constexpr int WARP_RHS = 4;
+
+// the front's factor columns into Ls (n x fs), the reciprocals of its pivots
+// into rd, the slab v (n x n_rhs) into z
+template <typename T, int NT>
+__device__ __forceinline__ void small_stage(const T* __restrict__ G, const double* __restrict__ v, int n, int fs,
+                                            int nr, T* z, T* rd, T* Ls) {
+  const int tot = n * fs;
+  for (int i0 = 0; i0 < tot; i0 += 8 * NT) {
+    T x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int idx = i0 + threadIdx.x + u * NT;
+      x[u] = idx < tot ? G[idx] : T(0);        // columns 0..fs-1 are contiguous (ld n)
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int idx = i0 + threadIdx.x + u * NT;
+      if (idx < tot) Ls[idx] = x[u];
+    }
+  }
+  for (int idx = threadIdx.x; idx < n * nr; idx += NT) z[idx] = (T)v[idx];
+  for (int j = threadIdx.x; j < fs; j += NT) rd[j] = T(1) / G[j + (int64_t)j * n];
+  __syncthreads();
+}
+
+// this thread's right-hand sides q0, q0 + qs, .. and rows i0, i0 + is, .. of a sweep
+struct SmallShare {
+  int q0, qs, i0, is;
+  bool warp;
+  __device__ __forceinline__ SmallShare(int nr, int nt) {
+    warp = nr >= WARP_RHS;
+    q0 = warp ? threadIdx.x >> 5 : 0;
+    qs = warp ? nt / 32 : 1;
+    i0 = warp ? threadIdx.x & 31 : threadIdx.x;
+    is = warp ? 32 : nt;
+  }
+  __device__ __forceinline__ void sync() const {
+    if (warp) __syncwarp();
+    else __syncthreads();
+  }
+};
+
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_fwd_small_staged(DevCtx c, const Item* __restrict__ items) {
-  using CT = T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, fs = f.fs, nr = c.n_rhs;
-  CT* z = reinterpret_cast<CT*>(smem_raw);
-  T* Ls = z + (size_t)n * nr;
-  const T* __restrict__ G = arena<T>(c) + f.off;
+  T* z = reinterpret_cast<T*>(smem_raw);
+  T* rd = z + (size_t)n * nr;
+  T* Ls = rd + fs;
   double* __restrict__ zg = c.vec + f.voff;
-  const int tot = n * fs;
-  for (int i0 = 0; i0 < tot; i0 += 8 * NT) {
-    T v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int idx = i0 + threadIdx.x + u * NT;
-      v[u] = idx < tot ? G[idx] : T(0);        // columns 0..fs-1 are contiguous (ld n)
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int idx = i0 + threadIdx.x + u * NT;
-      if (idx < tot) Ls[idx] = v[u];
+  small_stage<T, NT>(arena<T>(c) + f.off, zg, n, fs, nr, z, rd, Ls);
+  const SmallShare sh(nr, NT);
+  for (int q = sh.q0; q < nr; q += sh.qs) {
+    T* zq = z + q * n;
+    for (int j = 0; j < fs; ++j) {
+      const T zj = zq[j] * rd[j];
+      const T* col = Ls + j * n;
+      for (int i = j + 1 + sh.i0; i < n; i += sh.is) zq[i] -= col[i] * zj;
+      sh.sync();
     }
   }
-  for (int idx = threadIdx.x; idx < n * nr; idx += NT) z[idx] = (CT)zg[idx];
   __syncthreads();
-  for (int j = 0; j < fs; ++j) {
-    if (threadIdx.x < nr) z[j + threadIdx.x * n] /= (CT)Ls[j + j * n];
-    __syncthreads();
-    const int h = n - j - 1;
-    for (int q = 0; q < nr; ++q) {
-      const CT zj = z[j + q * n];
-      for (int i = j + 1 + threadIdx.x; i < n; i += NT) z[i + q * n] -= (CT)Ls[i + j * n] * zj;
-    }
-    (void)h;
-    __syncthreads();
-  }
   double* __restrict__ yg = zg + (int64_t)n * nr;
   for (int q = 0; q < nr; ++q)
     for (int i = threadIdx.x; i < n; i += NT) {
-      if (i < fs) yg[i + (int64_t)q * n] = (double)z[i + q * n];
+      if (i < fs) yg[i + (int64_t)q * n] = (double)(z[i + q * n] * rd[i]);
       else zg[i + (int64_t)q * n] = (double)z[i + q * n];
     }
 }
@@ -199,50 +233,39 @@ __global__ void __launch_bounds__(NT) k_fwd_small_staged(DevCtx c, const Item* _
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_bwd_small_staged(DevCtx c, const Item* __restrict__ items,
                                                          double* __restrict__ g, int64_t ldg) {
-  using CT = T;                       // the factor's precision, as in the forward sweep
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, fs = f.fs, nr = c.n_rhs;
-  CT* z = reinterpret_cast<CT*>(smem_raw);
-  CT* w = z + (size_t)n * nr;
-  T* Ls = w + fs;
-  const T* __restrict__ G = arena<T>(c) + f.off;
-  double* __restrict__ zg = c.vec + f.voff + (int64_t)n * nr;   // y slab
-  const int tot = n * fs;
-  for (int i0 = 0; i0 < tot; i0 += 8 * NT) {
-    T v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int idx = i0 + threadIdx.x + u * NT;
-      v[u] = idx < tot ? G[idx] : T(0);
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int idx = i0 + threadIdx.x + u * NT;
-      if (idx < tot) Ls[idx] = v[u];
-    }
-  }
-  for (int idx = threadIdx.x; idx < n * nr; idx += NT) z[idx] = (CT)zg[idx];
-  __syncthreads();
-  for (int q = 0; q < nr; ++q) {
-    CT* zq = z + q * n;
-    for (int j = threadIdx.x; j < fs; j += NT) {
-      CT sacc = CT(0);
+  T* z = reinterpret_cast<T*>(smem_raw);
+  T* rd = z + (size_t)n * nr;
+  T* Ls = rd + fs;
+  const double* __restrict__ yg = c.vec + f.voff + (int64_t)n * nr;   // y slab
+  small_stage<T, NT>(arena<T>(c) + f.off, yg, n, fs, nr, z, rd, Ls);
+  const SmallShare sh(nr, NT);
+  for (int q = sh.q0; q < nr; q += sh.qs) {
+    T* zq = z + q * n;
+    for (int j = sh.i0; j < fs; j += sh.is) {
+      T s0 = T(0), s1 = T(0);
       const T* col = Ls + (size_t)j * n;
-      for (int i = fs; i < n; ++i) sacc += (CT)col[i] * zq[i];
-      w[j] = zq[j] - sacc;
+      int i = fs;
+      for (; i + 1 < n; i += 2) {
+        s0 += col[i] * zq[i];
+        s1 += col[i + 1] * zq[i + 1];
+      }
+      if (i < n) s0 += col[i] * zq[i];
+      zq[j] -= s0 + s1;
     }
-    __syncthreads();
-    for (int j = fs - 1; j >= 0; --j) {
-      const CT xj = w[j] / (CT)Ls[j + j * n];
-      for (int i = threadIdx.x; i < j; i += NT) w[i] -= (CT)Ls[j + i * n] * xj;
-      if (threadIdx.x == 0) zq[j] = xj;
-      __syncthreads();
+    sh.sync();
+    for (int j = fs - 1; j > 0; --j) {
+      const T xj = zq[j] * rd[j];
+      for (int i = sh.i0; i < j; i += sh.is) zq[i] -= Ls[j + i * n] * xj;
+      sh.sync();
     }
   }
+  __syncthreads();
   for (int q = 0; q < nr; ++q)
-    for (int i = threadIdx.x; i < fs; i += NT) g[(f.g0 + i) + q * ldg] = (double)z[i + q * n];
+    for (int i = threadIdx.x; i < fs; i += NT) g[(f.g0 + i) + q * ldg] = (double)(z[i + q * n] * rd[i]);
 }
 
 void launch_fwd_small(const DevCtx& c, const Item* items, int n_items, int dtype, int method,
