@@ -584,108 +584,161 @@ __global__ void __launch_bounds__(256) k_potrf_diag(DevCtx c, const Item* __rest
 // TRSM use nothing else), and no multiply-add is spent on zeros.  GB300 does
 // about 2 FP64 multiply-adds per clock per SM, so a warp instruction costs its
 // scheduler ~64 clocks whatever its lanes do: the block is bound by their
-// count.  Tile (i, j), i >= j, of the 16 x 16 lower tiles (4 x 4 entries)
+// count and by the chain of pivots.  Tile (i, j), i >= j, of the 16 x 16 lower tiles (4 x 4 entries)
 // holds A until step j and X = L^{-1} after it; either way step q < i takes
 // the one rank-4 update  t -= L[tile i, q] B[:, tile j],  B[m][c] = L(c, P+m)
 // right of the pivot columns P .. P+3 (j > q) and X(P+m, c) left of them (j
-// <= q): 2 x 136 half tiles on 9 warps, in order of i, so that finished rows
-// leave whole warps idle.  The step's 64 vectors (rows of A below the pivot,
-// columns of X) take the same 4-step substitution, one thread each: warps 9
-// and 10 factor the pivot block (every thread) and solve them.  Measured on
-// GB300: 294 -> 67 us per block against the tile-per-thread form (k_potrf_diag),
-// which updates the full squares.
-constexpr int PD_BULK = 288, PD_THREADS = PD_BULK + 64;
+// <= q): 2 x 136 half tiles on 9 warps.  The step's 64 vectors (rows of A from
+// the pivot on, columns of X) take the same 4-step substitution, one thread each of
+// two solver warps, which factor the pivot block (every thread) as well.
+// The solvers run one step ahead: their vectors leave the tiles before the
+// update of the step before, which the solvers apply themselves, so that pivots
+// and bulk updates overlap; they hand over on named barriers.  The bulk warps
+// are spread so that the schedulers of the solver warps take fewer of them.
+// Measured on GB300: 294 us per block in the tile-per-thread form
+// (k_potrf_diag), which updates the full squares; 67 with the steps in
+// turn; 60 so (the solvers' chain of dependent FP64 operations, ~45 a step).
+constexpr int PD_BULK_WARPS = 9, PD_THREADS = 12 * 32;
+constexpr int PD_ALL = 32 * (PD_BULK_WARPS + 2);      // threads of a hand-over barrier
+// role of each warp: bulk chunk 0 .. 8 (tiles in order of i: the last chunks work
+// longest), 16 / 17 solver, -1 none; a warp's scheduler is its index mod 4
+__device__ __constant__ signed char pd_role[12] = {8, 2, 1, 7, 6, 0, -1, 5, 4, 16, 17, 3};
+
+__device__ __forceinline__ void pd_arrive(int id) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(PD_ALL) : "memory");
+}
+__device__ __forceinline__ void pd_sync(int id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(PD_ALL) : "memory");
+}
 
 __global__ void __launch_bounds__(PD_THREADS) k_potrf_inv64(DevCtx c, const Item* __restrict__ items) {
-  __shared__ __align__(16) double V[4][64], B[4][64];
+  __shared__ __align__(16) double V[2][4][64], B[2][4][64];
+  __shared__ double pv[4][4];
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, k0 = it.a;
   const int kb = min(64, f.fs - k0);
-  const double* __restrict__ G = c.a64 + f.off + k0 + (int64_t)k0 * n;
-  double* __restrict__ D = c.dinv64 + f.dinv_off + (int64_t)(k0 / 64) * 4096;
-  const int tid = threadIdx.x;
-  int i = -1, j = -1;                       // this thread's tile (none: i = -1)
-  if (tid < 2 * 136) {
-    const int t = tid >> 1;
-    i = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
-    while (i * (i + 1) / 2 > t) --i;
-    while ((i + 1) * (i + 2) / 2 <= t) ++i;
-    j = t - i * (i + 1) / 2;
-  }
-  const int r0 = 4 * i, c0 = 4 * j + 2 * (tid & 1);   // rows r0 .. r0+3, columns c0, c0+1
-  double a[4][2];
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 2; ++v) {
-      const int r = r0 + u, cc = c0 + v;
-      a[u][v] = i < 0 || r < cc ? 0.0 : (r < kb && cc < kb) ? G[r + (int64_t)cc * n] : (r == cc ? 1.0 : 0.0);
+  const int role = pd_role[threadIdx.x >> 5], lane = threadIdx.x & 31;
+  // barriers: 1 the solvers; 2, 3 vectors of step q (q mod 2) published; 4, 5 B of step q written
+  if (role >= 0 && role < 16) {
+    const double* __restrict__ G = c.a64 + f.off + k0 + (int64_t)k0 * n;
+    const int unit = 32 * role + lane;
+    int i = -1, j = -1;                       // this thread's tile (none: i = -1)
+    if (unit < 2 * 136) {
+      const int t = unit >> 1;
+      i = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
+      while (i * (i + 1) / 2 > t) --i;
+      while ((i + 1) * (i + 2) / 2 <= t) ++i;
+      j = t - i * (i + 1) / 2;
     }
-  bool bad = false;
+    const int r0 = 4 * i, c0 = 4 * j + 2 * (unit & 1);   // rows r0 .. r0+3, columns c0, c0+1
+    double a[4][2];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        const int r = r0 + u, cc = c0 + v;
+        a[u][v] = i < 0 || r < cc ? 0.0 : (r < kb && cc < kb) ? G[r + (int64_t)cc * n] : (r == cc ? 1.0 : 0.0);
+      }
+    // the vectors of step q leave the tiles of column q (A) and row q (X)
+    auto publish = [&](int q) {
+      double (*v)[64] = V[q & 1];
+      if (i >= q && j == q) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) Vec4<double>::st(&v[c0 + e - 4 * q][r0], {a[0][e], a[1][e], a[2][e], a[3][e]});
+      } else if (i == q && j < q - 1) {       // (column q - 1 starts at zero)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) *reinterpret_cast<double2*>(&v[u][c0]) = make_double2(a[u][0], a[u][1]);
+      }
+    };
+    publish(0);
+    publish(1);
+    pd_arrive(2);
 #pragma unroll 1
-  for (int q = 0; q < 16; ++q) {
-    const int P = 4 * q;
-    if (i >= q && j == q) {                 // A below (and on) the pivot columns
+    for (int q = 0; q < 14; ++q) {
+      pd_sync(4 + (q & 1));
+      if (i > q + 1 && j != q + 1) {
+        const double (*b)[64] = B[q & 1];
+        if (j == q) {
 #pragma unroll
-      for (int v = 0; v < 2; ++v) Vec4<double>::st(&V[c0 + v - P][r0], {a[0][v], a[1][v], a[2][v], a[3][v]});
-    } else if (i == q) {                    // X in the pivot rows
+          for (int u = 0; u < 4; ++u) a[u][0] = a[u][1] = 0.0;
+        }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) *reinterpret_cast<double2*>(&V[u][c0]) = make_double2(a[u][0], a[u][1]);
+        for (int m = 0; m < 4; ++m) {
+          double l[4];
+          Vec4<double>::ld(&b[m][r0], l);
+          const double2 x = *reinterpret_cast<const double2*>(&b[m][c0]);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            a[u][0] -= l[u] * x.x;
+            a[u][1] -= l[u] * x.y;
+          }
+        }
+      }
+      publish(q + 2);
+      pd_arrive(2 + (q & 1));
     }
-    __syncthreads();
-    if (tid >= PD_BULK) {
-      const int cc = tid - PD_BULK;
-      double lb[4][4], rd[4], t[4];
+  } else if (role >= 16) {
+    double* __restrict__ D = c.dinv64 + f.dinv_off + (int64_t)(k0 / 64) * 4096;
+    const int cc = 32 * (role - 16) + lane;
+    bool bad = false;
+#pragma unroll 1
+    for (int q = 0; q < 16; ++q) {
+      const int P = 4 * q;
+      if (q != 1) pd_sync(2 + (q & 1));
+      double t[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) t[m] = cc >= P - 4 && cc < P ? 0.0 : V[q & 1][m][cc];
+      if (q > 0) {
+        // the update of step q - 1
+        const double (*b)[64] = B[(q - 1) & 1];
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+          const double x = b[l][cc];
+          double y[4];
+          Vec4<double>::ld(&b[l][P], y);
+#pragma unroll
+          for (int m = 0; m < 4; ++m) t[m] -= y[m] * x;
+        }
+      }
+      const bool piv = cc >= P && cc < P + 4;
+      if (piv) Vec4<double>::st(&pv[cc - P][0], t);            // A(cc, P ..)
+      asm volatile("bar.sync 1, 64;" ::: "memory");
+      double lb[4][4], rd[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) Vec4<double>::ld(&pv[r][0], lb[r]);
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
-        double s = V[m][P + m];
+        double s = lb[m][m];
 #pragma unroll
         for (int l = 0; l < m; ++l) s -= lb[m][l] * lb[m][l];
         if (!(s > 0.0)) { bad = true; s = 1.0; }
         rd[m] = rsqrt(s);
 #pragma unroll
         for (int r = m + 1; r < 4; ++r) {
-          double w = V[m][P + r];
+          double w = lb[r][m];
 #pragma unroll
           for (int l = 0; l < m; ++l) w -= lb[r][l] * lb[m][l];
           lb[r][m] = w * rd[m];
         }
       }
-      const bool piv = cc >= P && cc < P + 4;
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
-        double w = piv ? (cc == P + m ? 1.0 : 0.0) : V[m][cc];
+        double w = piv ? (cc == P + m ? 1.0 : 0.0) : t[m];
 #pragma unroll
         for (int l = 0; l < m; ++l) w -= lb[m][l] * t[l];
         t[m] = w * rd[m];
-        B[m][cc] = t[m];
+        B[q & 1][m][cc] = t[m];
       }
+      asm volatile("bar.sync 1, 64;" ::: "memory");            // B of this step, before either warp's next
+      if (q < 14) pd_arrive(4 + (q & 1));
 #pragma unroll
       for (int m = 0; m < 4; ++m)
         if (cc >= P + 4 || P + m >= kb || cc >= kb) t[m] = 0.0;
       Vec4<double>::st(D + (int64_t)cc * 64 + P, t);
     }
-    __syncthreads();
-    if (i > q) {
-      if (j == q) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) a[u][0] = a[u][1] = 0.0;
-      }
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        double l[4];
-        Vec4<double>::ld(&B[m][r0], l);
-        const double2 b = *reinterpret_cast<const double2*>(&B[m][c0]);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          a[u][0] -= l[u] * b.x;
-          a[u][1] -= l[u] * b.y;
-        }
-      }
-    }
+    if (cc == 0 && bad) set_status(c, it.front, ST_NOT_SPD);
   }
-  if (tid == PD_BULK && bad) set_status(c, it.front, ST_NOT_SPD);
 }
 
 void launch_potrf_diag(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
