@@ -18,6 +18,7 @@
 // The sum is formed in the front's precision: FP64 fronts in FP64, FP32
 // fronts in FP32 (FP64 arithmetic runs at a small fraction of the FP32 rate
 // on this GPU, and the FP32 front stores the sum in FP32 either way).
+#include <cstddef>
 #include <cstdio>
 #include <stdexcept>
 #include <string>
@@ -1147,8 +1148,8 @@ void launch_getrf_panel(const DevCtx& c, const Item* items, int n_items, int dty
 // LU panel in shared memory: one CTA, a cluster, or a whole grid per front
 // ---------------------------------------------------------------------------
 // The panel (rows k0..n-1, columns k0..k0+kb-1) of each item is split into
-// chunks of R rows, one per CTA, held in shared memory (column-major, leading
-// dimension rmax).  For each column k of the panel, every CTA
+// chunks of R rows, one per CTA, held in shared memory (row-major: a thread
+// updates four columns of its row with 16-byte accesses).  For each column k of the panel, every CTA
 //   1. offers its candidate pivot: the largest |a| in column k among its rows
 //      in [k0+k, fs) (the reference searches the eliminated rows only), ties
 //      to the lowest row, with the row's kb values; the CTA holding row k0+k
@@ -1182,10 +1183,11 @@ void launch_getrf_panel(const DevCtx& c, const Item* items, int n_items, int dty
 // block barriers, one exchange, the reductions), then by the update's shared-
 // memory traffic (FP32) or multiply-adds (FP64).  Measured on GB300, the panels
 // of one factorisation, against a grid barrier on a counter per column: 24^3 p =
-// 3 FP32 141 + 2.5 (one-CTA panels in global memory) -> 69.0 ms, 12^3 p = 3
-// FP64 55.9 + 4.8 -> 25.7, 6^3 p = 3 4.9 + 2.0 -> 4.4.
+// 3 FP32 141 + 2.5 (one-CTA panels in global memory) -> 59.4 ms, 12^3 p = 3
+// FP64 55.9 + 4.8 -> 24.2, 6^3 p = 3 4.9 + 2.0 -> 4.3.  The chunk by columns instead
+// (one column of a row per access) took 69.0, 25.7 and 4.4: bank conflicts where a
+// row is read, and four times the shared-memory instructions.
 constexpr int GC_ERR = 3;
-constexpr int GC_BATCH = 4;                     // columns a thread updates at a time
 constexpr int GC_POLL = (GC_MAX_CTAS + 31) / 32;
 constexpr int64_t GC_REC = 2 + 2 * 64;          // words of one record: candidate, then a row (two per FP64 value)
 static_assert(gc_words(1, 1) == 4 * GC_REC, "record size of the launcher's callers");
@@ -1195,6 +1197,7 @@ UHM_DEFINE_WAIT_LIMIT(set_wait_limit_factor, 1u << 22)
 template <typename T> struct LuBits;
 template <> struct LuBits<double> {
   static constexpr int WORDS = 2;               // exchange words per value
+  static constexpr int LD = 66;                 // row of the chunk (16-byte loads of 8 rows hit every bank once)
   static __device__ __forceinline__ uint64_t key(double v) {
     return v == v ? (uint64_t)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull : 0ull;
   }
@@ -1205,6 +1208,7 @@ template <> struct LuBits<double> {
 };
 template <> struct LuBits<float> {
   static constexpr int WORDS = 1;
+  static constexpr int LD = 68;
   static __device__ __forceinline__ uint64_t key(float v) {
     return v == v ? (uint64_t)(__float_as_uint(v) & 0x7FFFFFFFu) : 0ull;
   }
@@ -1283,15 +1287,26 @@ __device__ __forceinline__ void lu_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ float lu_rcp(float v) { return 1.0f / v; }
-__device__ __forceinline__ double lu_rcp(double v) { return __drcp_rn(v); }
+// 1 / v by Chebyshev's iteration: an FP32 start x of the mantissa, then
+// x (1 + r + r^2), r = 1 - v x (the next term, r^3, is below 2^-66); three
+// dependent FP64 operations, 0.5000 ulp over 10^8 values of every exponent
+__device__ __forceinline__ double lu_rcp(double v) {
+  const int hi = __double2hiint(v), f = (hi >> 20) & 0x7FF;
+  if (f < 24 || f > 2022) return 1.0 / v;
+  const float m = __int_as_float((127 << 23) | (hi & 0xFFFFF) << 3 | (int)((unsigned)__double2loint(v) >> 29));
+  const uint32_t xb = __float_as_uint(1.0f / m);               // (1/2, 1]
+  const double x = __hiloint2double((int)((hi & 0x80000000u) | ((xb >> 3) + ((1023 - 127 - (f - 1023)) << 20))),
+                                    (int)(xb << 29));
+  const double r = fma(-v, x, 1.0);
+  return fma(x, fma(r, r, r), x);
+}
 
 // rows received in one column: of every candidate (CL) or of the pivot, then row k0 + k
 template <typename T, bool CL>
 struct LuRecv {
   T row[CL ? GC_CLUSTER : 1][64];
   T diag[64];
-  uint64_t key[CL ? GC_CLUSTER : 1];
-  uint64_t at[CL ? GC_CLUSTER : 1];
+  uint64_t cand[CL ? GC_CLUSTER : 1][2];        // key, row
 };
 
 template <typename T, bool CL, int NT>
@@ -1299,13 +1314,15 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
                                                    int pivot, int rmax, int csize, uint64_t* __restrict__ xbuf,
                                                    int* err) {
   extern __shared__ __align__(16) unsigned char gc_smem[];
-  constexpr int NW = NT / 32, WORDS = LuBits<T>::WORDS;
+  using LuRecvT = LuRecv<T, CL>;
+  constexpr int NW = NT / 32, WORDS = LuBits<T>::WORDS, SR = LuBits<T>::LD;
   __shared__ __align__(16) LuRecv<T, CL> recv[2];
   __shared__ uint64_t s_key[NW];
   __shared__ int s_row[NW];
   __shared__ int s_item, s_p;
   __shared__ T s_rinv;
-  T* S = reinterpret_cast<T*>(gc_smem);        // chunk, column-major, leading dimension rmax
+  T* S = reinterpret_cast<T*>(gc_smem);        // chunk, row-major, rows of SR
+  T* s_col = S + (int64_t)rmax * SR;           // the column to eliminate next, by parity
   const int total = gridDim.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) {
@@ -1313,6 +1330,7 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
     if (!CL) while (k + 1 < n_items && (int)blockIdx.x >= items[k + 1].b) ++k;
     s_item = CL ? blockIdx.x / csize : k;
   }
+  for (int e = tid; e < (int)(sizeof(recv) / sizeof(uint32_t)); e += NT) reinterpret_cast<uint32_t*>(recv)[e] = 0;
   __syncthreads();
   const Item it = items[s_item];
   const FrontDev f = c.fronts[it.front];
@@ -1326,7 +1344,7 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
   T* __restrict__ G = arena<T>(c) + f.off;
   // !CL: exchange records: per parity, one per CTA, then one per item (the row k0 + k)
   auto rec = [&](int par, int b) { return xbuf + ((int64_t)par * (total + n_items) + b) * GC_REC; };
-  // thread layout of the chunk: rows along lanes, ng column groups
+  // thread layout of the chunk: rows along lanes, ng groups of 4-column blocks
   const int rw = min(NT, (max(nr_my, 1) + 31) / 32 * 32), ng = NT / rw;
   const int tr = tid % rw, tg = tid / rw;
   uint64_t mk = 0;                             // this thread's best candidate of the next column
@@ -1336,11 +1354,14 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
     if (v == v && (mr == LU_NONE || key > mk || (key == mk && r < mr))) { mk = key; mr = r; }
   };
   if (tg < ng)
-    for (int j = tg; j < kb; j += ng)
+    for (int j = tg; j < 64; j += ng)
       for (int r = tr; r < nr_my; r += rw) {
-        const T v = G[(rbeg + r) + (int64_t)(k0 + j) * n];
-        S[j * rmax + r] = v;
-        if (pivot && j == 0 && rbeg + r < fs) offer(v, rbeg + r);
+        const T v = j < kb ? G[(rbeg + r) + (int64_t)(k0 + j) * n] : T(0);
+        S[r * SR + j] = v;
+        if (j == 0) {
+          s_col[r] = v;
+          if (pivot && rbeg + r < fs) offer(v, rbeg + r);
+        }
       }
   lu_best<T>(mk, mr);
   if (lane == 0) { s_key[warp] = mk; s_row[warp] = mr; }
@@ -1358,29 +1379,32 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
     const T* old = rc.diag;
     int p = gk;
     if constexpr (CL) {
-      // warp w serves CTAs w, w + NW, ..
-      for (int d = warp; d < csize; d += NW) {
-        if (lane == 0) {
-          lu_put(lu_mapa(lu_smem(&rc.key[q]), d), bk);
-          lu_put(lu_mapa(lu_smem(&rc.at[q]), d), (uint64_t)bi);
-        }
-        if (bi != LU_NONE) {
-          const uint32_t a = lu_mapa(lu_smem(&rc.row[q][0]), d);
-          for (int j = lane; j < kb; j += 32) lu_put(a + j * (uint32_t)sizeof(T), S[j * rmax + (bi - rbeg)]);
-        }
+      // warp w serves CTA w
+      if (warp < csize) {
+        const T* cs = S + (bi == LU_NONE ? 0 : bi - rbeg) * SR + lane;
+        const T* ds = S + (diag_mine ? gk - rbeg : 0) * SR + lane;
+        const T c0 = cs[0], c1 = cs[32], d0 = ds[0], d1 = ds[32];
+        const uint32_t a = lu_mapa(lu_smem(&rc), warp);
+        const uint32_t ar = a + (uint32_t)offsetof(LuRecvT, row) + (uint32_t)sizeof(T) * (64 * q + lane);
+        const uint32_t ad = a + (uint32_t)offsetof(LuRecvT, diag) + (uint32_t)sizeof(T) * lane;
+        lu_put(ar, c0);
+        lu_put(ar + 32 * (uint32_t)sizeof(T), c1);
         if (diag_mine) {
-          const uint32_t a = lu_mapa(lu_smem(&rc.diag[0]), d);
-          for (int j = lane; j < kb; j += 32) lu_put(a + j * (uint32_t)sizeof(T), S[j * rmax + (gk - rbeg)]);
+          lu_put(ad, d0);
+          lu_put(ad + 32 * (uint32_t)sizeof(T), d1);
         }
+        if (lane < 2)
+          lu_put(a + (uint32_t)offsetof(LuRecvT, cand) + 16u * q + 8u * lane, lane ? (uint64_t)bi : bk);
       }
       if (csize > 1) lu_cluster_sync();
       else __syncthreads();
       // 2. the item's pivot
-      uint64_t key = lane < csize ? rc.key[lane] : 0;
-      int r = lane < csize ? (int)rc.at[lane] : LU_NONE;
+      uint64_t key = lane < csize ? rc.cand[lane][0] : 0;
+      int r = lane < csize ? (int)rc.cand[lane][1] : LU_NONE, w = lane;
       lu_best<T>(key, r);
       if (r != LU_NONE) p = r;
-      u = p == gk ? rc.diag : rc.row[(p - k0) / R];
+      w = __ffs(__ballot_sync(0xffffffffu, lane < csize && (int)rc.cand[w & (GC_CLUSTER - 1)][1] == r)) - 1;
+      u = p == gk ? rc.diag : rc.row[max(w, 0)];
     } else {
       const uint64_t tag56 = (uint64_t)(k + 1) << 56;
       bool ok = true;
@@ -1392,10 +1416,10 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
                                                : (bk & 0xFFFFFFFFull)));
         if (bi != LU_NONE)
           for (int w = lane; w < kb * WORDS; w += 32)
-            gc_put(cb + 2 + w, tag56 | LuBits<T>::half(S[(w / WORDS) * rmax + (bi - rbeg)], w % WORDS));
+            gc_put(cb + 2 + w, tag56 | LuBits<T>::half(S[(bi - rbeg) * SR + w / WORDS], w % WORDS));
         // 2. the item's pivot
         uint64_t x0[GC_POLL], x1[GC_POLL], key = 0;
-        int r = LU_NONE, w = -1;
+        int r = LU_NONE;
         ok = gc_poll<GC_POLL>(rec(par, it.b), (int)GC_REC, P, k + 1, x0, err) &&
              gc_poll<GC_POLL>(rec(par, it.b) + 1, (int)GC_REC, P, k + 1, x1, err);
         if (ok) {
@@ -1412,13 +1436,12 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
         lu_best<T>(key, r);
         if (r != LU_NONE) p = r;
         if (lane == 0) s_p = p;
-        w = it.b + (p - k0) / R;
         if (ok && p != gk) {
           if (p >= rbeg && p < rend) {
-            for (int j = lane; j < kb; j += 32) rc.row[0][j] = S[j * rmax + (p - rbeg)];
+            for (int j = lane; j < kb; j += 32) rc.row[0][j] = S[(p - rbeg) * SR + j];
           } else {
             uint64_t x[2 * WORDS];
-            ok = gc_poll<2 * WORDS>(rec(par, w) + 2, 1, kb * WORDS, k + 1, x, err);
+            ok = gc_poll<2 * WORDS>(rec(par, it.b + (p - k0) / R) + 2, 1, kb * WORDS, k + 1, x, err);
 #pragma unroll
             for (int e = 0; e < 2 * WORDS; ++e) {
               const uint32_t v = (uint32_t)x[e], lo = __shfl_down_sync(0xffffffffu, v, 1);
@@ -1432,8 +1455,8 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
         uint64_t* dr = rec(par, total + s_item);
         if (diag_mine) {
           for (int w = lane; w < kb * WORDS; w += 32)
-            gc_put(dr + w, tag56 | LuBits<T>::half(S[(w / WORDS) * rmax + (gk - rbeg)], w % WORDS));
-          for (int j = lane; j < kb; j += 32) rc.diag[j] = S[j * rmax + (gk - rbeg)];
+            gc_put(dr + w, tag56 | LuBits<T>::half(S[(gk - rbeg) * SR + w / WORDS], w % WORDS));
+          for (int j = lane; j < kb; j += 32) rc.diag[j] = S[(gk - rbeg) * SR + j];
         } else {
           uint64_t x[2 * WORDS];
           ok = gc_poll<2 * WORDS>(dr, 1, kb * WORDS, k + 1, x, err);
@@ -1467,54 +1490,66 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
       rinv = lu_rcp(akk);
     }
     // 3. rows from the pivot row on: the two rows swapped, multiplier and
-    // rank-1 update of the panel's later columns below it
+    // rank-1 update of the panel's later columns below it; the 4-column
+    // blocks from that of column k + 1 on in turn over the groups
     mk = 0;
     mr = LU_NONE;
+    const int b0 = (k + 1) >> 2;
     if (tg < ng)
       for (int rl = max(rbeg, gk) - rbeg + tr; rl < nr_my; rl += rw) {
         const int r = rbeg + rl;
+        T* __restrict__ row = S + rl * SR;
         if (r == gk) {
           if (p != gk)
-            for (int j = tg; j < kb; j += ng) S[j * rmax + rl] = u[j];
+            for (int j = tg; j < 64; j += ng) row[j] = u[j];
           continue;
         }
+        T a[4], x[4];
         const bool sw = r == p;
-        const T l = (sw ? old[k] : S[k * rmax + rl]) * rinv;
+        const T* __restrict__ src = sw ? old : row;
+        const T l = (sw ? old[k] : s_col[par * rmax + rl]) * rinv;
         if (sw)
-          for (int j = tg; j < k; j += ng) S[j * rmax + rl] = old[j];
-        int j = k + 1 + tg;
-        if (tg == 0 && j < kb) {
-          const T v = (sw ? old[j] : S[j * rmax + rl]) - l * u[j];
-          S[j * rmax + rl] = v;
-          if (pivot && r < fs) offer(v, r);
-          j += ng;
-        }
-        for (; j + (GC_BATCH - 1) * ng < kb; j += GC_BATCH * ng) {
-          T a[GC_BATCH], b[GC_BATCH];
-#pragma unroll
-          for (int e = 0; e < GC_BATCH; ++e) {
-            a[e] = sw ? old[j + e * ng] : S[(j + e * ng) * rmax + rl];
-            b[e] = u[j + e * ng];
+          for (int b = tg; b < b0; b += ng) {
+            Vec4<T>::ld(old + 4 * b, a);
+            if (4 * b + 3 == k) a[3] = l;
+            Vec4<T>::st(row + 4 * b, a);
           }
+        int b = b0 + tg;
+        if (tg == 0) {
+          if ((k & 3) == 3 && !sw) row[k] = l; // column k in the block before
+          if (b < 16) {
+            Vec4<T>::ld(src + 4 * b, a);
+            Vec4<T>::ld(u + 4 * b, x);
 #pragma unroll
-          for (int e = 0; e < GC_BATCH; ++e) S[(j + e * ng) * rmax + rl] = a[e] - l * b[e];
+            for (int e = 0; e < 4; ++e) {
+              const int j = 4 * b + e;
+              if (j > k) a[e] -= l * x[e];
+              else if (j == k) a[e] = l;
+            }
+            Vec4<T>::st(row + 4 * b, a);
+            const int e1 = (k + 1) & 3;
+            const T v = e1 == 0 ? a[0] : e1 == 1 ? a[1] : e1 == 2 ? a[2] : a[3];
+            s_col[(par ^ 1) * rmax + rl] = v;
+            if (pivot && r < fs) offer(v, r);
+          }
+          b += ng;
         }
-        for (; j < kb; j += ng) S[j * rmax + rl] = (sw ? old[j] : S[j * rmax + rl]) - l * u[j];
+#pragma unroll 2
+        for (; b < 16; b += ng) {
+          Vec4<T>::ld(src + 4 * b, a);
+          Vec4<T>::ld(u + 4 * b, x);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[e] -= l * x[e];
+          Vec4<T>::st(row + 4 * b, a);
+        }
       }
     lu_best<T>(mk, mr);
     if (lane == 0) { s_key[warp] = mk; s_row[warp] = mr; }
     __syncthreads();
-    // the multipliers, once every group has read column k
-    if (tg == 0)
-      for (int rl = max(rbeg, gk + 1) - rbeg + tr; rl < nr_my; rl += rw) {
-        T* e = &S[k * rmax + rl];
-        *e = (rbeg + rl == p ? old[k] : *e) * rinv;
-      }
-    __syncthreads();
   }
   if (tg < ng)
     for (int j = tg; j < kb; j += ng)
-      for (int r = tr; r < nr_my; r += rw) G[(rbeg + r) + (int64_t)(k0 + j) * n] = S[j * rmax + r];
+      for (int r = tr; r < nr_my; r += rw) G[(rbeg + r) + (int64_t)(k0 + j) * n] = S[r * SR + j];
 }
 
 constexpr int GC_NT_CLUSTER = 512, GC_NT_GRID = 256;
@@ -1523,7 +1558,7 @@ template <typename T, bool CL>
 static cudaError_t getrf_smem_t(const DevCtx& c, const Item* items, int n_items, int n_ctas, int csize, int nb,
                                 int pivot, int rmax, uint64_t* xbuf, int* err, cudaStream_t s) {
   constexpr int NT = CL ? GC_NT_CLUSTER : GC_NT_GRID;
-  const size_t smem = (size_t)rmax * nb * sizeof(T);
+  const size_t smem = (size_t)rmax * (LuBits<T>::LD + 2) * sizeof(T);
   cudaFuncSetAttribute(k_getrf_smem<T, CL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(n_ctas);
