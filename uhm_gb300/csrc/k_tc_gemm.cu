@@ -8,23 +8,29 @@
 // Split precision: every FP32 entry a = hi + lo + (mid) with hi, lo (, mid)
 // BF16 (round to nearest); the product a*b is taken as the sum of BF16
 // products hi*hi + hi*lo + lo*hi ("bf16x3", ~2^-17 relative) or, with three
-// parts, the six terms of order <= 2^-16 ("bf16x6", FP32-class).  Terms are
-// laid end to end along K, so one GEMM with K' = terms * KB accumulates them
-// all in FP32 in tensor memory.
+// parts, the six terms of order <= 2^-16 ("bf16x6", FP32-class), all
+// accumulated in FP32 in tensor memory.
 //
-// Kernel: one persistent CTA per SM walks the 128 x 128 output tiles; warp 8
-// issues TMA loads (128-byte swizzle) into a 4-stage shared-memory ring
-// guarded by mbarriers, one thread of warp 9 issues tcgen05.mma (M=128,
-// N=128, K=16) into one of two 128-column TMEM accumulators, warps 0-7 read
-// TMEM back (tcgen05.ld; two warps per 32-lane quarter, one per column half)
-// and apply C -= acc to the FP32 panel while the next tile accumulates in
-// the other buffer.  Every wait is bounded: a wait that
-// gives up records an error flag and the CTA skips its stores.
+// Kernel: one persistent CTA per SM walks the 128 x 128 output tiles; warp 16
+// issues TMA loads (128-byte swizzle) into a shared-memory ring guarded by
+// mbarriers, warp 17 issues tcgen05.mma (M=128, N=128, K=16) into one of two
+// 128-column TMEM accumulators, warps 0-15 (a 32-lane quarter and 32 columns
+// each) read TMEM back (tcgen05.ld) and apply C -= acc to the FP32 panel while
+// the next tile accumulates in the other buffer.  Every wait is bounded: a wait
+// that gives up records an error flag and the CTA skips its stores.
+//
+// Bound by the memory traffic of C (read and written once: K = 256 leaves 24 flops
+// per byte) and by the operands' way from L2.  A ring slot holds every part of a
+// 64-column chunk of A and of B, so that a part used by two terms is loaded once
+// (256 KB instead of 384 per tile in bf16x3); a warp's 32 loads of C go out
+// before it waits for the products, 64 KB per SM, where eight warps staging C
+// through shared memory 16 loads at a time had 16 KB.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 
 #include <cstdio>
+#include <stdexcept>
 
 #include "k_common.cuh"
 #include "k_tc.cuh"
@@ -32,13 +38,13 @@
 
 namespace uhm_gpu {
 
-constexpr int TC_BM = 128, TC_BN = 128, TC_BK = 64, TC_STAGES = 4;
-constexpr int TC_THREADS = 320;     // warps 0-7 epilogue, 8 TMA producer, 9 MMA issuer
-constexpr int TC_EPI_THREADS = 256;
+constexpr int TC_BM = 128, TC_BN = 128, TC_BK = 64;
+constexpr int TC_EPI_WARPS = 16;
+constexpr int TC_THREADS = 32 * (TC_EPI_WARPS + 2);     // epilogue, TMA producer, MMA issuer
 constexpr uint32_t TC_TILE_BYTES = TC_BM * TC_BK * 2;   // 16 KB (A and B tiles alike)
-constexpr uint32_t TC_CPAD = TC_BN + 1;                 // padded row of the staged C tile
-constexpr uint32_t TC_CTILE_BYTES = TC_BM * TC_CPAD * 4;
-constexpr uint32_t TC_SMEM = 1024 + TC_STAGES * 2 * TC_TILE_BYTES + 256 + TC_CTILE_BYTES;
+constexpr uint32_t TC_RING = 12 * TC_TILE_BYTES;        // slots of 2 x parts tiles: 3 (bf16x3) or 2 (bf16x6)
+constexpr int TC_SLOTS_MAX = 3;
+constexpr uint32_t TC_SMEM = 1024 + TC_RING + 256;
 
 UHM_DEFINE_WAIT_LIMIT(set_wait_limit_tc, 1u << 24)
 
@@ -50,40 +56,42 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 
 // item: front, a = K0 (outer step start), b = tile row, c = tile col
 // (tiles counted from the trailing block's first row K0 + KB).
-// term_code: 2 bits per part index, 4 bits per term (A part, B part).
+// Operand parts: A 0 .. parts - 1, B pb0 .. pb0 + parts - 1; term_code: 4 bits
+// per term (A part, B part - pb0).
 //
 // Persistent: one CTA per SM walks the tile list with stride gridDim.x.  The
 // TMA ring (full / empty barriers) runs continuously across tiles; TMEM holds
 // two 128-column accumulators, so the epilogue of tile i (TMEM -> registers
 // -> C in global memory) overlaps the mainloop of tile i + 1.  acc_full[b]
-// is committed by the MMA thread when accumulator b holds a finished tile;
-// acc_empty[b] collects the 256 epilogue threads once they have read it.
+// is committed by the MMA warp when accumulator b holds a finished tile;
+// acc_empty[b] collects the epilogue warps once they have read it.
+// Measured on GB300, the LU trailing updates of 24^3 p = 3 (BF16X3, K = 256):
+// 21.7 -> 17.0 ms; 13,225 tiles 522 -> 428 us, of which C's traffic alone is 255.
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_tc_syrk(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __restrict__ ws_off,
-          const int64_t* __restrict__ ws_stride, const Item* __restrict__ items, int n_items, int nbo,
-          int nterms, uint32_t term_code, int lower_only, int* err) {
+          const int64_t* __restrict__ ws_stride, const Item* __restrict__ items, int n_items, int nbo, int parts,
+          int pb0, int nterms, uint32_t term_code, int lower_only, int* err) {
   extern __shared__ __align__(1024) uint8_t tc_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* tilesA = smem;
-  uint8_t* tilesB = smem + TC_STAGES * TC_TILE_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * TC_STAGES * TC_TILE_BYTES);
-  // bars[0..S) full, bars[S..2S) empty, bars[2S..2S+2) acc_full, bars[2S+2..2S+4) acc_empty
-  uint64_t* acc_full = bars + 2 * TC_STAGES;
-  uint64_t* acc_empty = bars + 2 * TC_STAGES + 2;
-  volatile int* s_abort = reinterpret_cast<volatile int*>(bars + 2 * TC_STAGES + 4);
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 2 * TC_STAGES + 5);
-  uint64_t* drain_bar = bars + 2 * TC_STAGES + 6;
-  float* s_c = reinterpret_cast<float*>(smem + 2 * TC_STAGES * TC_TILE_BYTES + 256);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TC_RING);
+  uint64_t* empty = bars + TC_SLOTS_MAX;
+  uint64_t* acc_full = empty + TC_SLOTS_MAX;
+  uint64_t* acc_empty = acc_full + 2;
+  uint64_t* drain_bar = acc_empty + 2;
+  volatile int* s_abort = reinterpret_cast<volatile int*>(drain_bar + 1);
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(drain_bar + 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t slot_bytes = 2 * (uint32_t)parts * TC_TILE_BYTES;
+  const int slots = min(TC_SLOTS_MAX, (int)(TC_RING / slot_bytes));
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < TC_STAGES; ++s) {
+    for (int s = 0; s < TC_SLOTS_MAX; ++s) {
       mbar_init(smem_u32(&bars[s]), 1);
-      mbar_init(smem_u32(&bars[TC_STAGES + s]), 1);
+      mbar_init(smem_u32(&empty[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&acc_full[b]), 1);
-      mbar_init(smem_u32(&acc_empty[b]), TC_EPI_THREADS);
+      mbar_init(smem_u32(&acc_empty[b]), TC_EPI_WARPS);
     }
     mbar_init(smem_u32(drain_bar), 1);
     *s_abort = 0;
@@ -98,147 +106,117 @@ k_tc_syrk(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *s_tmem;
 
-  // per-tile geometry, identical in every role
-  struct Tile {
-    int front, n, base, R0, C0, row0, prow, kpt, nk, off;
-  };
-  auto tile_of = [&](int t) {
-    const Item it = items[t];
-    const FrontDev f = c.fronts[it.front];
-    Tile T;
-    T.front = it.front;
-    T.n = f.n;
-    const int KB = min(nbo, f.fs - it.a);
-    T.base = it.a + KB;
-    T.R0 = T.base + it.b * TC_BM;
-    T.C0 = T.base + it.c * TC_BN;
-    // the whole BF16 workspace is one 2D tensor of rows of nbo elements;
-    // part p of this front starts at row (ws_off + p * ws_stride) / nbo
-    T.row0 = (int)(ws_off[it.front] / nbo);
-    T.prow = (int)(ws_stride[it.front] / nbo);
-    T.kpt = (KB + TC_BK - 1) / TC_BK;
-    T.nk = T.kpt * nterms;
-    T.off = (int)0;
-    (void)f;
-    return T;
-  };
-
-  if (warp == 8) {
+  if (warp == TC_EPI_WARPS) {
     if (lane == 0) {
       // TMA producer
-      uint32_t g = 0;       // chunks issued by this CTA so far
+      int s = 0;
+      uint32_t ph = 1;               // parity of the empty wait (the first round passes)
+      uint32_t issued = 0;           // chunks
       bool live = true;
       for (int t = blockIdx.x; t < n_items && live; t += gridDim.x) {
-        const Tile T = tile_of(t);
-        for (int kc = 0; kc < T.nk; ++kc, ++g) {
-          const uint32_t s = g % TC_STAGES;
-          if (g >= TC_STAGES &&
-              !mbar_wait(smem_u32(&bars[TC_STAGES + s]), ((g / TC_STAGES) + 1) & 1, s_abort, err)) {
+        const Item it = items[t];
+        const int KB = min(nbo, c.fronts[it.front].fs - it.a);
+        const int nk = (KB + TC_BK - 1) / TC_BK;
+        // the whole BF16 workspace is one 2D tensor of rows of nbo elements;
+        // part p of this front starts at row (ws_off + p * ws_stride) / nbo
+        const int prow = (int)(ws_stride[it.front] / nbo);
+        const int ra = (int)(ws_off[it.front] / nbo) + it.b * TC_BM;
+        const int rb = (int)(ws_off[it.front] / nbo) + pb0 * prow + it.c * TC_BN;
+        for (int kk = 0; kk < nk; ++kk) {
+          if (issued >= (uint32_t)slots && !mbar_wait(smem_u32(&empty[s]), ph, s_abort, err)) {
             live = false;
             break;
           }
-          const int term = kc / T.kpt, kk = kc % T.kpt;
-          const int pa = (term_code >> (4 * term)) & 3, pb = (term_code >> (4 * term + 2)) & 3;
-          const uint32_t fb = smem_u32(&bars[s]);
-          mbar_expect_tx(fb, 2 * TC_TILE_BYTES);
-          tma_load_2d(smem_u32(tilesA + s * TC_TILE_BYTES), &wsmap, kk * TC_BK,
-                      T.row0 + pa * T.prow + (T.R0 - T.base), fb);
-          tma_load_2d(smem_u32(tilesB + s * TC_TILE_BYTES), &wsmap, kk * TC_BK,
-                      T.row0 + pb * T.prow + (T.C0 - T.base), fb);
+          const uint32_t fb = smem_u32(&bars[s]), st = smem_u32(smem) + s * slot_bytes;
+          mbar_expect_tx(fb, slot_bytes);
+          for (int p = 0; p < parts; ++p) {
+            tma_load_2d(st + p * TC_TILE_BYTES, &wsmap, kk * TC_BK, ra + p * prow, fb);
+            tma_load_2d(st + (parts + p) * TC_TILE_BYTES, &wsmap, kk * TC_BK, rb + p * prow, fb);
+          }
+          ++issued;
+          if (++s == slots) { s = 0; ph ^= 1; }
         }
       }
-      // the last loads issued (one per stage at most) have landed before the
-      // CTA exits, whether or not the MMA thread consumed them
-      for (uint32_t g2 = g > TC_STAGES ? g - TC_STAGES : 0; g2 < g; ++g2)
-        mbar_drain(smem_u32(&bars[g2 % TC_STAGES]), (g2 / TC_STAGES) & 1);
+      // the last loads issued (one chunk per slot at most) have landed before
+      // the CTA exits, whether or not the MMA warp consumed them
+      const uint32_t cnt = issued < (uint32_t)slots ? issued : (uint32_t)slots;
+      for (uint32_t q = issued - cnt; q < issued; ++q) mbar_drain(smem_u32(&bars[q % slots]), (q / slots) & 1);
     }
-  } else if (warp == 9) {
-    if (lane == 0) {
-      // MMA issuer
-      const uint32_t idesc = idesc_bf16_f32(TC_BM, TC_BN);
-      uint32_t g = 0;
-      int i = 0;            // tiles processed by this CTA
-      bool live = true;
-      for (int t = blockIdx.x; t < n_items && live; t += gridDim.x, ++i) {
-        const Tile T = tile_of(t);
-        const int b = i & 1, u = i >> 1;
-        if (u >= 1 && !mbar_wait(smem_u32(&acc_empty[b]), (u - 1) & 1, s_abort, err)) break;
+  } else if (warp == TC_EPI_WARPS + 1) {
+    // MMA issuer: the whole warp, one elected lane issuing
+    const uint32_t elected = elect_one();
+    const uint32_t idesc = idesc_bf16_f32(TC_BM, TC_BN);
+    const uint32_t ring = smem_u32(smem), bar0 = smem_u32(bars), empty0 = smem_u32(empty);
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbar_wait(bar, parity, s_abort, err)) != 0;
+    };
+    int s = 0, i = 0;
+    uint32_t ph = 0;
+    bool live = true;
+    for (int t = blockIdx.x; t < n_items && live; t += gridDim.x, ++i) {
+      const Item it = items[t];
+      const int nk = __shfl_sync(0xffffffffu, (min(nbo, c.fronts[it.front].fs - it.a) + TC_BK - 1) / TC_BK, 0);
+      const int b = i & 1, u = i >> 1;
+      if (u >= 1 && !wait(smem_u32(&acc_empty[b]), (u - 1) & 1)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t acc = tmem + b * TC_BN;
+      uint32_t on = 0;
+      for (int kk = 0; kk < nk; ++kk) {
+        live = wait(bar0 + 8 * s, ph);
+        if (!live) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t acc = tmem + b * TC_BN;
-        for (int kc = 0; kc < T.nk; ++kc, ++g) {
-          const uint32_t s = g % TC_STAGES;
-          if (!mbar_wait(smem_u32(&bars[s]), (g / TC_STAGES) & 1, s_abort, err)) {
-            live = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a0 = smem_u32(tilesA + s * TC_TILE_BYTES);
-          const uint32_t b0 = smem_u32(tilesB + s * TC_TILE_BYTES);
+        const uint32_t a0 = sdesc_lo(ring + (uint32_t)s * slot_bytes);
+        const uint32_t b0 = sdesc_lo(ring + (uint32_t)s * slot_bytes + (uint32_t)parts * TC_TILE_BYTES);
+        for (int q = 0; q < nterms; ++q) {
+          const uint32_t at = a0 + ((term_code >> (4 * q)) & 3) * (TC_TILE_BYTES >> 4);
+          const uint32_t bt = b0 + ((term_code >> (4 * q + 2)) & 3) * (TC_TILE_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < TC_BK / 16; ++k)
-            umma_bf16(acc, sdesc_sw128(a0 + k * 32), sdesc_sw128(b0 + k * 32), idesc, (kc | k) != 0);
-          umma_commit(smem_u32(&bars[TC_STAGES + s]));
+          for (int k = 0; k < TC_BK / 16; ++k) {
+            umma_bf16_w(elected, acc, at + 2 * k, bt + 2 * k, SDESC_SW128_HI, idesc, on);
+            on = 1u;
+          }
         }
-        if (live) umma_commit(smem_u32(&acc_full[b]));
+        umma_commit_w(elected, empty0 + 8 * s);
+        if (++s == slots) { s = 0; ph ^= 1; }
       }
-      // every MMA this thread issued has completed before TMEM is freed
-      umma_commit(smem_u32(drain_bar));
-      mbar_drain(smem_u32(drain_bar), 0);
+      if (live) umma_commit_w(elected, smem_u32(&acc_full[b]));
     }
+    // every MMA issued has completed before TMEM is freed
+    umma_commit_w(elected, smem_u32(drain_bar));
+    mbar_drain(smem_u32(drain_bar), 0);
   } else {
-    // epilogue warps 0-7: warp w reads TMEM lanes [32 (w % 4), +32) (its
-    // lane quarter = tile rows) and handles the columns [64 (w / 4), +64).
-    // The thread's half-row of the next C tile is staged in shared memory
-    // while the mainloop runs (independent, coalesced loads); each thread
-    // reads back only what it staged, so no barrier is needed for s_c.
-    const int quarter = warp & 3, half = warp >> 2;
-    const int rl = quarter * 32 + lane;
-    constexpr int HW = TC_BN / 2;
-    float* crow = s_c + rl * TC_CPAD + half * HW;
+    // epilogue: warp w reads TMEM lanes [32 (w % 4), +32) (its lane quarter =
+    // tile rows) and handles the columns [32 (w / 4), +32); the entries of C are
+    // loaded while the products run
+    constexpr int NC = TC_BN / 4;
+    const int quarter = warp & 3, cg = warp >> 2;
     int i = 0;
     for (int t = blockIdx.x; t < n_items; t += gridDim.x, ++i) {
-      const Tile T = tile_of(t);
-      const FrontDev f = c.fronts[T.front];
-      float* __restrict__ G = c.a32 + f.off;
-      const int n = T.n;
-      const int row = T.R0 + rl;
-      const int cbase = T.C0 + half * HW;
-      const int jmax = lower_only ? min(n, row + 1) : n;     // columns < jmax are stored
-#pragma unroll 1
-      for (int j0 = 0; j0 < HW; j0 += 16) {
-        float v[16];
+      const Item it = items[t];
+      const FrontDev& f = c.fronts[it.front];
+      const int n = f.n, base = it.a + min(nbo, f.fs - it.a);
+      const int row = base + it.b * TC_BM + quarter * 32 + lane, c0 = base + it.c * TC_BN + cg * NC;
+      // columns c0 + j, j < cend, of this thread's row are updated
+      const int cend = row < n ? (lower_only ? min(n, row + 1) : n) - c0 : 0;
+      float* __restrict__ G = c.a32 + f.off + row + (int64_t)c0 * n;
+      float v[NC];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const int col = cbase + j0 + q;
-          v[q] = (row < n && col < jmax) ? __ldcg(G + row + (int64_t)col * n) : 0.0f;
-        }
-#pragma unroll
-        for (int q = 0; q < 16; ++q) crow[j0 + q] = v[q];
-      }
+      for (int j = 0; j < NC; ++j) v[j] = j < cend ? __ldcg(G + (int64_t)j * n) : 0.0f;
       const int b = i & 1, u = i >> 1;
-      const bool ok = mbar_wait(smem_u32(&acc_full[b]), u & 1, s_abort, err);
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_full[b]), u & 1, s_abort, err));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      float outv[HW / 32][32];
-#pragma unroll
-      for (int cc = 0; cc < HW / 32; ++cc) {
-        uint32_t v[32];
-        TC_LD32(tmem + ((uint32_t)(quarter * 32) << 16) + b * TC_BN + half * HW + cc * 32, v);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-        for (int j = 0; j < 32; ++j) outv[cc][j] = crow[cc * 32 + j] - __uint_as_float(v[j]);
-      }
+      uint32_t a[NC];
+      TC_LD32(tmem + ((uint32_t)(quarter * 32) << 16) + b * TC_BN + cg * NC, a);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       // accumulator b may be overwritten from here on
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      mbar_arrive(smem_u32(&acc_empty[b]));
-      if (!*s_abort && row < n) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&acc_empty[b]));
+      if (!*s_abort) {
 #pragma unroll
-        for (int cc = 0; cc < HW / 32; ++cc)
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int col = cbase + cc * 32 + j;
-            if (col < jmax) G[row + (int64_t)col * n] = outv[cc][j];
-          }
+        for (int j = 0; j < NC; ++j)
+          if (j < cend) G[(int64_t)j * n] = v[j] - __uint_as_float(a[j]);
       }
     }
   }
@@ -350,9 +328,10 @@ void launch_tc_pack(const DevCtx& c, const Item* items, int n_items, int nbo, in
 }
 
 void launch_tc_syrk(const DevCtx& c, const CUtensorMap& wsmap, const int64_t* ws_off,
-                    const int64_t* ws_stride, const Item* items, int n_items, int nbo, int nterms,
+                    const int64_t* ws_stride, const Item* items, int n_items, int nbo, int parts, int pb0, int nterms,
                     uint32_t term_code, int lower_only, int* err, cudaStream_t s) {
   if (!n_items) return;
+  if (parts < 1 || 2 * parts * TC_TILE_BYTES > TC_RING) throw std::invalid_argument("tc_syrk: 1 to 6 operand parts");
   static int n_sm = 0;
   if (!n_sm) {
     int dev = 0;
@@ -362,7 +341,7 @@ void launch_tc_syrk(const DevCtx& c, const CUtensorMap& wsmap, const int64_t* ws
   }
   cudaFuncSetAttribute(k_tc_syrk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
   const int grid = n_items < n_sm ? n_items : n_sm;   // one persistent CTA per SM
-  k_tc_syrk<<<grid, TC_THREADS, TC_SMEM, s>>>(c, wsmap, ws_off, ws_stride, items, n_items, nbo, nterms,
+  k_tc_syrk<<<grid, TC_THREADS, TC_SMEM, s>>>(c, wsmap, ws_off, ws_stride, items, n_items, nbo, parts, pb0, nterms,
                                               term_code, lower_only, err);
 }
 
