@@ -106,6 +106,20 @@ def test_lu_right_hand_sides(native_lib, method, n_rhs):
     assert np.abs(x - ref).max() <= 3 * 729 * U["fp64"] * 40 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("n_rhs", [2, 3, 5, 16])
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_cholesky_right_hand_sides(native_lib, prec, n_rhs):
+    """Groups of one, two and four right-hand sides (the last one ragged) through
+    the flag-driven Cholesky solves, ragged last blocks; the tolerance of _check."""
+    m, leaves, mats, rhs = _mesh(300, 129, True, 32, n_rhs)
+    if prec == "fp32":
+        m.set_mode(1, api.PREC_FP32, 1e-12, 10)
+    m.factor(uo.CHOL)
+    m.solve(uo.CHOL)
+    x, ref = _solutions(m, 300, 129, mats, rhs)
+    assert np.abs(x - ref).max() <= 3e-10 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("fs,ss", SIZES)
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_cholesky_front(native_lib, prec, fs, ss):

@@ -1642,8 +1642,8 @@ void Engine::build_programs(int method) {
         large.clear();
       }
       if (nr <= NR_FLAGS_MAX && !large.empty()) {
-        // one flag-driven launch for every large front of this level (per
-        // group of FLAG_NR right-hand sides)
+        // one flag-driven launch for every large front of this level (256-row
+        // CTAs: per group of FLAG_NR right-hand sides)
         std::vector<Item> fi, ai;
         const int RB = chol ? tune.solve_rows : 64;     // rows per CTA: 64 (k_fwd_flags) or 256 (k_fwd_flags4)
         const int per = RB / NB;
@@ -1658,14 +1658,9 @@ void Engine::build_programs(int method) {
           for (int k = 0; k * RB < f.ss; ++k) ai.push_back(Item{s, nfbr + k, 0, 0});
         }
         fi.insert(fi.end(), ai.begin(), ai.end());
-        int f0 = 1 << 30, f1 = 0;
-        for (int s : large) {
-          f0 = std::min(f0, fronts[s].flag_off);
-          f1 = std::max(f1, fronts[s].flag_off + (fronts[s].fs + NB - 1) / NB);
-        }
         const int64_t io = add_items(fi);
-        for (int q0 = 0; q0 < nr; q0 += FLAG_NR) {
-          Op op{OP_FWD_FLAGS, dt, f1 - f0, f0, io, (int)fi.size()};
+        for (int q0 = 0; q0 < nr; q0 += RB == 64 ? nr : FLAG_NR) {
+          Op op{OP_FWD_FLAGS, dt, 0, 0, io, (int)fi.size()};
           op.q0 = q0;
           op.aux = RB;
           fwd_ops.push_back(op);
@@ -1720,19 +1715,7 @@ void Engine::build_programs(int method) {
         for (int b = maxb - 1; b >= 0; --b)
           for (int s : large)
             if (b < ((fronts[s].fs + NB - 1) / NB + per - 1) / per) bi.push_back(Item{s, b, 0, 0});
-        int f0 = 1 << 30, f1 = 0;
-        for (int s : large) {
-          f0 = std::min(f0, fronts[s].flag_off);
-          f1 = std::max(f1, fronts[s].flag_off + (fronts[s].fs + NB - 1) / NB);
-        }
-        const int64_t io = add_items(bi);
-        const int qstep = chol && dt == F64 ? FLAG_NR_BWD_F64 : FLAG_NR;
-        for (int q0 = 0; q0 < nr; q0 += qstep) {
-          Op op{OP_BWD_FLAGS, dt, f1 - f0, f0, io, (int)bi.size()};
-          op.q0 = q0;
-          op.aux = NB;
-          bwd_ops.push_back(op);
-        }
+        push(bwd_ops, OP_BWD_FLAGS, dt, 0, 0, bi);
       }
       push(bwd_ops, OP_BWD_STORE, dt, 0, gm, st);
     }
@@ -2055,19 +2038,14 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
         if (op.aux == 256)
           launch_fwd_flags4(ctx, it, op.n_items, op.dtype, d_ticket, d_err, op.q0, st);
         else
-          launch_fwd_flags(ctx, it, op.n_items, op.dtype, d_ticket, ctx.flags + op.param, op.nb, d_err, op.q0,
-                           st);
+          launch_fwd_flags(ctx, it, op.n_items, op.dtype, d_ticket, d_err, st);
         break;
       case OP_FWD_CHAIN: launch_fwd_chain(ctx, it, op.n_items, d_ticket, d_err, op.q0, st); break;
       case OP_BWD_CHAIN: launch_bwd_chain(ctx, it, op.n_items, d_ticket, d_err, op.q0, st); break;
       case OP_LU_DINV: launch_lu_dinv(ctx, it, op.n_items, op.dtype, st); break;
       case OP_BWD_FLAGS:
-        if (!ctx.symmetric) {
-          launch_lu_bwd_flags(ctx, it, op.n_items, op.dtype, d_ticket, d_err, op.q0, st);
-          break;
-        }
-        launch_bwd_flags(ctx, it, op.n_items, op.dtype, d_ticket, ctx.flags + op.param, op.nb, d_err, op.q0,
-                           st);
+        if (!ctx.symmetric) launch_lu_bwd_flags(ctx, it, op.n_items, op.dtype, d_ticket, d_err, st);
+        else launch_bwd_flags(ctx, it, op.n_items, op.dtype, d_ticket, d_err, st);
         break;
       case OP_TC_PACK:
         launch_tc_pack(ctx, it, op.n_items, op.nb, op.param, d_ws, d_ws_off, d_ws_stride, op.q0, op.aux, st);

@@ -643,7 +643,7 @@ namespace uhm_gpu {
 // with L_bb^{-1} precomputed at factorisation (64 x 64, dinv arenas).
 // ===========================================================================
 constexpr int FB = 64;
-constexpr int SF_NR = FLAG_NR;    // right-hand sides handled by one launch
+constexpr int SF_NR = FLAG_NR;    // right-hand sides per launch (256-row and chain kernels)
 
 UHM_DEFINE_WAIT_LIMIT(set_wait_limit_solve, 1u << 22)
 
@@ -687,7 +687,7 @@ int solve_wait_where() {
   return v;
 }
 
-// Warp 0 of a CTA: the 64 hand-off words of one block and right-hand side
+// One warp: the 64 hand-off words of one block and right-hand side
 // (entries lane and lane + 32; entries at or past kb read as 0).
 struct HandWords {
   unsigned long long w0, w1;
@@ -724,10 +724,32 @@ struct HandWords {
   }
 };
 
+// The hand-off words of one block for NQ right-hand sides: warp q < nq polls and
+// stages right-hand side q (with one warp polling them in turn, each took a round
+// trip of its own on the chain of hand-offs).
+struct HandWarp {
+  HandWords hw;
+  bool mine, live;       // live: false once a wait has run out (no more waiting)
+  const double* base;    // this warp's right-hand side
+  __device__ __forceinline__ HandWarp(const double* slab, int n, int q0, int nq) {
+    const int q = threadIdx.x >> 5;
+    mine = live = q < nq;
+    base = slab + (int64_t)(q0 + (mine ? q : 0)) * n;
+  }
+  __device__ __forceinline__ void load(int j, int kb) {
+    if (mine) hw.load(base + j * FB, kb);
+  }
+  template <typename CT, int NQ>
+  __device__ __forceinline__ void take(int j, int kb, int* err, int where, CT (&dst)[NQ][FB]) {
+    if (!mine) return;
+    if (live) live = hw.wait(base + j * FB, kb, err, where);
+    hw.stage(dst[threadIdx.x >> 5]);
+  }
+};
+
 // acc[q] += sum over the column blocks j < jend of L[row, block j] y_j for
 // the CTA's rows (thread: row lane tid % 64, column group tid / 64), y_j read
-// from its hand-off words: warp 0 polls and stages them (the next block's
-// words already in flight), the other warps wait at the block barrier.
+// from its hand-off words (HandWarp), the other warps waiting at the block barrier.
 template <typename T, int NQ>
 __device__ __forceinline__ void fwd_gather_blocks(const DevCtx& c, const FrontDev& f, int row, bool rv, int jend,
                                                   int q0, int nq, int* err, T (&acc)[NQ], T (*ysh)[NQ][FB]) {
@@ -746,30 +768,17 @@ __device__ __forceinline__ void fwd_gather_blocks(const DevCtx& c, const FrontDe
       tile[u] = (rv && cc < kbj) ? (CT)G[row + (int64_t)(j * FB + cc) * n] : CT(0);
     }
   };
-  const bool w0 = threadIdx.x < 32;
-  HandWords hw;
-  bool live = true;      // warp 0: false once a wait has run out (no more waiting)
+  HandWarp hand(y, n, q0, nq);
   if (jend > 0) {
     load_tile(0);
-    if (w0) hw.load(y + (int64_t)q0 * n, min(FB, fs));
+    hand.load(0, min(FB, fs));
   }
   for (int j = 0; j < jend; ++j) {
     const int buf = j & 1;
-    if (w0) {
-      // y_j is read by every later block of the front at once: one warp
-      // per CTA polls and stages it (the next block's words already in flight)
-      const int kbj = min(FB, fs - j * FB);
-      const double* yj = y + j * FB;
-      if (live) live = hw.wait(yj + (int64_t)q0 * n, kbj, err, wait_code(1, j, row / FB));
-      hw.stage(ysh[buf][0]);
-      for (int q = 1; q < nq; ++q) {
-        HandWords hq;
-        hq.load(yj + (int64_t)(q0 + q) * n, kbj);
-        if (live) live = hq.wait(yj + (int64_t)(q0 + q) * n, kbj, err, wait_code(1, j, row / FB));
-        hq.stage(ysh[buf][q]);
-      }
-      if (j + 1 < jend) hw.load(y + (j + 1) * FB + (int64_t)q0 * n, min(FB, fs - (j + 1) * FB));
-    }
+    // y_j is read by every later block of the front at once: one warp per CTA
+    // and right-hand side polls and stages it (the next block's words already in flight)
+    hand.take(j, min(FB, fs - j * FB), err, wait_code(1, j, row / FB), ysh[buf]);
+    if (j + 1 < jend) hand.load(j + 1, min(FB, fs - (j + 1) * FB));
     CT cur[16];
 #pragma unroll
     for (int u = 0; u < 16; ++u) cur[u] = tile[u];
@@ -785,13 +794,11 @@ __device__ __forceinline__ void fwd_gather_blocks(const DevCtx& c, const FrontDe
 }
 
 // item: front, a = block index (factor blocks 0..nfb-1, ABL blocks nfb..);
-// right-hand sides q0 .. q0+nq-1, nq <= NQ <= SF_NR (more are solved by
-// further launches); NQ is the launch's right-hand sides rounded up to 1, 2
-// or 4, so that a launch for one right-hand side issues no products for
-// absent ones
+// a CTA per group of NQ right-hand sides (flags_nq), so that a launch for one
+// right-hand side issues no products for absent ones
 template <typename T, int NQ>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_fwd_flags(DevCtx c, const Item* __restrict__ items,
-                                                   int* ticket, int* err, int q0) {
+                                                   int* ticket, int* err, int ng) {
   using CT = T;
   __shared__ int s_t;
   __shared__ CT red[4][FB][NQ];
@@ -801,7 +808,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_fwd_flags(DevCt
   __shared__ CT ysh[2][NQ][FB];
   if (threadIdx.x == 0) s_t = atomicAdd(ticket, 1);
   __syncthreads();
-  const Item it = items[s_t];
+  const Item it = items[s_t / ng];
+  const int q0 = (s_t % ng) * NQ;
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, fs = f.fs, nr = c.n_rhs, b = it.a;
   const int nq = min(NQ, nr - q0);
@@ -1083,232 +1091,222 @@ void launch_fwd_flags4(const DevCtx& c, const Item* items, int n_items, int dtyp
   }
 }
 
-// acc[q][u] += sum over the rows r below the factor block (the ABL rows, x
-// known from the parent, then the factor blocks j = nfb - 1 down to stop + 1
-// as their hand-off words arrive) of L[r, 64 b + 16 g + u] x_r, for column
-// block b (thread: row lane tid % 64, column group tid / 64).  Warp 0 polls
-// and stages x_j (the next block's words already in flight).
+// Backward: item: front, a = factor block index, tickets in descending block
+// order, a CTA per group of NQ right-hand sides.  The 64-row blocks below the
+// factor block, the ABL rows (x known from the parent) first, then the factor
+// blocks from the last one up as their hand-off words arrive, pass through two
+// shared-memory tiles: loaded by rows (a warp's loads are consecutive rows of a
+// column), a block ahead in registers, and read by columns, so that a thread
+// sums a quarter of one column per right-hand side in NQ registers.  (With 16 NQ
+// sums per thread, one row each, only one CTA fitted an SM, and adding the 64 rows
+// up was on the chain of hand-offs.)
 template <typename T, int NQ>
-__device__ __forceinline__ void bwd_gather_rows(const DevCtx& c, const FrontDev& f, int b, int stop, int q0, int nq,
-                                                int* err, T (&acc)[NQ][16], T (*xsh)[NQ][FB]) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_bwd_flags(DevCtx c, const Item* __restrict__ items,
+                                                   int* ticket, int* err, int ng) {
   using CT = T;
-  const int n = f.n, fs = f.fs, nr = c.n_rhs;
-  const int nfb = (fs + FB - 1) / FB;
-  const int c0 = b * FB, kb = min(FB, fs - c0);
-  const T* __restrict__ G = arena<T>(c) + f.off;
-  const double* __restrict__ hx = c.vec + f.voff;                  // hand-off: the z slab's factor rows
-  const double* __restrict__ y = hx + (int64_t)n * nr;
-  const int rl = threadIdx.x % FB, g = threadIdx.x / FB;
-  // rows below block b: the ABL part (known) first, two row blocks per
-  // round with all loads issued before the arithmetic, then factor blocks
-  // from the last one down (they complete in that order)
-  for (int rs = fs; rs < n; rs += 2 * FB) {
-    CT xr[2][NQ], gv[2][16];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = rs + h * FB + rl;
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) xr[h][q] = (r < n && q < nq) ? (CT)y[r + (int64_t)(q0 + q) * n] : CT(0);
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int cc = g * 16 + u;
-        gv[h][u] = (r < n && cc < kb) ? (CT)G[r + (int64_t)(c0 + cc) * n] : CT(0);
-      }
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int u = 0; u < 16; ++u)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) acc[q][u] += gv[h][u] * xr[h][q];
-  }
-  // the factor tile of row block j does not depend on x: loaded one block
-  // ahead, so that only the loads of x_j follow the wait
-  CT tile[16];
-  auto load_tile = [&](int j) {
-    const int r = j * FB + rl;
-    const bool in = r < min(j * FB + FB, fs);
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int cc = g * 16 + u;
-      tile[u] = (in && cc < kb) ? (CT)G[r + (int64_t)(c0 + cc) * n] : CT(0);
-    }
-  };
-  const bool w0 = threadIdx.x < 32;
-  HandWords hw;
-  bool live = true;      // warp 0: false once a wait has run out (no more waiting)
-  if (nfb - 1 > stop) {
-    load_tile(nfb - 1);
-    if (w0) hw.load(hx + (nfb - 1) * FB + (int64_t)q0 * n, min(FB, fs - (nfb - 1) * FB));
-  }
-  for (int j = nfb - 1, k = 0; j > stop; --j, ++k) {
-    const int buf = k & 1;
-    if (w0) {
-      const int kbj = min(FB, fs - j * FB);
-      const double* xj = hx + j * FB;
-      if (live) live = hw.wait(xj + (int64_t)q0 * n, kbj, err, wait_code(2, j, b));
-      hw.stage(xsh[buf][0]);
-      for (int q = 1; q < nq; ++q) {
-        HandWords hq;
-        hq.load(xj + (int64_t)(q0 + q) * n, kbj);
-        if (live) live = hq.wait(xj + (int64_t)(q0 + q) * n, kbj, err, wait_code(2, j, b));
-        hq.stage(xsh[buf][q]);
-      }
-      if (j - 1 > stop) hw.load(hx + (j - 1) * FB + (int64_t)q0 * n, min(FB, fs - (j - 1) * FB));
-    }
-    CT cur[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) cur[u] = tile[u];
-    if (j - 1 > stop) load_tile(j - 1);
-    __syncthreads();
-    const int r = j * FB + rl;
-    if (r < min(j * FB + FB, fs)) {
-#pragma unroll
-      for (int u = 0; u < 16; ++u)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) acc[q][u] += cur[u] * xsh[buf][q][rl];
-    }
-  }
-}
-
-// item: front, a = factor block index, tickets in descending block order;
-// right-hand sides q0 .. q0+NQ-1, accumulated in the same pass over the
-// factor tiles (a pass per right-hand side would put NQ-1 un-overlapped
-// re-reads of the whole block column on the chain of hand-offs)
-template <typename T, int NQ>
-__global__ void __launch_bounds__(256) k_bwd_flags(DevCtx c, const Item* __restrict__ items,
-                                                   int* ticket, int* err, int q0) {
-  using CT = T;
-  __shared__ int s_t;
   extern __shared__ __align__(16) unsigned char bwd_dyn[];
-  CT (*red)[FB + 1] = reinterpret_cast<CT (*)[FB + 1]>(bwd_dyn);   // [row lane][column]
+  CT (*ts)[FB][FB + 1] = reinterpret_cast<CT (*)[FB][FB + 1]>(bwd_dyn);      // two tiles [row][column]
+  CT* dsh = reinterpret_cast<CT*>(bwd_dyn) + 2 * FB * (FB + 1);             // inverse diagonal block
+  __shared__ int s_t;
+  __shared__ CT red[4][FB][NQ];
   __shared__ CT v[FB][NQ];
-  __shared__ T dsh[FB * (FB + 1)];
-  // x_j staged by warp 0, two buffers alternating by block: one barrier per block
   __shared__ CT xsh[2][NQ][FB];
   if (threadIdx.x == 0) s_t = atomicAdd(ticket, 1);
   __syncthreads();
-  const Item it = items[s_t];
+  const Item it = items[s_t / ng];
+  const int q0 = (s_t % ng) * NQ;
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, fs = f.fs, nr = c.n_rhs, b = it.a;
-  const int nq = min(NQ, nr - q0);
+  const int nq = min(NQ, nr - q0), nfb = (fs + FB - 1) / FB;
   const int c0 = b * FB, kb = min(FB, fs - c0);
+  const T* __restrict__ G = arena<T>(c) + f.off;
   {
     const T* __restrict__ Dg = dinv_arena<T>(c) + f.dinv_off + (int64_t)b * FB * FB;
     for (int idx = threadIdx.x; idx < FB * FB; idx += 256) dsh[(idx / FB) * (FB + 1) + idx % FB] = Dg[idx];
   }
   double* __restrict__ hx = c.vec + f.voff;                  // hand-off: the z slab's factor rows
   double* __restrict__ y = hx + (int64_t)n * nr;
-  const int rl = threadIdx.x % FB, g = threadIdx.x / FB;   // row lane, column group
-  CT acc[NQ][16];
-#pragma unroll
-  for (int q = 0; q < NQ; ++q)
-#pragma unroll
-    for (int u = 0; u < 16; ++u) acc[q][u] = CT(0);
-  // this block's right-hand sides, loaded before any wait
-  CT yb[NQ];
-#pragma unroll
-  for (int q = 0; q < NQ; ++q)
-    yb[q] = (threadIdx.x < kb && q < nq) ? (CT)y[c0 + threadIdx.x + (int64_t)(q0 + q) * n] : CT(0);
-  bwd_gather_rows<T, NQ>(c, f, b, b, q0, nq, err, acc, xsh);
-  // the column sums over the 64 row lanes: four parts of 16 rows on all
-  // 256 threads (the loads issued together), then the parts in order
-  __shared__ CT part[4][FB];
+  // thread: column i (row i of a tile when loading), quarter g
+  const int i = threadIdx.x % FB, g = threadIdx.x / FB;
+  CT acc[NQ], yb[NQ];
 #pragma unroll
   for (int q = 0; q < NQ; ++q) {
+    acc[q] = CT(0);
+    // this block's right-hand sides, loaded before any wait
+    yb[q] = (threadIdx.x < kb && q < nq) ? (CT)y[c0 + threadIdx.x + (int64_t)(q0 + q) * n] : CT(0);
+  }
+  // FP64: the ABL rows without the tiles, a row per thread and 16 columns, the
+  // rows added up before any wait (the tiles' barriers and 64-bit accesses cost the
+  // levels that are bound by the FP64 products a quarter of their time)
+  constexpr bool ROWS = sizeof(T) == 8 && NQ == 1;
+  if constexpr (ROWS) {
+    if (fs < n) {
+      CT ar[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) ar[u] = CT(0);
+      for (int rs = fs; rs < n; rs += 2 * FB) {
+        CT xr[2], gv[2][16];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = rs + h * FB + i;
+          xr[h] = r < n ? (CT)y[r + (int64_t)q0 * n] : CT(0);
+#pragma unroll
+          for (int u = 0; u < 16; ++u) {
+            const int cc = g * 16 + u;
+            gv[h][u] = (r < n && cc < kb) ? (CT)G[r + (int64_t)(c0 + cc) * n] : CT(0);
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int u = 0; u < 16; ++u) ar[u] += gv[h][u] * xr[h];
+      }
+#pragma unroll
+      for (int u = 0; u < 16; ++u) ts[1][i][g * 16 + u] = ar[u];
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < 16; ++r) acc[0] += ts[1][g * 16 + r][i];
+    }
+  }
+  const int na = ROWS ? 0 : (n - fs + FB - 1) / FB, nblk = na + nfb - 1 - b;
+  auto first_row = [&](int k) { return k < na ? fs + k * FB : (nfb - 1 - (k - na)) * FB; };
+  auto rows_of = [&](int k) { return min(FB, (k < na ? n : fs) - first_row(k)); };
+  CT tile[16];
+  auto load_tile = [&](int k) {
+    const int r = first_row(k) + i;
+    const bool in = i < rows_of(k);
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int cc = g * 16 + u;
+      tile[u] = (in && cc < kb) ? (CT)G[r + (int64_t)(c0 + cc) * n] : CT(0);
+    }
+  };
+  HandWarp hand(hx, n, q0, nq);
+  const double* const ya = y + (int64_t)(q0 + (hand.mine ? threadIdx.x >> 5 : 0)) * n;
+  const int lane = threadIdx.x & 31;
+  auto load_x = [&](int k) {
+    if (!hand.mine) return;
+    const int r = first_row(k), m = rows_of(k);
+    if (k < na) {
+      hand.hw.w0 = lane < m ? (unsigned long long)__double_as_longlong(ya[r + lane]) : 0ull;
+      hand.hw.w1 = lane + 32 < m ? (unsigned long long)__double_as_longlong(ya[r + lane + 32]) : 0ull;
+    } else {
+      hand.hw.load(hand.base + r, m);
+    }
+  };
+  if (nblk > 0) {
+    load_tile(0);
+    load_x(0);
+  }
+  for (int k = 0; k < nblk; ++k) {
+    const int buf = k & 1;
+#pragma unroll
+    for (int u = 0; u < 16; ++u) ts[buf][i][g * 16 + u] = tile[u];
+    if (k + 1 < nblk) load_tile(k + 1);
+    if (hand.mine) {
+      const int r = first_row(k);
+      if (k >= na && hand.live) hand.live = hand.hw.wait(hand.base + r, rows_of(k), err, wait_code(2, r / FB, b));
+      hand.hw.stage(xsh[buf][threadIdx.x >> 5]);
+    }
+    if (k + 1 < nblk) load_x(k + 1);
     __syncthreads();
 #pragma unroll
-    for (int u = 0; u < 16; ++u) red[rl][g * 16 + u] = acc[q][u];
-    __syncthreads();
-    {
-      const int col = threadIdx.x % FB, pr = threadIdx.x / FB;
-      CT sp = CT(0);
+    for (int u = 0; u < 16; ++u) {
+      const CT t = ts[buf][g * 16 + u][i];
 #pragma unroll
-      for (int r = 0; r < 16; ++r) sp += red[16 * pr + r][col];
-      part[pr][col] = sp;
+      for (int q = 0; q < NQ; ++q) acc[q] += t * xsh[buf][q][g * 16 + u];
     }
-    __syncthreads();
-    if (threadIdx.x < FB) {
-      const CT sum = part[0][threadIdx.x] + part[1][threadIdx.x] + part[2][threadIdx.x] + part[3][threadIdx.x];
-      v[threadIdx.x][q] = (threadIdx.x < kb && q < nq) ? yb[q] - sum : CT(0);
-    }
+  }
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) red[g][i][q] = acc[q];
+  __syncthreads();
+  if (threadIdx.x < FB) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+      v[i][q] = (i < kb && q < nq) ? yb[q] - (red[0][i][q] + red[1][i][q] + red[2][i][q] + red[3][i][q]) : CT(0);
   }
   __syncthreads();
   // x = Dinv^T v : x_i = sum_{t >= i} Dinv[t, i] v_t   (column i of Dinv, staged at start),
-  // on all 256 threads: group gg sums t in [16 gg, 16 gg + 16), partial sums
-  // added in group order
-  {
-    const int ii = threadIdx.x % FB, gg = threadIdx.x / FB;
+  // on all 256 threads: group g sums t in [16 g, 16 g + 16), partial sums
+  // added in group order; Dinv[t][i] is zero for t < i and past kb: the
+  // unbranched sum is exact
+  CT xp[NQ];
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      CT xp = CT(0);
-      // Dinv[t][ii] is zero for t < ii and past kb: the unbranched sum is exact
+  for (int q = 0; q < NQ; ++q) xp[q] = CT(0);
 #pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int t = gg * 16 + u;
-        xp += (CT)dsh[ii * (FB + 1) + t] * v[t][q];
-      }
-      red[gg * NQ + q][ii] = xp;
-    }
+  for (int u = 0; u < 16; ++u) {
+    const CT d = dsh[i * (FB + 1) + g * 16 + u];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) xp[q] += d * v[g * 16 + u][q];
   }
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) red[g][i][q] = xp[q];
   __syncthreads();
   if (threadIdx.x < kb) {
-    const int ii = threadIdx.x;
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
       if (q >= nq) break;
-      const double x = (double)(red[q][ii] + red[NQ + q][ii] + red[2 * NQ + q][ii] + red[3 * NQ + q][ii]);
-      y[c0 + ii + (int64_t)(q0 + q) * n] = x;
-      st_hand(hx + c0 + ii + (int64_t)(q0 + q) * n, x);
+      const double x = (double)(red[0][i][q] + red[1][i][q] + red[2][i][q] + red[3][i][q]);
+      y[c0 + i + (int64_t)(q0 + q) * n] = x;
+      st_hand(hx + c0 + i + (int64_t)(q0 + q) * n, x);
     }
   }
 }
 
-void launch_fwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket,
-                      int* flag_base, int n_flags, int* err, int q0, cudaStream_t s) {
-  if (!n_items) return;
-  (void)flag_base; (void)n_flags;     // hand-off words, no flags
-  cudaMemsetAsync(ticket, 0, sizeof(int), s);
-  const int nq = c.n_rhs - q0 < FLAG_NR ? c.n_rhs - q0 : FLAG_NR;
-  // NQ covers every right-hand side of the group (3 of them take the 4-wide kernel)
-  if (dtype == F64) {
-    if (nq >= 3) k_fwd_flags<double, 4><<<n_items, 256, 0, s>>>(c, items, ticket, err, q0);
-    else if (nq == 2) k_fwd_flags<double, 2><<<n_items, 256, 0, s>>>(c, items, ticket, err, q0);
-    else k_fwd_flags<double, 1><<<n_items, 256, 0, s>>>(c, items, ticket, err, q0);
-  } else {
-    if (nq >= 3) k_fwd_flags<float, 4><<<n_items, 256, 0, s>>>(c, items, ticket, err, q0);
-    else if (nq == 2) k_fwd_flags<float, 2><<<n_items, 256, 0, s>>>(c, items, ticket, err, q0);
-    else k_fwd_flags<float, 1><<<n_items, 256, 0, s>>>(c, items, ticket, err, q0);
+// Right-hand sides per CTA; the other groups run beside it (consecutive
+// tickets: their reads of a tile of the factor meet in L2).  FP64: one, since its
+// products, 64 x 64 per block and right-hand side at about 1.1 us each, are
+// on the chain of hand-offs twice per block.  FP32: up to four (with eight the
+// levels of large fronts took 543 instead of 351 us forward and 316 instead of 195
+// backward, those of many fronts 120 to 300 instead of 160 to 340).
+// Measured on GB300, a launch per group before, forward and backward: 12^3 p = 4
+// FP64, 4 right-hand sides, root 12,698 rows: 2.69 + 3.86 -> 1.30 + 1.42 ms; FP32, 16
+// right-hand sides, 11,427 fronts up to 6,938 rows, two solves: 6.8 + 10.3 -> 2.1 +
+// 2.4; one right-hand side, 16^3 p = 4 FP64: 1.15 + 1.52 -> 1.15 + 1.35.
+template <typename T> static int flags_nq(int nr) { return sizeof(T) == 8 || nr == 1 ? 1 : nr == 2 ? 2 : 4; }
+
+template <typename T>
+static void fwd_flags_t(const DevCtx& c, const Item* items, int n_items, int* ticket, int* err, cudaStream_t s) {
+  const int nq = flags_nq<T>(c.n_rhs), ng = (c.n_rhs + nq - 1) / nq;
+  if (nq == 1) k_fwd_flags<T, 1><<<n_items * ng, 256, 0, s>>>(c, items, ticket, err, ng);
+  else if constexpr (sizeof(T) == 4) {
+    if (nq == 2) k_fwd_flags<T, 2><<<n_items * ng, 256, 0, s>>>(c, items, ticket, err, ng);
+    else k_fwd_flags<T, 4><<<n_items * ng, 256, 0, s>>>(c, items, ticket, err, ng);
   }
 }
 
+void launch_fwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket, int* err,
+                      cudaStream_t s) {
+  if (!n_items) return;
+  cudaMemsetAsync(ticket, 0, sizeof(int), s);
+  if (dtype == F64) fwd_flags_t<double>(c, items, n_items, ticket, err, s);
+  else fwd_flags_t<float>(c, items, n_items, ticket, err, s);
+}
+
 template <typename T, int NQ>
-static void bwd_flags_nq(const DevCtx& c, const Item* items, int n_items, int* ticket, int* err, int q0,
+static void bwd_flags_nq(const DevCtx& c, const Item* items, int n_items, int* ticket, int* err, int ng,
                          cudaStream_t s) {
-  const size_t dyn = sizeof(T) * FB * (FB + 1);
+  const size_t dyn = 3 * sizeof(T) * FB * (FB + 1);
   cudaFuncSetAttribute(k_bwd_flags<T, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-  k_bwd_flags<T, NQ><<<n_items, 256, dyn, s>>>(c, items, ticket, err, q0);
+  k_bwd_flags<T, NQ><<<n_items * ng, 256, dyn, s>>>(c, items, ticket, err, ng);
 }
 
 template <typename T>
-static void bwd_flags_t(const DevCtx& c, const Item* items, int n_items, int* ticket, int* err, int q0,
-                        int nq, cudaStream_t s) {
-  if (nq >= 3) bwd_flags_nq<T, 4>(c, items, n_items, ticket, err, q0, s);
-  else if (nq == 2) bwd_flags_nq<T, 2>(c, items, n_items, ticket, err, q0, s);
-  else bwd_flags_nq<T, 1>(c, items, n_items, ticket, err, q0, s);
+static void bwd_flags_t(const DevCtx& c, const Item* items, int n_items, int* ticket, int* err, cudaStream_t s) {
+  const int nq = flags_nq<T>(c.n_rhs), ng = (c.n_rhs + nq - 1) / nq;
+  if (nq == 1) bwd_flags_nq<T, 1>(c, items, n_items, ticket, err, ng, s);
+  else if constexpr (sizeof(T) == 4) {
+    if (nq == 2) bwd_flags_nq<T, 2>(c, items, n_items, ticket, err, ng, s);
+    else bwd_flags_nq<T, 4>(c, items, n_items, ticket, err, ng, s);
+  }
 }
 
-void launch_bwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket,
-                      int* flag_base, int n_flags, int* err, int q0, cudaStream_t s) {
+void launch_bwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket, int* err,
+                      cudaStream_t s) {
   if (!n_items) return;
-  (void)flag_base; (void)n_flags;     // hand-off words, no flags
   cudaMemsetAsync(ticket, 0, sizeof(int), s);
-  // right-hand sides of this launch: FLAG_NR, or FLAG_NR_BWD_F64 in FP64
-  // (register budget of the NQ x 16 accumulators)
-  const int grp = dtype == F64 ? FLAG_NR_BWD_F64 : FLAG_NR;
-  const int nq = c.n_rhs - q0 < grp ? c.n_rhs - q0 : grp;
-  if (dtype == F64) bwd_flags_t<double>(c, items, n_items, ticket, err, q0, nq, s);
-  else bwd_flags_t<float>(c, items, n_items, ticket, err, q0, nq, s);
+  if (dtype == F64) bwd_flags_t<double>(c, items, n_items, ticket, err, s);
+  else bwd_flags_t<float>(c, items, n_items, ticket, err, s);
 }
 
 // ===========================================================================
@@ -1324,7 +1322,7 @@ void launch_bwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype
 // ===========================================================================
 template <typename T, int NQ>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_lu_bwd_flags(DevCtx c, const Item* __restrict__ items,
-                                                                              int* ticket, int* err, int q0) {
+                                                                              int* ticket, int* err, int ng) {
   __shared__ int s_t;
   __shared__ T red[4][FB][NQ];
   __shared__ T v[FB][NQ];
@@ -1332,7 +1330,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_lu_bwd_flags(De
   __shared__ T xsh[2][NQ][FB];
   if (threadIdx.x == 0) s_t = atomicAdd(ticket, 1);
   __syncthreads();
-  const Item it = items[s_t];
+  const Item it = items[s_t / ng];
+  const int q0 = (s_t % ng) * NQ;
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, fs = f.fs, nr = c.n_rhs, b = it.a;
   const int nq = min(NQ, nr - q0), nfb = (fs + FB - 1) / FB;
@@ -1377,28 +1376,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_lu_bwd_flags(De
       tile[u] = (rv && cc < kbj) ? G[row + (int64_t)(j * FB + cc) * n] : T(0);
     }
   };
-  const bool w0 = threadIdx.x < 32;
-  HandWords hw;
-  bool live = true;      // warp 0: false once a wait has run out (no more waiting)
+  HandWarp hand(hx, n, q0, nq);
   if (nfb - 1 > b) {
     load_tile(nfb - 1);
-    if (w0) hw.load(hx + (nfb - 1) * FB + (int64_t)q0 * n, min(FB, fs - (nfb - 1) * FB));
+    hand.load(nfb - 1, min(FB, fs - (nfb - 1) * FB));
   }
   for (int j = nfb - 1; j > b; --j) {
     const int buf = j & 1;
-    if (w0) {
-      const int kbj = min(FB, fs - j * FB);
-      const double* xj = hx + j * FB;
-      if (live) live = hw.wait(xj + (int64_t)q0 * n, kbj, err, wait_code(2, j, b));
-      hw.stage(xsh[buf][0]);
-      for (int q = 1; q < nq; ++q) {
-        HandWords hq;
-        hq.load(xj + (int64_t)(q0 + q) * n, kbj);
-        if (live) live = hq.wait(xj + (int64_t)(q0 + q) * n, kbj, err, wait_code(2, j, b));
-        hq.stage(xsh[buf][q]);
-      }
-      if (j - 1 > b) hw.load(hx + (j - 1) * FB + (int64_t)q0 * n, min(FB, fs - (j - 1) * FB));
-    }
+    hand.take(j, min(FB, fs - j * FB), err, wait_code(2, j, b), xsh[buf]);
+    if (j - 1 > b) hand.load(j - 1, min(FB, fs - (j - 1) * FB));
     T cur[16];
 #pragma unroll
     for (int u = 0; u < 16; ++u) cur[u] = tile[u];
@@ -1445,20 +1431,21 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_lu_bwd_flags(De
 }
 
 template <typename T>
-static void lu_bwd_flags_t(const DevCtx& c, const Item* items, int n_items, int* ticket, int* err, int q0, int nq,
-                           cudaStream_t s) {
-  if (nq >= 3) k_lu_bwd_flags<T, 4><<<n_items, 256, 0, s>>>(c, items, ticket, err, q0);
-  else if (nq == 2) k_lu_bwd_flags<T, 2><<<n_items, 256, 0, s>>>(c, items, ticket, err, q0);
-  else k_lu_bwd_flags<T, 1><<<n_items, 256, 0, s>>>(c, items, ticket, err, q0);
+static void lu_bwd_flags_t(const DevCtx& c, const Item* items, int n_items, int* ticket, int* err, cudaStream_t s) {
+  const int nq = flags_nq<T>(c.n_rhs), ng = (c.n_rhs + nq - 1) / nq;
+  if (nq == 1) k_lu_bwd_flags<T, 1><<<n_items * ng, 256, 0, s>>>(c, items, ticket, err, ng);
+  else if constexpr (sizeof(T) == 4) {
+    if (nq == 2) k_lu_bwd_flags<T, 2><<<n_items * ng, 256, 0, s>>>(c, items, ticket, err, ng);
+    else k_lu_bwd_flags<T, 4><<<n_items * ng, 256, 0, s>>>(c, items, ticket, err, ng);
+  }
 }
 
-void launch_lu_bwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket, int* err, int q0,
+void launch_lu_bwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket, int* err,
                          cudaStream_t s) {
   if (!n_items) return;
   cudaMemsetAsync(ticket, 0, sizeof(int), s);
-  const int nq = c.n_rhs - q0 < FLAG_NR ? c.n_rhs - q0 : FLAG_NR;
-  if (dtype == F64) lu_bwd_flags_t<double>(c, items, n_items, ticket, err, q0, nq, s);
-  else lu_bwd_flags_t<float>(c, items, n_items, ticket, err, q0, nq, s);
+  if (dtype == F64) lu_bwd_flags_t<double>(c, items, n_items, ticket, err, s);
+  else lu_bwd_flags_t<float>(c, items, n_items, ticket, err, s);
 }
 
 // ===========================================================================

@@ -123,20 +123,19 @@ void launch_fwd_small(const DevCtx& c, const Item* items, int n_items, int dtype
                       int staged_bytes, cudaStream_t s);
 void launch_bwd_small(const DevCtx& c, const Item* items, int n_items, int dtype, int method,
                       double* g, int64_t ldg, int staged_bytes, cudaStream_t s);
-// flag-driven level solves of large Cholesky fronts (one launch per level and
-// group of FLAG_NR right-hand sides, starting at column q0): items ordered so
-// that every CTA waits only on CTAs with smaller tickets
-constexpr int FLAG_NR = 4;
-constexpr int FLAG_NR_BWD_F64 = 2;   // backward FP64 launches take two
-void launch_fwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket,
-                      int* flag_base, int n_flags, int* err, int q0, cudaStream_t s);
-// the same with 256-row CTAs (item a: 256-row block of the factor rows, then
+// flag-driven level solves of large fronts (one launch per level: the CTAs of
+// an item's groups of right-hand sides hold consecutive tickets): items ordered
+// so that every CTA waits only on CTAs with smaller tickets
+void launch_fwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket, int* err,
+                      cudaStream_t s);
+constexpr int FLAG_NR = 4;           // right-hand sides per launch of the kernels below
+// the same with 256-row CTAs and a launch per FLAG_NR right-hand sides from q0 on (item a: 256-row block of the factor rows, then
 // of ABL), each solving its own four 64-row blocks in turn; the same
 // hand-off words in and out
 void launch_fwd_flags4(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket, int* err, int q0,
                        cudaStream_t s);
-void launch_bwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket,
-                      int* flag_base, int n_flags, int* err, int q0, cudaStream_t s);
+void launch_bwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket, int* err,
+                      cudaStream_t s);
 // chain solves of large FP32 Cholesky fronts (one launch per level and group
 // of FLAG_NR right-hand sides).  Items: front, a = block, b = role: CH_CHAIN
 // (one per front, first), CH_HELPER (forward: row blocks b > CH_K in
@@ -160,7 +159,7 @@ int solve_wait_where();
 // and U (item: front, a = block; L's at dinv_off, U's behind them), and the
 // backward flag-driven solve (the forward one is launch_fwd_flags)
 void launch_lu_dinv(const DevCtx& c, const Item* items, int n_items, int dtype, cudaStream_t s);
-void launch_lu_bwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket, int* err, int q0,
+void launch_lu_bwd_flags(const DevCtx& c, const Item* items, int n_items, int dtype, int* ticket, int* err,
                          cudaStream_t s);
 void launch_bwd_prepare(const DevCtx& c, const Item* items, int n_items, int dtype, int method,
                         const double* g, int64_t ldg, cudaStream_t s);
