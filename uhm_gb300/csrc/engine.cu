@@ -27,9 +27,9 @@ static constexpr int LUROW_CB = 16;         // k_lu_row_update (k_factor.cu)
 static constexpr int LU_GOAL_F64 = 64, LU_GOAL_F32 = 192;
 // more rows than this per CTA of the largest cluster go to the whole GPU.
 // Measured on GB300 (us per 64-column panel): FP32, 16 CTAs, 115 at 100 rows each,
-// 172 at 384, 230 from 400 to 768, against 180 for the whole GPU from 6,200 to 9,800
-// rows and 195 at 14,911; FP64, 16 CTAs, 187 at 96 rows each, 205 at 128, 225 to 264
-// from 130 to 208, against 206 for the whole GPU from 2,100 to 3,300 rows and 230 at 6,938
+// 172 at 384, 230 from 400 to 768, against 155 to 170 for the whole GPU from 6,200 to 14,911
+// rows (four fronts at once: more); FP64, 16 CTAs, 187 at 96 rows each, 205 at 128, 225 to
+// 264 from 130 to 208, against 200 for the whole GPU from 2,100 to 3,300 rows and 218 at 6,938
 static constexpr int LU_CLUSTER_ROWS_F64 = 128, LU_CLUSTER_ROWS_F32 = 384;
 static constexpr int TILE = 64;             // trailing-update tile (k_tile_update)
 

@@ -1183,14 +1183,16 @@ void launch_getrf_panel(const DevCtx& c, const Item* items, int n_items, int dty
 // block barriers, one exchange, the reductions), then by the update's shared-
 // memory traffic (FP32) or multiply-adds (FP64).  Measured on GB300, the panels
 // of one factorisation, against a grid barrier on a counter per column: 24^3 p =
-// 3 FP32 141 + 2.5 (one-CTA panels in global memory) -> 59.4 ms, 12^3 p = 3
-// FP64 55.9 + 4.8 -> 24.2, 6^3 p = 3 4.9 + 2.0 -> 4.3.  The chunk by columns instead
+// 3 FP32 141 + 2.5 (one-CTA panels in global memory) -> 57.1 ms, 12^3 p = 3
+// FP64 55.9 + 4.8 -> 23.3, 6^3 p = 3 4.9 + 2.0 -> 4.3.  The chunk by columns instead
 // (one column of a row per access) took 69.0, 25.7 and 4.4: bank conflicts where a
-// row is read, and four times the shared-memory instructions.
+// row is read, and four times the shared-memory instructions.  !CL with each
+// candidate in front of its row and its two words polled one after the other: 59.4
+// and 24.2 (a panel of 152 CTAs 187 us FP32, 207 FP64, now 166 and 200).
 constexpr int GC_ERR = 3;
 constexpr int GC_POLL = (GC_MAX_CTAS + 31) / 32;
-constexpr int64_t GC_REC = 2 + 2 * 64;          // words of one record: candidate, then a row (two per FP64 value)
-static_assert(gc_words(1, 1) == 4 * GC_REC, "record size of the launcher's callers");
+constexpr int64_t GC_REC = 2 * 64;              // words of a row's record (two per FP64 value)
+static_assert(gc_words(1, 1) == 4 + 4 * GC_REC, "record size of the launcher's callers");
 
 UHM_DEFINE_WAIT_LIMIT(set_wait_limit_factor, 1u << 22)
 
@@ -1245,7 +1247,7 @@ __device__ __forceinline__ uint64_t gc_get(const uint64_t* p) {
 // words p[32 e + lane] (e < N, while < cnt), all loads in flight, until every
 // one carries the tag; false (and the error word set) when the wait gives up
 template <int N>
-__device__ __forceinline__ bool gc_poll(const uint64_t* p, int stride, int cnt, uint32_t tag, uint64_t (&x)[N], int* err) {
+__device__ __forceinline__ bool gc_poll(const uint64_t* p, int cnt, uint32_t tag, uint64_t (&x)[N], int* err) {
   const int lane = threadIdx.x & 31;
   const uint32_t lim = g_wait_limit;
   uint32_t open = 0;
@@ -1255,10 +1257,40 @@ __device__ __forceinline__ bool gc_poll(const uint64_t* p, int stride, int cnt, 
     uint64_t y[N];
 #pragma unroll
     for (int e = 0; e < N; ++e)
-      if ((open >> e) & 1) y[e] = gc_get(p + (int64_t)(lane + 32 * e) * stride);
+      if ((open >> e) & 1) y[e] = gc_get(p + lane + 32 * e);
 #pragma unroll
     for (int e = 0; e < N; ++e)
       if (((open >> e) & 1) && (uint32_t)(y[e] >> 56) == tag) { x[e] = y[e]; open &= ~(1u << e); }
+    if (!open) break;
+    if (i >= lim) { atomicExch(err, GC_ERR); return false; }
+    if ((i & 255) == 255 && *(volatile int*)err) return false;
+    if (i > 64) __nanosleep(20);
+  }
+  return true;
+}
+// the same for pairs of words: p[2 (32 e + lane)] and the word behind it
+template <int N>
+__device__ __forceinline__ bool gc_poll2(const uint64_t* p, int cnt, uint32_t tag, uint64_t (&x0)[N], uint64_t (&x1)[N],
+                                         int* err) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t lim = g_wait_limit;
+  uint32_t open = 0;
+#pragma unroll
+  for (int e = 0; e < N; ++e) open |= (lane + 32 * e < cnt ? 1u : 0u) << e;
+  for (uint32_t i = 0; open; ++i) {
+    uint64_t y0[N], y1[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+      if ((open >> e) & 1)
+        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                     : "=l"(y0[e]), "=l"(y1[e]) : "l"(p + 2 * (lane + 32 * e)) : "memory");
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+      if (((open >> e) & 1) && (uint32_t)(y0[e] >> 56) == tag && (uint32_t)(y1[e] >> 56) == tag) {
+        x0[e] = y0[e];
+        x1[e] = y1[e];
+        open &= ~(1u << e);
+      }
     if (!open) break;
     if (i >= lim) { atomicExch(err, GC_ERR); return false; }
     if ((i & 255) == 255 && *(volatile int*)err) return false;
@@ -1342,8 +1374,10 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
   const int rbeg = k0 + q * R, rend = min(rbeg + R, n);   // my rows [rbeg, rend)
   const int nr_my = max(0, rend - rbeg);
   T* __restrict__ G = arena<T>(c) + f.off;
-  // !CL: exchange records: per parity, one per CTA, then one per item (the row k0 + k)
-  auto rec = [&](int par, int b) { return xbuf + ((int64_t)par * (total + n_items) + b) * GC_REC; };
+  // !CL: per parity, the candidates of all CTAs side by side (two words each); then
+  // rows, per parity one per CTA and one per item (the row k0 + k)
+  auto cand = [&](int par, int b) { return xbuf + 2 * ((int64_t)par * total + b); };
+  auto rec = [&](int par, int b) { return xbuf + 4 * total + ((int64_t)par * (total + n_items) + b) * GC_REC; };
   // thread layout of the chunk: rows along lanes, ng groups of 4-column blocks
   const int rw = min(NT, (max(nr_my, 1) + 31) / 32 * 32), ng = NT / rw;
   const int tr = tid % rw, tg = tid / rw;
@@ -1412,16 +1446,15 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
         uint64_t* cb = rec(par, blockIdx.x);
         if (lane < 2)
           // key bits 63..32 and the row (24 bits) in the first word, key bits 31..0 in the second
-          gc_put(cb + lane, tag56 | (lane == 0 ? (uint64_t)(bi == LU_NONE ? 0xFFFFFFu : (uint32_t)(bi - k0)) << 32 | (bk >> 32)
+          gc_put(cand(par, blockIdx.x) + lane, tag56 | (lane == 0 ? (uint64_t)(bi == LU_NONE ? 0xFFFFFFu : (uint32_t)(bi - k0)) << 32 | (bk >> 32)
                                                : (bk & 0xFFFFFFFFull)));
         if (bi != LU_NONE)
           for (int w = lane; w < kb * WORDS; w += 32)
-            gc_put(cb + 2 + w, tag56 | LuBits<T>::half(S[(bi - rbeg) * SR + w / WORDS], w % WORDS));
+            gc_put(cb + w, tag56 | LuBits<T>::half(S[(bi - rbeg) * SR + w / WORDS], w % WORDS));
         // 2. the item's pivot
         uint64_t x0[GC_POLL], x1[GC_POLL], key = 0;
         int r = LU_NONE;
-        ok = gc_poll<GC_POLL>(rec(par, it.b), (int)GC_REC, P, k + 1, x0, err) &&
-             gc_poll<GC_POLL>(rec(par, it.b) + 1, (int)GC_REC, P, k + 1, x1, err);
+        ok = gc_poll2<GC_POLL>(cand(par, it.b), P, k + 1, x0, x1, err);
         if (ok) {
 #pragma unroll
           for (int e = 0; e < GC_POLL; ++e) {
@@ -1441,7 +1474,7 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
             for (int j = lane; j < kb; j += 32) rc.row[0][j] = S[(p - rbeg) * SR + j];
           } else {
             uint64_t x[2 * WORDS];
-            ok = gc_poll<2 * WORDS>(rec(par, it.b + (p - k0) / R) + 2, 1, kb * WORDS, k + 1, x, err);
+            ok = gc_poll<2 * WORDS>(rec(par, it.b + (p - k0) / R), kb * WORDS, k + 1, x, err);
 #pragma unroll
             for (int e = 0; e < 2 * WORDS; ++e) {
               const uint32_t v = (uint32_t)x[e], lo = __shfl_down_sync(0xffffffffu, v, 1);
@@ -1459,7 +1492,7 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
           for (int j = lane; j < kb; j += 32) rc.diag[j] = S[(gk - rbeg) * SR + j];
         } else {
           uint64_t x[2 * WORDS];
-          ok = gc_poll<2 * WORDS>(dr, 1, kb * WORDS, k + 1, x, err);
+          ok = gc_poll<2 * WORDS>(dr, kb * WORDS, k + 1, x, err);
 #pragma unroll
           for (int e = 0; e < 2 * WORDS; ++e) {
             const uint32_t v = (uint32_t)x[e], lo = __shfl_down_sync(0xffffffffu, v, 1);

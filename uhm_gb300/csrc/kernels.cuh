@@ -102,7 +102,7 @@ void launch_syrk_update(const DevCtx& c, const Item* items, int n_items, int dty
 // CTA, at most GC_RMAX_F64 / GC_RMAX_F32
 constexpr int GC_RMAX_F64 = 384, GC_RMAX_F32 = 768;
 constexpr int GC_MAX_CTAS = 160, GC_CLUSTER = 16;
-constexpr int64_t gc_words(int n_ctas, int n_items) { return 2 * (int64_t)(n_ctas + n_items) * (2 + 2 * 64); }
+constexpr int64_t gc_words(int n_ctas, int n_items) { return 4 * (int64_t)n_ctas + 2 * (int64_t)(n_ctas + n_items) * (2 * 64); }
 void launch_getrf_smem(const DevCtx& c, const Item* items, int n_items, int n_ctas, int csize, int dtype, int nb,
                        int pivot, int rmax, uint64_t* xbuf, int* err, cudaStream_t s);
 void launch_laswp(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, cudaStream_t s);
