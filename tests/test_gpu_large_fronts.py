@@ -120,6 +120,27 @@ def test_cholesky_right_hand_sides(native_lib, prec, n_rhs):
     assert np.abs(x - ref).max() <= 3e-10 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("method,prec", [(uo.CHOL, api.PREC_FP64), (uo.CHOL, api.PREC_FP32),
+                                         (uo.LU_PIV, api.PREC_FP64), (uo.LU_NOPIV, api.PREC_BF16X3)])
+def test_lookahead_changes_no_bit(native_lib, method, prec):
+    """Fronts of several outer panels whose updates run beside the next panel's
+    steps (more launches): every entry meets the same operations in the same order."""
+    got = []
+    m, leaves, mats, rhs = _mesh(2500, 500, method == uo.CHOL, 33)
+    for la in (0, 1):
+        if prec != api.PREC_FP64:
+            m.set_mode(1, prec, 1e-12, 10)
+        m.set_tunables(lookahead=la)
+        m.factor(method)
+        launches = m.timing()["kernel_launches"]
+        m.solve(method)
+        eid = m.fronts()[0]
+        got.append((launches, [m.front_block(int(e), "ABR") for e in eid[:2]],
+                    m.node_solution(np.arange(3, dtype=np.int32), np.array([2500, 2500, 500]), 1)))
+    assert got[1][0] > got[0][0]
+    assert all((a == b).all() for a, b in zip(got[0][1], got[1][1])) and (got[0][2] == got[1][2]).all()
+
+
 @pytest.mark.parametrize("fs,ss", SIZES)
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_cholesky_front(native_lib, prec, fs, ss):

@@ -97,7 +97,7 @@ void Engine::free_device() {
   d_ws2_row0 = nullptr;
   d_ws2b_row0 = d_linv_row0 = nullptr;
   d_xs = nullptr;
-  xs_ctx = XsCtx{};
+  xs_ctx = xs_in = XsCtx{};
   d_pflags = nullptr;
   d_hand = nullptr;
   d_err = nullptr;
@@ -725,6 +725,15 @@ void Engine::build_plan(int method) {
       if (method != UHM_CHOL) rows += r;
       f.xs_exp0 = exps;
       exps += (method == UHM_CHOL ? 1 : 2) * (int64_t)f.n;
+      // the 64-column steps of the next outer panel run beside the update that
+      // reads these: slices of their own
+      const int64_t ri = (int64_t)(f.prec == PREC_FP64 ? XS_S64 : XS_S32) * f.n;
+      f.xs_row0i = rows;
+      rows += ri;
+      f.xs_row0bi = method == UHM_CHOL ? f.xs_row0i : rows;
+      if (method != UHM_CHOL) rows += ri;
+      f.xs_exp0i = exps;
+      exps += (method == UHM_CHOL ? 1 : 2) * (int64_t)f.n;
     }
     xs_rows = std::max(xs_rows, rows);
     xs_exps = std::max(xs_exps, exps);
@@ -956,7 +965,7 @@ void Engine::build_programs(int method) {
   // the other columns), the rest one CTA per front.  nbo > 0 (tensor-core
   // fronts): rows are swapped only in columns below the outer panel's
   // trailing block, whose swaps come after the outer panel
-  auto push_lu_panel = [&](int dt, const std::vector<Item>& p_items, double fp, int nbo) {
+  auto push_lu_panel = [&](int dt, const std::vector<Item>& p_items, double fp, int nbo, int sms) {
     const int piv = method == UHM_LU_PIV ? 1 : 0;
     const int rcap = dt == F64 ? GC_RMAX_F64 : GC_RMAX_F32, rgoal = dt == F64 ? LU_GOAL_F64 : LU_GOAL_F32;
     auto col_end = [&](const Item& it) {
@@ -966,7 +975,7 @@ void Engine::build_programs(int method) {
     // a cluster per front up to the rows that fit its shared memory, the whole
     // GPU for the rest; in global memory where gc_min_rows was raised to ask for
     // one CTA on more rows than its shared memory holds
-    const int n_cta = std::min(n_sm, GC_MAX_CTAS);
+    const int n_cta = std::min(sms, GC_MAX_CTAS);      // sms: SMs that no concurrent update holds
     std::vector<Item> glob, tall, sw, cl[5];
     int rmax_cl[5] = {1, 1, 1, 1, 1};
     // clusters that keep the launch within one wave
@@ -1058,12 +1067,12 @@ void Engine::build_programs(int method) {
     return 2.0 * kb * area;
   };
   auto push_xs = [&](int dt, int nb, int region, const std::vector<Item>& pk, std::vector<Item>& tiles,
-                     double fl, double by) {
+                     double fl, double by, int cap = 0, int strm = 0) {
     if (tiles.empty()) return;
     push(fac_ops, OP_XS_PACK, dt, nb, 0, pk);
     // fewer tiles than SMs: tiles of half the width (a launch is as long as its
     // slowest CTA; one round of half tiles of K = 64 takes 19 us)
-    const bool narrow = (int)tiles.size() < n_sm;
+    const bool narrow = (int)tiles.size() < (cap > 0 ? cap : n_sm);
     if (narrow) {
       std::vector<Item> h;
       for (const Item& t : tiles)
@@ -1079,7 +1088,39 @@ void Engine::build_programs(int method) {
     op.aux = narrow ? 64 : XS_TILE;
     op.flops = fl;
     op.bytes = by;
+    op.cap = cap;
+    op.strm = strm;
     fac_ops.push_back(op);
+  };
+  // Lookahead: an outer panel's trailing update is split into the next panel's
+  // columns (on the engine's stream) and the rest, which runs on the side stream
+  // beside the next panel's 64-column steps, on SMs of its own.  Returns those
+  // SMs, 0: no split.  t0: the next panel's latency (us), chain: its work that
+  // more SMs shorten, upd: the rest's (SM us each; a tile beside the panel's
+  // kernels takes about 1.4 times what it takes alone).  The steps are latency bound,
+  // the update is not: measured on GB300, factorisations with every update after
+  // the one before and so, 24^3 p = 3 BF16X3 LU 100.3 -> 95.3 ms, 12^3 p = 3 FP64
+  // LU 42.8 -> 40.4, 16^3 p = 4 FP64 Cholesky 72.2 -> 68.6, 13^3 p = 4 FP32 12.0 ->
+  // 11.2.  Too few SMs cost more than too many (without the 1.4: 96.5, 40.5,
+  // 71.8, 12.7; with half of them 121, 54, 99, 18).  At most half the SMs for LU, whose
+  // panels on the whole GPU want them (110: 97.8, 40.7), 110 for Cholesky (half:
+  // 70.0, 11.9).
+  constexpr int EV_PACKED = 0, EV_REST = 1;
+  auto ev_op = [&](int kind, int id, int strm) {
+    Op op{kind, 0, 0, id, 0, 0};
+    op.strm = strm;
+    fac_ops.push_back(op);
+  };
+  auto split_sms = [&](double t0, double chain, double upd) {
+    if (!tune.lookahead || t0 <= 0 || upd <= 0) return 0;
+    upd *= 1.4;
+    int best = 0;
+    double tb = 0.97 * (t0 + (chain + upd) / n_sm);
+    for (int u = 2; u <= (chol ? n_sm * 110 / 152 : n_sm / 2); ++u) {
+      const double t = std::max(t0 + chain / (n_sm - u), upd / u);
+      if (t < tb) { tb = t; best = u; }
+    }
+    return best;
   };
   const int small_max[2] = {tune.small_max_f64, tune.small_max_f32};
   for (auto& lv : levels) {
@@ -1145,6 +1186,7 @@ void Engine::build_programs(int method) {
       // trailing block once per outer panel (K = XS_NBO)
       int maxfs = 0;
       for (int s : large) maxfs = std::max(maxfs, fronts[s].fs);
+      int side = 0;                  // SMs of the previous panel's concurrent update
       for (int K0 = 0; K0 < maxfs; K0 += XS_NBO) {
         const int k_end = std::min(K0 + XS_NBO, maxfs);
         for (int k0 = K0; k0 < k_end; k0 += NB) {
@@ -1180,11 +1222,13 @@ void Engine::build_programs(int method) {
           } else if (chol) {
             push_potrf_trsm(dt, p_items, t_items, fp, ft);
           } else {
-            push_lu_panel(dt, p_items, fp, XS_NBO);
+            push_lu_panel(dt, p_items, fp, XS_NBO, n_sm - side);
             push(fac_ops, OP_LUROW, dt, NB, 0, t_items, ft);
           }
-          push_xs(dt, NB, 1, pk, ut, fu, bu);
+          push_xs(dt, NB, 1, pk, ut, fu, bu, side ? n_sm - side : 0);
         }
+        if (side) ev_op(OP_EV_WAIT, EV_REST, 0);
+        side = 0;
         if (method == UHM_LU_PIV) {
           // the outer panel's row swaps on the columns right of it
           std::vector<Item> sw;
@@ -1214,9 +1258,12 @@ void Engine::build_programs(int method) {
           push(fac_ops, OP_LUROW, dt, NB, 0, t_items, ft);
           push_xs(dt, NB, 2, pk, ut, fu, bu);
         }
-        // the trailing block
-        std::vector<Item> pk, ut;
-        double fu = 0, bu = 0;
+        // the trailing block: the next panel's columns, the rest
+        std::vector<Item> pk, us, ut;
+        double fs_ = 0, fu = 0, bs = 0, bu = 0;
+        double t0 = 0, chain = 0;
+        const bool d = dt == F64;
+        bool fits = true;            // the next panel's rows in the shared memory of half the SMs (LU)
         for (int s : large) {
           const HostFront& f = fronts[s];
           if (f.fs <= K0) continue;
@@ -1224,9 +1271,33 @@ void Engine::build_programs(int method) {
           if (base >= f.n) continue;
           xs_pack_items(pk, XS_NBO, s, K0, base, f.n, 0);
           if (!chol) xs_pack_items(pk, XS_NBO, s, K0, base, f.n, 1);
-          fu += xs_tiles(ut, f, K0, KB, base, f.n, base, f.n, chol, bu);
+          fits = fits && (chol || f.n - base <= (d ? GC_RMAX_F64 : GC_RMAX_F32) * (n_sm / 2));
+          const int B = std::min(base + XS_NBO, f.fs), cs = base + (B - base + XS_TILE - 1) / XS_TILE * XS_TILE;
+          if (B > base) fs_ += xs_tiles(us, f, K0, KB, base, f.n, base, B, chol, bs);
+          if (cs < f.n) fu += xs_tiles(ut, f, K0, KB, chol ? cs : base, f.n, cs, f.n, chol, bu);
+          for (int k0 = base; k0 < B; k0 += NB) {
+            const double rows = f.n - k0;
+            // measured: a TRSM of 16 rows 10.6 SM us (FP32: 64 rows 5), a 128 x 128 tile of
+            // K = 64 20 (12)
+            if (chol) chain += d ? 10.6 * rows / 16 : 5.0 * rows / 64;
+            chain += (d ? 20.0 : 12.0) * std::ceil(rows / XS_TILE) * ((B - k0) / (double)XS_TILE);
+          }
+          // a step's launches at their shortest
+          t0 = std::max(t0, (B - base + NB - 1) / NB * (chol ? (d ? 80.0 : 40.0) : (d ? 250.0 : 215.0)));
         }
-        push_xs(dt, XS_NBO, 0, pk, ut, fu, bu);
+        const double tile = d ? 30.0 : 13.0;       // a tile of K = 256 (SM us)
+        side = fits ? split_sms(t0, chain + tile * us.size(), tile * ut.size()) : 0;
+        if (side) {
+          push(fac_ops, OP_XS_PACK, dt, XS_NBO, 0, pk);
+          ev_op(OP_EV_RECORD, EV_PACKED, 0);
+          ev_op(OP_EV_WAIT, EV_PACKED, 1);
+          push_xs(dt, XS_NBO, 0, {}, ut, fu, bu, side, 1);
+          ev_op(OP_EV_RECORD, EV_REST, 1);
+          push_xs(dt, XS_NBO, 0, {}, us, fs_, bs, n_sm - side);
+        } else {
+          us.insert(us.end(), ut.begin(), ut.end());
+          push_xs(dt, XS_NBO, 0, pk, us, fs_ + fu, bs + bu);
+        }
       }
       // tensor-core fronts: outer panels of tc_nbo columns; inside a panel the
       // SIMT kernels factor 64 columns at a time and update only the panel's
@@ -1236,6 +1307,7 @@ void Engine::build_programs(int method) {
       for (int s : tcf) maxfs_tc = std::max(maxfs_tc, fronts[s].fs);
       const int NBO = tune.tc_nbo;
       const int TB = tc_tile();
+      side = 0;
       for (int K0 = 0; !chol && K0 < maxfs_tc; K0 += NBO) {
         // LU tensor-core fronts, standard blocked LU with an outer panel of
         // NBO columns: inside it the 64-column steps swap rows and update
@@ -1262,7 +1334,7 @@ void Engine::build_programs(int method) {
                 if (base + tj * TILE < B) u_items.push_back(Item{s, k0, ti, tj});
             fu += get_flop_gemm(0, f.n - base, std::max(0, B - base), kb);
           }
-          push_lu_panel(dt, p_items, fp, NBO);
+          push_lu_panel(dt, p_items, fp, NBO, n_sm - side);
           push(fac_ops, OP_LUROW, dt, NB, 0, t_items, ft);
           {
             Op op{OP_GEMM, dt, NB, 0, add_items(u_items), (int)u_items.size()};
@@ -1272,6 +1344,8 @@ void Engine::build_programs(int method) {
             if (!u_items.empty()) fac_ops.push_back(op);
           }
         }
+        if (side) ev_op(OP_EV_WAIT, EV_REST, 0);
+        side = 0;
         // the outer panel's row swaps on the columns >= B
         if (method == UHM_LU_PIV) {
           std::vector<Item> sw;
@@ -1311,20 +1385,27 @@ void Engine::build_programs(int method) {
           if (!u_items.empty()) fac_ops.push_back(op);
         }
         // trailing block on the tensor cores: L21 (parts 0-1) and U12^T (parts 2-3)
-        std::vector<Item> pk, tt;
-        double ftc = 0, btc = 0;
+        std::vector<Item> pk, ts, tt;      // ts: tiles of the next panel's columns
+        double ftc = 0, btc = 0, fts = 0, bts = 0, t0 = 0, chain = 0;
+        bool fits = true;            // the next panel's rows in the shared memory of half the SMs
         for (int s : tcf) {
           const HostFront& f = fronts[s];
           if (f.fs <= K0) continue;
           const int KB = std::min(NBO, f.fs - K0);
           const int m = f.n - (K0 + KB);
           if (m <= 0) continue;
+          fits = fits && m <= GC_RMAX_F32 * (n_sm / 2);
           for (int rb = 0; rb < (m + 63) / 64; ++rb) pk.push_back(Item{s, K0, rb, 0});
-          const int T = (m + TB - 1) / TB;
+          const int T = (m + TB - 1) / TB, W = std::min(NBO, f.fs - (K0 + KB)), Ts = (W + TB - 1) / TB;
           for (int ti = 0; ti < T; ++ti)
-            for (int tj = 0; tj < T; ++tj) tt.push_back(Item{s, K0, ti, tj});
-          ftc += get_flop_gemm(0, m, m, KB);
-          btc += 8.0 * (double)m * m + 2.0 * 4 * (double)m * KB;
+            for (int tj = 0; tj < T; ++tj) (tj < Ts ? ts : tt).push_back(Item{s, K0, ti, tj});
+          const double ws = std::min(Ts * TB, m);
+          fts += get_flop_gemm(0, m, ws, KB);
+          ftc += get_flop_gemm(0, m, m - ws, KB);
+          bts += 8.0 * (double)m * ws;
+          btc += 8.0 * (double)m * (m - ws) + 2.0 * 4 * (double)m * KB;
+          for (int k0 = 0; k0 < W; k0 += NB) chain += 2.5 * std::ceil(m / 64.0) * ((W - k0) / 64);   // SIMT tiles
+          t0 = std::max(t0, (W + NB - 1) / NB * 210.0);      // a step's launches at their shortest
         }
         if (!pk.empty()) {
           Op pa{OP_TC_PACK, dt, NBO, 2, add_items(pk), (int)pk.size()};
@@ -1333,7 +1414,20 @@ void Engine::build_programs(int method) {
           pb.q0 = 1;        // transposed: U12^T
           pb.aux = 2;       // into parts 2-3
           fac_ops.push_back(pb);
-          push(fac_ops, OP_TC_GEMM, dt, NBO, 2, tt, ftc, btc);
+          side = fits ? split_sms(t0, chain + 4.5 * ts.size(), 4.5 * tt.size()) : 0;   // a tile: 4.5 SM us
+          if (side) {
+            ev_op(OP_EV_RECORD, EV_PACKED, 0);
+            ev_op(OP_EV_WAIT, EV_PACKED, 1);
+            push(fac_ops, OP_TC_GEMM, dt, NBO, 2, tt, ftc, btc);
+            fac_ops.back().cap = side;
+            fac_ops.back().strm = 1;
+            ev_op(OP_EV_RECORD, EV_REST, 1);
+            push(fac_ops, OP_TC_GEMM, dt, NBO, 2, ts, fts, bts);
+            fac_ops.back().cap = n_sm - side;
+          } else {
+            ts.insert(ts.end(), tt.begin(), tt.end());
+            push(fac_ops, OP_TC_GEMM, dt, NBO, 2, ts, fts + ftc, bts + btc);
+          }
         }
       }
       for (int K0 = 0; chol && K0 < maxfs_tc; K0 += NBO) {
@@ -1434,11 +1528,6 @@ void Engine::build_programs(int method) {
           op.q0 = diag_seq++;                // the launch's tag
           return op;
         };
-        auto ev_op = [&](int kind, int id, int strm) {
-          Op op{kind, 0, 0, id, 0, 0};
-          op.strm = strm;
-          return op;
-        };
         const bool la = tune.lookahead != 0;
         Op d0 = diag_op(0);
         fac_ops.push_back(d0);
@@ -1476,18 +1565,18 @@ void Engine::build_programs(int method) {
             }
           }
           push(fac_ops, OP_CHOL_PACK, F32, 0, 0, pit, 0, bp);
-          if (p > 0 && la) fac_ops.push_back(ev_op(OP_EV_WAIT, 2 * p, 0));   // diagonal kernel of panel p done
+          if (p > 0 && la) ev_op(OP_EV_WAIT, 2 * p, 0);   // diagonal kernel of panel p done
           push(fac_ops, OP_TC_CHOL_TRSM, F32, 0, 0, xit, fx, bx);
           if (next && la) {
             split_halves(tdiag);
             push(fac_ops, OP_TC_CHOL_TRAIL, F32, 0, 0, tdiag, fd, bd);
-            fac_ops.push_back(ev_op(OP_EV_RECORD, 2 * p + 1, 0));
-            fac_ops.push_back(ev_op(OP_EV_WAIT, 2 * p + 1, 1));
+            ev_op(OP_EV_RECORD, 2 * p + 1, 0);
+            ev_op(OP_EV_WAIT, 2 * p + 1, 1);
             Op dn = diag_op(K0 + W1);
             dn.strm = 1;
             const int reserve = std::min(dn.aux, 16);
             fac_ops.push_back(dn);
-            fac_ops.push_back(ev_op(OP_EV_RECORD, 2 * (p + 1), 1));
+            ev_op(OP_EV_RECORD, 2 * (p + 1), 1);
             Op tr{OP_TC_CHOL_TRAIL, F32, 0, 0, add_items(trest), (int)trest.size()};
             tr.flops = fr;
             tr.bytes = br;
@@ -1800,12 +1889,15 @@ void Engine::alloc_device(int method) {
     d_xs = dmalloc(bytes);
     CK(cudaMemsetAsync(d_xs, 0, bytes, stream));     // rows never packed are read by tiles that run over
     if (!xs_encode(&xs_map, d_xs, xs_rows + XS_SPARE_ROWS)) fail("tensor map encoding failed", 4);
-    std::vector<int64_t> v(3 * fronts.size(), 0);
+    std::vector<int64_t> v(6 * fronts.size(), 0);
     for (auto& f : fronts)
       if (f.xs) {
         v[f.slot] = f.xs_row0;
         v[fronts.size() + f.slot] = f.xs_row0b;
         v[2 * fronts.size() + f.slot] = f.xs_exp0;
+        v[3 * fronts.size() + f.slot] = f.xs_row0i;
+        v[4 * fronts.size() + f.slot] = f.xs_row0bi;
+        v[5 * fronts.size() + f.slot] = f.xs_exp0i;
       }
     int64_t* d = (int64_t*)dmalloc(sizeof(int64_t) * v.size());
     CK(cudaMemcpyAsync(d, v.data(), sizeof(int64_t) * v.size(), cudaMemcpyHostToDevice, stream));
@@ -1815,6 +1907,10 @@ void Engine::alloc_device(int method) {
     xs_ctx.row0b = d + fronts.size();
     xs_ctx.exp0 = d + 2 * fronts.size();
     xs_ctx.exps = (int*)dmalloc(sizeof(int) * (size_t)xs_exps);
+    xs_in = xs_ctx;
+    xs_in.row0 = d + 3 * fronts.size();
+    xs_in.row0b = d + 4 * fronts.size();
+    xs_in.exp0 = d + 5 * fronts.size();
   }
   if (pflags_n > 0) d_pflags = (int*)dmalloc(sizeof(int) * (size_t)pflags_n);
   if (hand_n > 0) {
@@ -2029,7 +2125,7 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
         break;
       case OP_POTRF: launch_potrf_diag(ctx, it, op.n_items, op.dtype, op.nb, st); break;
       case OP_TRSM:
-        if (op.dtype == F64) launch_xs_trsm(ctx, xs_ctx, it, op.n_items, st);
+        if (op.dtype == F64) launch_xs_trsm(ctx, xs_in, it, op.n_items, st);
         else launch_trsm_panel(ctx, it, op.n_items, op.dtype, op.nb, st);
         break;
       case OP_POTRF_TRSM: launch_potrf_trsm(ctx, it, op.n_items, op.dtype, st); break;
@@ -2052,11 +2148,14 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
         break;
       case OP_TC_SYRK:
         launch_tc_syrk(ctx, ws_map, d_ws_off, d_ws_stride, it, op.n_items, op.nb, op.param, 0,
-                       op.param == 3 ? 6 : 3, op.param == 3 ? TC_TERMS_BF16X6 : TC_TERMS_BF16X3, 1, d_err, st);
+                       op.param == 3 ? 6 : 3, op.param == 3 ? TC_TERMS_BF16X6 : TC_TERMS_BF16X3, 1, 0, d_err, st);
         break;
-      case OP_XS_PACK: launch_xs_pack(ctx, xs_ctx, it, op.n_items, op.dtype, op.nb, st); break;
+      case OP_XS_PACK:
+        launch_xs_pack(ctx, op.nb == NB ? xs_in : xs_ctx, it, op.n_items, op.dtype, op.nb, st);
+        break;
       case OP_XS_UPDATE:
-        launch_xs_update(ctx, xs_ctx, xs_map, it, op.n_items, op.dtype, op.nb, op.q0, op.param, op.aux, d_err, st);
+        launch_xs_update(ctx, op.nb == NB ? xs_in : xs_ctx, xs_map, it, op.n_items, op.dtype, op.nb, op.q0, op.param,
+                         op.aux, profiling ? 0 : op.cap, d_err, st);
         break;
       case OP_GETRF: launch_getrf_panel(ctx, it, op.n_items, op.dtype, op.nb, op.param, st); break;
       case OP_GETRF_COOP:
@@ -2068,8 +2167,8 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
       case OP_GEMM: launch_gemm_update(ctx, it, op.n_items, op.dtype, op.nb, op.q0, op.aux, st); break;
       case OP_TC_GEMM:
         // A parts 0-1 (L21), B parts 2-3 (U12^T)
-        launch_tc_syrk(ctx, ws_map, d_ws_off, d_ws_stride, it, op.n_items, op.nb, 2, 2, 3, TC_TERMS_BF16X3, 0, d_err,
-                       st);
+        launch_tc_syrk(ctx, ws_map, d_ws_off, d_ws_stride, it, op.n_items, op.nb, 2, 2, 3, TC_TERMS_BF16X3, 0,
+                       profiling ? 0 : op.cap, d_err, st);
         break;
       case OP_CLEAR_FLAGS:
         launch_clear_flags(d_pflags, op.q0, d_hand ? reinterpret_cast<unsigned*>(d_hand) : nullptr, st);

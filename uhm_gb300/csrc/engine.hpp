@@ -34,7 +34,8 @@ struct HostFront {
   bool tc = false;                 // trailing updates on tensor cores (BF16-split)
   bool tcc = false;                // ... through the cooperative panel kernel (BF16X3 Cholesky, k_chol_tc.cu)
   bool xs = false;                 // large FP64 / FP32 front: sliced tensor-core updates (k_xs.cu)
-  int64_t xs_row0 = 0, xs_row0b = 0, xs_exp0 = 0;   // its slices and row exponents in the level's workspace
+  int64_t xs_row0 = 0, xs_row0b = 0, xs_exp0 = 0;      // its slices and row exponents in the level's workspace
+  int64_t xs_row0i = 0, xs_row0bi = 0, xs_exp0i = 0;   // the same of a 64-column step
   int64_t ws_off = 0, ws_stride = 0;
   int64_t ws2_row0 = 0;            // first 128-byte row of its parts in the chunk-major workspace
   int64_t ws2b_row0 = 0;           // ... of the panel rows before their TRSM (tc_panel 256)
@@ -72,6 +73,7 @@ struct Op {
                       // region of the front (sliced update)
   int aux = 0;        // rows per CTA (cooperative LU panel, flag-driven solves)
   int strm = 0;       // 0: the engine's stream, 1: its side stream (panel lookahead)
+  int cap = 0;        // CTAs of a persistent update beside a concurrent launch (0: one per SM)
 };
 
 constexpr int N_OP_KINDS = 40;
@@ -114,7 +116,7 @@ struct Tunables {
                              // of the other tensor-core fronts
   int solve_rows = 64;       // rows (columns) per CTA of the flag-driven forward (backward) solves of
                              // large Cholesky fronts (64 or 256)
-  int lookahead = 1;         // panels of 256: the next panel's diagonal kernel overlaps the update
+  int lookahead = 1;         // the next outer panel (panels of 256: its diagonal kernel) overlaps the update
   int solve_chain = 0;       // 1: 64-row solves of FP32 fronts as chains (one CTA per front solves
                              // the diagonal blocks, helper CTAs the rest); 0: the flag-driven
                              // kernels, faster on the meshes measured (the chain CTA's per-step
@@ -306,7 +308,7 @@ class Engine {
   CUtensorMap ws2_map;
   void* d_xs = nullptr;              // operand slices of the current level's sliced updates
   int64_t xs_rows = 0, xs_exps = 0;  // its rows of 64 BF16 and row exponents (the largest level)
-  uhm_gpu::XsCtx xs_ctx{};
+  uhm_gpu::XsCtx xs_ctx{}, xs_in{};  // of the outer panels' updates, of those inside a panel
   CUtensorMap xs_map;
   int* d_pflags = nullptr;           // tickets and flags of the panel launches (cleared per factorisation)
   int64_t* d_ws2b_row0 = nullptr;

@@ -329,7 +329,7 @@ void launch_tc_pack(const DevCtx& c, const Item* items, int n_items, int nbo, in
 
 void launch_tc_syrk(const DevCtx& c, const CUtensorMap& wsmap, const int64_t* ws_off,
                     const int64_t* ws_stride, const Item* items, int n_items, int nbo, int parts, int pb0, int nterms,
-                    uint32_t term_code, int lower_only, int* err, cudaStream_t s) {
+                    uint32_t term_code, int lower_only, int cap, int* err, cudaStream_t s) {
   if (!n_items) return;
   if (parts < 1 || 2 * parts * TC_TILE_BYTES > TC_RING) throw std::invalid_argument("tc_syrk: 1 to 6 operand parts");
   static int n_sm = 0;
@@ -340,7 +340,8 @@ void launch_tc_syrk(const DevCtx& c, const CUtensorMap& wsmap, const int64_t* ws
     if (n_sm <= 0) n_sm = 1;
   }
   cudaFuncSetAttribute(k_tc_syrk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
-  const int grid = n_items < n_sm ? n_items : n_sm;   // one persistent CTA per SM
+  const int sms = cap > 0 && cap < n_sm ? cap : n_sm;
+  const int grid = n_items < sms ? n_items : sms;   // one persistent CTA per SM
   k_tc_syrk<<<grid, TC_THREADS, TC_SMEM, s>>>(c, wsmap, ws_off, ws_stride, items, n_items, nbo, parts, pb0, nterms,
                                               term_code, lower_only, err);
 }

@@ -602,7 +602,7 @@ bool xs_encode(CUtensorMap* map, void* base, int64_t rows) {
 
 template <typename T, int BN>
 static void xs_update_t(const DevCtx& c, const XsCtx& x, const CUtensorMap& map, const Item* items, int n_items,
-                        int nb, int region, int lower, int* err, cudaStream_t s) {
+                        int nb, int region, int lower, int cap, int* err, cudaStream_t s) {
   static int n_sm = 0;
   if (!n_sm) {
     int dev = 0;
@@ -611,21 +611,22 @@ static void xs_update_t(const DevCtx& c, const XsCtx& x, const CUtensorMap& map,
     if (n_sm <= 0) n_sm = 1;
   }
   cudaFuncSetAttribute(k_xs_update<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XS_SMEM);
-  const int grid = n_items < n_sm ? n_items : n_sm;
+  const int sms = cap > 0 && cap < n_sm ? cap : n_sm;
+  const int grid = n_items < sms ? n_items : sms;
   k_xs_update<T, BN><<<grid, XS_THREADS, XS_SMEM, s>>>(c, x, map, items, n_items, nb, region, lower, err);
 }
 
 void launch_xs_update(const DevCtx& c, const XsCtx& x, const CUtensorMap& map, const Item* items, int n_items,
-                      int dtype, int nb, int region, int lower, int tile_n, int* err, cudaStream_t s) {
+                      int dtype, int nb, int region, int lower, int tile_n, int cap, int* err, cudaStream_t s) {
   if (!n_items) return;
   if (nb > XS_NBO) throw std::invalid_argument("sliced update: panel wider than 256");
   if (tile_n != 64 && tile_n != XS_TILE) throw std::invalid_argument("sliced update: tiles are 64 or 128 columns wide");
   if (dtype == F64) {
-    if (tile_n == 64) xs_update_t<double, 64>(c, x, map, items, n_items, nb, region, lower, err, s);
-    else xs_update_t<double, 128>(c, x, map, items, n_items, nb, region, lower, err, s);
+    if (tile_n == 64) xs_update_t<double, 64>(c, x, map, items, n_items, nb, region, lower, cap, err, s);
+    else xs_update_t<double, 128>(c, x, map, items, n_items, nb, region, lower, cap, err, s);
   } else {
-    if (tile_n == 64) xs_update_t<float, 64>(c, x, map, items, n_items, nb, region, lower, err, s);
-    else xs_update_t<float, 128>(c, x, map, items, n_items, nb, region, lower, err, s);
+    if (tile_n == 64) xs_update_t<float, 64>(c, x, map, items, n_items, nb, region, lower, cap, err, s);
+    else xs_update_t<float, 128>(c, x, map, items, n_items, nb, region, lower, cap, err, s);
   }
 }
 

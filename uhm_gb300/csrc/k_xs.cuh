@@ -38,8 +38,9 @@ void launch_xs_trsm(const DevCtx& c, const XsCtx& x, const Item* items, int n_it
 // C -= A B^T over 128 x tile_n tiles (item: front, a = first row, b = first
 // column, c = K0 of the packed columns, W = min(nb, fs - K0)); lower: B is A
 // and only entries col <= row are updated.  region as for k_tile_update: 0
-// every entry, 1 columns below the outer panel's end, 2 rows below it
+// every entry, 1 columns below the outer panel's end, 2 rows below it; cap:
+// CTAs (0: one per SM)
 void launch_xs_update(const DevCtx& c, const XsCtx& x, const CUtensorMap& map, const Item* items, int n_items,
-                      int dtype, int nb, int region, int lower, int tile_n, int* err, cudaStream_t s);
+                      int dtype, int nb, int region, int lower, int tile_n, int cap, int* err, cudaStream_t s);
 
 }  // namespace uhm_gpu
