@@ -31,7 +31,7 @@ static constexpr int LU_GOAL_F64 = 64, LU_GOAL_F32 = 192;
 // rows (four fronts at once: more); FP64, 16 CTAs, 187 at 96 rows each, 205 at 128, 225 to
 // 264 from 130 to 208, against 200 for the whole GPU from 2,100 to 3,300 rows and 218 at 6,938
 static constexpr int LU_CLUSTER_ROWS_F64 = 128, LU_CLUSTER_ROWS_F32 = 384;
-static constexpr int TILE = 64;             // trailing-update tile (k_tile_update)
+static constexpr int TR = TILE_UPDATE_ROWS, TC = TILE_UPDATE_COLS;   // k_tile_update
 
 #define CK(x)                                                                          \
   do {                                                                                 \
@@ -1328,10 +1328,8 @@ void Engine::build_programs(int method) {
             fp += get_flop_lu(0, f.n - k0, kb);
             for (int c0 = base; c0 < B; c0 += LUROW_CB) t_items.push_back(Item{s, k0, c0, B});
             ft += get_flop_trsm_lower(0, kb, std::max(0, B - base));
-            const int T = (f.n - base + TILE - 1) / TILE;
-            for (int ti = 0; ti < T; ++ti)
-              for (int tj = 0; tj < T; ++tj)
-                if (base + tj * TILE < B) u_items.push_back(Item{s, k0, ti, tj});
+            for (int ti = 0; base + ti * TR < f.n; ++ti)
+              for (int tj = 0; base + tj * TC < B; ++tj) u_items.push_back(Item{s, k0, ti, tj});
             fu += get_flop_gemm(0, f.n - base, std::max(0, B - base), kb);
           }
           push_lu_panel(dt, p_items, fp, NBO, n_sm - side);
@@ -1369,12 +1367,8 @@ void Engine::build_programs(int method) {
             const int B = std::min(K0 + NBO, f.fs);
             for (int c0 = B; c0 < f.n; c0 += LUROW_CB) t_items.push_back(Item{s, k0, c0, 0});
             ft += get_flop_trsm_lower(0, kb, f.n - B);
-            const int T = (f.n - base + TILE - 1) / TILE;
-            for (int ti = 0; ti < T; ++ti) {
-              if (base + ti * TILE >= B) break;
-              for (int tj = 0; tj < T; ++tj)
-                if (base + (tj + 1) * TILE > B) u_items.push_back(Item{s, k0, ti, tj});
-            }
+            for (int ti = 0; base + ti * TR < B; ++ti)
+              for (int tj = (B - base) / TC; base + tj * TC < f.n; ++tj) u_items.push_back(Item{s, k0, ti, tj});
             fu += get_flop_gemm(0, std::max(0, B - base), f.n - B, kb);
           }
           push(fac_ops, OP_LUROW, dt, NB, 0, t_items, ft);
@@ -1444,10 +1438,9 @@ void Engine::build_programs(int method) {
             fp += get_flop_chol(0, kb);
             for (int r0 = base; r0 < f.n; r0 += TRSM_RB) t_items.push_back(Item{s, k0, r0, 0});
             ft += get_flop_trsm_lower(0, kb, f.n - base);
-            const int T = (f.n - base + TILE - 1) / TILE;
-            for (int ti = 0; ti < T; ++ti)
-              for (int tj = 0; tj <= ti; ++tj)
-                if (base + tj * TILE < cmax) u_items.push_back(Item{s, k0, ti, tj});
+            for (int ti = 0; base + ti * TR < f.n; ++ti)
+              for (int tj = 0; tj * TC < (ti + 1) * TR && base + tj * TC < cmax; ++tj)
+                u_items.push_back(Item{s, k0, ti, tj});
             const double w = std::max(0, cmax - base), mr = f.n - base;
             fu += 2.0 * kb * (w * mr - 0.5 * w * (w - 1));
           }

@@ -91,6 +91,7 @@ void launch_potrf_diag(const DevCtx& c, const Item* items, int n_items, int dtyp
                        cudaStream_t s);
 void launch_trsm_panel(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
                        cudaStream_t s);
+constexpr int TILE_UPDATE_ROWS = 128, TILE_UPDATE_COLS = 64;   // tiles of the FP32 updates inside a panel
 void launch_syrk_update(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
                         int nbo, cudaStream_t s);
 // LU (partial pivoting restricted to the factor rows, or none): a 64-column
