@@ -31,7 +31,7 @@ def _matrix(n, symmetric, rng):
     return a
 
 
-def _mesh(fs, ss, symmetric, seed, n_rhs=1):
+def _mesh(fs, ss, symmetric, seed, n_rhs=1, mats=None):
     rng = np.random.default_rng(seed)
     m = api.Mesh()
     nodes = [m.add_node(0, fs), m.add_node(1, fs), m.add_node(2, ss)]
@@ -44,7 +44,7 @@ def _mesh(fs, ss, symmetric, seed, n_rhs=1):
         m.add_child(root, e)
     m.lock()
     m.create_matrix_without_buffer(api.UHM_REAL, n_rhs)
-    mats = [_matrix(fs + ss, symmetric, rng) for _ in leaves]
+    mats = mats or [_matrix(fs + ss, symmetric, rng) for _ in leaves]
     rhs = [rng.standard_normal((fs + ss, n_rhs)) for _ in leaves]
     for k, e in enumerate(leaves):
         m.copy_in(e, [k, 2], api.UHM_LHS, mats[k])
@@ -52,8 +52,8 @@ def _mesh(fs, ss, symmetric, seed, n_rhs=1):
     return m, leaves, mats, rhs
 
 
-def _check(method, prec, fs, ss, seed):
-    m, leaves, mats, rhs = _mesh(fs, ss, method == uo.CHOL, seed)
+def _check(method, prec, fs, ss, seed, mats=None):
+    m, leaves, mats, rhs = _mesh(fs, ss, method == uo.CHOL, seed, mats=mats)
     if prec == "fp32":
         m.set_mode(1, api.PREC_FP32, 1e-12, 10)
     m.factor(method)
@@ -145,6 +145,18 @@ def test_lookahead_changes_no_bit(native_lib, method, prec):
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_cholesky_front(native_lib, prec, fs, ss):
     _check(uo.CHOL, prec, fs, ss, 200 + fs)
+
+
+@pytest.mark.parametrize("prec,digits", [("fp32", (63, 127, 127, 64)), ("fp64", (63, 127, 127, 127, 127, 127, 64))])
+def test_largest_digits(native_lib, prec, digits):
+    """Panels whose 8-bit digits are all near their largest: the sums of 256 products
+    pass 2^22 (and 2^24 between diagonals), beyond what a typical tile meets."""
+    fs, ss = 256, 129
+    v = sum(d * 256.0 ** -(k + 1) for k, d in enumerate(digits)) * 4
+    a = np.diag(np.r_[np.full(fs, 256.0), np.full(ss, 3.0)])     # L11 = 16 I, L21 = v / 16; condition number 200
+    a[fs:, :fs] = a[:fs, fs:] = v
+    a[fs:, fs:] += v * v
+    _check(uo.CHOL, prec, fs, ss, 35, mats=[a, a])
 
 
 @pytest.mark.parametrize("value", [np.nan, np.inf])

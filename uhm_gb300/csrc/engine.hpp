@@ -309,7 +309,7 @@ class Engine {
   void* d_xs = nullptr;              // operand slices of the current level's sliced updates
   int64_t xs_rows = 0, xs_exps = 0;  // its rows of 64 BF16 and row exponents (the largest level)
   uhm_gpu::XsCtx xs_ctx{}, xs_in{};  // of the outer panels' updates, of those inside a panel
-  CUtensorMap xs_map;
+  uhm_gpu::XsMaps xs_map;
   int* d_pflags = nullptr;           // tickets and flags of the panel launches (cleared per factorisation)
   int64_t* d_ws2b_row0 = nullptr;
   int64_t* d_linv_row0 = nullptr;

@@ -960,8 +960,7 @@ void launch_potrf_trsm(const DevCtx& c, const Item* items, int n_items, int dtyp
 // shared-memory words and two broadcast 16-byte ones per 32 multiply-adds.
 // Bound by those multiply-adds and, K being 64 at most, by the tile's loads.
 // Measured on GB300, the updates inside the panels of 24^3 p = 3 LU (14,911 rows
-// down): 14.3 (64 x 64 tiles, four by four entries a thread) -> 10.6 ms;
-// 229 tiles 31 -> 17 us.
+// down): 14.3 (64 x 64 tiles, four by four entries a thread) -> 10.6 ms.
 constexpr int TU_BM = TILE_UPDATE_ROWS, TU_BN = TILE_UPDATE_COLS, TU_K = 64;
 constexpr int TU_LDA = TU_BM + 1, TU_LDB = TU_BN + 4;
 constexpr size_t TU_SMEM = sizeof(float) * TU_K * (TU_LDA + TU_LDB);

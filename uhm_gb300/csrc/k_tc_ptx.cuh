@@ -148,6 +148,22 @@ __device__ __forceinline__ void umma_bf16_w(uint32_t elected, uint32_t tmem_d, u
       " @e tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %5, p;\n}\n" ::"r"(elected),
       "r"(tmem_d), "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate));
 }
+// the same, accumulating, in a row of MMAs with one A operand: the first one keeps
+// A in the tensor core's collector buffer, the others take it from there
+enum { UMMA_A_FILL, UMMA_A_USE, UMMA_A_LAST };
+template <int OP>
+__device__ __forceinline__ void umma_bf16_wa(uint32_t elected, uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t hi,
+                                             uint32_t idesc) {
+#define UMMA_WA(op)                                                                                          \
+  asm volatile("{\n .reg .pred p, e;\n .reg .b64 da, db;\n setp.ne.b32 e, %0, 0;\n setp.eq.b32 p, %0, %0;\n"  \
+               " mov.b64 da, {%2, %4};\n mov.b64 db, {%3, %4};\n"                                            \
+               " @e tcgen05.mma.cta_group::1.kind::f16.collector::a::" op " [%1], da, db, %5, p;\n}\n"       \
+               ::"r"(elected), "r"(tmem_d), "r"(alo), "r"(blo), "r"(hi), "r"(idesc))
+  if constexpr (OP == UMMA_A_FILL) UMMA_WA("fill");
+  else if constexpr (OP == UMMA_A_USE) UMMA_WA("use");
+  else UMMA_WA("lastuse");
+#undef UMMA_WA
+}
 __device__ __forceinline__ void umma_commit_w(uint32_t elected, uint32_t bar) {
   asm volatile(
       "{\n .reg .pred e;\n setp.ne.b32 e, %0, 0;\n"

@@ -30,8 +30,8 @@
 // measured for the SIMT update), against 1,906 TFLOP/s of BF16 products:
 // 36 products per FP64 one still leave 53.  FP32 fronts: 10 products leave
 // 190 TFLOP/s against 15 measured for the SIMT update.  Measured on GB300, the
-// updates of one factorisation: 16^3 p = 4 FP64 906 -> 34.5 ms (and 2.3 for the
-// slices), 13^3 p = 4 FP32 23.0 -> 6.5 (2.0), 12^3 p = 3 FP64 LU 196 -> 10.3 (2.7).
+// updates of one factorisation: 16^3 p = 4 FP64 906 -> 33.8 ms (and 2.3 for the
+// slices), 13^3 p = 4 FP32 23.0 -> 6.4 (2.0), 12^3 p = 3 FP64 LU 196 -> 10.2 (2.7).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -281,15 +281,51 @@ constexpr uint32_t XS_SMEM = 1024 + XS_SLOTS * XS_SLOT + 512;
         "=r"(v[14]), "=r"(v[15])                                                                  \
       : "r"(taddr))
 
+#define XS_LD8(taddr, v)                                                                          \
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"          \
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),          \
+                 "=r"(v[6]), "=r"(v[7])                                                           \
+               : "r"(taddr))
+
 // One tile takes S = 8 (FP64) in two passes over its columns: diagonals 4 ..
 // 7 (26 products of all slices), then diagonals 0 .. 3 (10 products of slices
 // 0 .. 3); S = 4 (FP32) only the second pass.  Diagonal d goes to accumulator
 // d mod 4, 128 x 128 FP32; the four fill tensor memory.
 
-// a += v 2^SH, v a diagonal's integer sum
+// a += i 2^SH
 template <int SH>
-__device__ __forceinline__ void xs_add(long long& a, uint32_t v) {
-  a += (long long)__float2int_rn(__uint_as_float(v)) << SH;
+__device__ __forceinline__ void xs_add(long long& a, int i) {
+  if constexpr (SH < 31) {
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(a) : "r"(i), "n"(1 << SH));
+  } else {
+    a += (long long)((unsigned long long)((unsigned)i << (SH - 32)) << 32);
+  }
+}
+
+// FP32 tiles: conversions to integers run at 16 per clock and SM, additions at 128:
+// the sum of an integer below 2^22 and 1.5 2^23 holds it in its low bits, as
+// XS_MAGIC + v.  A diagonal's sums can reach 1.75 2^24 (256 products of 8-bit
+// digits); then, a warp's vote, they are converted.  (FP64 tiles have no
+// registers left for it.)
+constexpr uint32_t XS_MAGIC = 0x4B400000u;
+__device__ __forceinline__ void xs_ints(uint32_t taddr, uint32_t (&v)[4][8]) {
+  uint32_t out = 0;
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[a][j] = __float_as_uint(__uint_as_float(v[a][j]) + 12582912.0f);
+      out |= v[a][j] ^ XS_MAGIC;               // bits 23.. are clear within [2^23, 2^24)
+    }
+  if (__any_sync(0xffffffffu, out >> 23)) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a) XS_LD8(taddr + a * XS_TILE, v[a]);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[a][j] = XS_MAGIC + (uint32_t)__float2int_rn(__uint_as_float(v[a][j]));
+  }
 }
 
 // a 2^E, rounded to nearest (E may leave the exponent range).  FP64 without
@@ -311,11 +347,14 @@ __device__ __forceinline__ double xs_scaled(long long a, int E, double) {
   if (a < 0) q |= 1ull << 63;
   return __longlong_as_double((long long)q);
 }
+// |a| < 2^45: a = h 2^23 + l, |h| < 2^22, both exact in FP32 (as above, without a
+// conversion), so that their sum rounds once
 __device__ __forceinline__ float xs_scaled(long long a, int E, float) {
-  const float x = __ll2float_rn(a);
+  const float h = __uint_as_float(XS_MAGIC + (uint32_t)(a >> 23)) - 12582912.0f;
+  const float l = __uint_as_float(0x4B000000u | ((uint32_t)a & 0x7FFFFFu)) - 8388608.0f;
+  const float x = fmaf(h, 8388608.0f, l);
   const int b = __float_as_int(x), f = (b >> 23) & 0xFF;
-  if (a == 0) return 0.f;
-  if ((unsigned)(f + E - 1) < 253u) return __int_as_float(b + (E << 23));
+  if ((unsigned)(f + E - 1) < 253u && f) return __int_as_float(b + (E << 23));
   const int e1 = max(-240, min(240, E)) / 2, e2 = max(-240, min(240, E)) - e1;
   return x * __int_as_float((127 + e1) << 23) * __int_as_float((127 + e2) << 23);
 }
@@ -329,16 +368,22 @@ __device__ __forceinline__ float xs_scaled(long long a, int E, float) {
 // Seven slots of 32 KB.  The four slices share
 // 128-byte rows because TMA takes a row at a time: with 32-byte rows a tile of K =
 // 256 took 64 us, with 64- and 128-byte ones 42, with the converged issue loop
-// (umma_bf16_w) 30; the tensor pipe alone needs 18.  BN = 64: tiles of half the width
+// (umma_bf16_w) 30, with slice p of A kept in the collector buffer for its products
+// (umma_bf16_wa) 27.5; FP32 tiles 13.1, then 11.9.  The tensor pipe alone needs 21 (6):
+// a 128 x 128 x 16 product reads 8 KB at 128 B a clock, as long as it takes, and the
+// loads (48 slots; 16) write beside it.  (Half of B from each of two CTAs by
+// multicast changed nothing: 65 B a clock and SM from L2 are there, 27 are used.)
+// FP32 tiles load C while their products run and read the four diagonals eight columns
+// at a time.  BN = 64: tiles of half the width
 // for launches with fewer 128 x 128 tiles than SMs, where a tile's own time
 // counts: half the products and half the FP64 additions of the epilogue, whose C
-// entries are loaded while the products run.  Bound: tensor pipe / shared-memory
+// entries are loaded while the products run.  Bound: shared-memory
 // reads of the 128 x 128 products; a tile of a small launch by its epilogue.
 // Measured on GB300 for up to 80 tiles
-// of K = 64 (256): 29 (60) us with whole tiles, 19 (35) with these.
+// of K = 64 (256): 29 (60) us with whole tiles, 18 (31) with these.
 template <typename T, int BN>
 __global__ void __launch_bounds__(XS_THREADS, 1)
-k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const Item* __restrict__ items, int n_items,
+k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ XsMaps maps, const Item* __restrict__ items, int n_items,
             int nb, int region, int lower, int* err) {
   constexpr int S = XsType<T>::S;
   extern __shared__ __align__(1024) uint8_t xs_raw[];
@@ -399,10 +444,10 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
                 break;
               }
               const uint32_t fb = smem_u32(&bars[s]), st = smem_u32(smem + s * XS_SLOT);
-              mbar_expect_tx(fb, XS_SLOT);
+              mbar_expect_tx(fb, XS_BOX + BN * 128);
               const int64_t dr = (int64_t)(p * 4 * nch + k) * n;
-              tma_load_2d(st, &wsmap, 0, (int)(ya + dr), fb);
-              tma_load_2d(st + XS_BOX, &wsmap, 0, (int)(yb + dr), fb);
+              tma_load_2d(st, &maps.m128, 0, (int)(ya + dr), fb);
+              tma_load_2d(st + XS_BOX, BN == 128 ? &maps.m128 : &maps.m64, 0, (int)(yb + dr), fb);
               ++issued;
               if (++s == XS_SLOTS) { s = 0; ph ^= 1; }
             }
@@ -451,6 +496,26 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
       if (k == nk - 1) umma_commit_w(elected, acc_bar + 8 * a);
       return true;
     };
+    // between the first and the last chunk: the products of diagonals D0 .. D0 + 3
+    // slice of A by slice of A, which is read from shared memory once
+    auto inner = [&](auto dd, uint32_t s0, uint32_t s1) {
+      constexpr int D0 = decltype(dd)::value, np = D0 ? S : 4;
+#pragma unroll
+      for (int p = 0; p < np; ++p) {
+        constexpr int LAST = D0 + 3;
+        const int qa = D0 > p ? D0 - p : 0, qb = LAST - p;       // slices of B: qa .. qb
+        const uint32_t alo = (p < 4 ? s0 : s1) + 2 * (p & 3);
+#pragma unroll
+        for (int q = 0; q < np; ++q) {
+          if (q < qa || q > qb) continue;
+          const uint32_t blo = (q < 4 ? s0 : s1) + (XS_BOX >> 4) + 2 * (q & 3), acc = tmem + ((p + q) & 3) * XS_TILE;
+          if (qa == qb) umma_bf16_w(elected, acc, alo, blo, SDESC_SW128_HI, idesc, 1u);
+          else if (q == qa) umma_bf16_wa<UMMA_A_FILL>(elected, acc, alo, blo, SDESC_SW128_HI, idesc);
+          else if (q == qb) umma_bf16_wa<UMMA_A_LAST>(elected, acc, alo, blo, SDESC_SW128_HI, idesc);
+          else umma_bf16_wa<UMMA_A_USE>(elected, acc, alo, blo, SDESC_SW128_HI, idesc);
+        }
+      }
+    };
     auto lo_of = [&](int q) { return sdesc_lo(ring + (uint32_t)q * XS_SLOT); };
     for (int t = blockIdx.x; t < n_items && live; t += gridDim.x) {
       const Item it = items[t];
@@ -463,10 +528,14 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
           if (!live) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t s0 = lo_of(s), s1 = lo_of(q);
-          live = diag(std::integral_constant<int, 4>{}, s0, s1, k, nk) &&
-                 diag(std::integral_constant<int, 5>{}, s0, s1, k, nk) &&
-                 diag(std::integral_constant<int, 6>{}, s0, s1, k, nk) &&
-                 diag(std::integral_constant<int, 7>{}, s0, s1, k, nk);
+          if (k > 0 && k < nk - 1) {
+            inner(std::integral_constant<int, 4>{}, s0, s1);
+          } else {
+            live = diag(std::integral_constant<int, 4>{}, s0, s1, k, nk) &&
+                   diag(std::integral_constant<int, 5>{}, s0, s1, k, nk) &&
+                   diag(std::integral_constant<int, 6>{}, s0, s1, k, nk) &&
+                   diag(std::integral_constant<int, 7>{}, s0, s1, k, nk);
+          }
           umma_commit_w(elected, bar0 + 8 * (XS_SLOTS + s));
           umma_commit_w(elected, bar0 + 8 * (XS_SLOTS + q));
           s = q + 1 == XS_SLOTS ? 0 : q + 1;
@@ -478,10 +547,14 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
         if (!live) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t s0 = lo_of(s);
-        live = diag(std::integral_constant<int, 0>{}, s0, s0, k, nk) &&
-               diag(std::integral_constant<int, 1>{}, s0, s0, k, nk) &&
-               diag(std::integral_constant<int, 2>{}, s0, s0, k, nk) &&
-               diag(std::integral_constant<int, 3>{}, s0, s0, k, nk);
+        if (k > 0 && k < nk - 1) {
+          inner(std::integral_constant<int, 0>{}, s0, s0);
+        } else {
+          live = diag(std::integral_constant<int, 0>{}, s0, s0, k, nk) &&
+                 diag(std::integral_constant<int, 1>{}, s0, s0, k, nk) &&
+                 diag(std::integral_constant<int, 2>{}, s0, s0, k, nk) &&
+                 diag(std::integral_constant<int, 3>{}, s0, s0, k, nk);
+        }
         umma_commit_w(elected, bar0 + 8 * (XS_SLOTS + s));
         if (++s == XS_SLOTS) { s = 0; ph ^= 1; }
       }
@@ -506,6 +579,54 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
       // columns c0 + j, j < cend, of this thread's row are updated
       const int cend = row < rmax ? min(cmax, lower ? row + 1 : cmax) - c0 : 0;
       T* __restrict__ G = arena<T>(c) + f.off + row + (int64_t)c0 * n;
+      if constexpr (S == 4 && BN == 128) {
+        // FP32: the products of a tile take less time than eight rounds of C
+        // accesses; C is loaded while they run, and the four diagonals are read
+        // eight columns at a time
+        T cv[NC];
+#pragma unroll
+        for (int j = 0; j < NC; ++j) cv[j] = j < cend ? __ldcg(G + (int64_t)j * n) : T(0);
+        const int* __restrict__ ex = x.exps + x.exp0[it.front];
+        const int ea = cend > 0 ? ex[row] - 36 : 0;
+        const int ebl = c0 + lane < cmax ? ex[(lower ? 0 : n) + c0 + lane] : 0;      // NC = 32 lanes
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+          live = live && mbar_wait_lim(smem_u32(&acc_full[a]), par & 1, s_abort, err, XS_ERR, lim);
+        live = __all_sync(0xffffffffu, live);
+        if (!live) break;
+        par ^= 1u;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int h = 0; h < NC / 8; ++h) {
+          uint32_t v[4][8];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) XS_LD8(tbase + a * XS_TILE + 8 * h, v[a]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          xs_ints(tbase + 8 * h, v);
+          if (h == NC / 8 - 1) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane < 4) mbar_arrive(smem_u32(&acc_empty[lane]));
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            long long s4 = -(long long)XS_MAGIC * 0x1010101ll;
+            xs_add<24>(s4, (int)v[0][j]);
+            xs_add<16>(s4, (int)v[1][j]);
+            xs_add<8>(s4, (int)v[2][j]);
+            xs_add<0>(s4, (int)v[3][j]);
+            const int E = ea + __shfl_sync(0xffffffffu, ebl, 8 * h + j);
+            T d = xs_scaled(s4, E, T(0));
+            if (E > XS_BAD / 2) d = T(NAN);
+            cv[8 * h + j] -= d;
+          }
+        }
+        if (*s_abort) break;
+#pragma unroll
+        for (int j = 0; j < NC; ++j)
+          if (j < cend) G[(int64_t)j * n] = cv[j];
+        continue;
+      }
       constexpr bool EARLY = BN == 64;
       T ce[EARLY ? NC : 1];
       if constexpr (EARLY) {
@@ -532,7 +653,7 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
             if (lane == 0) mbar_arrive(smem_u32(&acc_empty[a]));
           }
 #pragma unroll
-          for (int j = 0; j < 16; ++j) xs_add<SH>(acc[16 * h + j], v[j]);
+          for (int j = 0; j < 16; ++j) xs_add<SH>(acc[16 * h + j], __float2int_rn(__uint_as_float(v[j])));
         }
         return true;
       };
@@ -579,7 +700,7 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ CUtensorMap wsmap, const 
   }
 }
 
-bool xs_encode(CUtensorMap* map, void* base, int64_t rows) {
+bool xs_encode(XsMaps* maps, void* base, int64_t rows) {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   if (!encode) {
     void* fn = nullptr;
@@ -593,15 +714,19 @@ bool xs_encode(CUtensorMap* map, void* base, int64_t rows) {
   }
   cuuint64_t dims[2] = {64, (cuuint64_t)rows};
   cuuint64_t strides[1] = {128};
-  cuuint32_t box[2] = {64, 128};
   cuuint32_t estr[2] = {1, 1};
-  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  for (int h = 0; h < 2; ++h) {
+    cuuint32_t box[2] = {64, h ? 64u : 128u};
+    if (encode(h ? &maps->m64 : &maps->m128, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return false;
+  }
+  return true;
 }
 
 template <typename T, int BN>
-static void xs_update_t(const DevCtx& c, const XsCtx& x, const CUtensorMap& map, const Item* items, int n_items,
+static void xs_update_t(const DevCtx& c, const XsCtx& x, const XsMaps& maps, const Item* items, int n_items,
                         int nb, int region, int lower, int cap, int* err, cudaStream_t s) {
   static int n_sm = 0;
   if (!n_sm) {
@@ -613,20 +738,20 @@ static void xs_update_t(const DevCtx& c, const XsCtx& x, const CUtensorMap& map,
   cudaFuncSetAttribute(k_xs_update<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XS_SMEM);
   const int sms = cap > 0 && cap < n_sm ? cap : n_sm;
   const int grid = n_items < sms ? n_items : sms;
-  k_xs_update<T, BN><<<grid, XS_THREADS, XS_SMEM, s>>>(c, x, map, items, n_items, nb, region, lower, err);
+  k_xs_update<T, BN><<<grid, XS_THREADS, XS_SMEM, s>>>(c, x, maps, items, n_items, nb, region, lower, err);
 }
 
-void launch_xs_update(const DevCtx& c, const XsCtx& x, const CUtensorMap& map, const Item* items, int n_items,
+void launch_xs_update(const DevCtx& c, const XsCtx& x, const XsMaps& maps, const Item* items, int n_items,
                       int dtype, int nb, int region, int lower, int tile_n, int cap, int* err, cudaStream_t s) {
   if (!n_items) return;
   if (nb > XS_NBO) throw std::invalid_argument("sliced update: panel wider than 256");
   if (tile_n != 64 && tile_n != XS_TILE) throw std::invalid_argument("sliced update: tiles are 64 or 128 columns wide");
   if (dtype == F64) {
-    if (tile_n == 64) xs_update_t<double, 64>(c, x, map, items, n_items, nb, region, lower, cap, err, s);
-    else xs_update_t<double, 128>(c, x, map, items, n_items, nb, region, lower, cap, err, s);
+    if (tile_n == 64) xs_update_t<double, 64>(c, x, maps, items, n_items, nb, region, lower, cap, err, s);
+    else xs_update_t<double, 128>(c, x, maps, items, n_items, nb, region, lower, cap, err, s);
   } else {
-    if (tile_n == 64) xs_update_t<float, 64>(c, x, map, items, n_items, nb, region, lower, cap, err, s);
-    else xs_update_t<float, 128>(c, x, map, items, n_items, nb, region, lower, cap, err, s);
+    if (tile_n == 64) xs_update_t<float, 64>(c, x, maps, items, n_items, nb, region, lower, cap, err, s);
+    else xs_update_t<float, 128>(c, x, maps, items, n_items, nb, region, lower, cap, err, s);
   }
 }
 

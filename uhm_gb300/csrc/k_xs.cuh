@@ -25,8 +25,11 @@ struct XsCtx {
   int* exps;
 };
 
-// 2D map over the workspace's 128-byte rows: box 128 rows, 128-byte swizzle
-bool xs_encode(CUtensorMap* map, void* base, int64_t rows);
+// 2D maps over the workspace's 128-byte rows: boxes of 128 and of 64 rows, 128-byte swizzle
+struct XsMaps {
+  CUtensorMap m128, m64;
+};
+bool xs_encode(XsMaps* maps, void* base, int64_t rows);
 // slices of xs_pack_rows(nb) panel rows, columns K0 .. K0 + W, W = min(nb, fs - K0), nb 64 or XS_NBO (item:
 // front, a = K0, b = first row, c = 0; c = 1: the rows are the front's
 // columns (U12^T: entries (K0 + k, row)), written to the B region)
@@ -40,7 +43,7 @@ void launch_xs_trsm(const DevCtx& c, const XsCtx& x, const Item* items, int n_it
 // and only entries col <= row are updated.  region as for k_tile_update: 0
 // every entry, 1 columns below the outer panel's end, 2 rows below it; cap:
 // CTAs (0: one per SM)
-void launch_xs_update(const DevCtx& c, const XsCtx& x, const CUtensorMap& map, const Item* items, int n_items,
+void launch_xs_update(const DevCtx& c, const XsCtx& x, const XsMaps& maps, const Item* items, int n_items,
                       int dtype, int nb, int region, int lower, int tile_n, int cap, int* err, cudaStream_t s);
 
 }  // namespace uhm_gpu
