@@ -2140,8 +2140,7 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
         launch_tc_pack(ctx, it, op.n_items, op.nb, op.param, d_ws, d_ws_off, d_ws_stride, op.q0, op.aux, st);
         break;
       case OP_TC_SYRK:
-        launch_tc_syrk(ctx, ws_map, d_ws_off, d_ws_stride, it, op.n_items, op.nb, op.param, 0,
-                       op.param == 3 ? 6 : 3, op.param == 3 ? TC_TERMS_BF16X6 : TC_TERMS_BF16X3, 1, 0, d_err, st);
+        launch_tc_syrk(ctx, ws_map, d_ws_off, d_ws_stride, it, op.n_items, op.nb, op.param, 0, 1, 0, d_err, st);
         break;
       case OP_XS_PACK:
         launch_xs_pack(ctx, op.nb == NB ? xs_in : xs_ctx, it, op.n_items, op.dtype, op.nb, st);
@@ -2160,7 +2159,7 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
       case OP_GEMM: launch_gemm_update(ctx, it, op.n_items, op.dtype, op.nb, op.q0, op.aux, st); break;
       case OP_TC_GEMM:
         // A parts 0-1 (L21), B parts 2-3 (U12^T)
-        launch_tc_syrk(ctx, ws_map, d_ws_off, d_ws_stride, it, op.n_items, op.nb, 2, 2, 3, TC_TERMS_BF16X3, 0,
+        launch_tc_syrk(ctx, ws_map, d_ws_off, d_ws_stride, it, op.n_items, op.nb, 2, 2, 0,
                        profiling ? 0 : op.cap, d_err, st);
         break;
       case OP_CLEAR_FLAGS:

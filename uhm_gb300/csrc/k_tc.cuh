@@ -13,16 +13,11 @@ bool tc_encode_part(CUtensorMap* map, void* base, int64_t rows, int nbo);
 // trans = 1: the LU panel's U block right of it, transposed (B operand)
 void launch_tc_pack(const DevCtx& c, const Item* items, int n_items, int nbo, int nparts, void* ws,
                     const int64_t* ws_off, const int64_t* ws_stride, int trans, int poff, cudaStream_t s);
+// C -= A B^T, operands in BF16 parts: A 0 .. parts - 1, B pb0 .. pb0 + parts - 1, the
+// terms p + q < parts; cap: CTAs (0: one per SM)
 void launch_tc_syrk(const DevCtx& c, const CUtensorMap& wsmap, const int64_t* ws_off,
-                    const int64_t* ws_stride, const Item* items, int n_items, int nbo, int parts, int pb0, int nterms,
-                    uint32_t term_code, int lower_only, int cap, int* err, cudaStream_t s);
+                    const int64_t* ws_stride, const Item* items, int n_items, int nbo, int parts, int pb0,
+                    int lower_only, int cap, int* err, cudaStream_t s);
 int tc_tile();
-
-// cap: CTAs (0: one per SM); operands: A parts 0 .. parts - 1, B parts pb0 .. pb0 + parts - 1; term codes:
-// 4 bits per term = (A part) | (B part - pb0) << 2
-constexpr uint32_t TC_TERMS_BF16X3 = (0u | 0u << 2) | ((0u | 1u << 2) << 4) | ((1u | 0u << 2) << 8);
-constexpr uint32_t TC_TERMS_BF16X6 = (0u | 0u << 2) | ((0u | 1u << 2) << 4) | ((1u | 0u << 2) << 8) |
-                                     ((0u | 2u << 2) << 12) | ((1u | 1u << 2) << 16) |
-                                     ((2u | 0u << 2) << 20);
 
 }  // namespace uhm_gpu

@@ -56,8 +56,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 
 // item: front, a = K0 (outer step start), b = tile row, c = tile col
 // (tiles counted from the trailing block's first row K0 + KB).
-// Operand parts: A 0 .. parts - 1, B pb0 .. pb0 + parts - 1; term_code: 4 bits
-// per term (A part, B part - pb0).
+// Operand parts: A 0 .. PARTS - 1, B pb0 .. pb0 + PARTS - 1; the products of parts p
+// and q, p + q < PARTS (three terms for two parts, six for three).
 //
 // Persistent: one CTA per SM walks the tile list with stride gridDim.x.  The
 // TMA ring (full / empty barriers) runs continuously across tiles; TMEM holds
@@ -66,11 +66,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // is committed by the MMA warp when accumulator b holds a finished tile;
 // acc_empty[b] collects the epilogue warps once they have read it.
 // Measured on GB300, the LU trailing updates of 24^3 p = 3 (BF16X3, K = 256):
-// 21.7 -> 17.0 ms; 13,225 tiles 522 -> 428 us, of which C's traffic alone is 255.
+// 21.7 -> 15.6 ms; 13,000 tiles 513 -> 379 us, of which C's traffic alone is 251 (420
+// before the next tile's C was asked into L2 while a tile's products run and a part
+// of A was kept in the collector buffer).
+template <int PARTS>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_tc_syrk(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __restrict__ ws_off,
-          const int64_t* __restrict__ ws_stride, const Item* __restrict__ items, int n_items, int nbo, int parts,
-          int pb0, int nterms, uint32_t term_code, int lower_only, int* err) {
+          const int64_t* __restrict__ ws_stride, const Item* __restrict__ items, int n_items, int nbo,
+          int pb0, int lower_only, int* err) {
   extern __shared__ __align__(1024) uint8_t tc_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TC_RING);
@@ -81,8 +84,10 @@ k_tc_syrk(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __
   volatile int* s_abort = reinterpret_cast<volatile int*>(drain_bar + 1);
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(drain_bar + 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t slot_bytes = 2 * (uint32_t)parts * TC_TILE_BYTES;
-  const int slots = min(TC_SLOTS_MAX, (int)(TC_RING / slot_bytes));
+  constexpr int parts = PARTS;
+  constexpr uint32_t slot_bytes = 2 * (uint32_t)parts * TC_TILE_BYTES;
+  constexpr int slots = TC_RING / slot_bytes;
+  static_assert(slots >= 2 && slots <= TC_SLOTS_MAX, "ring");
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_SLOTS_MAX; ++s) {
@@ -167,15 +172,28 @@ k_tc_syrk(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a0 = sdesc_lo(ring + (uint32_t)s * slot_bytes);
         const uint32_t b0 = sdesc_lo(ring + (uint32_t)s * slot_bytes + (uint32_t)parts * TC_TILE_BYTES);
-        for (int q = 0; q < nterms; ++q) {
-          const uint32_t at = a0 + ((term_code >> (4 * q)) & 3) * (TC_TILE_BYTES >> 4);
-          const uint32_t bt = b0 + ((term_code >> (4 * q + 2)) & 3) * (TC_TILE_BYTES >> 4);
+        // per 16 columns, part of A by part of A: its products with parts 0 .. PARTS -
+        // 1 - p of B; A is read from shared memory once (collector buffer)
 #pragma unroll
-          for (int k = 0; k < TC_BK / 16; ++k) {
-            umma_bf16_w(elected, acc, at + 2 * k, bt + 2 * k, SDESC_SW128_HI, idesc, on);
-            on = 1u;
-          }
-        }
+        for (int k = 0; k < TC_BK / 16; ++k)
+#pragma unroll
+          for (int p = 0; p < PARTS; ++p)
+#pragma unroll
+            for (int q = 0; q < PARTS - p; ++q) {
+              const uint32_t at = a0 + p * (TC_TILE_BYTES >> 4) + 2 * k, bt = b0 + q * (TC_TILE_BYTES >> 4) + 2 * k;
+              if (k == 0 && p == 0 && q == 0) {
+                umma_bf16_w(elected, acc, at, bt, SDESC_SW128_HI, idesc, on);
+                on = 1u;
+              } else if (k == 0 && p == 0 || p == PARTS - 1) {
+                umma_bf16_w(elected, acc, at, bt, SDESC_SW128_HI, idesc, 1u);
+              } else if (q == 0) {
+                umma_bf16_wa<UMMA_A_FILL>(elected, acc, at, bt, SDESC_SW128_HI, idesc);
+              } else if (q < PARTS - p - 1) {
+                umma_bf16_wa<UMMA_A_USE>(elected, acc, at, bt, SDESC_SW128_HI, idesc);
+              } else {
+                umma_bf16_wa<UMMA_A_LAST>(elected, acc, at, bt, SDESC_SW128_HI, idesc);
+              }
+            }
         umma_commit_w(elected, empty0 + 8 * s);
         if (++s == slots) { s = 0; ph ^= 1; }
       }
@@ -189,19 +207,38 @@ k_tc_syrk(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __
     // tile rows) and handles the columns [32 (w / 4), +32); the entries of C are
     // loaded while the products run
     constexpr int NC = TC_BN / 4;
+    static_assert(NC == 32, "a lane per column of the prefetch");
     const int quarter = warp & 3, cg = warp >> 2;
-    int i = 0;
-    for (int t = blockIdx.x; t < n_items; t += gridDim.x, ++i) {
+    // columns c0 + j, j < cend, of this thread's row are updated, entry 0 at G
+    struct Geo { float* G; int n, cend; };
+    auto geo_of = [&](int t) {
       const Item it = items[t];
       const FrontDev& f = c.fronts[it.front];
       const int n = f.n, base = it.a + min(nbo, f.fs - it.a);
       const int row = base + it.b * TC_BM + quarter * 32 + lane, c0 = base + it.c * TC_BN + cg * NC;
-      // columns c0 + j, j < cend, of this thread's row are updated
-      const int cend = row < n ? (lower_only ? min(n, row + 1) : n) - c0 : 0;
-      float* __restrict__ G = c.a32 + f.off + row + (int64_t)c0 * n;
+      return Geo{c.a32 + f.off + row + (int64_t)c0 * n, n, row < n ? (lower_only ? min(n, row + 1) : n) - c0 : 0};
+    };
+    int i = 0;
+    Geo cur = {};
+    if ((int)blockIdx.x < n_items) cur = geo_of(blockIdx.x);
+    for (int t = blockIdx.x; t < n_items; t += gridDim.x, ++i) {
+      const int n = cur.n, cend = cur.cend;
+      float* __restrict__ G = cur.G;
       float v[NC];
 #pragma unroll
       for (int j = 0; j < NC; ++j) v[j] = j < cend ? __ldcg(G + (int64_t)j * n) : 0.0f;
+      // the next tile's C towards L2: lane j asks for the rows of column j, at its
+      // first and its last row
+      if (t + (int)gridDim.x < n_items) {
+        cur = geo_of(t + gridDim.x);
+        const float* p0 = cur.G - lane + (int64_t)lane * cur.n;
+        const int most = __reduce_max_sync(0xffffffffu, cur.cend);
+        const unsigned rows = __ballot_sync(0xffffffffu, cur.cend > 0);
+        if (lane < most) {
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(p0 + __ffs(rows) - 1));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(p0 + 31 - __clz(rows)));
+        }
+      }
       const int b = i & 1, u = i >> 1;
       const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_full[b]), u & 1, s_abort, err));
       if (!ok) break;
@@ -328,10 +365,10 @@ void launch_tc_pack(const DevCtx& c, const Item* items, int n_items, int nbo, in
 }
 
 void launch_tc_syrk(const DevCtx& c, const CUtensorMap& wsmap, const int64_t* ws_off,
-                    const int64_t* ws_stride, const Item* items, int n_items, int nbo, int parts, int pb0, int nterms,
-                    uint32_t term_code, int lower_only, int cap, int* err, cudaStream_t s) {
+                    const int64_t* ws_stride, const Item* items, int n_items, int nbo, int parts, int pb0,
+                    int lower_only, int cap, int* err, cudaStream_t s) {
   if (!n_items) return;
-  if (parts < 1 || 2 * parts * TC_TILE_BYTES > TC_RING) throw std::invalid_argument("tc_syrk: 1 to 6 operand parts");
+  if (parts != 2 && parts != 3) throw std::invalid_argument("tc_syrk: operands of two or three parts");
   static int n_sm = 0;
   if (!n_sm) {
     int dev = 0;
@@ -339,11 +376,11 @@ void launch_tc_syrk(const DevCtx& c, const CUtensorMap& wsmap, const int64_t* ws
     cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
     if (n_sm <= 0) n_sm = 1;
   }
-  cudaFuncSetAttribute(k_tc_syrk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
+  const auto kernel = parts == 2 ? k_tc_syrk<2> : k_tc_syrk<3>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
   const int sms = cap > 0 && cap < n_sm ? cap : n_sm;
   const int grid = n_items < sms ? n_items : sms;   // one persistent CTA per SM
-  k_tc_syrk<<<grid, TC_THREADS, TC_SMEM, s>>>(c, wsmap, ws_off, ws_stride, items, n_items, nbo, parts, pb0, nterms,
-                                              term_code, lower_only, err);
+  kernel<<<grid, TC_THREADS, TC_SMEM, s>>>(c, wsmap, ws_off, ws_stride, items, n_items, nbo, pb0, lower_only, err);
 }
 
 int tc_tile() { return TC_BM; }
