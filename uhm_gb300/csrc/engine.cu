@@ -932,14 +932,15 @@ void Engine::build_programs(int method) {
   };
   // one Cholesky step's diagonal block + panel TRSM: fused (every CTA of the
   // TRSM factors the block, the first writes its inverse) or two launches
+  // (slices: for an update by sliced products)
   auto push_potrf_trsm = [&](int dt, const std::vector<Item>& p_items, const std::vector<Item>& t_items,
-                             double fp, double ft) {
+                             double fp, double ft, int slices) {
     // every fused CTA repeats the latency-bound diagonal factorisation: fuse
     // only while the launch fits fuse_potrf_trsm waves of one CTA per SM
     const size_t n_fused = t_items.size() + p_items.size();
     if (!tune.fuse_potrf_trsm || n_fused > (size_t)tune.fuse_potrf_trsm * n_sm) {
       push(fac_ops, OP_POTRF, dt, NB, 0, p_items, fp);
-      push(fac_ops, OP_TRSM, dt, NB, 0, t_items, ft);
+      push(fac_ops, OP_TRSM, dt, NB, slices, t_items, ft);
       return;
     }
     // consecutive row blocks of a front grouped so that the launch is one wave
@@ -958,7 +959,7 @@ void Engine::build_programs(int method) {
         fi.push_back(Item{d.front, d.a, rows[g0], (g0 == 0 ? 1 : 0) | (cnt << 1)});
       }
     }
-    push(fac_ops, OP_POTRF_TRSM, dt, NB, 0, fi, fp + ft);
+    push(fac_ops, OP_POTRF_TRSM, dt, NB, slices, fi, fp + ft);
   };
   // one LU step's 64-column panel: tall panels (many rows below the
   // diagonal) on many CTAs at once (panel-only row swaps, then k_laswp for
@@ -1211,8 +1212,8 @@ void Engine::build_programs(int method) {
               for (int c0 = base; c0 < B; c0 += LUROW_CB) t_items.push_back(Item{s, k0, c0, B});
             }
             if (base >= B) continue;
-            // (FP64 Cholesky: the TRSM writes the slices)
-            if (!chol || dt == F32) xs_pack_items(pk, NB, s, k0, base, f.n, 0);
+            // (Cholesky: the TRSM writes the slices)
+            if (!chol) xs_pack_items(pk, NB, s, k0, base, f.n, 0);
             if (!chol) xs_pack_items(pk, NB, s, k0, base, B, 1);
             fu += xs_tiles(ut, f, k0, kb, base, f.n, base, B, chol, bu);
           }
@@ -1220,7 +1221,7 @@ void Engine::build_programs(int method) {
             push(fac_ops, OP_POTRF, dt, NB, 0, p_items, fp);
             push(fac_ops, OP_TRSM, dt, NB, 0, t_items, ft);
           } else if (chol) {
-            push_potrf_trsm(dt, p_items, t_items, fp, ft);
+            push_potrf_trsm(dt, p_items, t_items, fp, ft, 1);
           } else {
             push_lu_panel(dt, p_items, fp, XS_NBO, n_sm - side);
             push(fac_ops, OP_LUROW, dt, NB, 0, t_items, ft);
@@ -1444,7 +1445,7 @@ void Engine::build_programs(int method) {
             const double w = std::max(0, cmax - base), mr = f.n - base;
             fu += 2.0 * kb * (w * mr - 0.5 * w * (w - 1));
           }
-          push_potrf_trsm(dt, p_items, t_items, fp, ft);
+          push_potrf_trsm(dt, p_items, t_items, fp, ft, 0);
           push(fac_ops, OP_SYRK, dt, NB, NBO, u_items, fu);
         }
         std::vector<Item> pk, tt;
@@ -2119,9 +2120,9 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
       case OP_POTRF: launch_potrf_diag(ctx, it, op.n_items, op.dtype, op.nb, st); break;
       case OP_TRSM:
         if (op.dtype == F64) launch_xs_trsm(ctx, xs_in, it, op.n_items, st);
-        else launch_trsm_panel(ctx, it, op.n_items, op.dtype, op.nb, st);
+        else launch_trsm_panel(ctx, it, op.n_items, op.dtype, op.nb, xs_in, op.param, st);
         break;
-      case OP_POTRF_TRSM: launch_potrf_trsm(ctx, it, op.n_items, op.dtype, st); break;
+      case OP_POTRF_TRSM: launch_potrf_trsm(ctx, it, op.n_items, op.dtype, xs_in, op.param, st); break;
       case OP_SYRK: launch_syrk_update(ctx, it, op.n_items, op.dtype, op.nb, op.param, st); break;
       case OP_FWD_FLAGS:
         if (op.aux == 256)

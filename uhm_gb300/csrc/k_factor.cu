@@ -24,6 +24,7 @@
 #include <string>
 #include "k_common.cuh"
 #include "k_potrf.cuh"
+#include "k_xs_slices.cuh"
 
 namespace uhm_gpu {
 
@@ -757,7 +758,8 @@ constexpr int TRSM_RB = 64;   // rows per panel-TRSM block
 // X (rows r0..r0+RB of columns k0..k0+kb) <- X * L11^{-T}
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_trsm_panel(DevCtx c, const Item* __restrict__ items,
-                                                   int nb) {
+                                                   int nb, XsCtx x, int slices) {
+  __shared__ int s_f[4][64];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
@@ -812,6 +814,8 @@ __global__ void __launch_bounds__(NT) k_trsm_panel(DevCtx c, const Item* __restr
       const int j = jg * 16 + u;
       if (i < rb && j < kb) G[(r0 + i) + (int64_t)(k0 + j) * n] = acc[u];
     }
+    if (slices && k0 + kb < min(k0 / XS_NBO * XS_NBO + XS_NBO, f.fs))
+      xs_store_step<T>(x, it.front, n, r0 + i, i < rb, acc, s_f);
     return;
   }
   for (int idx = threadIdx.x; idx < kb * kb; idx += NT) {
@@ -840,13 +844,13 @@ __global__ void __launch_bounds__(NT) k_trsm_panel(DevCtx c, const Item* __restr
   }
 }
 
-void launch_trsm_panel(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
+void launch_trsm_panel(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, const XsCtx& x, int slices,
                        cudaStream_t s) {
   if (!n_items) return;
   if (dtype == F64) throw std::invalid_argument("trsm_panel: FP64 fronts take xs_trsm");
   size_t sm = (size_t)(64 * 68 + TRSM_RB * nb) * sizeof(float);
   cudaFuncSetAttribute(k_trsm_panel<float, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_trsm_panel<float, 256><<<n_items, 256, sm, s>>>(c, items, nb);
+  k_trsm_panel<float, 256><<<n_items, 256, sm, s>>>(c, items, nb, x, slices);
 }
 
 // Diagonal block and panel TRSM of one 64-column step in one launch.  Every
@@ -859,11 +863,14 @@ void launch_trsm_panel(const DevCtx& c, const Item* items, int n_items, int dtyp
 // CTAs still reading A's block, so the arena keeps A's diagonal block.  A CTA
 // takes several consecutive row blocks, so that a step's launch is one wave.
 // Item: front, a = k0, b = first row of the first block (n: none),
-// c = writer (bit 0) + 2 * number of row blocks.
+// c = writer (bit 0) + 2 * number of row blocks.  slices: the rows' slices for
+// the update inside the outer panel too (a launch of their own took 11 us and
+// more a step).
 constexpr int PT_LD = 68;   // row length of the transposed inverse in shared memory (16-byte rows)
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_potrf_trsm(DevCtx c, const Item* __restrict__ items) {
+__global__ void __launch_bounds__(256) k_potrf_trsm(DevCtx c, const Item* __restrict__ items, XsCtx xs, int slices) {
+  __shared__ int s_f[4][64];
   extern __shared__ __align__(16) unsigned char pt_smem[];
   PotrfShared<T>& sh = *reinterpret_cast<PotrfShared<T>*>(pt_smem);
   T* Lt = reinterpret_cast<T*>(pt_smem + ((sizeof(PotrfShared<T>) + 15) / 16) * 16);   // 64 x PT_LD
@@ -933,15 +940,18 @@ __global__ void __launch_bounds__(256) k_potrf_trsm(DevCtx c, const Item* __rest
       const int j = jg * 16 + u;
       if (i < rb && j < kb) A[(r0 + i) + (int64_t)(k0 + j) * n] = acc[u];
     }
+    if (slices && k0 + kb < min(k0 / XS_NBO * XS_NBO + XS_NBO, f.fs))
+      xs_store_step<T>(xs, it.front, n, r0 + i, i < rb, acc, s_f);
   }
 }
 
-void launch_potrf_trsm(const DevCtx& c, const Item* items, int n_items, int dtype, cudaStream_t s) {
+void launch_potrf_trsm(const DevCtx& c, const Item* items, int n_items, int dtype, const XsCtx& x, int slices,
+                       cudaStream_t s) {
   if (!n_items) return;
   if (dtype == F64) throw std::invalid_argument("potrf_trsm: FP64 fronts take potrf_diag and trsm_panel");
   const size_t sm = ((sizeof(PotrfShared<float>) + 15) / 16) * 16 + sizeof(float) * 64 * PT_LD;
   cudaFuncSetAttribute(k_potrf_trsm<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_potrf_trsm<float><<<n_items, 256, sm, s>>>(c, items);
+  k_potrf_trsm<float><<<n_items, 256, sm, s>>>(c, items, x, slices);
 }
 
 // FP32 update of one 128 x 64 tile of the front by a panel of kb <= 64 columns:

@@ -40,79 +40,17 @@
 #include "k_common.cuh"
 #include "k_tc_ptx.cuh"
 #include "k_xs.cuh"
+#include "k_xs_slices.cuh"
 
 namespace uhm_gpu {
 
 UHM_DEFINE_WAIT_LIMIT(set_wait_limit_xs, 1u << 22)
 
-// exponent of a row holding a NaN or an infinity: the update is NaN in that
-// whole row and column (an infinity becomes one in the panel's TRSM already:
-// the product with the zeros of the diagonal block's inverse)
-constexpr int XS_BAD = 1 << 28;
 constexpr int XS_ERR = 7;
-
-// 64-column chunks per slice of a front's layout in a launch of panel width nb
-__device__ __forceinline__ int xs_chunks(int nb, int fs) { return (min(nb, fs) + 63) / 64; }
 
 // ---------------------------------------------------------------------------
 // slices
 // ---------------------------------------------------------------------------
-template <typename T> struct XsType;
-template <> struct XsType<double> {
-  static constexpr int S = XS_S64;
-  static __device__ __forceinline__ int field(double v) { return (__double2hiint(v) >> 20) & 0x7FF; }
-  static constexpr int FMAX = 0x7FF, EBIAS = 1022;
-  // round(v 2^(62 - e)), e = fmax - EBIAS, fmax the largest exponent field of the row (at least 1)
-  static __device__ __forceinline__ long long fixed(double v, int fmax) {
-    const long long b = __double_as_longlong(v);
-    int f = (int)((b >> 52) & 0x7FF);
-    long long m = b & 0xFFFFFFFFFFFFFll;
-    if (f) m |= 1ll << 52;
-    else f = 1;
-    const int sh = fmax - f;
-    m <<= 9;
-    if (sh > 0) m = sh > 62 ? 0 : (m + (1ll << (sh - 1))) >> sh;
-    return b < 0 ? -m : m;
-  }
-};
-template <> struct XsType<float> {
-  static constexpr int S = XS_S32;
-  static __device__ __forceinline__ int field(float v) { return (__float_as_int(v) >> 23) & 0xFF; }
-  static constexpr int FMAX = 0xFF, EBIAS = 126;
-  // round(v 2^(30 - e))
-  static __device__ __forceinline__ long long fixed(float v, int fmax) {
-    const int b = __float_as_int(v);
-    int f = (b >> 23) & 0xFF;
-    int m = b & 0x7FFFFF;
-    if (f) m |= 1 << 23;
-    else f = 1;
-    const int sh = fmax - f;
-    m <<= 6;
-    if (sh > 0) m = sh > 31 ? 0 : (m + (1 << (sh - 1))) >> sh;
-    return b < 0 ? -m : m;
-  }
-};
-
-// the digits of one entry, as bits of exact floats (d[p] = slice p)
-template <int S>
-__device__ __forceinline__ void xs_digits(long long X, uint32_t (&d)[S]) {
-  // balanced digits: adding 128 to every place but the top turns each into its
-  // byte; float(2^23 + byte) - (2^23 + 128) is the digit
-  constexpr long long BIAS = S == 8 ? 0x0080808080808080ll : 0x0000000000808080ll;
-  const long long Y = X + BIAS;
-#pragma unroll
-  for (int p = 0; p < S; ++p) {
-    float dg;
-    if (p == 0) {
-      dg = __int_as_float(0x4B400000 + (int)(Y >> (8 * (S - 1)))) - 12582912.0f;
-    } else {
-      const uint32_t b = (uint32_t)(Y >> (8 * (S - 1 - p))) & 0xFFu;
-      dg = __int_as_float((int)(0x4B000000u | b)) - 8388736.0f;
-    }
-    d[p] = __float_as_uint(dg);
-  }
-}
-
 // A CTA cuts 256 / NG rows: thread r + (256 / NG) g holds 16 columns 16 g .. of
 // row r (a warp's loads of one column are consecutive rows), all its loads in
 // flight, and writes its digits as one or two whole rows of the workspace.  NG =
@@ -147,23 +85,7 @@ __global__ void __launch_bounds__(256) k_xs_pack(DevCtx c, XsCtx x, const Item* 
   if (!in || 16 * g >= 64 * nch) return;
   const bool bad = fm == XsType<T>::FMAX;
   if (g == 0) x.exps[x.exp0[it.front] + (trans ? n : 0) + row] = bad ? XS_BAD : fm - XsType<T>::EBIAS;
-  uint8_t* const w0 = reinterpret_cast<uint8_t*>(x.ws) +
-                      128 * ((trans ? x.row0b : x.row0)[it.front] + (int64_t)g * n + row);
-  uint32_t d[S][8];
-#pragma unroll
-  for (int u = 0; u < 16; u += 2) {
-    uint32_t d0[S], d1[S];
-    xs_digits<S>(bad ? 0 : XsType<T>::fixed(v[u], fm), d0);
-    xs_digits<S>(bad ? 0 : XsType<T>::fixed(v[u + 1], fm), d1);
-#pragma unroll
-    for (int p = 0; p < S; ++p) d[p][u / 2] = __byte_perm(d0[p], d1[p], 0x7632);
-  }
-#pragma unroll
-  for (int p = 0; p < S; ++p) {
-    uint4* w = reinterpret_cast<uint4*>(w0 + 128 * (int64_t)((p >> 2) * 4 * nch) * n + 32 * (p & 3));
-    w[0] = make_uint4(d[p][0], d[p][1], d[p][2], d[p][3]);
-    w[1] = make_uint4(d[p][4], d[p][5], d[p][6], d[p][7]);
-  }
+  xs_store16<T>(x, (trans ? x.row0b : x.row0)[it.front] + (int64_t)g * n + row, (int64_t)4 * nch * n, v, fm, bad);
 }
 
 void launch_xs_pack(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, int dtype, int nb,

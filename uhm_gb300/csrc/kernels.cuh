@@ -53,6 +53,8 @@ struct Item {
 // Status words written by kernels (breakdown detection): per front.
 enum Status : int { ST_OK = 0, ST_NOT_SPD = 1, ST_ZERO_PIVOT = 2, ST_NAN = 3, ST_WAIT = 4 };
 
+struct XsCtx;          // operand slices (k_xs.cuh)
+
 struct DevCtx {
   FrontDev* fronts;
   SrcDev* srcs;
@@ -86,10 +88,11 @@ void launch_small_factor(const DevCtx& c, const Item* items, int n_items, int dt
                          int max_n, cudaStream_t s);
 // diagonal block + panel TRSM of one 64-column step (every CTA factors the
 // block; item: front, a = k0, b = first row of the panel block, c = 1 writer)
-void launch_potrf_trsm(const DevCtx& c, const Item* items, int n_items, int dtype, cudaStream_t s);
+void launch_potrf_trsm(const DevCtx& c, const Item* items, int n_items, int dtype, const XsCtx& x, int slices,
+                       cudaStream_t s);
 void launch_potrf_diag(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
                        cudaStream_t s);
-void launch_trsm_panel(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
+void launch_trsm_panel(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, const XsCtx& x, int slices,
                        cudaStream_t s);
 constexpr int TILE_UPDATE_ROWS = 128, TILE_UPDATE_COLS = 64;   // tiles of the FP32 updates inside a panel
 void launch_syrk_update(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
