@@ -582,165 +582,293 @@ __global__ void __launch_bounds__(256) k_potrf_diag(DevCtx c, const Item* __rest
   if (nb == 64 && Dinv) potrf_store_inverse<T>(kb, x, Dinv + f.dinv_off + (int64_t)(k0 / 64) * 4096);
 }
 
+UHM_DEFINE_WAIT_LIMIT(set_wait_limit_factor, 1u << 22)
+
+// 1 / v by Chebyshev's iteration: an FP32 start x of the mantissa, then
+// x (1 + r + r^2), r = 1 - v x (the next term, r^3, is below 2^-66); three
+// dependent FP64 operations, 0.5000 ulp over 10^8 values of every exponent
+__device__ __forceinline__ double fp64_rcp(double v) {
+  const int hi = __double2hiint(v), f = (hi >> 20) & 0x7FF;
+  if (f < 24 || f > 2022) return 1.0 / v;
+  const float m = __int_as_float((127 << 23) | (hi & 0xFFFFF) << 3 | (int)((unsigned)__double2loint(v) >> 29));
+  const uint32_t xb = __float_as_uint(1.0f / m);               // (1/2, 1]
+  const double x = __hiloint2double((int)((hi & 0x80000000u) | ((xb >> 3) + ((1023 - 127 - (f - 1023)) << 20))),
+                                    (int)(xb << 29));
+  const double r = fma(-v, x, 1.0);
+  return fma(x, fma(r, r, r), x);
+}
+
 // The same for FP64 fronts: only the inverse is formed (the solves and the
 // TRSM use nothing else), and no multiply-add is spent on zeros.  GB300 does
 // about 2 FP64 multiply-adds per clock per SM, so a warp instruction costs its
 // scheduler ~64 clocks whatever its lanes do: the block is bound by their
-// count and by the chain of pivots.  Tile (i, j), i >= j, of the 16 x 16 lower tiles (4 x 4 entries)
-// holds A until step j and X = L^{-1} after it; either way step q < i takes
-// the one rank-4 update  t -= L[tile i, q] B[:, tile j],  B[m][c] = L(c, P+m)
-// right of the pivot columns P .. P+3 (j > q) and X(P+m, c) left of them (j
-// <= q): 2 x 136 half tiles on 9 warps.  The step's 64 vectors (rows of A from
-// the pivot on, columns of X) take the same 4-step substitution, one thread each of
-// two solver warps, which factor the pivot block (every thread) as well.
-// The solvers run one step ahead: their vectors leave the tiles before the
-// update of the step before, which the solvers apply themselves, so that pivots
-// and bulk updates overlap; they hand over on named barriers.  The bulk warps
-// are spread so that the schedulers of the solver warps take fewer of them.
+// count and by the chain of pivots, and is spread over a cluster of two CTAs.
+// Rank 0 factors A = U D U^T (U unit lower; a pivot costs its reciprocal, three
+// dependent FP64 operations, and a step's vectors no product after their
+// substitution); rank 1 forms Z = U^{-1} a step behind it, from the columns of U
+// that rank 0 writes into its shared memory, and stores L^{-1} = D^{-1/2} Z.
+//
+// Both keep 4 x 4 tiles (i, j), i >= j, in registers, half a tile per thread,
+// 4 x 4 tiles per warp (ten warps), so that whole warps are done early: step q (pivot
+// columns P .. P+3) takes t -= U[tile i, q] W[:, tile j], W the rows' products with
+// the pivots (A: j > q) or the solved rows P .. P+3 of Z (j <= q < i).  Two more
+// warps solve the step's 64 vectors by a 4-step substitution, one thread each, and,
+// rank 0, factor the pivot block (every thread).  Rank 0's solvers run one step
+// ahead: their vectors leave the tiles before the update of the step before,
+// which the solvers apply themselves, so that pivots and bulk updates overlap; they
+// hand over on named barriers.
 // Measured on GB300: 294 us per block in the tile-per-thread form
-// (k_potrf_diag), which updates the full squares; 67 with the steps in
-// turn; 60 so (the solvers' chain of dependent FP64 operations, ~45 a step).
-constexpr int PD_BULK_WARPS = 9, PD_THREADS = 12 * 32;
-constexpr int PD_ALL = 32 * (PD_BULK_WARPS + 2);      // threads of a hand-over barrier
-// role of each warp: bulk chunk 0 .. 8 (tiles in order of i: the last chunks work
-// longest), 16 / 17 solver, -1 none; a warp's scheduler is its index mod 4
-__device__ __constant__ signed char pd_role[12] = {8, 2, 1, 7, 6, 0, -1, 5, 4, 16, 17, 3};
+// (k_potrf_diag), which updates the full squares; one CTA for both 67 with the
+// steps in turn, 60 with the solvers ahead, 58 without square roots; 54 so.
+constexpr int PD_WARPS = 12, PD_THREADS = 32 * PD_WARPS;
+// role of each warp, by rank: tile group 0 .. 9 ((I, J), I >= J, by J), 16 / 17
+// solver; a warp's scheduler is its index mod 4 (rank 0: the solvers' take the groups
+// that are done first)
+__device__ __constant__ signed char pd_role[2][PD_WARPS] = {{16, 17, 4, 6, 0, 2, 5, 7, 1, 3, 9, 8},
+                                                            {16, 17, 1, 2, 0, 3, 4, 5, 7, 9, 6, 8}};
+__device__ __constant__ signed char pd_group[10][2] = {{0, 0}, {1, 0}, {2, 0}, {3, 0}, {1, 1},
+                                                       {2, 1}, {3, 1}, {2, 2}, {3, 2}, {3, 3}};
 
 __device__ __forceinline__ void pd_arrive(int id) {
-  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(PD_ALL) : "memory");
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(PD_THREADS) : "memory");
 }
 __device__ __forceinline__ void pd_sync(int id) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(PD_ALL) : "memory");
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(PD_THREADS) : "memory");
+}
+__device__ __forceinline__ uint32_t pd_peer(const void* p) {       // the same variable of rank 1
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 1;"
+               : "=r"(r) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))));
+  return r;
+}
+__device__ __forceinline__ void pd_put(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
 
+struct PdShared {
+  double V[2][4][64];        // vectors handed to the solvers
+  double W[2][4][64];        // their results
+  double B[16][4][64];       // columns of U: rank 0 the last two steps', rank 1 every step's
+  double l[16][4][4];        // U's pivot blocks
+  double ds[64];             // D (rank 1: then D^{-1/2})
+  double pv[4][4];           // rank 0
+  double Z[64][65];          // rank 1
+  unsigned long long bar[16];        // rank 1: step q's column has arrived
+};
+
 __global__ void __launch_bounds__(PD_THREADS) k_potrf_inv64(DevCtx c, const Item* __restrict__ items) {
-  __shared__ __align__(16) double V[2][4][64], B[2][4][64];
-  __shared__ double pv[4][4];
-  const Item it = items[blockIdx.x];
+  extern __shared__ __align__(16) unsigned char pd_smem[];
+  PdShared& sh = *reinterpret_cast<PdShared*>(pd_smem);
+  const Item it = items[blockIdx.x >> 1];
+  const int rank = blockIdx.x & 1;
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, k0 = it.a;
   const int kb = min(64, f.fs - k0);
-  const int role = pd_role[threadIdx.x >> 5], lane = threadIdx.x & 31;
-  // barriers: 1 the solvers; 2, 3 vectors of step q (q mod 2) published; 4, 5 B of step q written
+  const int role = pd_role[rank][threadIdx.x >> 5], lane = threadIdx.x & 31;
+  if (threadIdx.x < 16)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;"
+                 ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(&sh.bar[threadIdx.x]))));
+  if (threadIdx.x == 0) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  // this thread's half tile: rows r0 .. r0+3, columns c0, c0+1
+  int i = -1, j = -1;
   if (role >= 0 && role < 16) {
-    const double* __restrict__ G = c.a64 + f.off + k0 + (int64_t)k0 * n;
-    const int unit = 32 * role + lane;
-    int i = -1, j = -1;                       // this thread's tile (none: i = -1)
-    if (unit < 2 * 136) {
-      const int t = unit >> 1;
-      i = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
-      while (i * (i + 1) / 2 > t) --i;
-      while ((i + 1) * (i + 2) / 2 <= t) ++i;
-      j = t - i * (i + 1) / 2;
+    i = 4 * pd_group[role][0] + ((lane >> 1) & 3);
+    j = 4 * pd_group[role][1] + (lane >> 3);
+    if (i < j) i = -1;
+  }
+  const int r0 = 4 * i, c0 = 4 * j + 2 * (lane & 1);
+  double a[4][2];
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const int r = r0 + u, cc = c0 + v;
+      a[u][v] = rank || i < 0 || r < cc ? 0.0
+                : (r < kb && cc < kb)   ? c.a64[f.off + (k0 + r) + (int64_t)(k0 + cc) * n]
+                                        : (r == cc ? 1.0 : 0.0);
     }
-    const int r0 = 4 * i, c0 = 4 * j + 2 * (unit & 1);   // rows r0 .. r0+3, columns c0, c0+1
-    double a[4][2];
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  auto update = [&](const double (*b)[64], const double (*w)[64]) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int m = 0; m < 4; ++m) {
+      double l[4];
+      Vec4<double>::ld(&b[m][r0], l);
+      const double2 x = *reinterpret_cast<const double2*>(&w[m][c0]);
 #pragma unroll
-      for (int v = 0; v < 2; ++v) {
-        const int r = r0 + u, cc = c0 + v;
-        a[u][v] = i < 0 || r < cc ? 0.0 : (r < kb && cc < kb) ? G[r + (int64_t)cc * n] : (r == cc ? 1.0 : 0.0);
+      for (int u = 0; u < 4; ++u) {
+        a[u][0] -= l[u] * x.x;
+        a[u][1] -= l[u] * x.y;
       }
-    // the vectors of step q leave the tiles of column q (A) and row q (X)
-    auto publish = [&](int q) {
-      double (*v)[64] = V[q & 1];
-      if (i >= q && j == q) {
+    }
+  };
+  // barriers: 1 the solvers; 2, 3 vectors of step q (q mod 2) published; 4, 5 results of step q written
+  if (rank == 0 && role < 16) {
+    auto publish = [&](int q) {              // column q
+      if (j == q && i >= q) {
 #pragma unroll
-        for (int e = 0; e < 2; ++e) Vec4<double>::st(&v[c0 + e - 4 * q][r0], {a[0][e], a[1][e], a[2][e], a[3][e]});
-      } else if (i == q && j < q - 1) {       // (column q - 1 starts at zero)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) *reinterpret_cast<double2*>(&v[u][c0]) = make_double2(a[u][0], a[u][1]);
+        for (int e = 0; e < 2; ++e)
+          Vec4<double>::st(&sh.V[q & 1][c0 + e - 4 * q][r0], {a[0][e], a[1][e], a[2][e], a[3][e]});
       }
     };
     publish(0);
     publish(1);
     pd_arrive(2);
 #pragma unroll 1
-    for (int q = 0; q < 14; ++q) {
+    for (int q = 0; q < 16; ++q) {
       pd_sync(4 + (q & 1));
-      if (i > q + 1 && j != q + 1) {
-        const double (*b)[64] = B[q & 1];
-        if (j == q) {
+      if (i >= 0 && j > q + 1) update(sh.B[q & 1], sh.W[q & 1]);
+      if (role < 2) {
+        // (two groups that are done early) column q of U to rank 1, its pivot block, D
+        const int P = 4 * q, cc = 32 * role + lane;
+        if (cc >= P + 4) {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) a[u][0] = a[u][1] = 0.0;
+          for (int m = 0; m < 4; ++m) pd_put(pd_peer(&sh.B[q][m][cc]), sh.B[q & 1][m][cc]);
         }
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          double l[4];
-          Vec4<double>::ld(&b[m][r0], l);
-          const double2 x = *reinterpret_cast<const double2*>(&b[m][c0]);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            a[u][0] -= l[u] * x.x;
-            a[u][1] -= l[u] * x.y;
-          }
-        }
+        if (role == 0 && lane < 16) pd_put(pd_peer(&sh.l[q][0][0] + lane), (&sh.l[q][0][0])[lane]);
+        if (role == 1 && lane < 4) pd_put(pd_peer(&sh.ds[P + lane]), sh.ds[P + lane]);
+        __syncwarp();
+        if (lane == 0)
+          asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(pd_peer(&sh.bar[q])) : "memory");
       }
-      publish(q + 2);
-      pd_arrive(2 + (q & 1));
+      if (q < 14) {
+        publish(q + 2);
+        pd_arrive(2 + (q & 1));
+      }
     }
-  } else if (role >= 16) {
-    double* __restrict__ D = c.dinv64 + f.dinv_off + (int64_t)(k0 / 64) * 4096;
+  } else if (rank == 0) {
     const int cc = 32 * (role - 16) + lane;
     bool bad = false;
+    double w[4];                             // this row's results
 #pragma unroll 1
     for (int q = 0; q < 16; ++q) {
       const int P = 4 * q;
       if (q != 1) pd_sync(2 + (q & 1));
       double t[4];
 #pragma unroll
-      for (int m = 0; m < 4; ++m) t[m] = cc >= P - 4 && cc < P ? 0.0 : V[q & 1][m][cc];
+      for (int m = 0; m < 4; ++m) t[m] = cc >= P ? sh.V[q & 1][m][cc] : 0.0;
       if (q > 0) {
         // the update of step q - 1
-        const double (*b)[64] = B[(q - 1) & 1];
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
-          const double x = b[l][cc];
           double y[4];
-          Vec4<double>::ld(&b[l][P], y);
+          Vec4<double>::ld(&sh.B[(q - 1) & 1][l][P], y);
 #pragma unroll
-          for (int m = 0; m < 4; ++m) t[m] -= y[m] * x;
+          for (int m = 0; m < 4; ++m) t[m] -= y[m] * w[l];
         }
       }
-      const bool piv = cc >= P && cc < P + 4;
-      if (piv) Vec4<double>::st(&pv[cc - P][0], t);            // A(cc, P ..)
+      if (cc >= P && cc < P + 4) Vec4<double>::st(&sh.pv[cc - P][0], t);       // A(cc, P ..)
       asm volatile("bar.sync 1, 64;" ::: "memory");
-      double lb[4][4], rd[4];
+      double p[4][4], l[4][4], rd[4], d[4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) Vec4<double>::ld(&pv[r][0], lb[r]);
+      for (int r = 0; r < 4; ++r) Vec4<double>::ld(&sh.pv[r][0], p[r]);
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
-        double s = lb[m][m];
-#pragma unroll
-        for (int l = 0; l < m; ++l) s -= lb[m][l] * lb[m][l];
-        if (!(s > 0.0)) { bad = true; s = 1.0; }
-        rd[m] = rsqrt(s);
+        d[m] = p[m][m];
+        if (!(d[m] > 0.0)) { bad = true; d[m] = 1.0; }
+        rd[m] = fp64_rcp(d[m]);
 #pragma unroll
         for (int r = m + 1; r < 4; ++r) {
-          double w = lb[r][m];
+          l[r][m] = p[r][m] * rd[m];
 #pragma unroll
-          for (int l = 0; l < m; ++l) w -= lb[r][l] * lb[m][l];
-          lb[r][m] = w * rd[m];
+          for (int e = m + 1; e <= r; ++e) p[r][e] -= l[r][m] * p[e][m];
         }
       }
+      // (no row is left for the lower warp once its 32 are done)
+      if (__any_sync(0xffffffffu, cc >= P + 4)) {
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        double w = piv ? (cc == P + m ? 1.0 : 0.0) : t[m];
+        for (int m = 0; m < 4; ++m) {
+          w[m] = t[m];
 #pragma unroll
-        for (int l = 0; l < m; ++l) w -= lb[m][l] * t[l];
-        t[m] = w * rd[m];
-        B[q & 1][m][cc] = t[m];
+          for (int e = 0; e < m; ++e) w[m] -= l[m][e] * w[e];
+          sh.W[q & 1][m][cc] = w[m];
+          sh.B[q & 1][m][cc] = w[m] * rd[m];
+        }
+      }
+      if (role == 17 && lane < 4) {          // lane r: row r of the pivot block
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          if (lane == r) {
+            sh.ds[P + r] = d[r];
+#pragma unroll
+            for (int e = 0; e < r; ++e) sh.l[q][r][e] = l[r][e];
+          }
       }
       asm volatile("bar.sync 1, 64;" ::: "memory");            // B of this step, before either warp's next
-      if (q < 14) pd_arrive(4 + (q & 1));
-#pragma unroll
-      for (int m = 0; m < 4; ++m)
-        if (cc >= P + 4 || P + m >= kb || cc >= kb) t[m] = 0.0;
-      Vec4<double>::st(D + (int64_t)cc * 64 + P, t);
+      pd_arrive(4 + (q & 1));
     }
     if (cc == 0 && bad) set_status(c, it.front, ST_NOT_SPD);
+  } else if (role >= 0 && role < 16) {
+#pragma unroll 1
+    for (int q = 0; q < 15; ++q) {
+      pd_sync(4 + (q & 1));
+      if (j <= q && q < i) update(sh.B[q], sh.W[q & 1]);
+      if (i == q + 1 && j <= q) {            // row q + 1 of Z
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          *reinterpret_cast<double2*>(&sh.V[(q + 1) & 1][u][c0]) = make_double2(a[u][0], a[u][1]);
+      }
+      pd_arrive(2 + ((q + 1) & 1));
+    }
+  } else if (role >= 16) {
+    const int cc = 32 * (role - 16) + lane;
+    const uint32_t lim = g_wait_limit;
+    bool live = true;
+#pragma unroll 1
+    for (int q = 0; q < 16; ++q) {
+      const int P = 4 * q;
+      if (q > 0) pd_sync(2 + (q & 1));
+      for (uint32_t k = 0; live; ++k) {
+        uint32_t ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
+                     " selp.b32 %0, 1, 0, p;\n}\n"
+                     : "=r"(ok) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&sh.bar[q]))) : "memory");
+        if (ok) break;
+        if (k >= lim) live = false;
+      }
+      double z[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        double w = cc < P ? sh.V[q & 1][m][cc] : (cc == P + m ? 1.0 : 0.0);
+#pragma unroll
+        for (int e = 0; e < m; ++e) w -= sh.l[q][m][e] * z[e];
+        z[m] = w;
+        sh.W[q & 1][m][cc] = w;
+        sh.Z[P + m][cc] = w;
+      }
+      if (q < 15) pd_arrive(4 + (q & 1));
+    }
+    if (!live) set_status(c, it.front, ST_WAIT);
   }
+  __syncthreads();
+  if (rank == 1) {
+    if (threadIdx.x < 64) sh.ds[threadIdx.x] = rsqrt(sh.ds[threadIdx.x]);
+    __syncthreads();
+    double* __restrict__ D = c.dinv64 + f.dinv_off + (int64_t)(k0 / 64) * 4096;
+    for (int e = threadIdx.x; e < 4096; e += PD_THREADS) {
+      const int r = e & 63, cc = e >> 6;     // entry (r, cc)
+      D[e] = cc <= r && r < kb ? sh.Z[r][cc] * sh.ds[r] : 0.0;
+    }
+  }
+  // neither CTA leaves while the other may still write to it
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+static void launch_potrf_inv64(const DevCtx& c, const Item* items, int n_items, cudaStream_t s) {
+  cudaFuncSetAttribute(k_potrf_inv64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PdShared));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * n_items);
+  cfg.blockDim = dim3(PD_THREADS);
+  cfg.dynamicSmemBytes = sizeof(PdShared);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_potrf_inv64, c, items);
+  if (e != cudaSuccess) throw std::runtime_error(std::string("FP64 diagonal block launch failed: ") + cudaGetErrorString(e));
 }
 
 void launch_potrf_diag(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
@@ -748,7 +876,7 @@ void launch_potrf_diag(const DevCtx& c, const Item* items, int n_items, int dtyp
   if (!n_items) return;
   if (nb > 64) throw std::invalid_argument("potrf_diag: block wider than 64");
   if (dtype == F64)
-    k_potrf_inv64<<<n_items, PD_THREADS, 0, s>>>(c, items);
+    launch_potrf_inv64(c, items, n_items, s);
   else
     k_potrf_diag<float><<<n_items, 256, 0, s>>>(c, items, nb);
 }
@@ -1177,7 +1305,6 @@ constexpr int GC_POLL = (GC_MAX_CTAS + 31) / 32;
 constexpr int64_t GC_REC = 2 * 64;              // words of a row's record (two per FP64 value)
 static_assert(gc_words(1, 1) == 4 + 4 * GC_REC, "record size of the launcher's callers");
 
-UHM_DEFINE_WAIT_LIMIT(set_wait_limit_factor, 1u << 22)
 
 template <typename T> struct LuBits;
 template <> struct LuBits<double> {
@@ -1302,19 +1429,7 @@ __device__ __forceinline__ void lu_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ float lu_rcp(float v) { return 1.0f / v; }
-// 1 / v by Chebyshev's iteration: an FP32 start x of the mantissa, then
-// x (1 + r + r^2), r = 1 - v x (the next term, r^3, is below 2^-66); three
-// dependent FP64 operations, 0.5000 ulp over 10^8 values of every exponent
-__device__ __forceinline__ double lu_rcp(double v) {
-  const int hi = __double2hiint(v), f = (hi >> 20) & 0x7FF;
-  if (f < 24 || f > 2022) return 1.0 / v;
-  const float m = __int_as_float((127 << 23) | (hi & 0xFFFFF) << 3 | (int)((unsigned)__double2loint(v) >> 29));
-  const uint32_t xb = __float_as_uint(1.0f / m);               // (1/2, 1]
-  const double x = __hiloint2double((int)((hi & 0x80000000u) | ((xb >> 3) + ((1023 - 127 - (f - 1023)) << 20))),
-                                    (int)(xb << 29));
-  const double r = fma(-v, x, 1.0);
-  return fma(x, fma(r, r, r), x);
-}
+__device__ __forceinline__ double lu_rcp(double v) { return fp64_rcp(v); }
 
 // rows received in one column: of every candidate (CL) or of the pivot, then row k0 + k
 template <typename T, bool CL>
