@@ -1789,52 +1789,57 @@ constexpr int LUROW_LQ = 18;   // row of a lane's 16 L entries in shared memory 
 // A[k0:k0+kb, cols] <- L11^{-1} A[k0:k0+kb, cols]  (unit lower), cols >= k0+kb;
 // item: front, a = k0, b = first column of the chunk, c = column limit (0: n)
 //
-// Substitution in registers: four lanes hold one column (lane q rows q, q+4,
-// ..), a step's solved entry goes to the other three by one shuffle, L comes
+// Substitution in registers: Q lanes hold one column (lane q rows q, q+Q,
+// ..), a step's solved entry goes to the others by one shuffle, L comes
 // from shared memory in the lanes' order, and nothing waits at a block
-// barrier after L is staged.  Two warps take 16 columns; bound by the
+// barrier after L is staged.  Bound by the
 // multiply-adds (2016 per column; FP64 at about 2 per clock and SM, which
-// is why the chunk is narrow: 16 columns spread a panel over every SM) and,
-// FP32, by latency.  Measured on GB300 against the form it replaces (64
+// is why the chunk is narrow: 16 columns spread a panel over every SM) and by the
+// chain of 64 steps.  A warp's FP64 multiply-add takes its scheduler 64 clocks, so
+// FP64 columns take eight lanes (four warps per CTA, one per scheduler, and half
+// the multiply-adds between two steps), FP32 ones four.  Measured on GB300 against a
+// column per thread (64
 // columns per CTA, a block barrier per row): 24^3 p = 3 BF16-split LU, 534
-// launches, 38.7 -> 7.9 ms; 12^3 p = 3 FP64, 115 launches, 8.6 ->
-// 4.0 ms.
-template <typename T>
-__global__ void __launch_bounds__(4 * LUROW_CB) k_lu_row_update(DevCtx c, const Item* __restrict__ items, int nb) {
-  __shared__ __align__(16) T L[64 * 4 * LUROW_LQ];   // L[(4 k + q) LUROW_LQ + u] = L11[q + 4 u][k]
+// launches, 38.7 -> 7.9 ms; FP64, the smallest launches, four lanes 29 us, eight 18;
+// 12^3 p = 3, 200 launches, 6.5 -> 5.0 ms.
+template <typename T, int Q>
+__global__ void __launch_bounds__(Q * LUROW_CB) k_lu_row_update(DevCtx c, const Item* __restrict__ items, int nb) {
+  constexpr int NU = 64 / Q, LQ = NU + 2;      // rows per lane; their L entries' row in shared memory (no bank conflicts)
+  constexpr int NT = Q * LUROW_CB;
+  __shared__ __align__(16) T L[64 * Q * LQ];   // L[(Q k + q) LQ + u] = L11[q + Q u][k]
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, k0 = it.a;
   const int kb = min(nb, f.fs - k0);
   const int cend = it.c > 0 ? min(it.c, n) : n;    // columns < cend (item c; 0: all)
   T* __restrict__ G = arena<T>(c) + f.off;
-  const int q = threadIdx.x & 3, col = it.b + (threadIdx.x >> 2);
+  const int q = threadIdx.x & (Q - 1), col = it.b + threadIdx.x / Q;
   const bool in = col < cend;
   T* __restrict__ X = G + k0 + q + (int64_t)col * n;
-  T x[16];
+  T x[NU];
 #pragma unroll
-  for (int u = 0; u < 16; ++u) x[u] = in && q + 4 * u < kb ? X[4 * u] : T(0);
+  for (int u = 0; u < NU; ++u) x[u] = in && q + Q * u < kb ? X[Q * u] : T(0);
   {
-    const int i = threadIdx.x;                     // row of L11 (64 threads)
+    const int i = threadIdx.x & 63;            // row of L11
 #pragma unroll 16
-    for (int k = 0; k < 64; ++k)
-      L[(4 * k + (i & 3)) * LUROW_LQ + (i >> 2)] = i > k && i < kb ? G[(k0 + i) + (int64_t)(k0 + k) * n] : T(0);
+    for (int k = threadIdx.x >> 6; k < 64; k += NT / 64)
+      L[(Q * k + (i & (Q - 1))) * LQ + i / Q] = i > k && i < kb ? G[(k0 + i) + (int64_t)(k0 + k) * n] : T(0);
   }
   __syncthreads();
 #pragma unroll
-  for (int b = 0; b < 16; ++b) {
+  for (int b = 0; b < NU; ++b) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const T xk = __shfl_sync(0xffffffffu, x[b], r, 4);
-      const T* __restrict__ l = L + (4 * (4 * b + r) + q) * LUROW_LQ;
+    for (int r = 0; r < Q; ++r) {
+      const T xk = __shfl_sync(0xffffffffu, x[b], r, Q);
+      const T* __restrict__ l = L + (Q * (Q * b + r) + q) * LQ;
       if (q > r) x[b] -= l[b] * xk;
 #pragma unroll
-      for (int u = b + 1; u < 16; ++u) x[u] -= l[u] * xk;
+      for (int u = b + 1; u < NU; ++u) x[u] -= l[u] * xk;
     }
   }
 #pragma unroll
-  for (int u = 0; u < 16; ++u)
-    if (in && q + 4 * u < kb) X[4 * u] = x[u];
+  for (int u = 0; u < NU; ++u)
+    if (in && q + Q * u < kb) X[Q * u] = x[u];
 }
 
 void launch_lu_row_update(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
@@ -1842,8 +1847,8 @@ void launch_lu_row_update(const DevCtx& c, const Item* items, int n_items, int d
   (void)pivot;
   if (!n_items) return;
   if (nb != 64) throw std::invalid_argument("lu_row_update: panels are 64 columns wide");
-  if (dtype == F64) k_lu_row_update<double><<<n_items, 4 * LUROW_CB, 0, s>>>(c, items, nb);
-  else k_lu_row_update<float><<<n_items, 4 * LUROW_CB, 0, s>>>(c, items, nb);
+  if (dtype == F64) k_lu_row_update<double, 8><<<n_items, 8 * LUROW_CB, 0, s>>>(c, items, nb);
+  else k_lu_row_update<float, 4><<<n_items, 4 * LUROW_CB, 0, s>>>(c, items, nb);
 }
 
 // Inverses of a large LU front's diagonal blocks, for the flag-driven solves:
