@@ -1784,7 +1784,6 @@ void launch_laswp(const DevCtx& c, const Item* items, int n_items, int dtype, in
 }
 
 constexpr int LUROW_CB = 16;   // columns per row-panel block
-constexpr int LUROW_LQ = 18;   // row of a lane's 16 L entries in shared memory (16-byte rows, no bank conflicts)
 
 // A[k0:k0+kb, cols] <- L11^{-1} A[k0:k0+kb, cols]  (unit lower), cols >= k0+kb;
 // item: front, a = k0, b = first column of the chunk, c = column limit (0: n)
@@ -1854,60 +1853,63 @@ void launch_lu_row_update(const DevCtx& c, const Item* items, int n_items, int d
 // Inverses of a large LU front's diagonal blocks, for the flag-driven solves:
 // L_bb (unit lower) and U_bb, 64 x 64, zero outside their triangles and past
 // the block's kb rows.  Item: front, a = b.  Substitution in registers as in
-// k_lu_row_update, four lanes per column of the identity; U through its
+// k_lu_row_update; U through its
 // transpose, (U^T)^{-1} by rows being U^{-1} by columns.  One launch per level
-// after its fronts are factored: every block of every front at once.
-template <typename T>
-__global__ void __launch_bounds__(256) k_lu_dinv(DevCtx c, const Item* __restrict__ items) {
-  __shared__ __align__(16) T L[64 * 4 * LUROW_LQ];   // L[(4 k + q) LUROW_LQ + u] = M[q + 4 u][k]
+// after its fronts are factored: every block of every front at once, eight CTAs
+// each (L or U, 16 columns of the identity, whose rows above are zero and
+// skipped).  Bound by the multiply-adds of a CTA: measured on GB300, FP64, 6^3
+// p = 3 (25 and 19 blocks) 0.32 ms with one CTA per block, 0.15 so; 12^3 p = 3 0.77, 0.57.
+template <typename T, int Q>
+__global__ void __launch_bounds__(Q * LUROW_CB) k_lu_dinv(DevCtx c, const Item* __restrict__ items) {
+  constexpr int NU = 64 / Q, LQ = NU + 2, NT = Q * LUROW_CB;
+  __shared__ __align__(16) T L[64 * Q * LQ];   // L[(Q k + q) LQ + u] = M[q + Q u][k]
   __shared__ T rd[64];
-  const Item it = items[blockIdx.x];
+  const Item it = items[blockIdx.x >> 3];
+  const int upper = (blockIdx.x >> 2) & 1, first = LUROW_CB * (blockIdx.x & 3);     // first column
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, fs = f.fs, k0 = 64 * it.a;
   const int kb = min(64, fs - k0), nfb = (fs + 63) / 64;
   const T* __restrict__ G = arena<T>(c) + f.off + k0 + (int64_t)k0 * n;
   T* __restrict__ D = (sizeof(T) == 8 ? (T*)c.dinv64 : (T*)c.dinv32) + f.dinv_off + (int64_t)it.a * 4096;
-  const int q = threadIdx.x & 3, col = threadIdx.x >> 2;
-#pragma unroll 1
-  for (int upper = 0; upper < 2; ++upper) {
-    for (int e = threadIdx.x; e < 4096; e += 256) {
-      const int i = e & 63, k = e >> 6;              // entry (i, k) of the block, column k
-      const T v = i < kb && k < kb ? G[i + (int64_t)k * n] : (i == k ? T(1) : T(0));
-      if (!upper) L[(4 * k + (i & 3)) * LUROW_LQ + (i >> 2)] = i > k ? v : T(0);
-      else L[(4 * i + (k & 3)) * LUROW_LQ + (k >> 2)] = k > i ? v : T(0);   // U^T: entry (k, i)
-      if (i == k) rd[i] = upper ? v : T(1);
+  const int q = threadIdx.x & (Q - 1), col = first + threadIdx.x / Q;
+#pragma unroll 8
+  for (int e = threadIdx.x; e < 4096; e += NT) {
+    const int i = e & 63, k = e >> 6;              // entry (i, k) of the block, column k
+    const T v = i < kb && k < kb ? G[i + (int64_t)k * n] : (i == k ? T(1) : T(0));
+    if (!upper) L[(Q * k + (i & (Q - 1))) * LQ + i / Q] = i > k ? v : T(0);
+    else L[(Q * i + (k & (Q - 1))) * LQ + k / Q] = k > i ? v : T(0);   // U^T: entry (k, i)
+    if (i == k) rd[i] = upper ? v : T(1);
+  }
+  __syncthreads();
+  T x[NU];
+#pragma unroll
+  for (int u = 0; u < NU; ++u) x[u] = q + Q * u == col ? T(1) : T(0);
+#pragma unroll
+  for (int b = 0; b < NU; ++b) {
+    if (Q * b < first) continue;                   // rows above the columns' first one are zero
+#pragma unroll
+    for (int r = 0; r < Q; ++r) {
+      if (upper && q == r) x[b] /= rd[Q * b + r];
+      const T xk = __shfl_sync(0xffffffffu, x[b], r, Q);
+      const T* __restrict__ l = L + (Q * (Q * b + r) + q) * LQ;
+      if (q > r) x[b] -= l[b] * xk;
+#pragma unroll
+      for (int u = b + 1; u < NU; ++u) x[u] -= l[u] * xk;
     }
-    __syncthreads();
-    T x[16];
+  }
 #pragma unroll
-    for (int u = 0; u < 16; ++u) x[u] = q + 4 * u == col ? T(1) : T(0);
-#pragma unroll
-    for (int b = 0; b < 16; ++b) {
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        if (upper && q == r) x[b] /= rd[4 * b + r];
-        const T xk = __shfl_sync(0xffffffffu, x[b], r, 4);
-        const T* __restrict__ l = L + (4 * (4 * b + r) + q) * LUROW_LQ;
-        if (q > r) x[b] -= l[b] * xk;
-#pragma unroll
-        for (int u = b + 1; u < 16; ++u) x[u] -= l[u] * xk;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int i = q + 4 * u;                       // entry (i, col) of M^{-1}
-      const T v = i < kb && col < kb && i >= col ? x[u] : T(0);
-      if (!upper) D[col * 64 + i] = v;
-      else D[(int64_t)nfb * 4096 + i * 64 + col] = v;
-    }
-    __syncthreads();
+  for (int u = 0; u < NU; ++u) {
+    const int i = q + Q * u;                       // entry (i, col) of M^{-1}
+    const T v = i < kb && col < kb && i >= col ? x[u] : T(0);
+    if (!upper) D[col * 64 + i] = v;
+    else D[(int64_t)nfb * 4096 + i * 64 + col] = v;
   }
 }
 
 void launch_lu_dinv(const DevCtx& c, const Item* items, int n_items, int dtype, cudaStream_t s) {
   if (!n_items) return;
-  if (dtype == F64) k_lu_dinv<double><<<n_items, 256, 0, s>>>(c, items);
-  else k_lu_dinv<float><<<n_items, 256, 0, s>>>(c, items);
+  if (dtype == F64) k_lu_dinv<double, 8><<<8 * n_items, 8 * LUROW_CB, 0, s>>>(c, items);
+  else k_lu_dinv<float, 4><<<8 * n_items, 4 * LUROW_CB, 0, s>>>(c, items);
 }
 
 // ---------------------------------------------------------------------------
