@@ -291,12 +291,23 @@ __global__ void __launch_bounds__(NT) k_small_factor(DevCtx c, const Item* __res
     for (int i = (chol ? j : 0) + lane; i < n; i += 32) G[i + (int64_t)j * n] = A[i + (int64_t)j * n];
 }
 
+// v / d from r, an approximation of 1 / d (to an ulp or two): the quotient and
+// Markstein's correction by its remainder, rounded as a division but for rare
+// ties.  (Products with the reciprocal root instead: an error of r is common to its
+// whole column of L and, on a uniform mesh, to every element's front; the
+// solutions of 12^3 and 16^3 p = 4 Poisson meshes were 1.3 and 1.5 times further
+// from the exact ones than with a square root and divisions.)
+__device__ __forceinline__ double fp64_div(double v, double d, double r) {
+  const double q = v * r;
+  return fma(fma(-q, d, v), r, q);
+}
+
 // The factor panel of a small FP64 front in shared memory, four columns per
 // step: one thread per row factors the 4 x 4 pivot block and substitutes its
 // row, then 4 x 2 register tiles of the panel's lower triangle take the rank-4
 // update.  Bound by the FP64 multiply-adds (2 per clock and SM: 85 us of them on
 // a 125 x 125 front).  Measured on GB300 against an FP64 square root and division
-// per column with a barrier on either side: that front 275 -> 199 us.
+// per column with a barrier on either side: that front 275 -> 242 us.
 template <int NT>
 __device__ __forceinline__ void small_panel4(const DevCtx& c, int front, double* __restrict__ A, int n, int fs) {
   const int tid = threadIdx.x;
@@ -304,10 +315,10 @@ __device__ __forceinline__ void small_panel4(const DevCtx& c, int front, double*
     const int w = min(4, fs - P), r = P + tid;
     double t[4];
     if (r < n) {
-      double lb[4][4], rd[4];
+      double lb[4][4], rd[4], ld[4];
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
-        rd[m] = 1.0;
+        rd[m] = ld[m] = 1.0;
         if (m >= w) continue;
         double s = A[P + m + (P + m) * n];
 #pragma unroll
@@ -317,12 +328,17 @@ __device__ __forceinline__ void small_panel4(const DevCtx& c, int front, double*
           s = 1.0;
         }
         rd[m] = rsqrt(s);
+        {
+          const double h = s * rd[m];          // sqrt(s), corrected the same way
+          const double e = fma(-h, h, s);
+          ld[m] = fabs(e) < s ? fma(0.5 * rd[m], e, h) : h;
+        }
 #pragma unroll
         for (int i = m + 1; i < 4; ++i) {
           double v = i < w ? A[P + i + (P + m) * n] : 0.0;
 #pragma unroll
           for (int l = 0; l < m; ++l) v -= lb[i][l] * lb[m][l];
-          lb[i][m] = v * rd[m];
+          lb[i][m] = fp64_div(v, ld[m], rd[m]);
         }
       }
 #pragma unroll
@@ -330,7 +346,7 @@ __device__ __forceinline__ void small_panel4(const DevCtx& c, int front, double*
         double v = m < w ? A[r + (P + m) * n] : 0.0;
 #pragma unroll
         for (int l = 0; l < m; ++l) v -= lb[m][l] * t[l];
-        t[m] = v * rd[m];
+        t[m] = r == P + m ? ld[m] : fp64_div(v, ld[m], rd[m]);
       }
       // (a failed pivot's row keeps the pivot 1)
       if (r < P + w) {
