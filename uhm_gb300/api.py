@@ -375,8 +375,7 @@ class Mesh:
 
     OP_NAMES = ["assemble", "small_factor", "potrf_diag", "trsm_panel", "syrk_update",
                 "getrf_panel", "lu_row_update", "gemm_update", "fwd_gather", "fwd_small",
-                "trsv_fwd_step", "gemv_fwd", "bwd_prepare", "bwd_small", "gemv_bwd", "trsv_bwd_step",
-                "bwd_store", "tc_pack", "tc_syrk_bf16", "fwd_flags", "bwd_flags", "getrf_coop",
+                "bwd_prepare", "bwd_small", "bwd_store", "tc_pack", "tc_syrk_bf16", "fwd_flags", "bwd_flags", "getrf_coop",
                 "laswp", "potrf_trsm", "assemble_scatter", "tc_gemm_bf16", "chol_panel", "tc_chol_trail",
                 "tc_chol_schur", "clear_flags", "chol_diag", "chol_pack", "tc_chol_trsm", "event_record",
                 "event_wait", "fwd_chain", "bwd_chain", "xs_pack", "xs_update", "lu_dinv"]

@@ -690,23 +690,20 @@ void Engine::build_plan(int method) {
     f.piv_off = piv_n;
     piv_n += f.fs;
   }
-  // large fronts: inverses of their 64 x 64 diagonal blocks and one
-  // completion flag per block for the flag-driven solves
-  dinv64_n = dinv32_n = flags_n = 0;
+  // large fronts: inverses of their 64 x 64 diagonal blocks for the flag-driven solves
+  dinv64_n = dinv32_n = 0;
   {
     const int small_max_f[2] = {tune.small_max_f64, tune.small_max_f32};
     for (auto& f : fronts) {
       const int dt = f.prec == PREC_FP64 ? F64 : F32;
       f.blocked = f.tc || f.n > small_max_f[dt];
       f.xs = f.blocked && !f.tc;
-      f.flag_off = (int)flags_n;
       f.dinv_off = 0;
       if (!f.blocked) continue;
       const int nfb = (f.fs + NB - 1) / NB;
       int64_t& dn = dt == F64 ? dinv64_n : dinv32_n;
       f.dinv_off = dn;
       dn += (method == UHM_CHOL ? 1 : 2) * (int64_t)nfb * NB * NB;   // LU: of L's blocks, then of U's
-      flags_n += nfb;
     }
   }
   // operand slices of the current panel of every front with sliced updates;
@@ -816,7 +813,6 @@ void Engine::build_plan(int method) {
     d.src0 = f.src0;
     d.nsrc = f.nsrc;
     d.status_slot = f.slot;
-    d.flag_off = f.flag_off;
     d.dinv_off = f.dinv_off;
   }
   // element residual tables (elements with a matrix, in leaf order)
@@ -1846,7 +1842,6 @@ void Engine::alloc_device(int method) {
   ctx.status = (int*)dmalloc(sizeof(int) * fronts.size());
   ctx.dinv64 = dinv64_n ? (double*)dmalloc(sizeof(double) * dinv64_n) : nullptr;
   ctx.dinv32 = dinv32_n ? (float*)dmalloc(sizeof(float) * dinv32_n) : nullptr;
-  ctx.flags = (int*)dmalloc(sizeof(int) * std::max<int64_t>(1, flags_n));
   d_ticket = (int*)dmalloc(sizeof(int));
   ctx.n_rhs = nr;
   ctx.symmetric = method == UHM_CHOL ? 1 : 0;

@@ -41,7 +41,6 @@ struct HostFront {
   int64_t ws2b_row0 = 0;           // ... of the panel rows before their TRSM (tc_panel 256)
   int64_t linv_row0 = 0;           // ... of the current panel's Linv parts (tc_panel 256)
   bool blocked = false;            // large front: blocked kernels, 64-col diagonal blocks
-  int flag_off = 0;
   int64_t dinv_off = 0;
   int64_t off = 0, voff = 0, inv_off = 0, colptr_off = 0, sgi_off = 0, piv_off = 0;
   int src0 = 0, nsrc = 0;
@@ -84,8 +83,8 @@ struct OpProfile {
 
 enum OpKind : int {
   OP_ASSEMBLE, OP_SMALL_FACTOR, OP_POTRF, OP_TRSM, OP_SYRK, OP_GETRF, OP_LUROW, OP_GEMM,
-  OP_FWD_GATHER, OP_FWD_SMALL, OP_TRSV_F, OP_GEMV_F, OP_BWD_PREP, OP_BWD_SMALL, OP_GEMV_B,
-  OP_TRSV_B, OP_BWD_STORE, OP_TC_PACK, OP_TC_SYRK, OP_FWD_FLAGS, OP_BWD_FLAGS, OP_GETRF_COOP,
+  OP_FWD_GATHER, OP_FWD_SMALL, OP_BWD_PREP, OP_BWD_SMALL, OP_BWD_STORE,
+  OP_TC_PACK, OP_TC_SYRK, OP_FWD_FLAGS, OP_BWD_FLAGS, OP_GETRF_COOP,
   OP_LASWP, OP_POTRF_TRSM, OP_ASSEMBLE_SCATTER, OP_TC_GEMM, OP_CHOL_PANEL, OP_TC_CHOL_TRAIL,
   OP_TC_CHOL_SCHUR, OP_CLEAR_FLAGS, OP_CHOL_DIAG, OP_CHOL_PACK, OP_TC_CHOL_TRSM, OP_EV_RECORD, OP_EV_WAIT,
   OP_FWD_CHAIN, OP_BWD_CHAIN, OP_XS_PACK, OP_XS_UPDATE, OP_LU_DINV, OP_KIND_END
@@ -288,7 +287,7 @@ class Engine {
   size_t d_items_part_cap = 0;
   void build_partial(int method, const std::vector<char>& act);
   int64_t arena64_n = 0, arena32_n = 0, vec_n = 0, piv_n = 0;
-  int64_t dinv64_n = 0, dinv32_n = 0, flags_n = 0;
+  int64_t dinv64_n = 0, dinv32_n = 0;
   int* d_ticket = nullptr;
 
   // device memory

@@ -899,102 +899,71 @@ void launch_potrf_diag(const DevCtx& c, const Item* items, int n_items, int dtyp
 
 constexpr int TRSM_RB = 64;   // rows per panel-TRSM block
 
-// X (rows r0..r0+RB of columns k0..k0+kb) <- X * L11^{-T}
-template <typename T, int NT>
-__global__ void __launch_bounds__(NT) k_trsm_panel(DevCtx c, const Item* __restrict__ items,
-                                                   int nb, XsCtx x, int slices) {
+// X (rows r0..r0+RB of columns k0..k0+kb) <- X * L11^{-T}, as a product with
+// the inverse computed by the diagonal-block kernel (stored column-major 64 x
+// 64): no sequential sweep.  Both tiles are loaded in one batch of registers.
+__global__ void __launch_bounds__(256) k_trsm_panel(DevCtx c, const Item* __restrict__ items, XsCtx x, int slices) {
   __shared__ int s_f[4][64];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, k0 = it.a, r0 = it.b;
-  const int kb = min(nb, f.fs - k0);
+  const int kb = min(64, f.fs - k0);
   const int rb = min(TRSM_RB, n - r0);
-  T* L = reinterpret_cast<T*>(smem_raw);        // kb x kb (or 64 x 68 padded inverse)
-  T* X = L + 64 * 68;                           // TRSM_RB x kb, ld TRSM_RB
-  T* __restrict__ G = arena<T>(c) + f.off;
-  const T* Dinv = (sizeof(T) == 8 ? (const T*)c.dinv64 : (const T*)c.dinv32);
-  if (nb == 64 && Dinv) {
-    // X <- X * L11^{-T} as a product with the inverse computed by the
-    // diagonal-block kernel (stored column-major 64 x 64): no sequential
-    // sweep.  Both tiles are loaded in one batch of registers.
-    static_assert(NT == 256 && TRSM_RB == 64, "64 x 64 tiles over 256 threads");
-    Dinv += f.dinv_off + (int64_t)(k0 / 64) * 4096;
-    T xv[16], dv[16];
+  float* L = reinterpret_cast<float*>(smem_raw);        // the inverse, rows padded to 68
+  float* X = L + 64 * 68;                               // TRSM_RB x 64, ld TRSM_RB
+  float* __restrict__ G = c.a32 + f.off;
+  const float* __restrict__ Dinv = c.dinv32 + f.dinv_off + (int64_t)(k0 / 64) * 4096;
+  float xv[16], dv[16];
 #pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int idx = threadIdx.x + NT * u, i = idx % TRSM_RB, j = idx / TRSM_RB;
-      xv[u] = (i < rb && j < kb) ? G[(r0 + i) + (int64_t)(k0 + j) * n] : (T)0;
-      dv[u] = Dinv[idx];
-    }
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int idx = threadIdx.x + NT * u;
-      // Dinv is column-major: Dinv[t * 64 + j] = Linv[j][t]; keep it as
-      // rows t of length 64 padded to 68 (16-byte rows), L[t * 68 + j] = Linv[j][t]
-      const int t = idx / 64, j = idx % 64;
-      X[idx] = xv[u];
-      L[t * 68 + j] = (t < kb && j < kb) ? dv[u] : T(0);
-    }
-    __syncthreads();
-    const int i = threadIdx.x % TRSM_RB, jg = threadIdx.x / TRSM_RB;   // 4 column groups of 16
-    T acc[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) acc[u] = T(0);
-    // Linv is lower triangular: columns jg * 16 .. need t <= jg * 16 + 15
-    const int te = min(kb, 16 * jg + 16);
-    for (int t = 0; t < te; ++t) {
-      const T x = X[i + t * TRSM_RB];
-#pragma unroll
-      for (int u4 = 0; u4 < 16; u4 += 4) {
-        T l4[4];
-        Vec4<T>::ld(&L[t * 68 + jg * 16 + u4], l4);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[u4 + e] += x * l4[e];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int j = jg * 16 + u;
-      if (i < rb && j < kb) G[(r0 + i) + (int64_t)(k0 + j) * n] = acc[u];
-    }
-    if (slices && k0 + kb < min(k0 / XS_NBO * XS_NBO + XS_NBO, f.fs))
-      xs_store_step<T>(x, it.front, n, r0 + i, i < rb, acc, s_f);
-    return;
+  for (int u = 0; u < 16; ++u) {
+    const int idx = threadIdx.x + 256 * u, i = idx % TRSM_RB, j = idx / TRSM_RB;
+    xv[u] = (i < rb && j < kb) ? G[(r0 + i) + (int64_t)(k0 + j) * n] : 0.f;
+    dv[u] = Dinv[idx];
   }
-  for (int idx = threadIdx.x; idx < kb * kb; idx += NT) {
-    const int i = idx % kb, j = idx / kb;
-    L[idx] = i >= j ? G[(k0 + i) + (int64_t)(k0 + j) * n] : (T)0;
-  }
-  for (int idx = threadIdx.x; idx < TRSM_RB * kb; idx += NT) {
-    const int i = idx % TRSM_RB, j = idx / TRSM_RB;
-    X[idx] = i < rb ? G[(r0 + i) + (int64_t)(k0 + j) * n] : (T)0;
+#pragma unroll
+  for (int u = 0; u < 16; ++u) {
+    const int idx = threadIdx.x + 256 * u;
+    // Dinv is column-major: Dinv[t * 64 + j] = Linv[j][t]; keep it as
+    // rows t of length 64 padded to 68 (16-byte rows), L[t * 68 + j] = Linv[j][t]
+    const int t = idx / 64, j = idx % 64;
+    X[idx] = xv[u];
+    L[t * 68 + j] = (t < kb && j < kb) ? dv[u] : 0.f;
   }
   __syncthreads();
-  for (int j = 0; j < kb; ++j) {
-    const T ljj = L[j + j * kb];
-    for (int i = threadIdx.x; i < TRSM_RB; i += NT) X[i + j * TRSM_RB] /= ljj;
-    __syncthreads();
-    const int w = kb - j - 1;
-    for (int idx = threadIdx.x; idx < TRSM_RB * w; idx += NT) {
-      const int i = idx % TRSM_RB, t = j + 1 + idx / TRSM_RB;
-      X[i + t * TRSM_RB] -= X[i + j * TRSM_RB] * L[t + j * kb];
+  const int i = threadIdx.x % TRSM_RB, jg = threadIdx.x / TRSM_RB;   // 4 column groups of 16
+  float acc[16];
+#pragma unroll
+  for (int u = 0; u < 16; ++u) acc[u] = 0.f;
+  // Linv is lower triangular: columns jg * 16 .. need t <= jg * 16 + 15
+  const int te = min(kb, 16 * jg + 16);
+  for (int t = 0; t < te; ++t) {
+    const float xt = X[i + t * TRSM_RB];
+#pragma unroll
+    for (int u4 = 0; u4 < 16; u4 += 4) {
+      float l4[4];
+      Vec4<float>::ld(&L[t * 68 + jg * 16 + u4], l4);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[u4 + e] += xt * l4[e];
     }
-    __syncthreads();
   }
-  for (int idx = threadIdx.x; idx < TRSM_RB * kb; idx += NT) {
-    const int i = idx % TRSM_RB, j = idx / TRSM_RB;
-    if (i < rb) G[(r0 + i) + (int64_t)(k0 + j) * n] = X[idx];
+#pragma unroll
+  for (int u = 0; u < 16; ++u) {
+    const int j = jg * 16 + u;
+    if (i < rb && j < kb) G[(r0 + i) + (int64_t)(k0 + j) * n] = acc[u];
   }
+  if (slices && k0 + kb < min(k0 / XS_NBO * XS_NBO + XS_NBO, f.fs))
+    xs_store_step<float>(x, it.front, n, r0 + i, i < rb, acc, s_f);
 }
 
 void launch_trsm_panel(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, const XsCtx& x, int slices,
                        cudaStream_t s) {
   if (!n_items) return;
   if (dtype == F64) throw std::invalid_argument("trsm_panel: FP64 fronts take xs_trsm");
-  size_t sm = (size_t)(64 * 68 + TRSM_RB * nb) * sizeof(float);
-  cudaFuncSetAttribute(k_trsm_panel<float, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_trsm_panel<float, 256><<<n_items, 256, sm, s>>>(c, items, nb, x, slices);
+  if (nb != 64) throw std::invalid_argument("trsm_panel: panels are 64 columns wide");
+  const size_t sm = (size_t)(64 * 68 + TRSM_RB * 64) * sizeof(float);
+  cudaFuncSetAttribute(k_trsm_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_trsm_panel<<<n_items, 256, sm, s>>>(c, items, x, slices);
 }
 
 // Diagonal block and panel TRSM of one 64-column step in one launch.  Every

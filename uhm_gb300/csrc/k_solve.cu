@@ -675,10 +675,8 @@ namespace uhm_gpu {
 // starting at fs.  A CTA takes a ticket (atomic counter) and processes the
 // item of that rank; items are ordered so that each CTA only waits for blocks
 // owned by CTAs with smaller tickets, which are already running -- progress
-// is guaranteed whatever the residency.  The 64-row kernels publish a
-// finished block's solution as self-validating hand-off words (below); the
-// 256-row kernels publish it, then a release-store of the block's flag, and
-// readers acquire the flag before reading.  Every wait is bounded (error
+// is guaranteed whatever the residency.  A finished block's solution is
+// published as self-validating hand-off words (below).  Every wait is bounded (error
 // flag, no hang).
 // Forward:  x_b = L_bb^{-1} (z_b - sum_{j<b} L_bj x_j)
 // Backward: x_b = L_bb^{-T} (y_b - sum_{r > block b} L_rb^T x_r)

@@ -29,7 +29,6 @@ struct FrontDev {
   int g0;             // first global dof eliminated here
   int src0, nsrc;     // assembly sources [src0, src0 + nsrc)
   int status_slot;
-  int flag_off;       // first per-block flag of the flag-driven solves
   int64_t dinv_off;   // inverses of the 64 x 64 diagonal blocks (element offset)
 };
 
@@ -72,7 +71,6 @@ struct DevCtx {
   int* status;        // per-front status
   double* dinv64;     // inverted diagonal blocks of the factor (FP64 fronts)
   float* dinv32;      // ... (FP32 fronts)
-  int* flags;         // per-block completion flags of the flag-driven solves
   int n_rhs;
   int symmetric;      // Cholesky: lower triangles only
 };
