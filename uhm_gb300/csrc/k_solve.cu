@@ -1250,12 +1250,18 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_bwd_flags(DevCt
     }
     if (k + 1 < nblk) load_x(k + 1);
     __syncthreads();
+    // (a tile's sum by itself: n / 64 + 16 roundings in a row instead of n / 4)
+    CT p[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) p[q] = CT(0);
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
       const CT t = ts[buf][g * 16 + u][i];
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) acc[q] += t * xsh[buf][q][g * 16 + u];
+      for (int q = 0; q < NQ; ++q) p[q] += t * xsh[buf][q][g * 16 + u];
     }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) acc[q] += p[q];
   }
 #pragma unroll
   for (int q = 0; q < NQ; ++q) red[g][i][q] = acc[q];
