@@ -96,7 +96,7 @@ void Engine::free_device() {
   d_ws2 = nullptr;
   d_ws2_row0 = nullptr;
   d_ws2b_row0 = d_linv_row0 = nullptr;
-  d_xs = nullptr;
+  d_xs = d_xs_stat = nullptr;
   xs_ctx = xs_in = XsCtx{};
   d_pflags = nullptr;
   d_hand = nullptr;
@@ -708,7 +708,7 @@ void Engine::build_plan(int method) {
   }
   // operand slices of the current panel of every front with sliced updates;
   // the levels run one after the other and share the workspace
-  xs_rows = xs_exps = 0;
+  xs_rows = xs_exps = xs_near_n = 0;
   for (auto& lv : levels) {
     int64_t rows = 0, exps = 0;
     for (int s : lv) {
@@ -731,6 +731,8 @@ void Engine::build_plan(int method) {
       if (method != UHM_CHOL) rows += ri;
       f.xs_exp0i = exps;
       exps += (method == UHM_CHOL ? 1 : 2) * (int64_t)f.n;
+      f.xs_near0 = xs_near_n;
+      if (method != UHM_CHOL) xs_near_n += (f.fs + XS_NBO - 1) / XS_NBO * (XS_NBO / 32);
     }
     xs_rows = std::max(xs_rows, rows);
     xs_exps = std::max(xs_exps, exps);
@@ -959,10 +961,11 @@ void Engine::build_programs(int method) {
   };
   // one LU step's 64-column panel: tall panels (many rows below the
   // diagonal) on many CTAs at once (panel-only row swaps, then k_laswp for
-  // the other columns), the rest one CTA per front.  nbo > 0 (tensor-core
-  // fronts): rows are swapped only in columns below the outer panel's
-  // trailing block, whose swaps come after the outer panel
-  auto push_lu_panel = [&](int dt, const std::vector<Item>& p_items, double fp, int nbo, int sms) {
+  // the other columns), the rest one CTA per front.  nbo > 0: rows are swapped
+  // only in columns below the outer panel's trailing block, whose swaps come after
+  // the outer panel; xs (sliced updates): only in the outer panel's own columns, since an
+  // update on the side stream may read those left of it (xs_plain)
+  auto push_lu_panel = [&](int dt, const std::vector<Item>& p_items, double fp, int nbo, int sms, bool xs) {
     const int piv = method == UHM_LU_PIV ? 1 : 0;
     const int rcap = dt == F64 ? GC_RMAX_F64 : GC_RMAX_F32, rgoal = dt == F64 ? LU_GOAL_F64 : LU_GOAL_F32;
     auto col_end = [&](const Item& it) {
@@ -980,8 +983,9 @@ void Engine::build_programs(int method) {
     for (const Item& it : p_items) {
       const int rows = fronts[it.front].n - it.a;
       bool own_swaps = false;
+      const int cb = xs ? it.a / nbo * nbo : 0;                  // first column swapped
       if (rows > rcap && rows < tune.gc_min_rows && tune.gc_min_rows > 512) {
-        glob.push_back(Item{it.front, it.a, col_end(it), 0});
+        glob.push_back(Item{it.front, it.a, col_end(it), cb});
         own_swaps = true;
       } else {
         int lc = 0;
@@ -997,15 +1001,16 @@ void Engine::build_programs(int method) {
       }
       if (!piv) continue;
       const int ce = col_end(it), lim = ce > 0 ? ce : fronts[it.front].n;
-      if (own_swaps) sw.push_back(Item{it.front, it.a, -1, 0});      // the permutation only
-      else for (int c0 = 0; c0 < lim; c0 += 256) sw.push_back(Item{it.front, it.a, c0, ce});
+      sw.push_back(Item{it.front, it.a, -1, 0});      // the permutation
+      for (int c0 = cb; c0 < lim && !own_swaps; c0 += 256) sw.push_back(Item{it.front, it.a, c0, ce});
     }
     double fl = fp;                  // the panel's operations, on its first launch
-    push(fac_ops, OP_GETRF, dt, NB, piv, glob, glob.empty() ? 0.0 : fl);
+    const int par = piv | (xs ? 2 : 0);
+    push(fac_ops, OP_GETRF, dt, NB, par, glob, glob.empty() ? 0.0 : fl);
     if (!glob.empty()) fl = 0;
     for (int lc = 0; lc < 5; ++lc) {
       if (cl[lc].empty()) continue;
-      Op op{OP_GETRF_COOP, dt, NB, piv, add_items(cl[lc]), (int)cl[lc].size()};
+      Op op{OP_GETRF_COOP, dt, NB, par, add_items(cl[lc]), (int)cl[lc].size()};
       op.q0 = -(1 << lc);            // CTAs per item (a cluster)
       op.aux = rmax_cl[lc];
       op.flops = fl;
@@ -1037,7 +1042,7 @@ void Engine::build_programs(int method) {
         rmax = std::max(rmax, (rows + P - 1) / P);
         b += P;
       }
-      Op op{OP_GETRF_COOP, dt, NB, piv, add_items(g), (int)g.size()};
+      Op op{OP_GETRF_COOP, dt, NB, par, add_items(g), (int)g.size()};
       op.q0 = b;
       op.aux = rmax;
       op.flops = fl;
@@ -1066,7 +1071,7 @@ void Engine::build_programs(int method) {
   auto push_xs = [&](int dt, int nb, int region, const std::vector<Item>& pk, std::vector<Item>& tiles,
                      double fl, double by, int cap = 0, int strm = 0) {
     if (tiles.empty()) return;
-    push(fac_ops, OP_XS_PACK, dt, nb, 0, pk);
+    push(fac_ops, OP_XS_PACK, dt, nb, region, pk);
     // fewer tiles than SMs: tiles of half the width (a launch is as long as its
     // slowest CTA; one round of half tiles of K = 64 takes 19 us)
     const bool narrow = (int)tiles.size() < (cap > 0 ? cap : n_sm);
@@ -1219,19 +1224,20 @@ void Engine::build_programs(int method) {
           } else if (chol) {
             push_potrf_trsm(dt, p_items, t_items, fp, ft, 1);
           } else {
-            push_lu_panel(dt, p_items, fp, XS_NBO, n_sm - side);
-            push(fac_ops, OP_LUROW, dt, NB, 0, t_items, ft);
+            push_lu_panel(dt, p_items, fp, XS_NBO, n_sm - side, true);
+            push(fac_ops, OP_LUROW, dt, NB, 1, t_items, ft);
           }
           push_xs(dt, NB, 1, pk, ut, fu, bu, side ? n_sm - side : 0);
         }
         if (side) ev_op(OP_EV_WAIT, EV_REST, 0);
         side = 0;
         if (method == UHM_LU_PIV) {
-          // the outer panel's row swaps on the columns right of it
+          // the outer panel's row swaps on the columns left and right of it
           std::vector<Item> sw;
           for (int s : large) {
             const HostFront& f = fronts[s];
             if (f.fs <= K0) continue;
+            for (int c0 = 0; c0 < K0; c0 += 256) sw.push_back(Item{s, K0, c0, K0});
             for (int c0 = std::min(K0 + XS_NBO, f.fs); c0 < f.n; c0 += 256) sw.push_back(Item{s, K0, c0, 0});
           }
           push(fac_ops, OP_LASWP, dt, XS_NBO, 0, sw);
@@ -1252,7 +1258,7 @@ void Engine::build_programs(int method) {
             xs_pack_items(pk, NB, s, k0, B, f.n, 1);
             fu += xs_tiles(ut, f, k0, kb, base, B, B, f.n, false, bu);
           }
-          push(fac_ops, OP_LUROW, dt, NB, 0, t_items, ft);
+          push(fac_ops, OP_LUROW, dt, NB, 2, t_items, ft);
           push_xs(dt, NB, 2, pk, ut, fu, bu);
         }
         // the trailing block: the next panel's columns, the rest
@@ -1329,7 +1335,7 @@ void Engine::build_programs(int method) {
               for (int tj = 0; base + tj * TC < B; ++tj) u_items.push_back(Item{s, k0, ti, tj});
             fu += get_flop_gemm(0, f.n - base, std::max(0, B - base), kb);
           }
-          push_lu_panel(dt, p_items, fp, NBO, n_sm - side);
+          push_lu_panel(dt, p_items, fp, NBO, n_sm - side, false);
           push(fac_ops, OP_LUROW, dt, NB, 0, t_items, ft);
           {
             Op op{OP_GEMM, dt, NB, 0, add_items(u_items), (int)u_items.size()};
@@ -1644,6 +1650,10 @@ void Engine::build_programs(int method) {
     op.q0 = (int)pf;
     fac_ops.insert(fac_ops.begin(), op);
   }
+  if (xs_near_n > 0) {
+    // what the sliced updates' balance and check gather starts at zero as well
+    fac_ops.insert(fac_ops.begin(), Op{OP_XS_CLEAR, 0, 0, 0, 0, 0});
+  }
   if (!fac_mask) {
     pflags_n = pf;
     hand_n = hand_slots;
@@ -1878,9 +1888,10 @@ void Engine::alloc_device(int method) {
     d_xs = dmalloc(bytes);
     CK(cudaMemsetAsync(d_xs, 0, bytes, stream));     // rows never packed are read by tiles that run over
     if (!xs_encode(&xs_map, d_xs, xs_rows + XS_SPARE_ROWS)) fail("tensor map encoding failed", 4);
-    std::vector<int64_t> v(6 * fronts.size(), 0);
+    std::vector<int64_t> v(7 * fronts.size(), 0);
     for (auto& f : fronts)
       if (f.xs) {
+        v[6 * fronts.size() + f.slot] = f.xs_near0;
         v[f.slot] = f.xs_row0;
         v[fronts.size() + f.slot] = f.xs_row0b;
         v[2 * fronts.size() + f.slot] = f.xs_exp0;
@@ -1896,6 +1907,17 @@ void Engine::alloc_device(int method) {
     xs_ctx.row0b = d + fronts.size();
     xs_ctx.exp0 = d + 2 * fronts.size();
     xs_ctx.exps = (int*)dmalloc(sizeof(int) * (size_t)xs_exps);
+    if (xs_near_n > 0) {
+      const size_t km = sizeof(int) * 3 * (size_t)((piv_n + 7) / 8 * 8);
+      xs_stat_bytes = km + sizeof(uint32_t) * 4 * XS_USES * (size_t)xs_near_n;
+      d_xs_stat = dmalloc(xs_stat_bytes);
+      xs_ctx.kmax = (int*)d_xs_stat;
+      xs_ctx.kmax_n = (piv_n + 7) / 8 * 8;
+      xs_ctx.near = (uint32_t*)((char*)d_xs_stat + km);
+      xs_ctx.near_n = xs_near_n;
+      xs_ctx.near0 = d + 6 * fronts.size();
+      xs_ctx.masks = (uint32_t*)dmalloc(XS_NBO / 8 * (size_t)xs_exps);
+    }
     xs_in = xs_ctx;
     xs_in.row0 = d + 3 * fronts.size();
     xs_in.row0b = d + 4 * fronts.size();
@@ -2139,19 +2161,25 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
         launch_tc_syrk(ctx, ws_map, d_ws_off, d_ws_stride, it, op.n_items, op.nb, op.param, 0, 1, 0, d_err, st);
         break;
       case OP_XS_PACK:
-        launch_xs_pack(ctx, op.nb == NB ? xs_in : xs_ctx, it, op.n_items, op.dtype, op.nb, st);
+        launch_xs_pack(ctx, op.nb == NB ? xs_in : xs_ctx, it, op.n_items, op.dtype, op.nb, op.param, st);
         break;
       case OP_XS_UPDATE:
         launch_xs_update(ctx, op.nb == NB ? xs_in : xs_ctx, xs_map, it, op.n_items, op.dtype, op.nb, op.q0, op.param,
                          op.aux, profiling ? 0 : op.cap, d_err, st);
         break;
-      case OP_GETRF: launch_getrf_panel(ctx, it, op.n_items, op.dtype, op.nb, op.param, st); break;
+      case OP_XS_CLEAR: CK(cudaMemsetAsync(d_xs_stat, 0, xs_stat_bytes, st)); break;
+      case OP_GETRF:
+        launch_getrf_panel(ctx, it, op.n_items, op.dtype, op.nb, op.param & 1, op.param & 2 ? xs_ctx.kmax : nullptr, st);
+        break;
       case OP_GETRF_COOP:
-        launch_getrf_smem(ctx, it, op.n_items, std::max(op.q0, 0), std::max(-op.q0, 0), op.dtype, op.nb, op.param,
-                          op.aux, d_gc_xbuf, d_err, st);
+        launch_getrf_smem(ctx, it, op.n_items, std::max(op.q0, 0), std::max(-op.q0, 0), op.dtype, op.nb, op.param & 1,
+                          op.aux, d_gc_xbuf, op.param & 2 ? xs_ctx.kmax : nullptr, d_err, st);
         break;
       case OP_LASWP: launch_laswp(ctx, it, op.n_items, op.dtype, op.nb, st); break;
-      case OP_LUROW: launch_lu_row_update(ctx, it, op.n_items, op.dtype, op.nb, 0, st); break;
+      case OP_LUROW:
+        launch_lu_row_update(ctx, it, op.n_items, op.dtype, op.nb, 
+                             op.param ? xs_ctx.kmax + op.param * xs_ctx.kmax_n : nullptr, st);
+        break;
       case OP_GEMM: launch_gemm_update(ctx, it, op.n_items, op.dtype, op.nb, op.q0, op.aux, st); break;
       case OP_TC_GEMM:
         // A parts 0-1 (L21), B parts 2-3 (U12^T)

@@ -36,6 +36,7 @@ struct HostFront {
   bool xs = false;                 // large FP64 / FP32 front: sliced tensor-core updates (k_xs.cu)
   int64_t xs_row0 = 0, xs_row0b = 0, xs_exp0 = 0;      // its slices and row exponents in the level's workspace
   int64_t xs_row0i = 0, xs_row0bi = 0, xs_exp0i = 0;   // the same of a 64-column step
+  int64_t xs_near0 = 0;            // LU: its words of XsCtx::near
   int64_t ws_off = 0, ws_stride = 0;
   int64_t ws2_row0 = 0;            // first 128-byte row of its parts in the chunk-major workspace
   int64_t ws2b_row0 = 0;           // ... of the panel rows before their TRSM (tc_panel 256)
@@ -87,7 +88,7 @@ enum OpKind : int {
   OP_TC_PACK, OP_TC_SYRK, OP_FWD_FLAGS, OP_BWD_FLAGS, OP_GETRF_COOP,
   OP_LASWP, OP_POTRF_TRSM, OP_ASSEMBLE_SCATTER, OP_TC_GEMM, OP_CHOL_PANEL, OP_TC_CHOL_TRAIL,
   OP_TC_CHOL_SCHUR, OP_CLEAR_FLAGS, OP_CHOL_DIAG, OP_CHOL_PACK, OP_TC_CHOL_TRSM, OP_EV_RECORD, OP_EV_WAIT,
-  OP_FWD_CHAIN, OP_BWD_CHAIN, OP_XS_PACK, OP_XS_UPDATE, OP_LU_DINV, OP_KIND_END
+  OP_FWD_CHAIN, OP_BWD_CHAIN, OP_XS_PACK, OP_XS_UPDATE, OP_LU_DINV, OP_XS_CLEAR, OP_KIND_END
 };
 static_assert(OP_KIND_END <= N_OP_KINDS, "profile arrays hold N_OP_KINDS op kinds");
 
@@ -248,7 +249,7 @@ class Engine {
   void sync_anorm();                 // stream waits for it (it writes d_y, d_r and d_red[1536..])
   std::vector<cudaEvent_t> evpool;   // events ordering the two streams (by id)
   static bool is_kernel_op(int kind) {
-    return kind != OP_CLEAR_FLAGS && kind != OP_EV_RECORD && kind != OP_EV_WAIT;
+    return kind != OP_CLEAR_FLAGS && kind != OP_XS_CLEAR && kind != OP_EV_RECORD && kind != OP_EV_WAIT;
   }
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_mid = nullptr;
   int* h_words = nullptr;            // pinned: the fronts' status words and the wait error word, read back together
@@ -307,6 +308,9 @@ class Engine {
   CUtensorMap ws2_map;
   void* d_xs = nullptr;              // operand slices of the current level's sliced updates
   int64_t xs_rows = 0, xs_exps = 0;  // its rows of 64 BF16 and row exponents (the largest level)
+  int64_t xs_near_n = 0;             // LU: words of XsCtx::near per use and side
+  void* d_xs_stat = nullptr;         // LU: XsCtx::kmax, then XsCtx::near (cleared per factorisation)
+  size_t xs_stat_bytes = 0;
   uhm_gpu::XsCtx xs_ctx{}, xs_in{};  // of the outer panels' updates, of those inside a panel
   uhm_gpu::XsMaps xs_map;
   int* d_pflags = nullptr;           // tickets and flags of the panel launches (cleared per factorisation)

@@ -1188,14 +1188,14 @@ void launch_gemm_update(const DevCtx& c, const Item* items, int n_items, int dty
 // ---------------------------------------------------------------------------
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_getrf_panel(DevCtx c, const Item* __restrict__ items,
-                                                    int nb, int pivot) {
+                                                    int nb, int pivot, int* __restrict__ lmax) {
   __shared__ T s_v[NT / 32];
   __shared__ int s_i[NT / 32];
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, fs = f.fs, k0 = it.a;
   const int kb = min(nb, fs - k0);
-  const int jend = it.b > 0 ? min(it.b, n) : n;   // rows are swapped in columns < jend
+  const int jend = it.b > 0 ? min(it.b, n) : n;   // rows are swapped in columns it.c .. jend - 1
   T* __restrict__ G = arena<T>(c) + f.off;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int NW = NT / 32;
@@ -1210,7 +1210,7 @@ __global__ void __launch_bounds__(NT) k_getrf_panel(DevCtx c, const Item* __rest
       const int p = block_argmax<T, NT>(best, bi, s_v, s_i);
       if (threadIdx.x == 0) c.piv[f.piv_off + k] = p;
       if (p != k)
-        for (int j = threadIdx.x; j < jend; j += NT) {
+        for (int j = it.c + threadIdx.x; j < jend; j += NT) {
           T t = G[k + (int64_t)j * n];
           G[k + (int64_t)j * n] = G[p + (int64_t)j * n];
           G[p + (int64_t)j * n] = t;
@@ -1231,13 +1231,19 @@ __global__ void __launch_bounds__(NT) k_getrf_panel(DevCtx c, const Item* __rest
     }
     __syncthreads();
   }
+  for (int k = k0 + warp; lmax && k < k0 + kb; k += NW) {
+    int fm = 0;
+    for (int i = k0 + kb + lane; i < n; i += 32) fm = max(fm, XsType<T>::expo(G[i + (int64_t)k * n]));
+    fm = __reduce_max_sync(0xffffffffu, fm);
+    if (lane == 0) lmax[f.piv_off + k] = fm;
+  }
 }
 
 void launch_getrf_panel(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
-                        int pivot, cudaStream_t s) {
+                        int pivot, int* lmax, cudaStream_t s) {
   if (!n_items) return;
-  if (dtype == F64) k_getrf_panel<double, 512><<<n_items, 512, 0, s>>>(c, items, nb, pivot);
-  else k_getrf_panel<float, 512><<<n_items, 512, 0, s>>>(c, items, nb, pivot);
+  if (dtype == F64) k_getrf_panel<double, 512><<<n_items, 512, 0, s>>>(c, items, nb, pivot, lmax);
+  else k_getrf_panel<float, 512><<<n_items, 512, 0, s>>>(c, items, nb, pivot, lmax);
 }
 
 // ---------------------------------------------------------------------------
@@ -1258,7 +1264,9 @@ void launch_getrf_panel(const DevCtx& c, const Item* items, int n_items, int dty
 //      k + 1 first, whose candidates are found on the way.
 // The result is the reference's partial pivoting (FLA_LU_piv inside the
 // eliminated block) exactly; only the panel's own columns are swapped here,
-// the other columns of the front by k_laswp afterwards.
+// the other columns of the front by k_laswp afterwards.  lmax (null: not wanted):
+// the largest exponent field of each column below the panel's diagonal block, what
+// the slices of the updates are balanced with (k_xs.cu).
 //
 // Two ways to hand candidates and rows over:
 // CL: the item's CTAs are a cluster (1 .. 16 of them) and write into each
@@ -1424,10 +1432,26 @@ struct LuRecv {
   uint64_t cand[CL ? GC_CLUSTER : 1][2];        // key, row
 };
 
+// the largest exponent field of each of the columns of m rows of a chunk, into out
+// (a function of its own: inlined, it cost the kernel's column loop 5 us of 200).  One
+// request per CTA and 32 columns: hundreds of CTAs meet at two L2 lines.
+template <typename T, int NT>
+__device__ __noinline__ void lu_column_max(const T* S, int m, int kb, int* s_max, int* out) {
+  const int tid = threadIdx.x, j = tid & 63;
+  if (tid < 64) s_max[tid] = 0;
+  __syncthreads();
+  int fm = 0;
+#pragma unroll 4
+  for (int r = tid >> 6; r < m; r += NT / 64) fm = max(fm, XsType<T>::expo(S[r * LuBits<T>::LD + j]));
+  if (fm) atomicMax(&s_max[j], fm);
+  __syncthreads();
+  if (tid < kb && s_max[tid]) atomicMax(out + tid, s_max[tid]);
+}
+
 template <typename T, bool CL, int NT>
 __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restrict__ items, int n_items, int nb,
                                                    int pivot, int rmax, int csize, uint64_t* __restrict__ xbuf,
-                                                   int* err) {
+                                                   int* __restrict__ lmax, int* err) {
   extern __shared__ __align__(16) unsigned char gc_smem[];
   using LuRecvT = LuRecv<T, CL>;
   constexpr int NW = NT / 32, WORDS = LuBits<T>::WORDS, SR = LuBits<T>::LD;
@@ -1666,13 +1690,16 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
   if (tg < ng)
     for (int j = tg; j < kb; j += ng)
       for (int r = tr; r < nr_my; r += rw) G[(rbeg + r) + (int64_t)(k0 + j) * n] = S[r * SR + j];
+  if (lmax)
+    lu_column_max<T, NT>(S + (int64_t)max(0, k0 + kb - rbeg) * SR, nr_my - max(0, k0 + kb - rbeg), kb,
+                         reinterpret_cast<int*>(recv), lmax + f.piv_off + k0);
 }
 
 constexpr int GC_NT_CLUSTER = 512, GC_NT_GRID = 256;
 
 template <typename T, bool CL>
 static cudaError_t getrf_smem_t(const DevCtx& c, const Item* items, int n_items, int n_ctas, int csize, int nb,
-                                int pivot, int rmax, uint64_t* xbuf, int* err, cudaStream_t s) {
+                                int pivot, int rmax, uint64_t* xbuf, int* lmax, int* err, cudaStream_t s) {
   constexpr int NT = CL ? GC_NT_CLUSTER : GC_NT_GRID;
   const size_t smem = (size_t)rmax * (LuBits<T>::LD + 2) * sizeof(T);
   cudaFuncSetAttribute(k_getrf_smem<T, CL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1694,23 +1721,23 @@ static cudaError_t getrf_smem_t(const DevCtx& c, const Item* items, int n_items,
   }
   cfg.attrs = attr;
   cfg.numAttrs = CL && csize == 1 ? 0 : 1;
-  return cudaLaunchKernelEx(&cfg, k_getrf_smem<T, CL, NT>, c, items, n_items, nb, pivot, rmax, csize, xbuf, err);
+  return cudaLaunchKernelEx(&cfg, k_getrf_smem<T, CL, NT>, c, items, n_items, nb, pivot, rmax, csize, xbuf, lmax, err);
 }
 
 void launch_getrf_smem(const DevCtx& c, const Item* items, int n_items, int n_ctas, int csize, int dtype, int nb,
-                       int pivot, int rmax, uint64_t* xbuf, int* err, cudaStream_t s) {
+                       int pivot, int rmax, uint64_t* xbuf, int* lmax, int* err, cudaStream_t s) {
   if (!n_items) return;
   if (nb > 64) throw std::invalid_argument("getrf_smem: panel wider than 64");
   if (csize > GC_CLUSTER) throw std::invalid_argument("getrf_smem: cluster too large");
   cudaError_t e;
   if (csize > 0) {
-    e = dtype == F64 ? getrf_smem_t<double, true>(c, items, n_items, n_items * csize, csize, nb, pivot, rmax, nullptr, err, s)
-                     : getrf_smem_t<float, true>(c, items, n_items, n_items * csize, csize, nb, pivot, rmax, nullptr, err, s);
+    e = dtype == F64 ? getrf_smem_t<double, true>(c, items, n_items, n_items * csize, csize, nb, pivot, rmax, nullptr, lmax, err, s)
+                     : getrf_smem_t<float, true>(c, items, n_items, n_items * csize, csize, nb, pivot, rmax, nullptr, lmax, err, s);
   } else {
     if (n_ctas > GC_MAX_CTAS) throw std::invalid_argument("getrf_smem: too many CTAs");
     cudaMemsetAsync(xbuf, 0, sizeof(uint64_t) * (size_t)gc_words(n_ctas, n_items), s);
-    e = dtype == F64 ? getrf_smem_t<double, false>(c, items, n_items, n_ctas, 0, nb, pivot, rmax, xbuf, err, s)
-                     : getrf_smem_t<float, false>(c, items, n_items, n_ctas, 0, nb, pivot, rmax, xbuf, err, s);
+    e = dtype == F64 ? getrf_smem_t<double, false>(c, items, n_items, n_ctas, 0, nb, pivot, rmax, xbuf, lmax, err, s)
+                     : getrf_smem_t<float, false>(c, items, n_items, n_ctas, 0, nb, pivot, rmax, xbuf, lmax, err, s);
   }
   if (e != cudaSuccess)
     throw std::runtime_error(std::string("LU panel launch failed: ") + cudaGetErrorString(e));
@@ -1719,9 +1746,8 @@ void launch_getrf_smem(const DevCtx& c, const Item* items, int n_items, int n_ct
 // Row interchanges of a panel (pivots of rows k0..k0+kb-1, kb = min(nb,
 // fs - k0), applied in order) on the front's columns outside the panel and
 // below a column limit.  Item: front, a = k0, b = first column of a
-// 256-column chunk, c = column limit (0: n); one thread per column.  The
-// last warp of chunk 0 (of b = -1: no columns) applies them to the front's
-// row permutation, which the solves gather by.
+// 256-column chunk, c = column limit (0: n); one thread per column.  b = -1: no
+// columns, but the front's row permutation, which the solves gather by.
 constexpr int LASWP_THREADS = 256 + 32;
 
 template <typename T>
@@ -1732,7 +1758,7 @@ __global__ void __launch_bounds__(LASWP_THREADS) k_laswp(DevCtx c, const Item* _
   const int kb = min(nb, f.fs - k0);
   const int32_t* __restrict__ pv = c.piv + f.piv_off;
   if (threadIdx.x >= 256) {
-    if (it.b > 0) return;
+    if (it.b >= 0) return;
     int32_t* __restrict__ perm = c.perm + f.piv_off;
     if (k0 == 0)
       for (int i = threadIdx.x - 256; i < f.fs; i += 32) perm[i] = i;
@@ -1771,7 +1797,8 @@ void launch_laswp(const DevCtx& c, const Item* items, int n_items, int dtype, in
 constexpr int LUROW_CB = 16;   // columns per row-panel block
 
 // A[k0:k0+kb, cols] <- L11^{-1} A[k0:k0+kb, cols]  (unit lower), cols >= k0+kb;
-// item: front, a = k0, b = first column of the chunk, c = column limit (0: n)
+// item: front, a = k0, b = first column of the chunk, c = column limit (0: n);
+// umax (null: not wanted): the rows' largest exponent fields, as lmax of k_getrf_smem
 //
 // Substitution in registers: Q lanes hold one column (lane q rows q, q+Q,
 // ..), a step's solved entry goes to the others by one shuffle, L comes
@@ -1787,7 +1814,8 @@ constexpr int LUROW_CB = 16;   // columns per row-panel block
 // launches, 38.7 -> 7.9 ms; FP64, the smallest launches, four lanes 29 us, eight 18;
 // 12^3 p = 3, 200 launches, 6.5 -> 5.0 ms.
 template <typename T, int Q>
-__global__ void __launch_bounds__(Q * LUROW_CB) k_lu_row_update(DevCtx c, const Item* __restrict__ items, int nb) {
+__global__ void __launch_bounds__(Q * LUROW_CB) k_lu_row_update(DevCtx c, const Item* __restrict__ items, int nb,
+                                                                int* __restrict__ umax) {
   constexpr int NU = 64 / Q, LQ = NU + 2;      // rows per lane; their L entries' row in shared memory (no bank conflicts)
   constexpr int NT = Q * LUROW_CB;
   __shared__ __align__(16) T L[64 * Q * LQ];   // L[(Q k + q) LQ + u] = L11[q + Q u][k]
@@ -1824,15 +1852,29 @@ __global__ void __launch_bounds__(Q * LUROW_CB) k_lu_row_update(DevCtx c, const 
 #pragma unroll
   for (int u = 0; u < NU; ++u)
     if (in && q + Q * u < kb) X[Q * u] = x[u];
+  if (!umax) return;
+  // the largest exponent field of each row over the CTA's columns
+  int* s_max = reinterpret_cast<int*>(L);
+  __syncthreads();                             // L has been read
+  if (threadIdx.x < 64) s_max[threadIdx.x] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < NU; ++u) {
+    int fm = in && q + Q * u < kb ? XsType<T>::expo(x[u]) : 0;
+#pragma unroll
+    for (int o = Q; o < 32; o <<= 1) fm = max(fm, __shfl_xor_sync(0xffffffffu, fm, o));
+    if ((threadIdx.x & 31) < Q && fm) atomicMax(&s_max[q + Q * u], fm);
+  }
+  __syncthreads();
+  if (threadIdx.x < kb && s_max[threadIdx.x]) atomicMax(umax + f.piv_off + k0 + threadIdx.x, s_max[threadIdx.x]);
 }
 
-void launch_lu_row_update(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
-                          int pivot, cudaStream_t s) {
-  (void)pivot;
+void launch_lu_row_update(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, int* umax,
+                          cudaStream_t s) {
   if (!n_items) return;
   if (nb != 64) throw std::invalid_argument("lu_row_update: panels are 64 columns wide");
-  if (dtype == F64) k_lu_row_update<double, 8><<<n_items, 8 * LUROW_CB, 0, s>>>(c, items, nb);
-  else k_lu_row_update<float, 4><<<n_items, 4 * LUROW_CB, 0, s>>>(c, items, nb);
+  if (dtype == F64) k_lu_row_update<double, 8><<<n_items, 8 * LUROW_CB, 0, s>>>(c, items, nb, umax);
+  else k_lu_row_update<float, 4><<<n_items, 4 * LUROW_CB, 0, s>>>(c, items, nb, umax);
 }
 
 // Inverses of a large LU front's diagonal blocks, for the flag-driven solves:

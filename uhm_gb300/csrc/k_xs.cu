@@ -1,6 +1,6 @@
-// Trailing updates C -= A B^T of FP64 and FP32 fronts on the tensor cores,
-// without loss of precision: the operands are cut into 8-bit slices whose
-// BF16 products add up exactly.
+// Trailing updates C -= A B^T of FP64 and FP32 fronts on the tensor cores, at
+// the precision of multiply-adds in the front's own type: the operands are cut
+// into 8-bit slices whose BF16 products add up exactly.
 //
 // Restates the trailing SYRK / GEMM of the front's blocked factorisation
 // (LINAL/src/dense/chol.cxx:78-82, lu_piv.cxx:95-105 and the front-level
@@ -26,6 +26,28 @@
 // close as the SIMT update's (seven slices without diagonal 7 were 3 to 10
 // times further off).
 //
+// All that is relative to the product of two row maxima, and a multiply-add's error
+// to the sum of the products' magnitudes.  Cholesky: both are bounded by
+// sqrt(a_ii a_jj), as for a factorisation in the type itself.  LU: the maxima of a
+// row of L21 and a column of U12 can lie at different inner k, where l_ik scales as
+// 1 / d_k and u_kj as d_k with the unit d_k of an eliminated equation (rows in
+// units of 1 and 10^10: solutions of an FP64 front 10^6 to 10^8 times further off).  So
+//  - column k of L21 and row k of U12 are multiplied by 2^t and 2^-t before they are
+//    cut, t half the difference of the exponents of their largest entries: exact,
+//    the products stay, and units of equations, of unknowns and of both are balanced;
+//  - each row keeps which of the panel's columns come within 2^4 (FP32 2^3) of its
+//    maximum, each front which of them some row of the other operand has so near its own.
+//    A row or column of a tile where no column is both (of the front's own part, or
+//    of its shared part, whichever the tile is in) goes by plain multiply-adds
+//    (xs_plain).  The rest differs from the sum of magnitudes by 2^8 (2^6) at
+//    most, over its row and over its column, which is the bound of 256
+//    multiply-adds in a row.
+// Measured (tests/test_gpu_lu_scaling.py: units to 2^33, rows that no balance serves)
+// errors are 0.4 to 0.9 times those of multiply-adds.  On convection-diffusion
+// fronts less than 0.3 % of the 32 x 32 blocks have such a row or column.  Cost:
+// 12^3 p = 3 FP64 LU factorisation 38.0 -> 39.4 ms (updates 0.8, slices 0.2, panels 0.4),
+// 6^3 6.5 -> 6.75.
+//
 // Why: GB300 does about 2 FP64 multiply-adds per clock per SM (1.17 TFLOP/s
 // measured for the SIMT update), against 1,906 TFLOP/s of BF16 products:
 // 36 products per FP64 one still leave 53.  FP32 fronts: 10 products leave
@@ -36,6 +58,7 @@
 #include <cudaTypedefs.h>
 
 #include <stdexcept>
+#include <type_traits>
 
 #include "k_common.cuh"
 #include "k_tc_ptx.cuh"
@@ -59,13 +82,18 @@ constexpr int XS_ERR = 7;
 // no FP64.  Measured on GB300 for 256 columns: 29 us with 64 rows per CTA and
 // its 64-column chunks in turn (whatever their number), 11 with 16 rows.
 template <typename T, int NG>
-__global__ void __launch_bounds__(256) k_xs_pack(DevCtx c, XsCtx x, const Item* __restrict__ items, int nb) {
+__global__ void __launch_bounds__(256) k_xs_pack(DevCtx c, XsCtx x, const Item* __restrict__ items, int nb,
+                                                  int use) {
   constexpr int S = XsType<T>::S, ROWS = 256 / NG;
-  __shared__ int s_f[NG][ROWS];
+  constexpr int NEAR = S == 8 ? XS_NEAR64 : XS_NEAR32;
+  __shared__ int s_f[NG][ROWS], s_r[NG][ROWS];
+  __shared__ __align__(16) int s_t[16 * NG];
+  __shared__ uint32_t s_or[2][8];
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, K0 = it.a, trans = it.c;
   const int W = min(nb, f.fs - K0), nch = xs_chunks(nb, f.fs);
+  const bool lu = x.kmax != nullptr;
   const int r = threadIdx.x % ROWS, g = threadIdx.x / ROWS;
   const int row = it.b + r;
   const T* __restrict__ G = arena<T>(c) + f.off;
@@ -75,29 +103,96 @@ __global__ void __launch_bounds__(256) k_xs_pack(DevCtx c, XsCtx x, const Item* 
   T v[16];
 #pragma unroll
   for (int u = 0; u < 16; ++u) v[u] = in && 16 * g + u < W ? G[base + (16 * g + u) * step] : T(0);
-  int fm = 1;
+  if (lu && threadIdx.x < 16 * NG) {
+    // this side's share of the balance of column K0 + k
+    int t = 0;
+    if ((int)threadIdx.x < W) {
+      const int64_t k = (int64_t)f.piv_off + K0 + threadIdx.x;
+      const int l = x.kmax[k], u = NG == 4 ? x.kmax[x.kmax_n + k] : max(x.kmax[x.kmax_n + k], x.kmax[2 * x.kmax_n + k]);
+      t = l && u ? (u - l) >> 1 : 0;
+    }
+    s_t[threadIdx.x] = trans ? -t : t;
+  }
+  const int64_t row0 = (trans ? x.row0b : x.row0)[it.front] + (int64_t)g * n + row;
+  if (!lu) {
+    int fm = 1;
 #pragma unroll
-  for (int u = 0; u < 16; ++u) fm = max(fm, XsType<T>::field(v[u]));
+    for (int u = 0; u < 16; ++u) fm = max(fm, XsType<T>::field(v[u]));
+    s_f[g][r] = fm;
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < NG; ++e) fm = max(fm, s_f[e][r]);
+    if (!in || 16 * g >= 64 * nch) return;
+    const bool bad = fm == XsType<T>::FMAX;
+    if (g == 0) x.exps[x.exp0[it.front] + row] = bad ? XS_BAD : fm - XsType<T>::EBIAS;
+    xs_store16<T>(x, row0, (int64_t)4 * nch * n, v, fm, bad);
+    return;
+  }
+  __syncthreads();                             // s_t
+  // (a zero counts as the smallest number for the row's exponent and is never near)
+  int e[16], fr = 0, fm = -XS_BAD;
+#pragma unroll
+  for (int u = 0; u < 16; u += 4) {
+    const int4 t4 = *reinterpret_cast<const int4*>(s_t + 16 * g + u);
+    const int t[4] = {t4.x, t4.y, t4.z, t4.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int fu = XsType<T>::field(v[u + q]);
+      fr = max(fr, fu);
+      e[u + q] = max(fu, 1) + t[q];
+      fm = max(fm, e[u + q]);
+    }
+  }
+  if (fr == XsType<T>::FMAX) fm = XS_BAD;
   s_f[g][r] = fm;
+  s_r[g][r] = fr;
   __syncthreads();
 #pragma unroll
-  for (int e = 0; e < NG; ++e) fm = max(fm, s_f[e][r]);
-  if (!in || 16 * g >= 64 * nch) return;
-  const bool bad = fm == XsType<T>::FMAX;
-  if (g == 0) x.exps[x.exp0[it.front] + (trans ? n : 0) + row] = bad ? XS_BAD : fm - XsType<T>::EBIAS;
-  xs_store16<T>(x, (trans ? x.row0b : x.row0)[it.front] + (int64_t)g * n + row, (int64_t)4 * nch * n, v, fm, bad);
+  for (int q = 0; q < NG; ++q) {
+    fm = max(fm, s_f[q][r]);
+    fr = max(fr, s_r[q][r]);
+  }
+  const bool bad = fm == XS_BAD, some = fr > 0 && !bad;
+  // the columns near the row's maximum; a row without any counts as near in all
+  uint32_t mask = 0;
+#pragma unroll
+  for (int u = 0; u < 16; ++u)
+    if (e[u] >= fm - NEAR && XsType<T>::field(v[u])) mask |= 1u << u;
+  // their union over the CTA's own and its shared rows (region 2 takes region 1's: xs_check)
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t all = __reduce_or_sync(0xffffffffu, some && (row >= f.fs) == h ? mask << (16 * (g & 1)) : 0u);
+    if ((threadIdx.x & 31) == 0) s_or[h][threadIdx.x >> 5] = all;
+  }
+  if (in && 16 * g < 64 * nch) {
+    const int64_t at = x.exp0[it.front] + (trans ? n : 0) + row;
+    reinterpret_cast<uint16_t*>(x.masks)[at * (XS_NBO / 16) + g] = (uint16_t)(some ? mask : 0xFFFFu);
+    if (g == 0) x.exps[at] = bad ? XS_BAD : fm - XsType<T>::EBIAS;
+    xs_store16<T>(x, row0, (int64_t)4 * nch * n, v, fm, bad, s_t + 16 * g);
+  }
+  if (use == 2 && !trans) return;
+  __syncthreads();
+  // (one request per CTA: hundreds meet at one L2 line)
+  const int h = threadIdx.x / (NG / 2), w = threadIdx.x % (NG / 2);
+  if (h < 2) {
+    uint32_t all = 0;
+#pragma unroll
+    for (int e = 0; e < 16 / NG; ++e) all |= s_or[h][NG == 16 ? w : 4 * w + e];
+    if (all) atomicOr(x.near + (4 * use + 2 * trans + h) * x.near_n + x.near0[it.front] + K0 / 32 + w, all);
+  }
 }
 
-void launch_xs_pack(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, int dtype, int nb,
+void launch_xs_pack(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, int dtype, int nb, int use,
                     cudaStream_t s) {
   if (!n_items) return;
   if (nb != 64 && nb != XS_NBO) throw std::invalid_argument("slices: panel width must be 64 or 256");
+  if (use < 0 || use >= XS_USES) throw std::invalid_argument("slices: the update's region must be 0, 1 or 2");
   if (dtype == F64) {
-    if (nb == 64) k_xs_pack<double, 4><<<n_items, 256, 0, s>>>(c, x, items, nb);
-    else k_xs_pack<double, 16><<<n_items, 256, 0, s>>>(c, x, items, nb);
+    if (nb == 64) k_xs_pack<double, 4><<<n_items, 256, 0, s>>>(c, x, items, nb, use);
+    else k_xs_pack<double, 16><<<n_items, 256, 0, s>>>(c, x, items, nb, use);
   } else {
-    if (nb == 64) k_xs_pack<float, 4><<<n_items, 256, 0, s>>>(c, x, items, nb);
-    else k_xs_pack<float, 16><<<n_items, 256, 0, s>>>(c, x, items, nb);
+    if (nb == 64) k_xs_pack<float, 4><<<n_items, 256, 0, s>>>(c, x, items, nb, use);
+    else k_xs_pack<float, 16><<<n_items, 256, 0, s>>>(c, x, items, nb, use);
   }
 }
 
@@ -193,6 +288,7 @@ constexpr uint32_t XS_BOX = 128 * 128;                  // 128 rows of four slic
 constexpr uint32_t XS_SLOT = 2 * XS_BOX;                // four slices of A and of B, 16 columns
 constexpr int XS_SLOTS = 7;
 constexpr uint32_t XS_SMEM = 1024 + XS_SLOTS * XS_SLOT + 512;
+static_assert(8 * (2 * XS_SLOTS + 13) + 8 * XS_EPI_WARPS <= 512, "barriers and the epilogue's words");
 
 #define XS_LD16(taddr, v)                                                                        \
   asm volatile(                                                                                  \
@@ -281,6 +377,91 @@ __device__ __forceinline__ float xs_scaled(long long a, int E, float) {
   return x * __int_as_float((127 + e1) << 23) * __int_as_float((127 + e2) << 23);
 }
 
+// LU: the rows (bits of left[0]) and columns (left[1]) of this warp's 32 x NC entries
+// that the slices do not serve: none of the panel columns near its own maximum is near the maximum of
+// any row of the other operand (of the front's own rows, or of its shared ones,
+// whichever the entries lie in; a panel that is zero there serves them).
+template <int NC>
+__device__ __forceinline__ void xs_check(const XsCtx& x, int front, int K0, int n, int fs, int nb, int use, int row,
+                                         int rmax, int c0, int cmax, volatile uint32_t* left) {
+  const int lane = threadIdx.x & 31, r0 = row - lane;
+  const bool rin = row < rmax, cin = lane < NC && c0 + lane < cmax;
+  const int64_t e0 = x.exp0[front], w0 = x.near0[front] + K0 / 32;
+  const uint2* ma = reinterpret_cast<const uint2*>(x.masks + (e0 + (rin ? row : 0)) * (XS_NBO / 32));
+  const uint2* mb = reinterpret_cast<const uint2*>(x.masks + (e0 + n + (cin ? c0 + lane : 0)) * (XS_NBO / 32));
+  // side A's unions of region 1 serve region 2 (its rows are among them), where region 1's
+  // columns join side B's (the balance is the same): own rows, shared rows
+  const uint2* na = reinterpret_cast<const uint2*>(x.near + 4 * (use ? 1 : 0) * x.near_n + w0);
+  const uint2* nbv = reinterpret_cast<const uint2*>(x.near + (4 * use + 2) * x.near_n + w0);
+  const uint2* nb1 = reinterpret_cast<const uint2*>(x.near + 6 * x.near_n + w0);
+  const int64_t own = x.near_n / 2;
+  uint32_t hr[2] = {0, 0}, hc[2] = {0, 0}, sa[2] = {0, 0}, sb[2] = {0, 0};
+#pragma unroll 2
+  for (int w = 0; w < nb / 64; ++w) {          // (every load of a round in flight)
+    const uint2 a = ma[w], b = mb[w];
+    uint2 pa[2], pb[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      pa[h] = na[w + h * own];
+      pb[h] = nbv[w + h * own];
+      if (use == 2) {
+        const uint2 p1 = nb1[w + h * own];
+        pb[h].x |= p1.x;
+        pb[h].y |= p1.y;
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      hr[h] |= (a.x & pb[h].x) | (a.y & pb[h].y);
+      hc[h] |= (b.x & pa[h].x) | (b.y & pa[h].y);
+      sa[h] |= pa[h].x | pa[h].y;
+      sb[h] |= pb[h].x | pb[h].y;
+    }
+  }
+  bool okr = true, okc = true;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const bool cols = h ? min(c0 + NC, cmax) > fs : c0 < fs, rows = h ? min(r0 + 32, rmax) > fs : r0 < fs;
+    okr = okr && (!cols || hr[h] || !sb[h]);
+    okc = okc && (!rows || hc[h] || !sa[h]);
+  }
+  const uint32_t wr = __ballot_sync(0xffffffffu, rin && !okr), wc = __ballot_sync(0xffffffffu, cin && !okc);
+  if (lane == 0) {
+    left[0] = wr;
+    left[1] = wc;
+  }
+  __syncwarp();
+}
+// the exponent of a row or column left to xs_plain: its slices' sums become zero
+__device__ __forceinline__ int xs_exp(int e, bool left) { return left ? -(1 << 29) : e; }
+
+// ... and their entries by multiply-adds in the front's precision, 64 columns of
+// the panel at a time: a row's columns along the lanes, then a column's rows.
+template <typename T, int NC>
+__device__ __noinline__ void xs_plain(T* G, int n, int K0, int W, int row, int rmax, int c0, int cmax,
+                                      volatile uint32_t* left) {
+  const int lane = threadIdx.x & 31, row0 = row - lane;
+  const uint32_t wr = left[0], wc = left[1];
+  __syncwarp();                                // C, unchanged in these rows and columns, is stored
+  auto entry = [&](int r, int col) {
+    T v = __ldcg(G + r + (int64_t)col * n);
+    const T* __restrict__ l = G + r + (int64_t)K0 * n;
+    const T* __restrict__ u = G + K0 + (int64_t)col * n;
+    for (int k0 = 0; k0 < W; k0 += 64) {
+      const int k1 = min(k0 + 64, W);
+      T s = T(0);
+#pragma unroll 8
+      for (int k = k0; k < k1; ++k) s += l[(int64_t)k * n] * u[k];
+      v -= s;
+    }
+    G[r + (int64_t)col * n] = v;
+  };
+  for (uint32_t m = wr; m; m &= m - 1)
+    if (lane < NC && c0 + lane < cmax) entry(row0 + __ffs(m) - 1, c0 + lane);
+  for (uint32_t m = wc; m; m &= m - 1)
+    if (row < rmax && !(wr >> lane & 1)) entry(row, c0 + __ffs(m) - 1);
+}
+
 // Persistent: one CTA per SM walks the 128 x 128 tiles.  Warp 16 loads four
 // slices of A and B (16 columns, 128-byte swizzle) per ring slot, one thread of
 // warp 17 issues the products of a chunk,
@@ -303,10 +484,11 @@ __device__ __forceinline__ float xs_scaled(long long a, int E, float) {
 // reads of the 128 x 128 products; a tile of a small launch by its epilogue.
 // Measured on GB300 for up to 80 tiles
 // of K = 64 (256): 29 (60) us with whole tiles, 18 (31) with these.
-template <typename T, int BN>
+template <typename T, int BN, bool LOWER>
 __global__ void __launch_bounds__(XS_THREADS, 1)
 k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ XsMaps maps, const Item* __restrict__ items, int n_items,
-            int nb, int region, int lower, int* err) {
+            int nb, int region, int* err) {
+  constexpr bool lower = LOWER;
   constexpr int S = XsType<T>::S;
   extern __shared__ __align__(1024) uint8_t xs_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(xs_raw) + 1023) & ~uintptr_t(1023));
@@ -489,6 +671,9 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ XsMaps maps, const Item* 
     constexpr int NC = BN / 4;       // columns per thread
     const int quarter = warp & 3, cg = warp >> 2;
     const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + cg * NC;
+    // LU: what of the warp's entries is left to xs_plain (in shared memory: no register is
+    // free while the accumulators are read)
+    volatile uint32_t* const left = reinterpret_cast<volatile uint32_t*>(drain_bar + 4) + 2 * warp;
     uint32_t par = 0;              // bit a: parity of the next use of accumulator a
     bool live = true;
     for (int t = blockIdx.x; t < n_items && live; t += gridDim.x) {
@@ -508,9 +693,10 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ XsMaps maps, const Item* 
         T cv[NC];
 #pragma unroll
         for (int j = 0; j < NC; ++j) cv[j] = j < cend ? __ldcg(G + (int64_t)j * n) : T(0);
+        if constexpr (!lower) xs_check<NC>(x, it.front, K0, n, f.fs, nb, region, row, rmax, c0, cmax, left);
         const int* __restrict__ ex = x.exps + x.exp0[it.front];
-        const int ea = cend > 0 ? ex[row] - 36 : 0;
-        const int ebl = c0 + lane < cmax ? ex[(lower ? 0 : n) + c0 + lane] : 0;      // NC = 32 lanes
+        const int ea = cend > 0 ? xs_exp(ex[row], !lower && (left[0] >> lane & 1)) - 36 : 0;
+        const int ebl = c0 + lane < cmax ? xs_exp(ex[(lower ? 0 : n) + c0 + lane], !lower && (left[1] >> lane & 1)) : 0;  // NC = 32 lanes
 #pragma unroll
         for (int a = 0; a < 4; ++a)
           live = live && mbar_wait_lim(smem_u32(&acc_full[a]), par & 1, s_abort, err, XS_ERR, lim);
@@ -547,6 +733,8 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ XsMaps maps, const Item* 
 #pragma unroll
         for (int j = 0; j < NC; ++j)
           if (j < cend) G[(int64_t)j * n] = cv[j];
+        if constexpr (!lower)
+          if (left[0] | left[1]) xs_plain<T, NC>(arena<T>(c) + f.off, n, K0, min(nb, f.fs - K0), row, rmax, c0, cmax, left);
         continue;
       }
       constexpr bool EARLY = BN == 64;
@@ -555,6 +743,7 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ XsMaps maps, const Item* 
 #pragma unroll
         for (int j = 0; j < NC; ++j) ce[j] = j < cend ? __ldcg(G + (int64_t)j * n) : T(0);
       }
+      if constexpr (!lower) xs_check<NC>(x, it.front, K0, n, f.fs, nb, region, row, rmax, c0, cmax, left);
       long long acc[NC];
 #pragma unroll
       for (int j = 0; j < NC; ++j) acc[j] = 0;
@@ -593,7 +782,8 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ XsMaps maps, const Item* 
       if (cend > 0) {
         const int* __restrict__ ex = x.exps + x.exp0[it.front];
         const int* __restrict__ ebp = ex + (lower ? 0 : n) + c0;
-        const int ea = ex[row] - (S == 8 ? 54 : 36);
+        const int ea = xs_exp(ex[row], !lower && (left[0] >> lane & 1)) - (S == 8 ? 54 : 36);
+        const uint32_t wc = lower ? 0u : left[1];
 #pragma unroll
         for (int j0 = 0; j0 < NC; j0 += 4) {
           T cv[4];
@@ -605,7 +795,7 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ XsMaps maps, const Item* 
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             if (j0 + j < cend) {
-              const int E = ea + __ldg(ebp + j0 + j);
+              const int E = ea + xs_exp(__ldg(ebp + j0 + j), !lower && (wc >> (j0 + j) & 1));
               T d = xs_scaled(acc[j0 + j], E, T(0));
               if (E > XS_BAD / 2) d = T(NAN);
               G[(int64_t)j * n] = cv[j] - d;
@@ -613,6 +803,8 @@ k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ XsMaps maps, const Item* 
           G += 4 * (int64_t)n;
         }
       }
+      if constexpr (!lower)
+        if (left[0] | left[1]) xs_plain<T, NC>(arena<T>(c) + f.off, n, K0, min(nb, f.fs - K0), row, rmax, c0, cmax, left);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -647,9 +839,9 @@ bool xs_encode(XsMaps* maps, void* base, int64_t rows) {
   return true;
 }
 
-template <typename T, int BN>
+template <typename T, int BN, bool LOWER>
 static void xs_update_t(const DevCtx& c, const XsCtx& x, const XsMaps& maps, const Item* items, int n_items,
-                        int nb, int region, int lower, int cap, int* err, cudaStream_t s) {
+                        int nb, int region, int cap, int* err, cudaStream_t s) {
   static int n_sm = 0;
   if (!n_sm) {
     int dev = 0;
@@ -657,10 +849,10 @@ static void xs_update_t(const DevCtx& c, const XsCtx& x, const XsMaps& maps, con
     cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
     if (n_sm <= 0) n_sm = 1;
   }
-  cudaFuncSetAttribute(k_xs_update<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XS_SMEM);
+  cudaFuncSetAttribute(k_xs_update<T, BN, LOWER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XS_SMEM);
   const int sms = cap > 0 && cap < n_sm ? cap : n_sm;
   const int grid = n_items < sms ? n_items : sms;
-  k_xs_update<T, BN><<<grid, XS_THREADS, XS_SMEM, s>>>(c, x, maps, items, n_items, nb, region, lower, err);
+  k_xs_update<T, BN, LOWER><<<grid, XS_THREADS, XS_SMEM, s>>>(c, x, maps, items, n_items, nb, region, err);
 }
 
 void launch_xs_update(const DevCtx& c, const XsCtx& x, const XsMaps& maps, const Item* items, int n_items,
@@ -668,13 +860,17 @@ void launch_xs_update(const DevCtx& c, const XsCtx& x, const XsMaps& maps, const
   if (!n_items) return;
   if (nb > XS_NBO) throw std::invalid_argument("sliced update: panel wider than 256");
   if (tile_n != 64 && tile_n != XS_TILE) throw std::invalid_argument("sliced update: tiles are 64 or 128 columns wide");
-  if (dtype == F64) {
-    if (tile_n == 64) xs_update_t<double, 64>(c, x, maps, items, n_items, nb, region, lower, cap, err, s);
-    else xs_update_t<double, 128>(c, x, maps, items, n_items, nb, region, lower, cap, err, s);
-  } else {
-    if (tile_n == 64) xs_update_t<float, 64>(c, x, maps, items, n_items, nb, region, lower, cap, err, s);
-    else xs_update_t<float, 128>(c, x, maps, items, n_items, nb, region, lower, cap, err, s);
-  }
+  if (!lower && !x.near) throw std::invalid_argument("sliced update: LU operands without their check");
+  const auto run = [&](auto t, auto low) {
+    using T = decltype(t);
+    constexpr bool L = decltype(low)::value;
+    if (tile_n == 64) xs_update_t<T, 64, L>(c, x, maps, items, n_items, nb, region, cap, err, s);
+    else xs_update_t<T, XS_TILE, L>(c, x, maps, items, n_items, nb, region, cap, err, s);
+  };
+  if (dtype == F64 && lower) run(double(), std::true_type());
+  else if (dtype == F64) run(double(), std::false_type());
+  else if (lower) run(float(), std::true_type());
+  else run(float(), std::false_type());
 }
 
 }  // namespace uhm_gpu

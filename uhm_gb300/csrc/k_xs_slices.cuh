@@ -17,6 +17,12 @@ template <typename T> struct XsType;
 template <> struct XsType<double> {
   static constexpr int S = XS_S64;
   static __device__ __forceinline__ int field(double v) { return (__double2hiint(v) >> 20) & 0x7FF; }
+  // the field, 1 for a subnormal number, 0 for zero (in integers: an FP64 comparison costs
+  // as much as a multiply-add)
+  static __device__ __forceinline__ int expo(double v) {
+    const int f = field(v);
+    return f ? f : (__double2hiint(v) << 1 | __double2loint(v)) != 0;
+  }
   static constexpr int FMAX = 0x7FF, EBIAS = 1022;
   // round(v 2^(62 - e)), e = fmax - EBIAS, fmax the largest exponent field of the row (at least 1)
   static __device__ __forceinline__ long long fixed(double v, int fmax) {
@@ -34,6 +40,10 @@ template <> struct XsType<double> {
 template <> struct XsType<float> {
   static constexpr int S = XS_S32;
   static __device__ __forceinline__ int field(float v) { return (__float_as_int(v) >> 23) & 0xFF; }
+  static __device__ __forceinline__ int expo(float v) {
+    const int f = field(v);
+    return f ? f : (__float_as_int(v) << 1) != 0;
+  }
   static constexpr int FMAX = 0xFF, EBIAS = 126;
   // round(v 2^(30 - e))
   static __device__ __forceinline__ long long fixed(float v, int fmax) {
@@ -70,17 +80,19 @@ __device__ __forceinline__ void xs_digits(long long X, uint32_t (&d)[S]) {
 }
 
 // slices of 16 columns of a row, v, whose row's largest exponent field is fm: row
-// `at` of the workspace, and, S = 8, the one `group` rows behind it
+// `at` of the workspace, and, S = 8, the one `group` rows behind it; t: powers
+// of two that the columns are multiplied by (fm with them), null: none
 template <typename T>
-__device__ __forceinline__ void xs_store16(const XsCtx& x, int64_t at, int64_t group, const T (&v)[16], int fm, bool bad) {
+__device__ __forceinline__ void xs_store16(const XsCtx& x, int64_t at, int64_t group, const T (&v)[16], int fm, bool bad,
+                                           const int* t = nullptr) {
   constexpr int S = XsType<T>::S;
   uint8_t* const w0 = reinterpret_cast<uint8_t*>(x.ws) + 128 * at;
   uint32_t d[S][8];
 #pragma unroll
   for (int u = 0; u < 16; u += 2) {
     uint32_t d0[S], d1[S];
-    xs_digits<S>(bad ? 0 : XsType<T>::fixed(v[u], fm), d0);
-    xs_digits<S>(bad ? 0 : XsType<T>::fixed(v[u + 1], fm), d1);
+    xs_digits<S>(bad ? 0 : XsType<T>::fixed(v[u], t ? fm - t[u] : fm), d0);
+    xs_digits<S>(bad ? 0 : XsType<T>::fixed(v[u + 1], t ? fm - t[u + 1] : fm), d1);
 #pragma unroll
     for (int p = 0; p < S; ++p) d[p][u / 2] = __byte_perm(d0[p], d1[p], 0x7632);
   }
