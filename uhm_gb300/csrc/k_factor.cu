@@ -296,7 +296,8 @@ __global__ void __launch_bounds__(NT) k_small_factor(DevCtx c, const Item* __res
 // ties.  (Products with the reciprocal root instead: an error of r is common to its
 // whole column of L and, on a uniform mesh, to every element's front; the
 // solutions of 12^3 and 16^3 p = 4 Poisson meshes were 1.3 and 1.5 times further
-// from the exact ones than with a square root and divisions.)
+// from the exact ones than with a square root and divisions.)  An infinite
+// d (r = 0) is given as 0: the quotients of finite numbers are then zero, as by division.
 __device__ __forceinline__ double fp64_div(double v, double d, double r) {
   const double q = v * r;
   return fma(fma(-q, d, v), r, q);
@@ -316,9 +317,11 @@ __device__ __forceinline__ void small_panel4(const DevCtx& c, int front, double*
     double t[4];
     if (r < n) {
       double lb[4][4], rd[4], ld[4];
+      bool inf[4];
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
         rd[m] = ld[m] = 1.0;
+        inf[m] = false;
         if (m >= w) continue;
         double s = A[P + m + (P + m) * n];
 #pragma unroll
@@ -332,6 +335,8 @@ __device__ __forceinline__ void small_panel4(const DevCtx& c, int front, double*
           const double h = s * rd[m];          // sqrt(s), corrected the same way
           const double e = fma(-h, h, s);
           ld[m] = fabs(e) < s ? fma(0.5 * rd[m], e, h) : h;
+          inf[m] = (__double2hiint(s) & 0x7FF00000) == 0x7FF00000;
+          if (inf[m]) ld[m] = 0.0;
         }
 #pragma unroll
         for (int i = m + 1; i < 4; ++i) {
@@ -346,13 +351,7 @@ __device__ __forceinline__ void small_panel4(const DevCtx& c, int front, double*
         double v = m < w ? A[r + (P + m) * n] : 0.0;
 #pragma unroll
         for (int l = 0; l < m; ++l) v -= lb[m][l] * t[l];
-        t[m] = r == P + m ? ld[m] : fp64_div(v, ld[m], rd[m]);
-      }
-      // (a failed pivot's row keeps the pivot 1)
-      if (r < P + w) {
-#pragma unroll
-        for (int m = 0; m < 4; ++m)
-          if (r == P + m && !(t[m] > 0.0)) t[m] = 1.0;
+        t[m] = r == P + m ? (inf[m] ? HUGE_VAL : ld[m]) : fp64_div(v, ld[m], rd[m]);
       }
     }
     __syncthreads();                     // the pivot block has been read
