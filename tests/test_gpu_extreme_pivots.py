@@ -5,6 +5,7 @@ import pytest
 
 from oracle import uhm_oracle as uo
 from tests.test_gpu_large_fronts import _matrix, _mesh, _solutions
+from tests.test_gpu_lu_scaling import _check_front
 from uhm_gb300 import api
 
 pytestmark = pytest.mark.gpu
@@ -34,3 +35,21 @@ def test_infinite_pivot_of_a_small_front(native_lib, ss, at):
     ref = np.zeros((n, 1))
     ref[keep] = np.linalg.solve(full[np.ix_(keep, keep)], b[keep])
     assert np.abs(x - ref).max() <= 12 * n * 2.0 ** -53 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("prec,unit,fs,ss", [("fp64", 513, 130, 140), ("fp32", 65, 130, 140), ("fp64", 513, 300, 2000)])
+@pytest.mark.parametrize("method", [uo.LU_NOPIV, uo.CHOL])
+def test_subnormal_pivots(native_lib, method, prec, unit, fs, ss):
+    """Unknowns in units of 2^-unit: their pivots are subnormal, their reciprocals beyond
+    the range, the multipliers near 2^unit.  Panels of a cluster and of many CTAs; the
+    tolerance of _check_front."""
+    if method == uo.CHOL and prec == "fp32":
+        pytest.skip("an FP32 Cholesky step takes reciprocal square roots, which do not overflow")
+    rng = np.random.default_rng(80)
+    d = np.ones(fs + ss)
+    d[[10, 63, 64, 70, fs - 1]] = 2.0 ** -unit
+    base = [_matrix(fs + ss, method == uo.CHOL, rng) for _ in range(2)]
+    mats = [d[:, None] * b * d[None, :] for b in base]
+    if prec == "fp32":
+        mats = [a.astype(np.float32).astype(np.float64) for a in mats]
+    _check_front(method, prec, fs, ss, mats, d, d)

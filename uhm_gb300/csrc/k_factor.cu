@@ -668,6 +668,7 @@ struct PdShared {
   double ds[64];             // D (rank 1: then D^{-1/2})
   double pv[4][4];           // rank 0
   double Z[64][65];          // rank 1
+  int sc[64];                // powers of two of a badly scaled block's rows and columns
   unsigned long long bar[16];        // rank 1: step q's column has arrived
 };
 
@@ -702,6 +703,26 @@ __global__ void __launch_bounds__(PD_THREADS) k_potrf_inv64(DevCtx c, const Item
                 : (r < kb && cc < kb)   ? c.a64[f.off + (k0 + r) + (int64_t)(k0 + cc) * n]
                                         : (r == cc ? 1.0 : 0.0);
     }
+  // Diagonal entries below 2^-895: reciprocals of their pivots may overflow where the
+  // entries of U are ordinary numbers.  The block is then factored with its rows and
+  // columns scaled to a diagonal near 1, the inverse's columns scaled back.
+  bool small = false;
+  if (threadIdx.x < kb) {
+    const double v = c.a64[f.off + (int64_t)(k0 + threadIdx.x) * (n + 1)];
+    const int e = XsType<double>::expo(v);
+    small = v > 0.0 && e < 128;
+    sh.sc[threadIdx.x] = v > 0.0 ? (1023 - e) / 2 : 0;
+  }
+  const bool scaled = __syncthreads_or(small);
+  if (scaled && rank == 0 && i >= 0) {
+#pragma unroll 1
+    for (int e = 0; e < 8; ++e)
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 2; ++v)
+          if (e == 2 * u + v && r0 + u < kb && c0 + v < kb) a[u][v] = scalbn(a[u][v], sh.sc[r0 + u] + sh.sc[c0 + v]);
+  }
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   auto update = [&](const double (*b)[64], const double (*w)[64]) {
 #pragma unroll
@@ -862,6 +883,10 @@ __global__ void __launch_bounds__(PD_THREADS) k_potrf_inv64(DevCtx c, const Item
     for (int e = threadIdx.x; e < 4096; e += PD_THREADS) {
       const int r = e & 63, cc = e >> 6;     // entry (r, cc)
       D[e] = cc <= r && r < kb ? sh.Z[r][cc] * sh.ds[r] : 0.0;
+    }
+    if (scaled) {
+      __syncthreads();
+      for (int e = threadIdx.x; e < 64 * kb; e += PD_THREADS) D[e] = scalbn(D[e], sh.sc[e >> 6]);
     }
   }
   // neither CTA leaves while the other may still write to it
@@ -1616,6 +1641,16 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
     if (akk == (T)0 || akk != akk) {
       if (q == 0 && tid == 0) set_status(c, it.front, akk != akk ? ST_NAN : ST_ZERO_PIVOT);
       akk = (T)1;
+    }
+    if (XsType<T>::field(akk) == 0) {
+      // a subnormal pivot: its reciprocal may overflow where the quotients are ordinary
+      // numbers, so it and the column are scaled up first
+      constexpr T UP = T(sizeof(T) == 8 ? 0x1p128 : 0x1p64);
+      __syncthreads();                         // every thread has read it
+      for (int r = tid; r < nr_my; r += NT) s_col[par * rmax + r] *= UP;
+      if (tid == 0) rc.diag[k] *= UP;
+      akk *= UP;
+      __syncthreads();
     }
     T rinv;
     if constexpr (sizeof(T) == 8) {            // a reciprocal costs every FP64 warp that takes it
