@@ -31,6 +31,11 @@ static constexpr int LU_GOAL_F64 = 64, LU_GOAL_F32 = 192;
 // rows (four fronts at once: more); FP64, 16 CTAs, 187 at 96 rows each, 205 at 128, 225 to
 // 264 from 130 to 208, against 200 for the whole GPU from 2,100 to 3,300 rows and 218 at 6,938
 static constexpr int LU_CLUSTER_ROWS_F64 = 128, LU_CLUSTER_ROWS_F32 = 384;
+// 128-byte rows of operand slices held at a time (1 GiB; a single front may need more).
+// Slices are up to 1.5 times (LU 3 times) the panels of fronts of 180 to 600 rows, so a
+// wide level of them goes in batches.  One batch fills the GPU: 200 FP64 fronts of 1,000
+// rows, 1,300 of 200; the largest level of the meshes measured takes 680 MB (512 fronts).
+static constexpr int64_t XS_BATCH_ROWS = (int64_t)1 << 23;
 static constexpr int TR = TILE_UPDATE_ROWS, TC = TILE_UPDATE_COLS;   // k_tile_update
 
 #define CK(x)                                                                          \
@@ -706,37 +711,42 @@ void Engine::build_plan(int method) {
       dn += (method == UHM_CHOL ? 1 : 2) * (int64_t)nfb * NB * NB;   // LU: of L's blocks, then of U's
     }
   }
-  // operand slices of the current panel of every front with sliced updates;
-  // the levels run one after the other and share the workspace
+  // operand slices of the current panel of every front with sliced updates; the levels
+  // and types run one after the other and share the workspace, and so do batches of
+  // fronts of one level and type beyond XS_BATCH_ROWS
   xs_rows = xs_exps = xs_near_n = 0;
-  for (auto& lv : levels) {
-    int64_t rows = 0, exps = 0;
-    for (int s : lv) {
-      HostFront& f = fronts[s];
-      if (!f.xs) continue;
-      const int64_t r = (int64_t)(f.prec == PREC_FP64 ? XS_S64 : XS_S32) *
-                        ((std::min(f.fs, XS_NBO) + 63) / 64) * f.n;
-      f.xs_row0 = rows;
-      rows += r;
-      f.xs_row0b = method == UHM_CHOL ? f.xs_row0 : rows;
-      if (method != UHM_CHOL) rows += r;
-      f.xs_exp0 = exps;
-      exps += (method == UHM_CHOL ? 1 : 2) * (int64_t)f.n;
-      // the 64-column steps of the next outer panel run beside the update that
-      // reads these: slices of their own
-      const int64_t ri = (int64_t)(f.prec == PREC_FP64 ? XS_S64 : XS_S32) * f.n;
-      f.xs_row0i = rows;
-      rows += ri;
-      f.xs_row0bi = method == UHM_CHOL ? f.xs_row0i : rows;
-      if (method != UHM_CHOL) rows += ri;
-      f.xs_exp0i = exps;
-      exps += (method == UHM_CHOL ? 1 : 2) * (int64_t)f.n;
-      f.xs_near0 = xs_near_n;
-      if (method != UHM_CHOL) xs_near_n += (f.fs + XS_NBO - 1) / XS_NBO * (XS_NBO / 32);
+  const int sides = method == UHM_CHOL ? 1 : 2;      // LU: U12^T beside L21
+  for (auto& lv : levels)
+    for (int dt = 0; dt < 2; ++dt) {
+      int64_t rows = 0, exps = 0;
+      int batch = 0;
+      for (int s : lv) {
+        HostFront& f = fronts[s];
+        if (!f.xs || (f.prec == PREC_FP64 ? F64 : F32) != dt) continue;
+        // of an outer panel, and of a 64-column step: the steps of the next outer panel
+        // run beside the update that reads the former
+        const int64_t ri = (int64_t)(dt == F64 ? XS_S64 : XS_S32) * f.n;
+        const int64_t r = ri * ((std::min(f.fs, XS_NBO) + 63) / 64);
+        if (rows > 0 && rows + sides * (r + ri) > XS_BATCH_ROWS) {
+          ++batch;
+          rows = exps = 0;
+        }
+        f.xs_batch = batch;
+        f.xs_row0 = rows;
+        f.xs_row0b = rows + (sides - 1) * r;
+        rows += sides * r;
+        f.xs_row0i = rows;
+        f.xs_row0bi = rows + (sides - 1) * ri;
+        rows += sides * ri;
+        f.xs_exp0 = exps;
+        f.xs_exp0i = exps + sides * (int64_t)f.n;
+        exps += 2 * sides * (int64_t)f.n;
+        f.xs_near0 = xs_near_n;
+        if (method != UHM_CHOL) xs_near_n += (f.fs + XS_NBO - 1) / XS_NBO * (XS_NBO / 32);
+        xs_rows = std::max(xs_rows, rows);
+        xs_exps = std::max(xs_exps, exps);
+      }
     }
-    xs_rows = std::max(xs_rows, rows);
-    xs_exps = std::max(xs_exps, exps);
-  }
   if (xs_rows + XS_SPARE_ROWS > ((int64_t)1 << 31) - 1) fail("operand workspace beyond the tensor map's row range", 4);
   // assembly sources in summation order: the element matrix (copy_in), then
   // the children in child order (op_merge, UHM/src/operation/element.cxx:150-162)
@@ -1125,6 +1135,11 @@ void Engine::build_programs(int method) {
     return best;
   };
   const int small_max[2] = {tune.small_max_f64, tune.small_max_f32};
+  auto max_fs = [&](const std::vector<int>& v) {
+    int m = 0;
+    for (int s : v) m = std::max(m, fronts[s].fs);
+    return m;
+  };
   for (auto& lv : levels) {
     for (int dt = 0; dt < 2; ++dt) {
       std::vector<int> fl;
@@ -1186,10 +1201,15 @@ void Engine::build_programs(int method) {
       // columns at a time, every update by sliced tensor-core products
       // (k_xs.cu): the panel's own columns after each step (K = 64), the
       // trailing block once per outer panel (K = XS_NBO)
-      int maxfs = 0;
-      for (int s : large) maxfs = std::max(maxfs, fronts[s].fs);
+      // (a batch of them after the other: they share a workspace)
       int side = 0;                  // SMs of the previous panel's concurrent update
-      for (int K0 = 0; K0 < maxfs; K0 += XS_NBO) {
+      std::vector<std::vector<int>> batches;
+      for (int s : large) {
+        if ((int)batches.size() <= fronts[s].xs_batch) batches.resize(fronts[s].xs_batch + 1);
+        batches[fronts[s].xs_batch].push_back(s);
+      }
+      for (const std::vector<int>& large : batches)
+      for (int K0 = 0, maxfs = max_fs(large); K0 < maxfs; K0 += XS_NBO) {
         const int k_end = std::min(K0 + XS_NBO, maxfs);
         for (int k0 = K0; k0 < k_end; k0 += NB) {
           std::vector<Item> p_items, t_items, pk, ut;

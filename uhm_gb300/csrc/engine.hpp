@@ -37,6 +37,7 @@ struct HostFront {
   int64_t xs_row0 = 0, xs_row0b = 0, xs_exp0 = 0;      // its slices and row exponents in the level's workspace
   int64_t xs_row0i = 0, xs_row0bi = 0, xs_exp0i = 0;   // the same of a 64-column step
   int64_t xs_near0 = 0;            // LU: its words of XsCtx::near
+  int xs_batch = 0;                // fronts of a level and type that share the workspace at a time
   int64_t ws_off = 0, ws_stride = 0;
   int64_t ws2_row0 = 0;            // first 128-byte row of its parts in the chunk-major workspace
   int64_t ws2b_row0 = 0;           // ... of the panel rows before their TRSM (tc_panel 256)
@@ -306,8 +307,8 @@ class Engine {
   int64_t ws2_rows = 0;              // its size in rows of 64 BF16
   int64_t* d_ws2_row0 = nullptr;     // per front: first row of its parts
   CUtensorMap ws2_map;
-  void* d_xs = nullptr;              // operand slices of the current level's sliced updates
-  int64_t xs_rows = 0, xs_exps = 0;  // its rows of 64 BF16 and row exponents (the largest level)
+  void* d_xs = nullptr;              // operand slices of the current batch's sliced updates
+  int64_t xs_rows = 0, xs_exps = 0;  // its rows of 64 BF16 and row exponents (the largest batch)
   int64_t xs_near_n = 0;             // LU: words of XsCtx::near per use and side
   void* d_xs_stat = nullptr;         // LU: XsCtx::kmax, then XsCtx::near (cleared per factorisation)
   size_t xs_stat_bytes = 0;
