@@ -2869,8 +2869,7 @@ int Engine::autotune(int method, int reps) {
     for (const auto* ops : {&fac_ops, &fwd_ops, &bwd_ops})
       for (const Op& o : *ops) {
         sig.push_back(o.kind);
-        sig.push_back(o.n_items);
-        sig.push_back(o.dtype);
+        for (int64_t v : {o.n_items, o.dtype, o.nb, o.param, o.q0, o.aux, o.cap, o.strm}) sig.push_back(v);
       }
     return sig;
   };
@@ -2895,10 +2894,9 @@ int Engine::autotune(int method, int reps) {
   if (!lu) knobs.push_back({&tune.fuse_potrf_trsm, {0, 1, 2, 4}});
   if (!lu) knobs.push_back({&tune.tc_panel, {0, 256, 512}});
   if (!lu) knobs.push_back({&tune.solve_rows, {64, 256}});
-  if (!lu) knobs.push_back({&tune.lookahead, {0, 1}});
+  knobs.push_back({&tune.lookahead, {0, 1}});
   if (!lu) knobs.push_back({&tune.solve_chain, {0, 1}});
   if (!lu) knobs.push_back({&tune.tc_nbo, {128, 256, 512}});
-  if (lu) knobs.push_back({&tune.gc_min_rows, {256, 512, 1024, 2048, 1 << 30}});
   int timed = 0;
   prec_dirty = true;
   double best_t = time_now();

@@ -106,7 +106,11 @@ struct Tunables {
   int small_max_f64 = 160;   // whole front in shared memory up to this n (FP64; kernel limit 160)
   int small_max_f32 = 224;   // same for FP32 fronts (kernel limit 224)
   int tc_min_n = 512;        // BF16-split Cholesky fronts use the tensor cores from this n
-  int gc_min_rows = 512;     // LU panels with this many rows below the diagonal use many CTAs
+  int gc_min_rows = 512;     // LU panels: clusters of up to 16 CTAs, and the whole GPU from this many
+                             // rows (of those that leave a cluster's CTA more than 128 FP64 or 384
+                             // FP32 rows).  Above 512: panels of fewer rows than this, but more than
+                             // one CTA's shared memory holds (384, 768), take one CTA in global
+                             // memory (not tried by autotune)
   int fuse_potrf_trsm = 2;   // Cholesky step: diagonal block + panel TRSM in one launch when it
                              // has at most this many CTAs per SM (0: never)
   int tc_nbo = 256;          // outer panel width of tensor-core fronts (128, 256 or 512)
