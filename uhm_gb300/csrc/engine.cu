@@ -887,10 +887,9 @@ void Engine::build_programs(int method) {
     ops.push_back(op);
   };
   // The Schur pass of the tensor-core Cholesky fronts of a level, ABR -=
-  // ABL ABL^T with K = fs: 128 x 256 tiles of the lower triangle, launched in
-  // clusters of two whose CTAs take the two row tiles of one column pair (a
-  // filler where a column has an odd count) and share the column's B
-  // operand; the last partial round of pairs is spread over half tiles.
+  // ABL ABL^T with K = fs: 128 x 256 tiles of the lower triangle, column of tiles by
+  // column of tiles (the CTAs of a round meet at the same B rows in L2); the last
+  // partial round is spread over half tiles.
   auto push_schur = [&](std::vector<Op>& ops, const std::vector<int>& tccf) {
     const int TM = TCC_TILE_M, TN = TCC_TILE_N;
     std::vector<Item> tt;
@@ -899,44 +898,21 @@ void Engine::build_programs(int method) {
       const HostFront& f = fronts[sl];
       if (f.ss <= 0) continue;
       const int nch = (f.fs + 63) / 64;
-      for (int c0 = f.fs; c0 < f.n; c0 += TN) {
-        std::vector<int> rows;
+      for (int c0 = f.fs; c0 < f.n; c0 += TN)
         for (int r0 = f.fs; r0 < f.n; r0 += TM)
-          if (c0 <= r0 + TM - 1) rows.push_back(r0);
-        for (size_t k = 0; k < rows.size(); k += 2) {
-          const Item a{sl, rows[k], c0, 0 | (nch << 16)};
-          tt.push_back(a);
-          if (k + 1 < rows.size()) {
-            tt.push_back(Item{sl, rows[k + 1], c0, a.c});
-          } else {
-            Item d = a;
-            d.c = (int)((unsigned)d.c | (1u << 29));
-            tt.push_back(d);
-          }
-        }
-      }
+          if (c0 <= r0 + TM - 1) tt.push_back(Item{sl, r0, c0, 0 | (nch << 16)});
       ft += get_flop_syrk(0, f.fs, f.ss);
       bt += 8.0 * 0.5 * (double)f.ss * (f.ss + 1) + 2.0 * 2.0 * f.ss * 64.0 * nch;
     }
     if (tt.empty()) return;
-    // the last partial round of pairs (one pair per cluster of two SMs) as half-tile pairs
-    const int nclu = std::max(1, n_sm / 2), npair = (int)tt.size() / 2, rem = npair % nclu;
-    if (npair >= nclu && rem > 0 && 2 * rem <= nclu) {
-      std::vector<Item> out(tt.begin(), tt.end() - 2 * rem);
-      for (int k = npair - rem; k < npair; ++k)
-        for (unsigned h = 1; h <= 2; ++h)
-          for (int m = 0; m < 2; ++m) {
-            Item x = tt[2 * k + m];
-            x.c = (int)((unsigned)x.c | (h << 30));
-            out.push_back(x);
-          }
-      tt.swap(out);
+    const int rem = (int)tt.size() % n_sm;
+    if ((int)tt.size() >= n_sm && rem > 0 && 2 * rem <= n_sm) {
+      std::vector<Item> last(tt.end() - rem, tt.end());
+      split_halves(last);
+      tt.resize(tt.size() - rem);
+      tt.insert(tt.end(), last.begin(), last.end());
     }
-    Op op{OP_TC_CHOL_SCHUR, F32, 0, 0, add_items(tt), (int)tt.size()};
-    op.flops = ft;
-    op.bytes = bt;
-    op.aux = 1;             // paired launch
-    ops.push_back(op);
+    push(ops, OP_TC_CHOL_SCHUR, F32, 0, 0, tt, ft, bt);
   };
   // one Cholesky step's diagonal block + panel TRSM: fused (every CTA of the
   // TRSM factors the block, the first writes its inverse) or two launches
@@ -2218,7 +2194,7 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
       case OP_TC_CHOL_TRAIL:
       case OP_TC_CHOL_SCHUR:
         launch_tc_chol(ctx, ws2_map, d_ws2_row0, it, op.n_items, d_err, st, 0, nullptr, nullptr, nullptr,
-                       profiling ? 0 : op.q0, op.kind == OP_TC_CHOL_SCHUR ? op.aux : 0);
+                       profiling ? 0 : op.q0);
         break;
       case OP_CHOL_DIAG:
         launch_chol_diag(ctx, it, op.n_items, d_pflags + op.param, d_hand + CD_HAND_HEAD,

@@ -683,8 +683,6 @@ constexpr int TCC_ERR = 6;
 // 128 x 256 tile, 1 / 2 its first / second 128 columns), so that the last
 // round of a launch can be spread over twice as many CTAs
 __device__ __forceinline__ int tcc_half(const Item& it) { return (int)(((unsigned)it.c >> 30) & 3u); }
-// a filler item of a pair (bit 29): computed with its partner's rows, stored nowhere
-__device__ __forceinline__ bool tcc_dummy(const Item& it) { return ((unsigned)it.c >> 29) & 1u; }
 
 // Two modes.
 // mode 0 (update): item front, a = first row r0, b = first column c0,
@@ -693,13 +691,6 @@ __device__ __forceinline__ bool tcc_dummy(const Item& it) { return ((unsigned)it
 // stop at fs for tiles of the factor block (c0 < fs) and at n for tiles of
 // ABR (c0 >= fs); only entries with col <= row are stored (Cholesky keeps
 // the lower triangle).
-// Paired (pair = 1, mode 0, launched in clusters of 2): items 2p and 2p + 1
-// share front, columns and chunks (two row tiles of one column of tiles, or
-// a tile and a filler), and CTA rank r of a cluster takes the items with
-// index = r mod 2.  Each CTA loads its own A and half of the shared B, sent
-// to both CTAs of the cluster (TMA multicast); a stage is reused once both
-// CTAs' MMAs have released it (the MMA completion arrives on the empty
-// barrier of both).  Operand traffic per tile falls from 1.5 to 1 KB per K.
 // mode 1 (TRSM below a panel's diagonal block): item front, a = r0, b = c0
 // (column within the panel), c = K0; X = A Linv^T with A the panel's rows
 // r0.. packed at row0b and B the packed rows c0.. of Linv (linv_row0), K =
@@ -708,7 +699,7 @@ __device__ __forceinline__ bool tcc_dummy(const Item& it) { return ((unsigned)it
 __global__ void __launch_bounds__(TCC_THREADS, 1)
 k_tc_chol(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __restrict__ ws_row0,
           const Item* __restrict__ items, int n_items, int* err, int mode, const int64_t* __restrict__ row0b,
-          const int64_t* __restrict__ linv_row0, __nv_bfloat16* __restrict__ ws, int pair) {
+          const int64_t* __restrict__ linv_row0, __nv_bfloat16* __restrict__ ws) {
   extern __shared__ __align__(1024) uint8_t tcc_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tcc_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TCC_STAGES * TCC_STAGE);
@@ -723,7 +714,7 @@ k_tc_chol(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __
   if (threadIdx.x == 0) {
     for (int s = 0; s < TCC_STAGES; ++s) {
       mbar_init(smem_u32(&bars[s]), 1);
-      mbar_init(smem_u32(&bars[TCC_STAGES + s]), pair ? 2 : 1);
+      mbar_init(smem_u32(&bars[TCC_STAGES + s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&acc_full[b]), 1);
@@ -740,11 +731,8 @@ k_tc_chol(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __
   }
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  // the peer's barriers are initialised before any multicast reaches them
-  if (pair) cluster_sync_all();
   const uint32_t tmem = *s_tmem;
   const uint32_t lim = g_wait_limit;
-  const uint32_t rank = pair ? cluster_rank() : 0;
 
   if (warp == 8) {
     if (lane == 0) {
@@ -796,21 +784,10 @@ k_tc_chol(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __
           const int64_t da = (int64_t)(kc - kc0) * ya_step, db = (int64_t)(kc - kc0) * yb_step;
           tma_load_2d(st + 0 * TCC_BOX, &wsmap, xq, (int)(ya_h + da), fb);
           tma_load_2d(st + 1 * TCC_BOX, &wsmap, xq, (int)(ya_l + da), fb);
-          if (!pair) {
-            tma_load_2d(st + 2 * TCC_BOX, &wsmap, xq, (int)(yb_h + db), fb);
-            if (!hsel) tma_load_2d(st + 3 * TCC_BOX, &wsmap, xq, (int)(yb_h + db + 128), fb);
-            tma_load_2d(st + 4 * TCC_BOX, &wsmap, xq, (int)(yb_l + db), fb);
-            if (!hsel) tma_load_2d(st + 5 * TCC_BOX, &wsmap, xq, (int)(yb_l + db + 128), fb);
-          } else if (hsel) {
-            // half tiles: rank 0 sends the hi box, rank 1 the lo box
-            if (rank == 0) tma_load_2d_mc(st + 2 * TCC_BOX, &wsmap, xq, (int)(yb_h + db), fb, 3);
-            else tma_load_2d_mc(st + 4 * TCC_BOX, &wsmap, xq, (int)(yb_l + db), fb, 3);
-          } else {
-            // rank r sends rows 128 r .. 128 r + 127 of both B parts
-            const int off = (int)rank * 128;
-            tma_load_2d_mc(st + (2 + rank) * TCC_BOX, &wsmap, xq, (int)(yb_h + db + off), fb, 3);
-            tma_load_2d_mc(st + (4 + rank) * TCC_BOX, &wsmap, xq, (int)(yb_l + db + off), fb, 3);
-          }
+          tma_load_2d(st + 2 * TCC_BOX, &wsmap, xq, (int)(yb_h + db), fb);
+          if (!hsel) tma_load_2d(st + 3 * TCC_BOX, &wsmap, xq, (int)(yb_h + db + 128), fb);
+          tma_load_2d(st + 4 * TCC_BOX, &wsmap, xq, (int)(yb_l + db), fb);
+          if (!hsel) tma_load_2d(st + 5 * TCC_BOX, &wsmap, xq, (int)(yb_l + db + 128), fb);
         }
       }
       // the last loads issued (one per stage at most) land before the CTA exits
@@ -856,8 +833,7 @@ k_tc_chol(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __
           for (int k = 0; k < 2; ++k) umma_bf16(acc, sdesc_sw64(ah + k * 32), sdesc_sw64(bl + k * 32), idesc, 1u);
 #pragma unroll
           for (int k = 0; k < 2; ++k) umma_bf16(acc, sdesc_sw64(al + k * 32), sdesc_sw64(bh + k * 32), idesc, 1u);
-          if (pair) umma_commit_mc(smem_u32(&bars[TCC_STAGES + s]), 3);
-          else umma_commit(smem_u32(&bars[TCC_STAGES + s]));
+          umma_commit(smem_u32(&bars[TCC_STAGES + s]));
         }
         if (live) umma_commit(smem_u32(&acc_full[b]));
       }
@@ -927,7 +903,7 @@ k_tc_chol(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __
         TC_LD32(tmem + ((uint32_t)(quarter * 32) << 16) + b * TCC_BN + half * 128 + cc * 32, v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         const int cb = cbase + half * 128 + cc * 32;
-        const bool rok = row < n && !*s_abort && !tcc_dummy(it);
+        const bool rok = row < n && !*s_abort;
         float cv[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
@@ -946,8 +922,6 @@ k_tc_chol(DevCtx c, const __grid_constant__ CUtensorMap wsmap, const int64_t* __
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  // neither CTA of a pair leaves while the other may still send it operands
-  if (pair) cluster_sync_all();
   if (warp == 0) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TCC_BN));
   }
@@ -1016,7 +990,7 @@ void launch_chol_pack(const DevCtx& c, const Item* items, int n_items, void* ws,
 
 void launch_tc_chol(const DevCtx& c, const CUtensorMap& map, const int64_t* ws_row0, const Item* items, int n_items,
                     int* err, cudaStream_t s, int mode, const int64_t* row0b, const int64_t* linv_row0, void* ws,
-                    int reserve, int pair) {
+                    int reserve) {
   if (!n_items) return;
   static int n_sm = 0;
   if (!n_sm) {
@@ -1027,29 +1001,9 @@ void launch_tc_chol(const DevCtx& c, const CUtensorMap& map, const int64_t* ws_r
   }
   cudaFuncSetAttribute(k_tc_chol, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TCC_SMEM);
   const int slots = n_sm - reserve > 1 ? n_sm - reserve : 1;
-  if (pair) {
-    // clusters of two CTAs (items come in pairs, n_items even)
-    const int clusters = n_items / 2 < slots / 2 ? n_items / 2 : slots / 2;
-    if (clusters < 1) return;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * clusters);
-    cfg.blockDim = dim3(TCC_THREADS);
-    cfg.dynamicSmemBytes = TCC_SMEM;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_tc_chol, c, map, ws_row0, items, n_items, err, mode, row0b, linv_row0,
-                       (__nv_bfloat16*)ws, 1);
-    return;
-  }
   const int grid = n_items < slots ? n_items : slots;
   k_tc_chol<<<grid, TCC_THREADS, TCC_SMEM, s>>>(c, map, ws_row0, items, n_items, err, mode, row0b, linv_row0,
-                                                (__nv_bfloat16*)ws, 0);
+                                                (__nv_bfloat16*)ws);
 }
 
 int chol_panel_max_w1() { return 512; }

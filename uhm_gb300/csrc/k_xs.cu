@@ -474,8 +474,7 @@ __device__ __noinline__ void xs_plain(T* G, int n, int K0, int W, int row, int r
 // (umma_bf16_w) 30, with slice p of A kept in the collector buffer for its products
 // (umma_bf16_wa) 27.5; FP32 tiles 13.1, then 11.9.  The tensor pipe alone needs 21 (6):
 // a 128 x 128 x 16 product reads 8 KB at 128 B a clock, as long as it takes, and the
-// loads (48 slots; 16) write beside it.  (Half of B from each of two CTAs by
-// multicast changed nothing: 65 B a clock and SM from L2 are there, 27 are used.)
+// loads (48 slots; 16) write beside it. 
 // FP32 tiles load C while their products run and read the four diagonals eight columns
 // at a time.  BN = 64: tiles of half the width
 // for launches with fewer 128 x 128 tiles than SMs, where a tile's own time
