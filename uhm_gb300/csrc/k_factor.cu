@@ -573,15 +573,15 @@ void launch_small_factor(const DevCtx& c, const Item* items, int n_items, int dt
 // X are independent, so rows go through shared memory per warp).  One block
 // barrier per phase, 16 in all.  A warp does only the factor work that
 // reaches its columns and only the inverse work whose rows are nonzero in
-// them.  Blocks narrower than 64 are padded with the identity.  FP32 pivots
-// use rsqrt (the factor is refined in FP64 by the mixed path); FP64 uses sqrt
-// and a divide.  Measured alternatives: one column per phase (64 barriers)
+// them.  Blocks narrower than 64 are padded with the identity.  Pivots
+// use rsqrt (the factor is refined in FP64 by the mixed path; FP64 blocks:
+// k_potrf_inv64).  Measured alternatives: one column per phase (64 barriers)
 // took 2x as long; a fully unrolled left-looking version (one row per
 // thread, ~100 KB of straight-line code) was bound by instruction fetch;
 // hand-offs between warps on mbarriers or shared flags instead of the block
 // barrier were slower (their wake-up latency).
-template <typename T>
 __global__ void __launch_bounds__(256) k_potrf_diag(DevCtx c, const Item* __restrict__ items, int nb) {
+  using T = float;
   __shared__ __align__(16) PotrfShared<T> sh;
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(256) k_potrf_diag(DevCtx c, const Item* __rest
   // L is written over the block in place: only this CTA reads it
   potrf_block<T>(G, n, kb, sh, x, bad, G);
   if (bad && threadIdx.x == 0) set_status(c, it.front, ST_NOT_SPD);
-  T* Dinv = (sizeof(T) == 8 ? (T*)c.dinv64 : (T*)c.dinv32);
+  T* Dinv = c.dinv32;
   if (nb == 64 && Dinv) potrf_store_inverse<T>(kb, x, Dinv + f.dinv_off + (int64_t)(k0 / 64) * 4096);
 }
 
@@ -613,7 +613,7 @@ __device__ __forceinline__ double fp64_rcp(double v) {
   return fma(x, fma(r, r, r), x);
 }
 
-// The same for FP64 fronts: only the inverse is formed (the solves and the
+// The diagonal block of FP64 fronts: only the inverse is formed (the solves and the
 // TRSM use nothing else), and no multiply-add is spent on zeros.  GB300 does
 // about 2 FP64 multiply-adds per clock per SM, so a warp instruction costs its
 // scheduler ~64 clocks whatever its lanes do: the block is bound by their
@@ -633,7 +633,7 @@ __device__ __forceinline__ double fp64_rcp(double v) {
 // which the solvers apply themselves, so that pivots and bulk updates overlap; they
 // hand over on named barriers.
 // Measured on GB300: 294 us per block in the tile-per-thread form
-// (k_potrf_diag), which updates the full squares; one CTA for both 67 with the
+// (k_potrf_diag's), which updates the full squares; one CTA for both 67 with the
 // steps in turn, 60 with the solvers ahead, 58 without square roots; 54 so.
 constexpr int PD_WARPS = 12, PD_THREADS = 32 * PD_WARPS;
 // role of each warp, by rank: tile group 0 .. 9 ((I, J), I >= J, by J), 16 / 17
@@ -918,7 +918,7 @@ void launch_potrf_diag(const DevCtx& c, const Item* items, int n_items, int dtyp
   if (dtype == F64)
     launch_potrf_inv64(c, items, n_items, s);
   else
-    k_potrf_diag<float><<<n_items, 256, 0, s>>>(c, items, nb);
+    k_potrf_diag<<<n_items, 256, 0, s>>>(c, items, nb);
 }
 
 constexpr int TRSM_RB = 64;   // rows per panel-TRSM block
@@ -1005,8 +1005,8 @@ void launch_trsm_panel(const DevCtx& c, const Item* items, int n_items, int dtyp
 // more a step).
 constexpr int PT_LD = 68;   // row length of the transposed inverse in shared memory (16-byte rows)
 
-template <typename T>
 __global__ void __launch_bounds__(256) k_potrf_trsm(DevCtx c, const Item* __restrict__ items, XsCtx xs, int slices) {
+  using T = float;
   __shared__ int s_f[4][64];
   extern __shared__ __align__(16) unsigned char pt_smem[];
   PotrfShared<T>& sh = *reinterpret_cast<PotrfShared<T>*>(pt_smem);
@@ -1025,8 +1025,7 @@ __global__ void __launch_bounds__(256) k_potrf_trsm(DevCtx c, const Item* __rest
   const int nrb = it.c >> 1;
   if (writer) {
     if (bad && tid == 0) set_status(c, it.front, ST_NOT_SPD);
-    T* Dinv = (sizeof(T) == 8 ? (T*)c.dinv64 : (T*)c.dinv32);
-    potrf_store_inverse<T>(kb, x, Dinv + f.dinv_off + (int64_t)(k0 / 64) * 4096);
+    potrf_store_inverse<T>(kb, x, c.dinv32 + f.dinv_off + (int64_t)(k0 / 64) * 4096);
   }
   if (it.b >= n || nrb == 0) return;
   // L^{-1} transposed into Lt (Lt[t * PT_LD + j] = Linv[j][t]); the panel
@@ -1085,10 +1084,10 @@ __global__ void __launch_bounds__(256) k_potrf_trsm(DevCtx c, const Item* __rest
 void launch_potrf_trsm(const DevCtx& c, const Item* items, int n_items, int dtype, const XsCtx& x, int slices,
                        cudaStream_t s) {
   if (!n_items) return;
-  if (dtype == F64) throw std::invalid_argument("potrf_trsm: FP64 fronts take potrf_diag and trsm_panel");
+  if (dtype == F64) throw std::invalid_argument("potrf_trsm: FP64 fronts take potrf_diag and xs_trsm");
   const size_t sm = ((sizeof(PotrfShared<float>) + 15) / 16) * 16 + sizeof(float) * 64 * PT_LD;
-  cudaFuncSetAttribute(k_potrf_trsm<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_potrf_trsm<float><<<n_items, 256, sm, s>>>(c, items, x, slices);
+  cudaFuncSetAttribute(k_potrf_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_potrf_trsm<<<n_items, 256, sm, s>>>(c, items, x, slices);
 }
 
 // FP32 update of one 128 x 64 tile of the front by a panel of kb <= 64 columns:

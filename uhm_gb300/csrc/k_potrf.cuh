@@ -8,14 +8,9 @@
 
 namespace uhm_gpu {
 
-template <typename T> __device__ __forceinline__ void pivot_root(T s, T& d, T& rd);
-template <> __device__ __forceinline__ void pivot_root<float>(float s, float& d, float& rd) {
+__device__ __forceinline__ void pivot_root(float s, float& d, float& rd) {
   rd = rsqrtf(s);
   d = s * rd;
-}
-template <> __device__ __forceinline__ void pivot_root<double>(double s, double& d, double& rd) {
-  d = sqrt(s);
-  rd = 1.0 / d;
 }
 
 template <typename T> struct Vec4;
@@ -108,7 +103,7 @@ __device__ __forceinline__ void potrf_block(const T* __restrict__ G, int n, int 
       for (int m = 0; m < j; ++m) s -= lb[j][m] * lb[j][m];
       if (!(s > T(0))) { bad = true; s = T(1); }
       T d;
-      pivot_root<T>(s, d, rd[j]);
+      pivot_root(s, d, rd[j]);
       lb[j][j] = d;
 #pragma unroll
       for (int i = j + 1; i < 4; ++i) {
@@ -272,7 +267,7 @@ __device__ __forceinline__ void la_pivot(PotrfLaShared<T>& sh, int q1, const T (
     for (int m = 0; m < j; ++m) s -= lb[j][m] * lb[j][m];
     if (!(s > T(0))) { bad = true; s = T(1); }
     T d;
-    pivot_root<T>(s, d, rd[j]);
+    pivot_root(s, d, rd[j]);
     lb[j][j] = d;
 #pragma unroll
     for (int i = j + 1; i < 4; ++i) {

@@ -322,8 +322,9 @@ __device__ __forceinline__ void xs_add(long long& a, int i) {
 
 // FP32 tiles: conversions to integers run at 16 per clock and SM, additions at 128:
 // the sum of an integer below 2^22 and 1.5 2^23 holds it in its low bits, as
-// XS_MAGIC + v.  A diagonal's sums can reach 1.75 2^24 (256 products of 8-bit
-// digits); then, a warp's vote, they are converted.  (FP64 tiles have no
+// XS_MAGIC + v.  The sums of diagonals 0 .. 3 reach 0.75 2^24 (256 times two products of
+// two 8-bit digits and two with a leading one of at most 64); beyond 2^22, a warp's
+// vote, they are converted.  (FP64 tiles have no
 // registers left for it.)
 constexpr uint32_t XS_MAGIC = 0x4B400000u;
 __device__ __forceinline__ void xs_ints(uint32_t taddr, uint32_t (&v)[4][8]) {
@@ -483,6 +484,8 @@ __device__ __noinline__ void xs_plain(T* G, int n, int K0, int W, int row, int r
 // reads of the 128 x 128 products; a tile of a small launch by its epilogue.
 // Measured on GB300 for up to 80 tiles
 // of K = 64 (256): 29 (60) us with whole tiles, 18 (31) with these.
+// Registers: 18 warps are allotted as 20, which leaves 96 a thread; the compiler spills up to 260
+// bytes of <double, 128>, 72 of <double, 64> and 88 of the FP32 forms, all of epilogue warps.
 template <typename T, int BN, bool LOWER>
 __global__ void __launch_bounds__(XS_THREADS, 1)
 k_xs_update(DevCtx c, XsCtx x, const __grid_constant__ XsMaps maps, const Item* __restrict__ items, int n_items,
