@@ -379,7 +379,7 @@ class Mesh:
                 "laswp", "potrf_trsm", "assemble_scatter", "tc_gemm_bf16", "chol_panel", "tc_chol_trail",
                 "tc_chol_schur", "clear_flags", "chol_diag", "chol_pack", "tc_chol_trsm", "event_record",
                 "event_wait", "fwd_chain", "bwd_chain", "xs_pack", "xs_update", "lu_dinv",
-                "xs_clear"]
+                "xs_clear", "xs_scale"]
 
     def set_profiling(self, on=True):
         self._check(self.L.uhm_gpu_set_profiling(C.byref(self.h), int(on)))

@@ -991,12 +991,11 @@ void Engine::build_programs(int method) {
       for (int c0 = cb; c0 < lim && !own_swaps; c0 += 256) sw.push_back(Item{it.front, it.a, c0, ce});
     }
     double fl = fp;                  // the panel's operations, on its first launch
-    const int par = piv | (xs ? 2 : 0);
-    push(fac_ops, OP_GETRF, dt, NB, par, glob, glob.empty() ? 0.0 : fl);
+    push(fac_ops, OP_GETRF, dt, NB, piv, glob, glob.empty() ? 0.0 : fl);
     if (!glob.empty()) fl = 0;
     for (int lc = 0; lc < 5; ++lc) {
       if (cl[lc].empty()) continue;
-      Op op{OP_GETRF_COOP, dt, NB, par, add_items(cl[lc]), (int)cl[lc].size()};
+      Op op{OP_GETRF_COOP, dt, NB, piv, add_items(cl[lc]), (int)cl[lc].size()};
       op.q0 = -(1 << lc);            // CTAs per item (a cluster)
       op.aux = rmax_cl[lc];
       op.flops = fl;
@@ -1028,7 +1027,7 @@ void Engine::build_programs(int method) {
         rmax = std::max(rmax, (rows + P - 1) / P);
         b += P;
       }
-      Op op{OP_GETRF_COOP, dt, NB, par, add_items(g), (int)g.size()};
+      Op op{OP_GETRF_COOP, dt, NB, piv, add_items(g), (int)g.size()};
       op.q0 = b;
       op.aux = rmax;
       op.flops = fl;
@@ -1258,7 +1257,7 @@ void Engine::build_programs(int method) {
           push_xs(dt, NB, 2, pk, ut, fu, bu);
         }
         // the trailing block: the next panel's columns, the rest
-        std::vector<Item> pk, us, ut;
+        std::vector<Item> sc, pk, us, ut;
         double fs_ = 0, fu = 0, bs = 0, bu = 0;
         double t0 = 0, chain = 0;
         const bool d = dt == F64;
@@ -1270,6 +1269,7 @@ void Engine::build_programs(int method) {
           if (base >= f.n) continue;
           xs_pack_items(pk, XS_NBO, s, K0, base, f.n, 0);
           if (!chol) xs_pack_items(pk, XS_NBO, s, K0, base, f.n, 1);
+          for (int c0 = base; !chol && c0 < f.n; c0 += XS_SCALE_COLS) sc.push_back(Item{s, K0, c0, 0});
           fits = fits && (chol || f.n - base <= (d ? GC_RMAX_F64 : GC_RMAX_F32) * (n_sm / 2));
           const int B = std::min(base + XS_NBO, f.fs), cs = base + (B - base + XS_TILE - 1) / XS_TILE * XS_TILE;
           if (B > base) fs_ += xs_tiles(us, f, K0, KB, base, f.n, base, B, chol, bs);
@@ -1286,6 +1286,7 @@ void Engine::build_programs(int method) {
         }
         const double tile = d ? 30.0 : 13.0;       // a tile of K = 256 (SM us)
         side = fits ? split_sms(t0, chain + tile * us.size(), tile * ut.size()) : 0;
+        push(fac_ops, OP_XS_SCALE, dt, 0, 0, sc);
         if (side) {
           push(fac_ops, OP_XS_PACK, dt, XS_NBO, 0, pk);
           ev_op(OP_EV_RECORD, EV_PACKED, 0);
@@ -1647,7 +1648,7 @@ void Engine::build_programs(int method) {
     fac_ops.insert(fac_ops.begin(), op);
   }
   if (xs_near_n > 0) {
-    // what the sliced updates' balance and check gather starts at zero as well
+    // what the sliced updates' scaling and check gather starts at zero as well
     fac_ops.insert(fac_ops.begin(), Op{OP_XS_CLEAR, 0, 0, 0, 0, 0});
   }
   if (!fac_mask) {
@@ -1906,11 +1907,11 @@ void Engine::alloc_device(int method) {
     xs_ctx.exp0 = d + 2 * fronts.size();
     xs_ctx.exps = (int*)dmalloc(sizeof(int) * (size_t)xs_exps);
     if (xs_near_n > 0) {
-      const size_t km = sizeof(int) * 3 * (size_t)((piv_n + 7) / 8 * 8);
+      xs_ctx.scale_n = (piv_n + 7) / 8 * 8;
+      const size_t km = sizeof(int) * XS_USES * (size_t)xs_ctx.scale_n;
       xs_stat_bytes = km + sizeof(uint32_t) * 4 * XS_USES * (size_t)xs_near_n;
       d_xs_stat = dmalloc(xs_stat_bytes);
-      xs_ctx.kmax = (int*)d_xs_stat;
-      xs_ctx.kmax_n = (piv_n + 7) / 8 * 8;
+      xs_ctx.scale = (int*)d_xs_stat;
       xs_ctx.near = (uint32_t*)((char*)d_xs_stat + km);
       xs_ctx.near_n = xs_near_n;
       xs_ctx.near0 = d + 6 * fronts.size();
@@ -2167,17 +2168,18 @@ void Engine::launch_ops(const std::vector<Op>& ops, double* g_in, double* g_out,
         break;
       case OP_XS_CLEAR: CK(cudaMemsetAsync(d_xs_stat, 0, xs_stat_bytes, st)); break;
       case OP_GETRF:
-        launch_getrf_panel(ctx, it, op.n_items, op.dtype, op.nb, op.param & 1, op.param & 2 ? xs_ctx.kmax : nullptr, st);
+        launch_getrf_panel(ctx, it, op.n_items, op.dtype, op.nb, op.param, st);
         break;
       case OP_GETRF_COOP:
-        launch_getrf_smem(ctx, it, op.n_items, std::max(op.q0, 0), std::max(-op.q0, 0), op.dtype, op.nb, op.param & 1,
-                          op.aux, d_gc_xbuf, op.param & 2 ? xs_ctx.kmax : nullptr, d_err, st);
+        launch_getrf_smem(ctx, it, op.n_items, std::max(op.q0, 0), std::max(-op.q0, 0), op.dtype, op.nb, op.param,
+                          op.aux, d_gc_xbuf, d_err, st);
         break;
       case OP_LASWP: launch_laswp(ctx, it, op.n_items, op.dtype, op.nb, st); break;
       case OP_LUROW:
-        launch_lu_row_update(ctx, it, op.n_items, op.dtype, op.nb, 
-                             op.param ? xs_ctx.kmax + op.param * xs_ctx.kmax_n : nullptr, st);
+        launch_lu_row_update(ctx, it, op.n_items, op.dtype, op.nb,
+                             op.param ? xs_ctx.scale + op.param * xs_ctx.scale_n : nullptr, st);
         break;
+      case OP_XS_SCALE: launch_xs_scale(ctx, xs_ctx, it, op.n_items, op.dtype, st); break;
       case OP_GEMM: launch_gemm_update(ctx, it, op.n_items, op.dtype, op.nb, op.q0, op.aux, st); break;
       case OP_TC_GEMM:
         // A parts 0-1 (L21), B parts 2-3 (U12^T)

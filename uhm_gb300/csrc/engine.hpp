@@ -89,7 +89,7 @@ enum OpKind : int {
   OP_TC_PACK, OP_TC_SYRK, OP_FWD_FLAGS, OP_BWD_FLAGS, OP_GETRF_COOP,
   OP_LASWP, OP_POTRF_TRSM, OP_ASSEMBLE_SCATTER, OP_TC_GEMM, OP_CHOL_PANEL, OP_TC_CHOL_TRAIL,
   OP_TC_CHOL_SCHUR, OP_CLEAR_FLAGS, OP_CHOL_DIAG, OP_CHOL_PACK, OP_TC_CHOL_TRSM, OP_EV_RECORD, OP_EV_WAIT,
-  OP_FWD_CHAIN, OP_BWD_CHAIN, OP_XS_PACK, OP_XS_UPDATE, OP_LU_DINV, OP_XS_CLEAR, OP_KIND_END
+  OP_FWD_CHAIN, OP_BWD_CHAIN, OP_XS_PACK, OP_XS_UPDATE, OP_LU_DINV, OP_XS_CLEAR, OP_XS_SCALE, OP_KIND_END
 };
 static_assert(OP_KIND_END <= N_OP_KINDS, "profile arrays hold N_OP_KINDS op kinds");
 
@@ -314,7 +314,7 @@ class Engine {
   void* d_xs = nullptr;              // operand slices of the current batch's sliced updates
   int64_t xs_rows = 0, xs_exps = 0;  // its rows of 64 BF16 and row exponents (the largest batch)
   int64_t xs_near_n = 0;             // LU: words of XsCtx::near per use and side
-  void* d_xs_stat = nullptr;         // LU: XsCtx::kmax, then XsCtx::near (cleared per factorisation)
+  void* d_xs_stat = nullptr;         // LU: XsCtx::scale, then XsCtx::near (cleared per factorisation)
   size_t xs_stat_bytes = 0;
   uhm_gpu::XsCtx xs_ctx{}, xs_in{};  // of the outer panels' updates, of those inside a panel
   uhm_gpu::XsMaps xs_map;

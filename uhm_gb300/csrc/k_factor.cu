@@ -1211,7 +1211,7 @@ void launch_gemm_update(const DevCtx& c, const Item* items, int n_items, int dty
 // ---------------------------------------------------------------------------
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_getrf_panel(DevCtx c, const Item* __restrict__ items,
-                                                    int nb, int pivot, int* __restrict__ lmax) {
+                                                    int nb, int pivot) {
   __shared__ T s_v[NT / 32];
   __shared__ int s_i[NT / 32];
   const Item it = items[blockIdx.x];
@@ -1254,19 +1254,13 @@ __global__ void __launch_bounds__(NT) k_getrf_panel(DevCtx c, const Item* __rest
     }
     __syncthreads();
   }
-  for (int k = k0 + warp; lmax && k < k0 + kb; k += NW) {
-    int fm = 0;
-    for (int i = k0 + kb + lane; i < n; i += 32) fm = max(fm, XsType<T>::expo(G[i + (int64_t)k * n]));
-    fm = __reduce_max_sync(0xffffffffu, fm);
-    if (lane == 0) lmax[f.piv_off + k] = fm;
-  }
 }
 
 void launch_getrf_panel(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
-                        int pivot, int* lmax, cudaStream_t s) {
+                        int pivot, cudaStream_t s) {
   if (!n_items) return;
-  if (dtype == F64) k_getrf_panel<double, 512><<<n_items, 512, 0, s>>>(c, items, nb, pivot, lmax);
-  else k_getrf_panel<float, 512><<<n_items, 512, 0, s>>>(c, items, nb, pivot, lmax);
+  if (dtype == F64) k_getrf_panel<double, 512><<<n_items, 512, 0, s>>>(c, items, nb, pivot);
+  else k_getrf_panel<float, 512><<<n_items, 512, 0, s>>>(c, items, nb, pivot);
 }
 
 // ---------------------------------------------------------------------------
@@ -1287,9 +1281,7 @@ void launch_getrf_panel(const DevCtx& c, const Item* items, int n_items, int dty
 //      k + 1 first, whose candidates are found on the way.
 // The result is the reference's partial pivoting (FLA_LU_piv inside the
 // eliminated block) exactly; only the panel's own columns are swapped here,
-// the other columns of the front by k_laswp afterwards.  lmax (null: not wanted):
-// the largest exponent field of each column below the panel's diagonal block, what
-// the slices of the updates are balanced with (k_xs.cu).
+// the other columns of the front by k_laswp afterwards.
 //
 // Two ways to hand candidates and rows over:
 // CL: the item's CTAs are a cluster (1 .. 16 of them) and write into each
@@ -1455,26 +1447,23 @@ struct LuRecv {
   uint64_t cand[CL ? GC_CLUSTER : 1][2];        // key, row
 };
 
-// the largest exponent field of each of the columns of m rows of a chunk, into out
-// (a function of its own: inlined, it cost the kernel's column loop 5 us of 200).  One
-// request per CTA and 32 columns: hundreds of CTAs meet at two L2 lines.
+// A subnormal pivot's reciprocal may overflow where the quotients by it are ordinary
+// numbers: it and its column are scaled up first.  (Every thread of the CTA; out of
+// line, so that the column loop's registers stay as they are.)
 template <typename T, int NT>
-__device__ __noinline__ void lu_column_max(const T* S, int m, int kb, int* s_max, int* out) {
-  const int tid = threadIdx.x, j = tid & 63;
-  if (tid < 64) s_max[tid] = 0;
+__device__ __noinline__ T lu_scale_up(T* col, int rows, T* diag, T akk) {
+  constexpr T UP = T(sizeof(T) == 8 ? 0x1p128 : 0x1p64);
+  __syncthreads();                             // every thread has read the pivot
+  for (int r = threadIdx.x; r < rows; r += NT) col[r] *= UP;
+  if (threadIdx.x == 0) *diag *= UP;
   __syncthreads();
-  int fm = 0;
-#pragma unroll 4
-  for (int r = tid >> 6; r < m; r += NT / 64) fm = max(fm, XsType<T>::expo(S[r * LuBits<T>::LD + j]));
-  if (fm) atomicMax(&s_max[j], fm);
-  __syncthreads();
-  if (tid < kb && s_max[tid]) atomicMax(out + tid, s_max[tid]);
+  return akk * UP;
 }
 
 template <typename T, bool CL, int NT>
 __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restrict__ items, int n_items, int nb,
                                                    int pivot, int rmax, int csize, uint64_t* __restrict__ xbuf,
-                                                   int* __restrict__ lmax, int* err) {
+                                                   int* err) {
   extern __shared__ __align__(16) unsigned char gc_smem[];
   using LuRecvT = LuRecv<T, CL>;
   constexpr int NW = NT / 32, WORDS = LuBits<T>::WORDS, SR = LuBits<T>::LD;
@@ -1641,16 +1630,7 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
       if (q == 0 && tid == 0) set_status(c, it.front, akk != akk ? ST_NAN : ST_ZERO_PIVOT);
       akk = (T)1;
     }
-    if (XsType<T>::field(akk) == 0) {
-      // a subnormal pivot: its reciprocal may overflow where the quotients are ordinary
-      // numbers, so it and the column are scaled up first
-      constexpr T UP = T(sizeof(T) == 8 ? 0x1p128 : 0x1p64);
-      __syncthreads();                         // every thread has read it
-      for (int r = tid; r < nr_my; r += NT) s_col[par * rmax + r] *= UP;
-      if (tid == 0) rc.diag[k] *= UP;
-      akk *= UP;
-      __syncthreads();
-    }
+    if (XsType<T>::field(akk) == 0) akk = lu_scale_up<T, NT>(s_col + par * rmax, nr_my, &rc.diag[k], akk);
     T rinv;
     if constexpr (sizeof(T) == 8) {            // a reciprocal costs every FP64 warp that takes it
       if (warp == 0) {
@@ -1723,16 +1703,13 @@ __global__ void __launch_bounds__(NT) k_getrf_smem(DevCtx c, const Item* __restr
   if (tg < ng)
     for (int j = tg; j < kb; j += ng)
       for (int r = tr; r < nr_my; r += rw) G[(rbeg + r) + (int64_t)(k0 + j) * n] = S[r * SR + j];
-  if (lmax)
-    lu_column_max<T, NT>(S + (int64_t)max(0, k0 + kb - rbeg) * SR, nr_my - max(0, k0 + kb - rbeg), kb,
-                         reinterpret_cast<int*>(recv), lmax + f.piv_off + k0);
 }
 
 constexpr int GC_NT_CLUSTER = 512, GC_NT_GRID = 256;
 
 template <typename T, bool CL>
 static cudaError_t getrf_smem_t(const DevCtx& c, const Item* items, int n_items, int n_ctas, int csize, int nb,
-                                int pivot, int rmax, uint64_t* xbuf, int* lmax, int* err, cudaStream_t s) {
+                                int pivot, int rmax, uint64_t* xbuf, int* err, cudaStream_t s) {
   constexpr int NT = CL ? GC_NT_CLUSTER : GC_NT_GRID;
   const size_t smem = (size_t)rmax * (LuBits<T>::LD + 2) * sizeof(T);
   cudaFuncSetAttribute(k_getrf_smem<T, CL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1754,23 +1731,23 @@ static cudaError_t getrf_smem_t(const DevCtx& c, const Item* items, int n_items,
   }
   cfg.attrs = attr;
   cfg.numAttrs = CL && csize == 1 ? 0 : 1;
-  return cudaLaunchKernelEx(&cfg, k_getrf_smem<T, CL, NT>, c, items, n_items, nb, pivot, rmax, csize, xbuf, lmax, err);
+  return cudaLaunchKernelEx(&cfg, k_getrf_smem<T, CL, NT>, c, items, n_items, nb, pivot, rmax, csize, xbuf, err);
 }
 
 void launch_getrf_smem(const DevCtx& c, const Item* items, int n_items, int n_ctas, int csize, int dtype, int nb,
-                       int pivot, int rmax, uint64_t* xbuf, int* lmax, int* err, cudaStream_t s) {
+                       int pivot, int rmax, uint64_t* xbuf, int* err, cudaStream_t s) {
   if (!n_items) return;
   if (nb > 64) throw std::invalid_argument("getrf_smem: panel wider than 64");
   if (csize > GC_CLUSTER) throw std::invalid_argument("getrf_smem: cluster too large");
   cudaError_t e;
   if (csize > 0) {
-    e = dtype == F64 ? getrf_smem_t<double, true>(c, items, n_items, n_items * csize, csize, nb, pivot, rmax, nullptr, lmax, err, s)
-                     : getrf_smem_t<float, true>(c, items, n_items, n_items * csize, csize, nb, pivot, rmax, nullptr, lmax, err, s);
+    e = dtype == F64 ? getrf_smem_t<double, true>(c, items, n_items, n_items * csize, csize, nb, pivot, rmax, nullptr, err, s)
+                     : getrf_smem_t<float, true>(c, items, n_items, n_items * csize, csize, nb, pivot, rmax, nullptr, err, s);
   } else {
     if (n_ctas > GC_MAX_CTAS) throw std::invalid_argument("getrf_smem: too many CTAs");
     cudaMemsetAsync(xbuf, 0, sizeof(uint64_t) * (size_t)gc_words(n_ctas, n_items), s);
-    e = dtype == F64 ? getrf_smem_t<double, false>(c, items, n_items, n_ctas, 0, nb, pivot, rmax, xbuf, lmax, err, s)
-                     : getrf_smem_t<float, false>(c, items, n_items, n_ctas, 0, nb, pivot, rmax, xbuf, lmax, err, s);
+    e = dtype == F64 ? getrf_smem_t<double, false>(c, items, n_items, n_ctas, 0, nb, pivot, rmax, xbuf, err, s)
+                     : getrf_smem_t<float, false>(c, items, n_items, n_ctas, 0, nb, pivot, rmax, xbuf, err, s);
   }
   if (e != cudaSuccess)
     throw std::runtime_error(std::string("LU panel launch failed: ") + cudaGetErrorString(e));
@@ -1831,7 +1808,7 @@ constexpr int LUROW_CB = 16;   // columns per row-panel block
 
 // A[k0:k0+kb, cols] <- L11^{-1} A[k0:k0+kb, cols]  (unit lower), cols >= k0+kb;
 // item: front, a = k0, b = first column of the chunk, c = column limit (0: n);
-// umax (null: not wanted): the rows' largest exponent fields, as lmax of k_getrf_smem
+// scale (null: not wanted): XsCtx::scale, raised by these columns
 //
 // Substitution in registers: Q lanes hold one column (lane q rows q, q+Q,
 // ..), a step's solved entry goes to the others by one shuffle, L comes
@@ -1848,7 +1825,7 @@ constexpr int LUROW_CB = 16;   // columns per row-panel block
 // 12^3 p = 3, 200 launches, 6.5 -> 5.0 ms.
 template <typename T, int Q>
 __global__ void __launch_bounds__(Q * LUROW_CB) k_lu_row_update(DevCtx c, const Item* __restrict__ items, int nb,
-                                                                int* __restrict__ umax) {
+                                                                int* __restrict__ scale) {
   constexpr int NU = 64 / Q, LQ = NU + 2;      // rows per lane; their L entries' row in shared memory (no bank conflicts)
   constexpr int NT = Q * LUROW_CB;
   __shared__ __align__(16) T L[64 * Q * LQ];   // L[(Q k + q) LQ + u] = L11[q + Q u][k]
@@ -1885,29 +1862,35 @@ __global__ void __launch_bounds__(Q * LUROW_CB) k_lu_row_update(DevCtx c, const 
 #pragma unroll
   for (int u = 0; u < NU; ++u)
     if (in && q + Q * u < kb) X[Q * u] = x[u];
-  if (!umax) return;
-  // the largest exponent field of each row over the CTA's columns
-  int* s_max = reinterpret_cast<int*>(L);
-  __syncthreads();                             // L has been read
-  if (threadIdx.x < 64) s_max[threadIdx.x] = 0;
-  __syncthreads();
+  if (!scale) return;
+  // how near each row comes to a column's largest entry, over the CTA's columns
+  int* s_e = reinterpret_cast<int*>(L);        // [row][column], rows of 17
+  static_assert(sizeof(L) >= 64 * (LUROW_CB + 1) * sizeof(int), "room for the words");
+  int e[NU], cm = 0;
 #pragma unroll
   for (int u = 0; u < NU; ++u) {
-    int fm = in && q + Q * u < kb ? XsType<T>::expo(x[u]) : 0;
-#pragma unroll
-    for (int o = Q; o < 32; o <<= 1) fm = max(fm, __shfl_xor_sync(0xffffffffu, fm, o));
-    if ((threadIdx.x & 31) < Q && fm) atomicMax(&s_max[q + Q * u], fm);
+    e[u] = in && q + Q * u < kb ? XsType<T>::expo(x[u]) : 0;
+    cm = max(cm, e[u]);
   }
+#pragma unroll
+  for (int o = 1; o < Q; o <<= 1) cm = max(cm, __shfl_xor_sync(0xffffffffu, cm, o));
+  __syncthreads();                             // L has been read
+#pragma unroll
+  for (int u = 0; u < NU; ++u) s_e[(q + Q * u) * (LUROW_CB + 1) + threadIdx.x / Q] = e[u] ? XS_SCALE0 + e[u] - cm : 0;
   __syncthreads();
-  if (threadIdx.x < kb && s_max[threadIdx.x]) atomicMax(umax + f.piv_off + k0 + threadIdx.x, s_max[threadIdx.x]);
+  if (threadIdx.x >= kb) return;
+  int v = 0;
+#pragma unroll
+  for (int j = 0; j < LUROW_CB; ++j) v = max(v, s_e[threadIdx.x * (LUROW_CB + 1) + j]);
+  if (v) atomicMax(scale + f.piv_off + k0 + threadIdx.x, v);
 }
 
-void launch_lu_row_update(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, int* umax,
+void launch_lu_row_update(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, int* scale,
                           cudaStream_t s) {
   if (!n_items) return;
   if (nb != 64) throw std::invalid_argument("lu_row_update: panels are 64 columns wide");
-  if (dtype == F64) k_lu_row_update<double, 8><<<n_items, 8 * LUROW_CB, 0, s>>>(c, items, nb, umax);
-  else k_lu_row_update<float, 4><<<n_items, 4 * LUROW_CB, 0, s>>>(c, items, nb, umax);
+  if (dtype == F64) k_lu_row_update<double, 8><<<n_items, 8 * LUROW_CB, 0, s>>>(c, items, nb, scale);
+  else k_lu_row_update<float, 4><<<n_items, 4 * LUROW_CB, 0, s>>>(c, items, nb, scale);
 }
 
 // Inverses of a large LU front's diagonal blocks, for the flag-driven solves:

@@ -32,21 +32,26 @@
 // row of L21 and a column of U12 can lie at different inner k, where l_ik scales as
 // 1 / d_k and u_kj as d_k with the unit d_k of an eliminated equation (rows in
 // units of 1 and 10^10: solutions of an FP64 front 10^6 to 10^8 times further off).  So
-//  - column k of L21 and row k of U12 are multiplied by 2^t and 2^-t before they are
-//    cut, t half the difference of the exponents of their largest entries: exact,
-//    the products stay, and units of equations, of unknowns and of both are balanced;
-//  - each row keeps which of the panel's columns come within 2^4 (FP32 2^3) of its
-//    maximum, each front which of them some row of the other operand has so near its own.
-//    A row or column of a tile where no column is both (of the front's own part, or
-//    of its shared part, whichever the tile is in) goes by plain multiply-adds
-//    (xs_plain).  The rest differs from the sum of magnitudes by 2^8 (2^6) at
-//    most, over its row and over its column, which is the bound of 256
-//    multiply-adds in a row.
-// Measured (tests/test_gpu_lu_scaling.py: units to 2^33, rows that no balance serves)
-// errors are 0.4 to 0.9 times those of multiply-adds.  On convection-diffusion
-// fronts less than 0.3 % of the 32 x 32 blocks have such a row or column.  Cost:
-// 12^3 p = 3 FP64 LU factorisation 38.0 -> 39.4 ms (updates 0.8, slices 0.2, panels 0.4),
-// 6^3 6.5 -> 6.75.
+//  - before they are cut, row k of U12 is divided and column k of L21 multiplied by 2^t,
+//    t <= 0 how near the row comes to a column's largest entry, at its best column:
+//    exact, and the products stay.  Units of equations cancel, every row reaches some
+//    column's maximum, and no column's maximum grows, so that the error stays
+//    small in proportion to each column, which is what the solution sees.  (Half the
+//    difference of the largest exponents of the column and the row balances
+//    units as well, but an FP64 convection-diffusion solve of 24^3, coefficients 1 to
+//    10^4, had a backward error 140 times larger; so scaled that the largest entry of
+//    each column of L21 is near 1, 3 % of the blocks below were left to multiply-adds.)
+//  - each row keeps which of the panel's columns come within 2^6 of its maximum, each
+//    front which of them some row of the other operand has so near its own.  A row
+//    or column of a tile where no column is both (of the front's own part, or of its
+//    shared part, whichever the tile is in; columns of region 2, rows of U themselves,
+//    are not checked) goes by plain multiply-adds (xs_plain).
+// Measured: errors of fronts with units to 2^33 and of rows that no scaling serves are 0.4
+// to 2.8 times those of multiply-adds (tests/test_gpu_lu_scaling.py); backward errors
+// of 12^3, 16^3 and 24^3 convection-diffusion 4.4e-19, 3.0e-19 and 2.3e-19 (3.8e-19, 2.1e-19
+// and 2.1e-19 without scaling).  Less than 0.5 % of the 32 x 32 blocks have such a row or column.
+// Cost: factorisations 6^3 p = 3 FP64 LU 6.5 -> 6.65 ms, 12^3 38.0 -> 39.2, 24^3 273 -> 288
+// (multiply-adds 8, the check 4.5), FP32 119 -> 129.
 //
 // Why: GB300 does about 2 FP64 multiply-adds per clock per SM (1.17 TFLOP/s
 // measured for the SIMT update), against 1,906 TFLOP/s of BF16 products:
@@ -93,7 +98,7 @@ __global__ void __launch_bounds__(256) k_xs_pack(DevCtx c, XsCtx x, const Item* 
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, K0 = it.a, trans = it.c;
   const int W = min(nb, f.fs - K0), nch = xs_chunks(nb, f.fs);
-  const bool lu = x.kmax != nullptr;
+  const bool lu = x.scale != nullptr;
   const int r = threadIdx.x % ROWS, g = threadIdx.x / ROWS;
   const int row = it.b + r;
   const T* __restrict__ G = arena<T>(c) + f.off;
@@ -104,12 +109,10 @@ __global__ void __launch_bounds__(256) k_xs_pack(DevCtx c, XsCtx x, const Item* 
 #pragma unroll
   for (int u = 0; u < 16; ++u) v[u] = in && 16 * g + u < W ? G[base + (16 * g + u) * step] : T(0);
   if (lu && threadIdx.x < 16 * NG) {
-    // this side's share of the balance of column K0 + k
     int t = 0;
     if ((int)threadIdx.x < W) {
-      const int64_t k = (int64_t)f.piv_off + K0 + threadIdx.x;
-      const int l = x.kmax[k], u = NG == 4 ? x.kmax[x.kmax_n + k] : max(x.kmax[x.kmax_n + k], x.kmax[2 * x.kmax_n + k]);
-      t = l && u ? (u - l) >> 1 : 0;
+      const int v = x.scale[use * x.scale_n + f.piv_off + K0 + threadIdx.x];
+      t = v ? v - XS_SCALE0 : 0;
     }
     s_t[threadIdx.x] = trans ? -t : t;
   }
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(256) k_xs_pack(DevCtx c, XsCtx x, const Item* 
 #pragma unroll
   for (int u = 0; u < 16; ++u)
     if (e[u] >= fm - NEAR && XsType<T>::field(v[u])) mask |= 1u << u;
-  // their union over the CTA's own and its shared rows (region 2 takes region 1's: xs_check)
+  // their union over the CTA's own and its shared rows (side A of region 2: not checked)
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const uint32_t all = __reduce_or_sync(0xffffffffu, some && (row >= f.fs) == h ? mask << (16 * (g & 1)) : 0u);
@@ -194,6 +197,55 @@ void launch_xs_pack(const DevCtx& c, const XsCtx& x, const Item* items, int n_it
     if (nb == 64) k_xs_pack<float, 4><<<n_items, 256, 0, s>>>(c, x, items, nb, use);
     else k_xs_pack<float, 16><<<n_items, 256, 0, s>>>(c, x, items, nb, use);
   }
+}
+
+// How near each of an outer panel's rows of U12 comes to a column's largest entry, at
+// its best column: a warp takes four columns, whose entries are contiguous.
+template <typename T>
+__global__ void __launch_bounds__(256) k_xs_scale(DevCtx c, XsCtx x, const Item* __restrict__ items) {
+  __shared__ int s_near[XS_NBO];
+  const Item it = items[blockIdx.x];
+  const FrontDev f = c.fronts[it.front];
+  const int n = f.n, K0 = it.a, W = min(XS_NBO, f.fs - K0), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const T* __restrict__ G = arena<T>(c) + f.off + K0;
+  s_near[threadIdx.x] = 0;
+  int best[XS_NBO / 32];
+#pragma unroll
+  for (int i = 0; i < XS_NBO / 32; ++i) best[i] = 0;
+  T v[2][XS_NBO / 32];
+  auto load = [&](int j, T (&w)[XS_NBO / 32]) {
+    const int col = it.b + 4 * warp + j;
+#pragma unroll
+    for (int i = 0; i < XS_NBO / 32; ++i) w[i] = col < n && lane + 32 * i < W ? G[lane + 32 * i + (int64_t)col * n] : T(0);
+  };
+  load(0, v[0]);
+#pragma unroll
+  for (int j = 0; j < XS_SCALE_COLS / 8; ++j) {
+    if (j + 1 < XS_SCALE_COLS / 8) load(j + 1, v[(j + 1) & 1]);
+    int e[XS_NBO / 32], cm = 0;
+#pragma unroll
+    for (int i = 0; i < XS_NBO / 32; ++i) {
+      e[i] = XsType<T>::expo(v[j & 1][i]);
+      cm = max(cm, e[i]);
+    }
+    cm = __reduce_max_sync(0xffffffffu, cm);
+#pragma unroll
+    for (int i = 0; i < XS_NBO / 32; ++i)
+      if (e[i]) best[i] = max(best[i], XS_SCALE0 + e[i] - cm);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < XS_NBO / 32; ++i)
+    if (best[i]) atomicMax(&s_near[lane + 32 * i], best[i]);
+  __syncthreads();
+  if (s_near[threadIdx.x]) atomicMax(x.scale + f.piv_off + K0 + threadIdx.x, s_near[threadIdx.x]);
+}
+
+void launch_xs_scale(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, int dtype, cudaStream_t s) {
+  if (!n_items) return;
+  static_assert(XS_NBO == 256 && XS_SCALE_COLS == 32, "a thread per row of the panel, four columns a warp");
+  if (dtype == F64) k_xs_scale<double><<<n_items, 256, 0, s>>>(c, x, items);
+  else k_xs_scale<float><<<n_items, 256, 0, s>>>(c, x, items);
 }
 
 // FP64 Cholesky panel TRSM, X = A Linv^T below a 64-column diagonal block (its
@@ -390,11 +442,9 @@ __device__ __forceinline__ void xs_check(const XsCtx& x, int front, int K0, int 
   const int64_t e0 = x.exp0[front], w0 = x.near0[front] + K0 / 32;
   const uint2* ma = reinterpret_cast<const uint2*>(x.masks + (e0 + (rin ? row : 0)) * (XS_NBO / 32));
   const uint2* mb = reinterpret_cast<const uint2*>(x.masks + (e0 + n + (cin ? c0 + lane : 0)) * (XS_NBO / 32));
-  // side A's unions of region 1 serve region 2 (its rows are among them), where region 1's
-  // columns join side B's (the balance is the same): own rows, shared rows
-  const uint2* na = reinterpret_cast<const uint2*>(x.near + 4 * (use ? 1 : 0) * x.near_n + w0);
+  // (the unions over own rows, then over shared rows)
+  const uint2* na = reinterpret_cast<const uint2*>(x.near + 4 * use * x.near_n + w0);
   const uint2* nbv = reinterpret_cast<const uint2*>(x.near + (4 * use + 2) * x.near_n + w0);
-  const uint2* nb1 = reinterpret_cast<const uint2*>(x.near + 6 * x.near_n + w0);
   const int64_t own = x.near_n / 2;
   uint32_t hr[2] = {0, 0}, hc[2] = {0, 0}, sa[2] = {0, 0}, sb[2] = {0, 0};
 #pragma unroll 2
@@ -405,11 +455,6 @@ __device__ __forceinline__ void xs_check(const XsCtx& x, int front, int K0, int 
     for (int h = 0; h < 2; ++h) {
       pa[h] = na[w + h * own];
       pb[h] = nbv[w + h * own];
-      if (use == 2) {
-        const uint2 p1 = nb1[w + h * own];
-        pb[h].x |= p1.x;
-        pb[h].y |= p1.y;
-      }
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -424,7 +469,7 @@ __device__ __forceinline__ void xs_check(const XsCtx& x, int front, int K0, int 
   for (int h = 0; h < 2; ++h) {
     const bool cols = h ? min(c0 + NC, cmax) > fs : c0 < fs, rows = h ? min(r0 + 32, rmax) > fs : r0 < fs;
     okr = okr && (!cols || hr[h] || !sb[h]);
-    okc = okc && (!rows || hc[h] || !sa[h]);
+    okc = okc && (!rows || hc[h] || !sa[h] || use == 2);
   }
   const uint32_t wr = __ballot_sync(0xffffffffu, rin && !okr), wc = __ballot_sync(0xffffffffu, cin && !okc);
   if (lane == 0) {
@@ -451,7 +496,7 @@ __device__ __noinline__ void xs_plain(T* G, int n, int K0, int W, int row, int r
     for (int k0 = 0; k0 < W; k0 += 64) {
       const int k1 = min(k0 + 64, W);
       T s = T(0);
-#pragma unroll 8
+#pragma unroll 16
       for (int k = k0; k < k1; ++k) s += l[(int64_t)k * n] * u[k];
       v -= s;
     }

@@ -13,7 +13,8 @@ constexpr int XS_TRSM_ROWS = 16;  // rows per item of the FP64 panel TRSM
 constexpr int XS_S64 = 8, XS_S32 = 4;   // slices of an FP64 / FP32 front's operands
 constexpr int XS_SPARE_ROWS = 256;      // workspace rows past the last front's (tiles run over)
 // LU: entries within 2^XS_NEAR of their row's maximum count as near it (k_xs.cu)
-constexpr int XS_NEAR64 = 4, XS_NEAR32 = 3;
+constexpr int XS_NEAR64 = 6, XS_NEAR32 = 6;
+constexpr int XS_SCALE0 = 1 << 12;      // (a word of scale that nothing has raised is zero)
 constexpr int XS_USES = 3;        // pairs of operands of a panel column: the update's region (0, 1, 2)
 
 // Where the operand slices live: 128-byte rows of four slices x 16 columns (BF16),
@@ -26,15 +27,14 @@ struct XsCtx {
   const int64_t* row0b;
   const int64_t* exp0;     // first exponent of the front's A rows; its B rows follow at + n
   int* exps;
-  // LU (otherwise null), what balances and checks the slices (k_xs.cu): per factor
-  // column (at the front's pivots) the largest exponent field of L below its 64-column
-  // step's diagonal block, then, kmax_n behind, of U right of it in the outer panel,
-  // then of U beyond the outer panel; per row of exps
-  // XS_NBO bits, one for each of the panel's columns near the row's maximum; per use, side (A, B),
-  // group (own, shared rows) and front the union of these over its rows, near_n words
-  // each, from near0[front] on
-  int* kmax;
-  int64_t kmax_n;
+  // LU (otherwise null), what scales and checks the slices (k_xs.cu): per use (the
+  // update's region, scale_n words each) and factor column (at the front's pivots)
+  // XS_SCALE0 plus the power of two of its row of U12; per row of exps XS_NBO bits, one for
+  // each of the panel's columns near the row's maximum; per use, side (A, B), group
+  // (own, shared rows) and front the union of these over its rows, near_n words each,
+  // from near0[front] on
+  int* scale;
+  int64_t scale_n;
   uint32_t* masks;
   uint32_t* near;
   int64_t near_n;
@@ -52,6 +52,10 @@ bool xs_encode(XsMaps* maps, void* base, int64_t rows);
 // region of the update that takes them
 void launch_xs_pack(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, int dtype, int nb, int use,
                     cudaStream_t s);
+// LU, nb = XS_NBO: the powers of two that the slices of U12 are scaled by, from its 32
+// columns at a time (item: front, a = K0, b = first column)
+constexpr int XS_SCALE_COLS = 32;
+void launch_xs_scale(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, int dtype, cudaStream_t s);
 // FP64 Cholesky: panel rows times the inverse of the diagonal block and, c = 1,
 // their slices for an update with nb = 64 (item: front, a = k0, b = first row)
 void launch_xs_trsm(const DevCtx& c, const XsCtx& x, const Item* items, int n_items, cudaStream_t s);

@@ -102,19 +102,19 @@ void launch_syrk_update(const DevCtx& c, const Item* items, int n_items, int dty
 // csize CTAs (a cluster, a power of two up to GC_CLUSTER) per item (front, a =
 // k0); csize = 0: a cooperative launch of n_ctas CTAs (item: front, a = k0, b =
 // first CTA, c = CTAs; xbuf: gc_words(n_ctas, n_items) words).  rmax = rows per
-// CTA, at most GC_RMAX_F64 / GC_RMAX_F32.  lmax / umax of the row update (null: not
-// wanted): largest exponent fields, XsCtx::kmax
+// CTA, at most GC_RMAX_F64 / GC_RMAX_F32
 constexpr int GC_RMAX_F64 = 384, GC_RMAX_F32 = 768;
 constexpr int GC_MAX_CTAS = 160, GC_CLUSTER = 16;
 constexpr int64_t gc_words(int n_ctas, int n_items) { return 4 * (int64_t)n_ctas + 2 * (int64_t)(n_ctas + n_items) * (2 * 64); }
 void launch_getrf_smem(const DevCtx& c, const Item* items, int n_items, int n_ctas, int csize, int dtype, int nb,
-                       int pivot, int rmax, uint64_t* xbuf, int* lmax, int* err, cudaStream_t s);
+                       int pivot, int rmax, uint64_t* xbuf, int* err, cudaStream_t s);
 void launch_laswp(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, cudaStream_t s);
 // the same panel in global memory, one CTA per front (any height), rows
 // swapped in columns c .. b - 1 (b = 0: c .. n - 1) as it goes (item: front, a = k0, b, c)
 void launch_getrf_panel(const DevCtx& c, const Item* items, int n_items, int dtype, int nb,
-                        int pivot, int* lmax, cudaStream_t s);
-void launch_lu_row_update(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, int* umax,
+                        int pivot, cudaStream_t s);
+// (scale: the use's words of XsCtx::scale; null: not wanted)
+void launch_lu_row_update(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, int* scale,
                           cudaStream_t s);
 // LU trailing GEMM tiles; nbo / region as for k_tile_update (0 / 0: every entry)
 void launch_gemm_update(const DevCtx& c, const Item* items, int n_items, int dtype, int nb, int nbo,
