@@ -31,11 +31,11 @@ static constexpr int LU_GOAL_F64 = 64, LU_GOAL_F32 = 192;
 // rows (four fronts at once: more); FP64, 16 CTAs, 187 at 96 rows each, 205 at 128, 225 to
 // 264 from 130 to 208, against 200 for the whole GPU from 2,100 to 3,300 rows and 218 at 6,938
 static constexpr int LU_CLUSTER_ROWS_F64 = 128, LU_CLUSTER_ROWS_F32 = 384;
-// 128-byte rows of operand slices held at a time (1 GiB; a single front may need more).
-// Slices are up to 1.5 times (LU 3 times) the panels of fronts of 180 to 600 rows, so a
-// wide level of them goes in batches.  One batch fills the GPU: 200 FP64 fronts of 1,000
-// rows, 1,300 of 200; the largest level of the meshes measured takes 680 MB (512 fronts).
-static constexpr int64_t XS_BATCH_ROWS = (int64_t)1 << 23;
+// 128-byte rows of operand slices held at a time: 4 GiB, or 1 GiB where the fronts and
+// elements take more than half of the device (a single front may need more).  Slices are
+// up to 1.5 times (LU 3 times) the panels of fronts of 180 to 600 rows, so a wide level of
+// them goes in batches.
+static constexpr int64_t XS_BATCH_ROWS = (int64_t)1 << 25, XS_BATCH_ROWS_TIGHT = (int64_t)1 << 23;
 static constexpr int TR = TILE_UPDATE_ROWS, TC = TILE_UPDATE_COLS;   // k_tile_update
 
 #define CK(x)                                                                          \
@@ -713,8 +713,12 @@ void Engine::build_plan(int method) {
   }
   // operand slices of the current panel of every front with sliced updates; the levels
   // and types run one after the other and share the workspace, and so do batches of
-  // fronts of one level and type beyond XS_BATCH_ROWS
+  // fronts of one level and type beyond batch_rows
   xs_rows = xs_exps = xs_near_n = 0;
+  size_t mem_free = 0, mem_total = 0;
+  CK(cudaMemGetInfo(&mem_free, &mem_total));
+  const bool tight = (size_t)(8 * arena64_n + 4 * arena32_n + 8 * emat_total) > mem_total / 2;
+  const int64_t batch_rows = tight ? XS_BATCH_ROWS_TIGHT : XS_BATCH_ROWS;
   const int sides = method == UHM_CHOL ? 1 : 2;      // LU: U12^T beside L21
   for (auto& lv : levels)
     for (int dt = 0; dt < 2; ++dt) {
@@ -727,7 +731,7 @@ void Engine::build_plan(int method) {
         // run beside the update that reads the former
         const int64_t ri = (int64_t)(dt == F64 ? XS_S64 : XS_S32) * f.n;
         const int64_t r = ri * ((std::min(f.fs, XS_NBO) + 63) / 64);
-        if (rows > 0 && rows + sides * (r + ri) > XS_BATCH_ROWS) {
+        if (rows > 0 && rows + sides * (r + ri) > batch_rows) {
           ++batch;
           rows = exps = 0;
         }
