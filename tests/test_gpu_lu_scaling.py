@@ -13,7 +13,7 @@ import pytest
 
 from oracle import uhm_oracle as uo
 from tests.test_gpu_large_fronts import _matrix, _mesh, _solutions
-from uhm_gb300 import api
+from uhm_gb300 import api, hpfem
 
 pytestmark = pytest.mark.gpu
 
@@ -188,3 +188,27 @@ def test_lookahead_changes_no_bit_with_units(native_lib):
         eid = m.fronts()[0]
         got.append([m.front_block(int(e), q) for e in eid[:2] for q in ("ATL", "ATR", "ABL", "ABR")])
     assert all((x == y).all() for x, y in zip(*got))
+
+
+def test_strong_coefficients(native_lib):
+    """Convection-diffusion with coefficients of 1 to 10^4 and no units of its own: errors
+    have to stay small in proportion to each column, or soft regions' large solutions see
+    them.  Backward error at most 4 times that of the oracle's FP64 elimination of the
+    same fronts."""
+    spec = hpfem.convdiff3d(16, 3, seed=0)
+    m = api.load_spec(spec)
+    m.factor(uo.LU_PIV)
+    m.solve(uo.LU_PIV)
+    assert m.backward_error() <= 4 * uo.backward_error(spec, uo.solve_mesh(spec, uo.LU_PIV).x)
+
+
+@pytest.mark.parametrize("kind,step", [("both", 20), ("both", 27), ("random", 12)])
+@pytest.mark.parametrize("prec,fs,ss", [("fp64", 300, 129), ("fp32", 320, 200), ("fp64", 260, 1300)])
+def test_cholesky_units(native_lib, prec, fs, ss, kind, step):
+    """Symmetric fronts with units: a row of L is bounded by its diagonal entry's root, so
+    that a shared exponent needs no scaling."""
+    step = min(step, 20) if prec == "fp32" else step
+    rng = np.random.default_rng(2000 + step)
+    d = _units(kind, step, fs + ss, rng)[0] if kind == "random" else _units(kind, step, fs + ss, rng)[1]
+    base = [_matrix(fs + ss, True, rng) for _ in range(2)]
+    _check_front(uo.CHOL, prec, fs, ss, [d[:, None] * b * d[None, :] for b in base], d, d)
