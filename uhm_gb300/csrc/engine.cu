@@ -1678,9 +1678,7 @@ void Engine::build_programs(int method) {
       const size_t b = (size_t)f.n * nr * 8 + (size_t)f.fs * 8 + (size_t)f.n * f.fs * (dt == F64 ? 8 : 4);
       mx = std::max(mx, b);
     }
-    // the unstaged kernels solve FP32 fronts in FP64, the staged ones in FP32: FP32
-    // launches stay unstaged from the 96 KB on
-    return mx <= (dt == F64 ? 216 : 96) * 1024 ? (int)((mx + 15) / 16 * 16) : 0;
+    return mx <= 216 * 1024 ? (int)((mx + 15) / 16 * 16) : 0;
   };
   constexpr int GATHER_ROWS = 1024;   // rows per CTA of the forward gather (no pivots)
   constexpr int NR_FLAGS_MAX = 16;    // right-hand sides taken by the flag-driven solves

@@ -164,7 +164,8 @@ __global__ void __launch_bounds__(NT) k_fwd_small(DevCtx c, const Item* __restri
 // (no global round trip per column).  The right-hand sides are solved in the
 // factor's precision (as in the flag-driven solves of large fronts): FP32
 // fronts take no FP64 arithmetic, which runs at a small fraction of the FP32 rate
-// on this GPU.  The pivots' reciprocals are formed once, all at a time (a
+// on this GPU; only where a launch's largest panel and right-hand sides pass
+// SMALL_SOLVE_FP32 bytes do they, as without staging.  The pivots' reciprocals are formed once, all at a time (a
 // division per column was most of an FP64 step); the solved entries are scaled by them
 // where they are used.  From WARP_RHS right-hand sides on each warp takes its own
 // ones and no block barrier is left in the sweep; below, the block shares
@@ -173,12 +174,13 @@ __global__ void __launch_bounds__(NT) k_fwd_small(DevCtx c, const Item* __restri
 // staged too); 4,096 fronts of 125 (27) 106 -> 77 and 240 -> 68; 12 meshes, 16
 // right-hand sides, FP32 1.08 -> 0.80 ms and 1.95 -> 1.03.
 constexpr int WARP_RHS = 4;
+constexpr int SMALL_SOLVE_FP32 = 96 * 1024;
 
 // the front's factor columns into Ls (n x fs), the reciprocals of its pivots
 // into rd, the slab v (n x n_rhs) into z
-template <typename T, int NT>
+template <typename T, typename CT, int NT>
 __device__ __forceinline__ void small_stage(const T* __restrict__ G, const double* __restrict__ v, int n, int fs,
-                                            int nr, T* z, T* rd, T* Ls) {
+                                            int nr, CT* z, CT* rd, T* Ls) {
   const int tot = n * fs;
   for (int i0 = 0; i0 < tot; i0 += 8 * NT) {
     T x[8];
@@ -193,8 +195,8 @@ __device__ __forceinline__ void small_stage(const T* __restrict__ G, const doubl
       if (idx < tot) Ls[idx] = x[u];
     }
   }
-  for (int idx = threadIdx.x; idx < n * nr; idx += NT) z[idx] = (T)v[idx];
-  for (int j = threadIdx.x; j < fs; j += NT) rd[j] = T(1) / G[j + (int64_t)j * n];
+  for (int idx = threadIdx.x; idx < n * nr; idx += NT) z[idx] = (CT)v[idx];
+  for (int j = threadIdx.x; j < fs; j += NT) rd[j] = CT(1) / (CT)G[j + (int64_t)j * n];
   __syncthreads();
 }
 
@@ -215,24 +217,24 @@ struct SmallShare {
   }
 };
 
-template <typename T, int NT>
+template <typename T, typename CT, int NT>
 __global__ void __launch_bounds__(NT) k_fwd_small_staged(DevCtx c, const Item* __restrict__ items) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, fs = f.fs, nr = c.n_rhs;
-  T* z = reinterpret_cast<T*>(smem_raw);
-  T* rd = z + (size_t)n * nr;
-  T* Ls = rd + fs;
+  CT* z = reinterpret_cast<CT*>(smem_raw);
+  CT* rd = z + (size_t)n * nr;
+  T* Ls = reinterpret_cast<T*>(rd + fs);
   double* __restrict__ zg = c.vec + f.voff;
-  small_stage<T, NT>(arena<T>(c) + f.off, zg, n, fs, nr, z, rd, Ls);
+  small_stage<T, CT, NT>(arena<T>(c) + f.off, zg, n, fs, nr, z, rd, Ls);
   const SmallShare sh(nr, NT);
   for (int q = sh.q0; q < nr; q += sh.qs) {
-    T* zq = z + q * n;
+    CT* zq = z + q * n;
     for (int j = 0; j < fs; ++j) {
-      const T zj = zq[j] * rd[j];
+      const CT zj = zq[j] * rd[j];
       const T* col = Ls + j * n;
-      for (int i = j + 1 + sh.i0; i < n; i += sh.is) zq[i] -= col[i] * zj;
+      for (int i = j + 1 + sh.i0; i < n; i += sh.is) zq[i] -= (CT)col[i] * zj;
       sh.sync();
     }
   }
@@ -247,36 +249,36 @@ __global__ void __launch_bounds__(NT) k_fwd_small_staged(DevCtx c, const Item* _
 
 // x_F = L_FF^{-T} (y_F - L_SF^T x_S): the Schur-row products for all factor
 // columns at once, then the small triangular solve column by column.
-template <typename T, int NT>
+template <typename T, typename CT, int NT>
 __global__ void __launch_bounds__(NT) k_bwd_small_staged(DevCtx c, const Item* __restrict__ items,
                                                          double* __restrict__ g, int64_t ldg) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Item it = items[blockIdx.x];
   const FrontDev f = c.fronts[it.front];
   const int n = f.n, fs = f.fs, nr = c.n_rhs;
-  T* z = reinterpret_cast<T*>(smem_raw);
-  T* rd = z + (size_t)n * nr;
-  T* Ls = rd + fs;
+  CT* z = reinterpret_cast<CT*>(smem_raw);
+  CT* rd = z + (size_t)n * nr;
+  T* Ls = reinterpret_cast<T*>(rd + fs);
   const double* __restrict__ yg = c.vec + f.voff + (int64_t)n * nr;   // y slab
-  small_stage<T, NT>(arena<T>(c) + f.off, yg, n, fs, nr, z, rd, Ls);
+  small_stage<T, CT, NT>(arena<T>(c) + f.off, yg, n, fs, nr, z, rd, Ls);
   const SmallShare sh(nr, NT);
   for (int q = sh.q0; q < nr; q += sh.qs) {
-    T* zq = z + q * n;
+    CT* zq = z + q * n;
     for (int j = sh.i0; j < fs; j += sh.is) {
-      T s0 = T(0), s1 = T(0);
+      CT s0 = CT(0), s1 = CT(0);
       const T* col = Ls + (size_t)j * n;
       int i = fs;
       for (; i + 1 < n; i += 2) {
-        s0 += col[i] * zq[i];
-        s1 += col[i + 1] * zq[i + 1];
+        s0 += (CT)col[i] * zq[i];
+        s1 += (CT)col[i + 1] * zq[i + 1];
       }
-      if (i < n) s0 += col[i] * zq[i];
+      if (i < n) s0 += (CT)col[i] * zq[i];
       zq[j] -= s0 + s1;
     }
     sh.sync();
     for (int j = fs - 1; j > 0; --j) {
-      const T xj = zq[j] * rd[j];
-      for (int i = sh.i0; i < j; i += sh.is) zq[i] -= Ls[j + i * n] * xj;
+      const CT xj = zq[j] * rd[j];
+      for (int i = sh.i0; i < j; i += sh.is) zq[i] -= (CT)Ls[j + i * n] * xj;
       sh.sync();
     }
   }
@@ -289,13 +291,11 @@ void launch_fwd_small(const DevCtx& c, const Item* items, int n_items, int dtype
                       int staged_bytes, cudaStream_t s) {
   if (!n_items) return;
   if (method == M_CHOL && staged_bytes > 0) {
-    if (dtype == F64) {
-      cudaFuncSetAttribute(k_fwd_small_staged<double, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, staged_bytes);
-      k_fwd_small_staged<double, 128><<<n_items, 128, staged_bytes, s>>>(c, items);
-    } else {
-      cudaFuncSetAttribute(k_fwd_small_staged<float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, staged_bytes);
-      k_fwd_small_staged<float, 128><<<n_items, 128, staged_bytes, s>>>(c, items);
-    }
+    const auto kernel = dtype == F64                       ? k_fwd_small_staged<double, double, 128>
+                        : staged_bytes <= SMALL_SOLVE_FP32 ? k_fwd_small_staged<float, float, 128>
+                                                           : k_fwd_small_staged<float, double, 128>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, staged_bytes);
+    kernel<<<n_items, 128, staged_bytes, s>>>(c, items);
     return;
   }
   // the largest small front bounds the shared slab; 64 KB covers n*n_rhs <= 8192
@@ -381,13 +381,11 @@ void launch_bwd_small(const DevCtx& c, const Item* items, int n_items, int dtype
                       double* g, int64_t ldg, int staged_bytes, cudaStream_t s) {
   if (!n_items) return;
   if (method == M_CHOL && staged_bytes > 0) {
-    if (dtype == F64) {
-      cudaFuncSetAttribute(k_bwd_small_staged<double, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, staged_bytes);
-      k_bwd_small_staged<double, 128><<<n_items, 128, staged_bytes, s>>>(c, items, g, ldg);
-    } else {
-      cudaFuncSetAttribute(k_bwd_small_staged<float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, staged_bytes);
-      k_bwd_small_staged<float, 128><<<n_items, 128, staged_bytes, s>>>(c, items, g, ldg);
-    }
+    const auto kernel = dtype == F64                       ? k_bwd_small_staged<double, double, 128>
+                        : staged_bytes <= SMALL_SOLVE_FP32 ? k_bwd_small_staged<float, float, 128>
+                                                           : k_bwd_small_staged<float, double, 128>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, staged_bytes);
+    kernel<<<n_items, 128, staged_bytes, s>>>(c, items, g, ldg);
     return;
   }
   size_t sm = 8192 * sizeof(double);
