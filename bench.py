@@ -44,11 +44,11 @@ sys.path.insert(0, ROOT)
 METRIC = "factor+solve s at 16³ p=4: plain FP64 vs mixed+IR+learned, bwd err≤1e-12"
 # DRAM traffic of the tensor-core Schur pass per algorithmic byte, from one ncu
 # capture (dram__bytes_read.sum + dram__bytes_write.sum) of its launch on tree
-# level -2 of the 12^3 p=4 mesh (27 fronts, fs 631, 145.0 MB against 177.4 MB
+# level -2 of the 12^3 p=4 mesh (27 fronts, fs 631, 142.2 MB against 177.4 MB
 # algorithmic); scaled to the benchmark's launches by their algorithmic bytes
-SCHUR_TRAFFIC_PER_ALG_BYTE = 145.03 / 177.36
+SCHUR_TRAFFIC_PER_ALG_BYTE = 142.25 / 177.36
 SCHUR_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the Schur launch of poisson3d_12_p4 "
-                        "(profiles/tc_chol_schur_poisson3d_12_p4.md), 0.82 x its algorithmic bytes, scaled")
+                        "(profiles/tc_chol_schur_poisson3d_12_p4.md), 0.80 x its algorithmic bytes, scaled")
 WORKLOAD = "3D Poisson 16^3 hex p=4 Legendre-hierarchic, Dirichlet, octree ND, Cholesky fronts, 1 RHS"
 
 
